@@ -14,7 +14,7 @@
 //                                operands' copies fast enough)
 //   warps 7..11 (384-thread variants; warp 7 alone in the 256-thread ones)
 //               communication  : all-gather: send this rank's A shard, peer by peer or once by multimem.st
-//                                (raw shards of any pitch; with one rank this is the padding prologue);
+//                                (raw shards of any pitch);
 //               reducers       : pull flavour: wait for a tile's W stamps, read the sum of all ranks' partials
 //                                through the switch (multimem.ld_reduce), store it or broadcast it + done stamp
 //
@@ -346,8 +346,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
   const int kps = (!CTA2 && BN <= 64) ? 2 : kKPS;
   const int sub_bytes = (kps != kKPS) ? (kABytes + BN * 128) : kSubBytes;
   const int num_kb = ceil_div(p.K, p.bk * kps);   // pipeline stages per tile
-  // (a raw-shard all-gather runs on one rank too: the padding prologue of a local GEMM)
-  const bool fused = (p.mode != MODE_LOCAL) && (p.W > 1 || (p.mode == MODE_AG && p.ag_raw != 0));
+  const bool fused = (p.mode != MODE_LOCAL) && (p.W > 1);
   const bool pull = kPull && fused && (p.pull != 0) && (p.mode == MODE_RS || p.mode == MODE_AR);
   // Pair flavour: `sub` is this CTA's half of the 256-row tile, work is dealt out per pair.
   const int sub = CTA2 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
@@ -377,8 +376,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
     tail->abort_flag = 0;
     // A fused launch that finds an earlier failure latched in the status block does nothing: the
     // ranks' epochs no longer agree, so every wait would only run into its time limit again.
-    tail->dead = (p.mode != MODE_LOCAL && (p.W > 1 || (p.mode == MODE_AG && p.ag_raw != 0)) &&
-                  ptx::ld_relaxed_sys_u32(p.status) != 0u) ? 1u : 0u;
+    tail->dead = (fused && ptx::ld_relaxed_sys_u32(p.status) != 0u) ? 1u : 0u;
     ptx::mbar_fence_init();
     ptx::prefetch_tmap(&p.tm_a);
     ptx::prefetch_tmap(&p.tm_b);

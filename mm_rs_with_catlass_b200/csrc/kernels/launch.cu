@@ -194,7 +194,7 @@ static bool wants_ag_multicast(const CatcocOpArgs& a) {
 }
 
 static TileSched build_sched(const CatcocOpArgs& a, int bm, int bn, int seg_dim) {
-  const bool fused = a.mode != CATCOC_MODE_LOCAL && (a.W > 1 || (a.mode == CATCOC_MODE_AG && a.ag_raw != 0));
+  const bool fused = a.mode != CATCOC_MODE_LOCAL && a.W > 1;
   const int W = fused ? a.W : 1;
   int first = 0;
   if (fused) first = (a.mode == CATCOC_MODE_AG) ? a.rank : (a.rank + 1) % W;
@@ -309,7 +309,7 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     return CATCOC_E_BAD_ARG;
   }
   const bool ag_raw = (a.mode == CATCOC_MODE_AG) && (a.ag_raw != 0);
-  const bool fused = a.mode != CATCOC_MODE_LOCAL && (a.W > 1 || ag_raw);
+  const bool fused = a.mode != CATCOC_MODE_LOCAL && a.W > 1;
   if (fused && (a.W > kMaxWorld || a.W < 1 || a.rank < 0 || a.rank >= a.W)) {
     set_error("bad rank/world %d/%d", a.rank, a.W);
     return CATCOC_E_BAD_ARG;

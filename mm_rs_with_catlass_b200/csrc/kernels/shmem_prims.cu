@@ -80,17 +80,6 @@ __global__ void mc_reduce_bf16_kernel(shmem::Ctx c, uint8_t* dst, int64_t src_of
     ptx::st_global_v4(dst + (i << 4), ptx::multimem_ld_reduce_add_bf16x2_v4(mc + (i << 4)));
 }
 
-// 2-D copy with independent pitches and zero fill of the padding columns: makes a TMA-legal
-// (16-byte pitch) copy of a matrix whose leading dimension is not.
-__global__ void pad2d_kernel(uint8_t* dst, int64_t dst_pitch, const uint8_t* src, int64_t src_pitch, int64_t rows,
-                             int64_t row_bytes) {
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
-    const uint8_t* s = src + r * src_pitch;
-    uint8_t* d = dst + r * dst_pitch;
-    for (int64_t b = threadIdx.x; b < dst_pitch; b += blockDim.x) d[b] = (b < row_bytes) ? s[b] : uint8_t(0);
-  }
-}
-
 }  // namespace
 
 extern "C" int catcoc_shmem_barrier_all(const CatcocShmemCtx* ctx, uint32_t epoch, uint64_t timeout_ns,
@@ -157,17 +146,6 @@ extern "C" int catcoc_shmem_mc_reduce_bf16(const CatcocShmemCtx* ctx, void* dst,
   if ((src_off & 15) || (n_elems & 7) || (reinterpret_cast<uintptr_t>(dst) & 15)) { host::set_error("mc_reduce: 16-byte alignment required"); return CATCOC_E_ALIGNMENT; }
   mc_reduce_bf16_kernel<<<64, 256, 0, static_cast<cudaStream_t>(stream)>>>(to_ctx(ctx), static_cast<uint8_t*>(dst),
                                                                            src_off, n_elems);
-  CATCOC_CUDA_OK(cudaGetLastError());
-  return CATCOC_OK;
-}
-
-extern "C" int catcoc_pad2d(void* dst, int64_t dst_pitch, const void* src, int64_t src_pitch, int64_t rows,
-                            int64_t row_bytes, void* stream) {
-  if (rows <= 0) return CATCOC_OK;
-  const int grid = rows < 1184 ? static_cast<int>(rows) : 1184;
-  pad2d_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<uint8_t*>(dst), dst_pitch,
-                                                                    static_cast<const uint8_t*>(src), src_pitch, rows,
-                                                                    row_bytes);
   CATCOC_CUDA_OK(cudaGetLastError());
   return CATCOC_OK;
 }

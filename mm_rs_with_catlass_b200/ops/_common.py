@@ -90,6 +90,9 @@ class Operand:
     ld: int
     trans: bool
     copied: bool = False  # the storage is a fresh padded copy of the caller's data (not reusable)
+    # how that copy was made from the caller's own storage: (src ptr, src pitch, rows, row bytes, dst pitch); None
+    # when it was made from a temporary
+    pad: Optional[Tuple[int, int, int, int, int]] = None
 
 
 def _tma_legal(t: torch.Tensor) -> bool:
@@ -101,16 +104,25 @@ def pad_rows(t: torch.Tensor) -> torch.Tensor:
     """Returns a copy of the 2-D row-major tensor whose row pitch is a multiple of 16 bytes,
     made by the library's own pad kernel (the analogue of the reference's padding prologue,
     3rdparty/catlass/include/catlass/gemm/kernel/padding_matmul.hpp:32-347)."""
+    src = t if t.stride(-1) == 1 else t.contiguous()
+    pad = pad_geometry(src)
+    buf = torch.empty((pad[2], pad[4] // t.element_size()), dtype=t.dtype, device=t.device)
+    run_pad(pad, buf)
+    return buf
+
+
+def pad_geometry(t: torch.Tensor) -> Tuple[int, int, int, int, int]:
+    """(src ptr, src pitch, rows, row bytes, dst pitch) of the padded copy of a row-major matrix."""
     elt = t.element_size()
     rows, cols = t.shape
-    per16 = 16 // elt
-    ld = (cols + per16 - 1) // per16 * per16
-    buf = torch.empty((rows, ld), dtype=t.dtype, device=t.device)
-    src = t if t.stride(-1) == 1 else t.contiguous()
-    stream = torch.cuda.current_stream(t.device).cuda_stream
-    N.check(N.lib().catcoc_pad2d(buf.data_ptr(), ld * elt, src.data_ptr(), src.stride(0) * elt, rows, cols * elt,
-                                 C.c_void_p(stream)))
-    return buf
+    return t.data_ptr(), t.stride(0) * elt, rows, cols * elt, (cols * elt + 15) // 16 * 16
+
+
+def run_pad(pad: Tuple[int, int, int, int, int], buf: torch.Tensor) -> None:
+    """Queues the pad kernel on the current stream; ``buf`` holds rows x dst pitch bytes."""
+    src, pitch, rows, row_bytes, dst_pitch = pad
+    stream = torch.cuda.current_stream(buf.device).cuda_stream
+    N.check(N.lib().catcoc_pad2d(buf.data_ptr(), dst_pitch, src, pitch, rows, row_bytes, C.c_void_p(stream)))
 
 
 def as_operand(x: torch.Tensor, trans: bool) -> Operand:
@@ -126,11 +138,13 @@ def as_operand(x: torch.Tensor, trans: bool) -> Operand:
     if x.stride(-1) != 1 and x.stride(0) == 1 and x.shape[0] > 1 and x.shape[1] > 1:
         x = x.t()
         trans = not trans
-    copied = False
+    copied, pad = False, None
     if not _tma_legal(x):
+        if x.stride(-1) == 1:
+            pad = pad_geometry(x)
         x = pad_rows(x)
         copied = True
-    return Operand(x, x.data_ptr(), x.stride(0), trans, copied)
+    return Operand(x, x.data_ptr(), x.stride(0), trans, copied, pad)
 
 
 def tkey(t: Optional[torch.Tensor]):
