@@ -242,6 +242,12 @@ int catcoc_shmem_put_blocks(void);  /* blocks a put launches: each adds signal_v
 int catcoc_pad2d(void* dst, int64_t dst_pitch, const void* src, int64_t src_pitch, int64_t rows,
                  int64_t row_bytes, void* stream);
 
+/* block-scaled fp8 (csrc/kernels/mx_quant.cu): x (fp16 / bf16 / fp32, `elems` contiguous elements, whole blocks of 32)
+ * -> q = fp8(x / 2^e), scales = e + 127 per block with e = ceil(log2(amax / fp8_max)), 0 for an all-zero block; and the
+ * repacking of scales [rows, kb] into [ceil(rows / 128), ceil(kb / 4), 512] blocks, padded with 127 */
+int catcoc_mx_quantize(const void* x, int fmt, int64_t elems, int e5m2, void* q, void* scales, void* stream);
+int catcoc_mx_pack_scales(const void* scales, int rows, int kb, void* out, void* stream);
+
 /* out = cast(alpha * sum over `slices` fp32 partials [rows, cols] (slice s at parts + s * slice_elems)
  *            + beta * c_src + bias[cols]); finishes a split-K product */
 int catcoc_splitk_reduce(const float* parts, int slices, int64_t slice_elems, int rows, int cols, void* out,

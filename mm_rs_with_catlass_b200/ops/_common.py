@@ -181,17 +181,20 @@ def default_timeout_ns() -> int:
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
+def stream_of(device: torch.device) -> int:
+    """Raw handle of the current stream of ``device``."""
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream
+
+
 def launch(args: N.OpArgs, device: torch.device, timeout_ns: Optional[int] = None) -> None:
     """Queues the kernel on the current stream of ``device`` (which must be the current device).
     The wait budget is re-read on every launch so that a cached argument block follows
     ``CATCOC_TIMEOUT_MS``."""
     args.timeout_ns = timeout_ns if timeout_ns is not None else default_timeout_ns()
     args.events, args.events_cap = _event_ring
-    if _raw_stream is not None and device.index is not None:
-        stream = _raw_stream(device.index)
-    else:
-        stream = torch.cuda.current_stream(device).cuda_stream
-    code = N.lib().catcoc_fused_launch(C.byref(args), C.c_void_p(stream))
+    code = N.lib().catcoc_fused_launch(C.byref(args), C.c_void_p(stream_of(device)))
     if code < 0:
         N.check(code)
     global _launches

@@ -10,6 +10,7 @@ blocks the tensor core reads (128 rows x 4 K-blocks, row r at ``(r % 32) * 16 + 
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Optional, Tuple
 
 import torch
@@ -31,13 +32,24 @@ def quantize_mxf8(x: torch.Tensor, fmt: str = "e4m3") -> Tuple[torch.Tensor, tor
     rows, k = x.shape
     if k % BLOCK:
         raise ValueError("K must be a multiple of 32 for block scaling (K=%d)" % k)
+    dt = torch.float8_e4m3fn if fmt == "e4m3" else torch.float8_e5m2
+    if x.is_cuda and fmt in _FP8_MAX and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and x.numel():
+        # one pass of the quantisation kernel: the same values as the passes below
+        x = x.contiguous()
+        if x.data_ptr() % 16:
+            x = x.clone()
+        q = torch.empty((rows, k), dtype=dt, device=x.device)
+        scales = torch.empty((rows, k // BLOCK), dtype=torch.uint8, device=x.device)
+        with torch.cuda.device(x.device):
+            N.check(N.lib().catcoc_mx_quantize(x.data_ptr(), cm.out_fmt(x.dtype), rows * k, int(fmt == "e5m2"), q.data_ptr(),
+                                               scales.data_ptr(), C.c_void_p(cm.stream_of(x.device))))
+        return q, scales
     xb = x.float().reshape(rows, k // BLOCK, BLOCK)
     amax = xb.abs().amax(dim=-1)
     exp = torch.ceil(torch.log2(torch.clamp(amax, min=2.0 ** -126) / _FP8_MAX[fmt]))
     exp = torch.clamp(exp, -127, 127)
     exp = torch.where(amax > 0, exp, torch.zeros_like(exp))
     q = xb / torch.exp2(exp)[..., None]
-    dt = torch.float8_e4m3fn if fmt == "e4m3" else torch.float8_e5m2
     return q.reshape(rows, k).to(dt), (exp + 127).to(torch.uint8)
 
 
@@ -52,6 +64,15 @@ def pack_scales(scales: torch.Tensor) -> torch.Tensor:
     layout; rows and K-blocks are padded with the neutral scale 127 (= 1.0)."""
     rows, kb = scales.shape
     rt, kt = (rows + 127) // 128, (kb + 3) // 4
+    if scales.is_cuda and scales.dtype == torch.uint8 and scales.numel():
+        scales = scales.contiguous()
+        if scales.data_ptr() % 4:
+            scales = scales.clone()
+        out = torch.empty((rt, kt, 512), dtype=torch.uint8, device=scales.device)
+        with torch.cuda.device(scales.device):
+            N.check(N.lib().catcoc_mx_pack_scales(scales.data_ptr(), rows, kb, out.data_ptr(),
+                                                  C.c_void_p(cm.stream_of(scales.device))))
+        return out
     pad = torch.full((rt * 128, kt * 4), 127, dtype=torch.uint8, device=scales.device)
     pad[:rows, :kb] = scales
     # row = rt*128 + j*32 + l  ->  [rt, kt, l, j, s]
