@@ -43,6 +43,7 @@ SOURCES = [
     "kernels/mx_quant.cu",
     "kernels/small_allreduce.cu",
     "kernels/flash_attn.cu",
+    "kernels/flash_decode.cu",
     "kernels/mla_decode.cu",
     "shmem/host.cu",
     "oracle/oracle.cpp",

@@ -292,6 +292,13 @@ int catcoc_flash_attention(const void* q, const void* k, const void* v, void* ou
                            int Sk, int D, int fmt, int causal, float scale, uint32_t* status, uint64_t timeout_ns,
                            void* stream);
 
+/* The same function for few query rows per key / value head (csrc/kernels/flash_decode.cu): the keys are cut over the SMs.
+ * catcoc_flash_decode_workspace_bytes says whether the kernel takes a call (-1: no) and how much scratch it needs. */
+int64_t catcoc_flash_decode_workspace_bytes(int B, int Hq, int Hk, int Sq, int Sk, int D);
+int catcoc_flash_decode(const void* q, const void* k, const void* v, void* out, void* workspace, int B, int Hq, int Hk,
+                        int Sq, int Sk, int D, int fmt, int causal, float scale, uint32_t* status, uint64_t timeout_ns,
+                        void* stream);
+
 /* ---- multi-head latent attention, decode step over a paged cache (csrc/kernels/mla_decode.cu) ----
  * q_nope [T, H, 512], q_rope [T, H, 64] (T = B * q_len new tokens, q_len 1..4), latent cache [num_pages, 128, 512],
  * rotary cache [num_pages, 128, 64], block_table [B, max_pages] and kv_lens [B] (device int32), out [T, H, 512]; all

@@ -1,0 +1,85 @@
+// One query row's share of an online-softmax step, for the attention kernels whose scores and probabilities live in
+// TMEM (one row per lane, 128 keys per block).
+//
+// All 128 scores of the row are read ONCE into registers (four 32-column tcgen05.ld in flight together) and stay
+// there for the maximum, the exponentials and the sum; a second read would put the TMEM latency into every block's
+// serial chain again. Scale, shift and sum run on register pairs (fma / add .f32x2) and the maximum takes three
+// operands per instruction, so that the special-function unit (32 lanes of ex2 take 8 cycles on a scheduler) and not
+// instruction issue is the longest of the warp's pipes.
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include "catcoc/params.h"
+#include "catcoc/ptx.cuh"
+
+namespace catcoc {
+namespace attn {
+
+constexpr int kRowKeys = 128;            // keys per block
+constexpr float kLazyRescale = 8.0f;     // log2 units the running maximum may exceed the reference by
+
+template <int FMT>
+CATCOC_DEVICE uint32_t pack16(float lo, float hi) {
+  if constexpr (FMT == FMT_BF16) { __nv_bfloat162 hh = __floats2bfloat162_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&hh); }
+  else { __half2 hh = __floats2half2_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&hh); }
+}
+
+// m: reference maximum (log2 domain), l: running sum
+struct RowState {
+  float m = -INFINITY, l = 0.0f;
+};
+
+// Reads 128 scores at TMEM address `t_s`, writes the packed probabilities over them (64 columns) and updates the
+// state. Returns the factor that O has to be multiplied by, and sets `move` (the same in all lanes) when that is not
+// 1 for some row of the warp. `vis_left`: keys of this block the row sees (used when `masked`).
+template <int FMT>
+CATCOC_DEVICE float softmax_row_block(uint32_t t_s, bool masked, int vis_left, float sc, RowState& st, bool& move) {
+  uint32_t v[4][32];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32b_x32(t_s + c * 32, v[c]);
+  ptx::tcgen05_wait_ld();
+  if (masked) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (c * 32 + i >= vis_left) v[c][i] = 0xff800000u;   // -inf: its probability is exactly zero
+  }
+  float mx[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    mx[c] = fmaxf(__uint_as_float(v[c][0]), __uint_as_float(v[c][1]));
+#pragma unroll
+    for (int i = 2; i < 32; i += 2) mx[c] = ptx::max3(mx[c], __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
+  }
+  const float m_new = fmaxf(st.m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc);
+  move = __any_sync(0xffffffffu, m_new > st.m + kLazyRescale);   // -inf + 8 = -inf: the first block moves
+  const float m_use = move ? m_new : st.m;
+  const float m_safe = (m_use == -INFINITY) ? 0.0f : m_use;      // a row that sees nothing yet
+  const float alpha = !move ? 1.0f : ((st.m == -INFINITY) ? 0.0f : ptx::ex2_approx(st.m - m_safe));
+  const uint64_t sc2 = ptx::pack_f32x2(sc, sc), nm2 = ptx::pack_f32x2(-m_safe, -m_safe);
+  uint64_t sum2[2] = {0ull, 0ull};
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t w[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const int c = 2 * h + (i >> 4), e = (i & 15) * 2;
+      float x0, x1;
+      ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1])), sc2, nm2), x0, x1);
+      x0 = ptx::ex2_approx(x0);
+      x1 = ptx::ex2_approx(x1);
+      sum2[i & 1] = ptx::add_f32x2(sum2[i & 1], ptx::pack_f32x2(x0, x1));
+      w[i] = pack16<FMT>(x0, x1);
+    }
+    ptx::tmem_st_32x32b_x32(t_s + h * 32, w);
+  }
+  float s0, s1;
+  ptx::unpack_f32x2(ptx::add_f32x2(sum2[0], sum2[1]), s0, s1);
+  st.l = st.l * alpha + (s0 + s1);
+  st.m = m_use;
+  return alpha;
+}
+
+}  // namespace attn
+}  // namespace catcoc

@@ -1,4 +1,6 @@
-"""Flash attention forward on the library's own tcgen05 kernel (``csrc/kernels/flash_attn.cu``).
+"""Flash attention forward on the library's own tcgen05 kernels (``csrc/kernels/flash_attn.cu`` and, when the
+query heads that share a key / value head have at most 128 rows between them, ``flash_decode.cu``: the
+general structure below with the key blocks dealt out over the SMs).
 
 One CTA per 256 query rows (two tiles of 128) of one (batch, head): ``S = Q K^T`` and
 ``O += P V`` run on the tensor cores with all four accumulators in TMEM. The softmax warps of a
@@ -61,11 +63,17 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal
     if not scale > 0.0:
         raise ValueError("the softmax scale must be positive")
     with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        N.check(N.lib().catcoc_flash_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), b, hq, hk, sq,
-                                               sk, d, cm.out_fmt(q.dtype), int(causal), float(scale),
-                                               cm.local_status(dev).data_ptr(), cm.default_timeout_ns(),
-                                               C.c_void_p(stream)))
+        lib, stream = N.lib(), C.c_void_p(cm.stream_of(dev))
+        tail = (b, hq, hk, sq, sk, d, cm.out_fmt(q.dtype), int(causal), float(scale), cm.local_status(dev).data_ptr(),
+                cm.default_timeout_ns(), stream)
+        # few query rows per key / value head (decode steps): the keys are cut over the SMs instead of the queries
+        need = int(lib.catcoc_flash_decode_workspace_bytes(b, hq, hk, sq, sk, d))
+        if need >= 0:
+            ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+            N.check(lib.catcoc_flash_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                                            ws.data_ptr() if need else None, *tail))
+        else:
+            N.check(lib.catcoc_flash_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), *tail))
     return out
 
 
