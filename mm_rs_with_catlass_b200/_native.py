@@ -111,6 +111,8 @@ def _declare(lib) -> None:
         "catcoc_is_checked_build": (i32, []),
         "catcoc_num_sms": (i32, [i32]),
         "catcoc_fused_launch": (i32, [P(OpArgs), vp]),
+        "catcoc_slice_k_workspace_bytes": (i64, [i32]),
+        "catcoc_slice_k_launch": (i32, [P(OpArgs), vp, vp, vp]),
         "catcoc_stage_bytes": (i64, [i32, i32, i32, i32, i32, i32, i32]),
         "catcoc_arrive_words": (i64, [i32, i32, i32, i32, i32, i32]),
         "catcoc_done_words": (i64, [i32, i32, i32, i32, i32, i32]),

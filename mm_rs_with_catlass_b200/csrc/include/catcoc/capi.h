@@ -134,6 +134,13 @@ int catcoc_is_checked_build(void);   /* 1: device-side bounds checks compiled in
 /* Launches the fused kernel on `stream` (a cudaStream_t). */
 int catcoc_fused_launch(const CatcocOpArgs* args, void* stream);
 
+/* Products over ragged ranges of K in one launch (weight gradients of grouped products): group g of args->num_groups
+ * multiplies the K rows [k_range[2 g], k_range[2 g + 1]) (host memory; an empty range leaves its output untouched) of
+ * an A stored [K, M_g] and a B stored [K, N]; M_g = args->group_rows, args->K counts all K rows, the outputs are
+ * stacked along rows. `workspace`: catcoc_slice_k_workspace_bytes(groups) bytes of device memory, 128-byte aligned. */
+int64_t catcoc_slice_k_workspace_bytes(int groups);
+int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void* workspace, void* stream);
+
 /* Workspace sizes (bytes / words) for given problem + tiling, identical on every rank. */
 int64_t catcoc_stage_bytes(int M, int N, int W, int seg_dim, int bn, int cta_pair, int partial_fmt);
 int64_t catcoc_arrive_words(int M, int N, int W, int seg_dim, int bn, int cta_pair);

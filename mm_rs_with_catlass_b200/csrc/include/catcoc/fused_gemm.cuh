@@ -429,6 +429,14 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
         a_row -= ti.seg * p.g_a_row_back;
         a_k_off = ti.seg * p.g_a_k;
       }
+      int tile_kb = num_kb;
+      if (p.gk_range != nullptr) {
+        const int2 r = __ldg(p.gk_range + ti.seg);
+        a_k_off = r.x;
+        tile_kb = ceil_div(r.y - r.x, p.bk * kps);   // an empty range has no tile: every role skips it
+        tma = p.gk_maps + 2 * ti.seg;
+        if (tile_kb > 0) ptx::tmap_acquire(tma);
+      }
       if (p.mode == MODE_AG && fused) {
         if (ti.seg == p.rank && p.ag_raw == 0) {
           a_row = ti.mi * sched.BM + sub * kBM;  // row inside the local shard
@@ -480,7 +488,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
         }
       }
       if (lane == 0) emit_event(p, EV_PRODUCER, EV_BEGIN, static_cast<uint32_t>(t));
-      for (int kb = 0; kb < num_kb; ++kb) {
+      for (int kb = 0; kb < tile_kb; ++kb) {
         tick.lap(c_issue);
         const bool got = ptx::mbar_wait(&tail->empty[stage], phase ^ 1u, p.timeout_ns, abort_flag);
         tick.lap(c_wait);
@@ -575,7 +583,15 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
       unsigned long long c_full = 0, c_acc = 0, c_issue = 0;
       Tick tick(tr);
       bool probed = false;
+      GroupWalk walk = group_walk_begin(p);
       for (int t = worker; ok && t < total_tiles; t += num_workers) {
+        int tile_k = K, tile_kb = num_kb;
+        if (p.gk_range != nullptr) {
+          const int2 r = __ldg(p.gk_range + walk_tile(p, t, walk).seg);
+          tile_k = r.y - r.x;
+          tile_kb = ceil_div(tile_k, p.bk * kps);
+          if (tile_kb <= 0) continue;
+        }
         tick.lap(c_issue);
         const bool got_acc = ptx::mbar_wait(&tail->acc_empty[acc], acc_phase ^ 1u, p.timeout_ns, abort_flag);
         tick.lap(c_acc);
@@ -589,7 +605,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
         ptx::tcgen05_fence_after();
         if (lane == 0) emit_event(p, EV_MMA, EV_BEGIN, static_cast<uint32_t>(t));
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc) * acc_stride;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = 0; kb < tile_kb; ++kb) {
           tick.lap(c_issue);
           // `probed` is the answer of a non-blocking probe issued before the previous stage's
           // MMAs: its latency was hidden behind their issue, so a ready stage costs nothing here
@@ -606,7 +622,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
           }
           ptx::tcgen05_fence_after();
           // K tail: TMA zero-fills beyond K, MMAs entirely out of range are skipped.
-          const int k_mmas = ceil_div(K, umma_k);                    // MMAs along K for a whole tile
+          const int k_mmas = ceil_div(tile_k, umma_k);               // MMAs along K for a whole tile
           const int k_first = kb * kps * k_per_stage;                // index of this stage's first MMA
           const uint64_t da = da0 + static_cast<uint64_t>(stage * stage_inc);
           const uint64_t db = db0 + static_cast<uint64_t>(stage * stage_inc);
@@ -640,7 +656,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
                 }
               }
               ptx::tcgen05_commit(&tail->empty[stage]);
-              if (kb == num_kb - 1) ptx::tcgen05_commit(&tail->acc_full[acc]);
+              if (kb == tile_kb - 1) ptx::tcgen05_commit(&tail->acc_full[acc]);
             }
           } else if (ptx::elect_one()) {
 #pragma unroll
@@ -664,7 +680,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
             // frees this smem stage (in both CTAs of a pair) once the MMAs above retire
             if (CTA2) ptx::tcgen05_commit_pair(&tail->empty[stage], 3);
             else ptx::tcgen05_commit(&tail->empty[stage]);
-            if (kb == num_kb - 1) {
+            if (kb == tile_kb - 1) {
               if (CTA2) ptx::tcgen05_commit_pair(&tail->acc_full[acc], 3);
               else ptx::tcgen05_commit(&tail->acc_full[acc]);
             }
@@ -728,6 +744,10 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
     GroupWalk walk = group_walk_begin(p);
     for (int t = worker; ok && t < total_tiles; t += num_workers) {
       const TileInfo ti = walk_tile(p, t, walk);
+      if (p.gk_range != nullptr) {
+        const int2 r = __ldg(p.gk_range + ti.seg);
+        if (r.y <= r.x) continue;
+      }
       const bool own = !kReduce || !fused || (p.mode == MODE_AG) || (ti.seg == p.rank);
       const bool reduce_here = kReduce && fused && own && (p.mode == MODE_RS || p.mode == MODE_AR);
       const int st_fmt = (own && !pull) ? p.out_fmt : pfmt;   // format of what this tile's epilogue stores
@@ -1228,7 +1248,16 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
         b_col += ti.seg * p.g_b_row;
         b_k_off = ti.seg * p.g_b_k;
       }
-      for (int kb = 0; kb < num_kb; ++kb) {
+      const CUtensorMap* tmb = &p.tm_b;
+      int tile_kb = num_kb;
+      if (p.gk_range != nullptr) {
+        const int2 r = __ldg(p.gk_range + ti.seg);
+        b_k_off = r.x;
+        tile_kb = ceil_div(r.y - r.x, p.bk * kps);
+        tmb = p.gk_maps + 2 * ti.seg + 1;
+        if (tile_kb > 0) ptx::tmap_acquire(tmb);
+      }
+      for (int kb = 0; kb < tile_kb; ++kb) {
         if (!ptx::mbar_wait(&tail->empty[stage], phase ^ 1u, p.timeout_ns, abort_flag)) {
           if (lane == 0) {
             report_status(p, STATUS_TIMEOUT_PIPELINE, 4u, static_cast<uint32_t>(t), static_cast<uint32_t>(kb), 0u);
@@ -1256,21 +1285,21 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
             const int k0 = (kb * kps + j) * p.bk + b_k_off;
             if (!CTA2) {
               if (!p.b_mn_major) {
-                ptx::tma_load_2d(sb, &p.tm_b, &tail->full[stage], k0, b_col);
+                ptx::tma_load_2d(sb, tmb, &tail->full[stage], k0, b_col);
               } else if (p.b_3d) {
-                ptx::tma_load_3d(sb, &p.tm_b, &tail->full[stage], 0, k0, b_col / per_box);
+                ptx::tma_load_3d(sb, tmb, &tail->full[stage], 0, k0, b_col / per_box);
               } else {
                 for (int b = 0; b < b_cols_cta / per_box; ++b)
-                  ptx::tma_load_2d(sb + b * (p.bk * 128), &p.tm_b, &tail->full[stage], b_col + b * per_box, k0);
+                  ptx::tma_load_2d(sb + b * (p.bk * 128), tmb, &tail->full[stage], b_col + b * per_box, k0);
               }
             } else {
               if (!p.b_mn_major) {
-                ptx::tma_load_2d_pair(sb, &p.tm_b, bar, k0, b_col);
+                ptx::tma_load_2d_pair(sb, tmb, bar, k0, b_col);
               } else if (p.b_3d) {
-                ptx::tma_load_3d_pair(sb, &p.tm_b, bar, 0, k0, b_col / per_box);
+                ptx::tma_load_3d_pair(sb, tmb, bar, 0, k0, b_col / per_box);
               } else {
                 for (int b = 0; b < b_cols_cta / per_box; ++b)
-                  ptx::tma_load_2d_pair(sb + b * (p.bk * 128), &p.tm_b, bar, b_col + b * per_box, k0);
+                  ptx::tma_load_2d_pair(sb + b * (p.bk * 128), tmb, bar, b_col + b * per_box, k0);
               }
             }
           }

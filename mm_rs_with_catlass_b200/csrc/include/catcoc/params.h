@@ -177,6 +177,11 @@ struct alignas(64) FusedParams {
   int g_b_row;                // N coordinate of B (stored [N, K]) starts at  g * g_b_row
   int g_b_k;                  // K coordinate of B starts at  g * g_b_k
   int g_nvec;                 // scale_n / bias / bias_f of group g start at  g * g_nvec
+  // Ragged K ranges (null: off): group g multiplies the K rows [gk_range[g].x, gk_range[g].y) of an A stored [K, M] and
+  // a B stored [K, N]. Its two tensor maps (A, B) end at the range's last row, so that the tail of the last K block
+  // reads as zeros and not as the next group's rows. Device memory, written ahead of the launch.
+  const CUtensorMap* gk_maps;
+  const int2* gk_range;
 
   // block-scaled fp8: scale factors packed in 512-byte blocks of 128 rows x 4 K-blocks
   // (row r, K-block s at (r % 32) * 16 + (r / 32) * 4 + s); block (row_tile, k128) at

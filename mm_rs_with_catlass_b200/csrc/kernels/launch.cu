@@ -818,3 +818,78 @@ extern "C" int catcoc_fused_launch(const CatcocOpArgs* args, void* stream) {
   const int threads = (cw >= 1 && cw <= 5) ? (7 + cw) * 32 : 0;
   return catcoc_launch_params(p, kind, grid, pair, threads, static_cast<cudaStream_t>(stream));
 }
+
+// ---- ragged K ranges in one launch ----
+namespace {
+// The maps travel as a kernel argument (no host buffer has to outlive the call, and the launch can be captured).
+constexpr int kMapBatch = 48;
+struct alignas(64) MapBatch {
+  CUtensorMap map[2 * kMapBatch];
+  int2 range[kMapBatch];
+  int first, count;
+};
+
+__global__ void __launch_bounds__(128) store_maps_kernel(const __grid_constant__ MapBatch m, CUtensorMap* maps, int2* range) {
+  const uint4* src = reinterpret_cast<const uint4*>(m.map);
+  uint4* dst = reinterpret_cast<uint4*>(maps + 2 * m.first);
+  for (int i = threadIdx.x; i < m.count * 2 * static_cast<int>(sizeof(CUtensorMap) / 16); i += blockDim.x) dst[i] = src[i];
+  for (int i = threadIdx.x; i < m.count; i += blockDim.x) range[m.first + i] = m.range[i];
+  ptx::tmap_release();
+}
+}  // namespace
+
+extern "C" int64_t catcoc_slice_k_workspace_bytes(int groups) {
+  return groups > 0 ? static_cast<int64_t>(groups) * (2 * sizeof(CUtensorMap) + sizeof(int2)) : 0;
+}
+
+extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void* workspace, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (args == nullptr || k_range == nullptr || workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 127) != 0) {
+    set_error("slice_k: null argument, or a workspace that is not 128-byte aligned");
+    return CATCOC_E_BAD_ARG;
+  }
+  const CatcocOpArgs& a = *args;
+  if (a.num_groups <= 0 || a.group_ends != nullptr || !a.trans_a || a.trans_b || a.g_a_k != 0 || a.g_b_k != 0 || a.g_b_row != 0) {
+    set_error("slice_k takes uniform groups of an A stored [K, M] and a B stored [K, N]");
+    return CATCOC_E_UNSUPPORTED;
+  }
+  for (int g = 0; g < a.num_groups; ++g) {
+    if (k_range[2 * g] < 0 || k_range[2 * g + 1] < k_range[2 * g] || k_range[2 * g + 1] > a.K) {
+      set_error("slice_k: K range [%d, %d) of group %d lies outside [0, %d)", k_range[2 * g], k_range[2 * g + 1], g, a.K);
+      return CATCOC_E_BAD_ARG;
+    }
+  }
+  FusedParams p;
+  int kind = 0, grid = 0, pair = 0;
+  int rc = catcoc_build_params(args, &p, &kind, &grid, &pair);
+  if (rc != 0) return rc;
+  Resolved rf;
+  rc = resolve_format(a.in_fmt, &rf);
+  if (rc != 0) return rc;
+  CUtensorMap* maps = static_cast<CUtensorMap*>(workspace);
+  int2* range = reinterpret_cast<int2*>(maps + 2 * a.num_groups);
+  const int per128 = 128 / rf.elt;
+  const int b_cols = pair ? p.sched.BN / 2 : p.sched.BN;
+  MapBatch batch;
+  for (int g0 = 0; g0 < a.num_groups; g0 += kMapBatch) {
+    batch.first = g0;
+    batch.count = imin(kMapBatch, a.num_groups - g0);
+    for (int i = 0; i < batch.count; ++i) {
+      const int begin = k_range[2 * (g0 + i)], end = k_range[2 * (g0 + i) + 1];
+      batch.range[i] = make_int2(begin, end);
+      if (end <= begin) continue;                         // never read
+      CUtensorMap* ma = &batch.map[2 * i];
+      rc = p.a_3d ? encode_3d_blocks(ma, a.a, rf.elt, rf.dt, end, a.a_rows_total, a.lda, rf.bk, kBM / per128)
+                  : encode_2d(ma, a.a, rf.elt, rf.dt, end, a.a_rows_total, a.lda, per128, rf.bk);
+      if (rc == 0)
+        rc = p.b_3d ? encode_3d_blocks(ma + 1, a.b, rf.elt, rf.dt, end, a.b_n_total, a.ldb, rf.bk, b_cols / per128)
+                    : encode_2d(ma + 1, a.b, rf.elt, rf.dt, end, a.b_n_total, a.ldb, per128, rf.bk);
+      if (rc != 0) return rc;
+    }
+    store_maps_kernel<<<1, 128, 0, stream>>>(batch, maps, range);
+    CATCOC_CUDA_OK(cudaGetLastError());
+  }
+  p.gk_maps = maps;
+  p.gk_range = range;
+  return catcoc_launch_params(p, kind, grid, pair, 0, stream);
+}
