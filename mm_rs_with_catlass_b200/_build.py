@@ -45,6 +45,7 @@ SOURCES = [
     "kernels/flash_attn.cu",
     "kernels/flash_decode.cu",
     "kernels/mla_decode.cu",
+    "kernels/mla_rows.cu",
     "shmem/host.cu",
     "oracle/oracle.cpp",
 ]

@@ -171,6 +171,8 @@ def _declare(lib) -> None:
         "catcoc_flash_decode": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, vp, u64, vp]),
         "catcoc_mla_workspace_bytes": (i64, [i32, i32, i32, i32]),
         "catcoc_mla_decode": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, C.c_float, i32, vp, u64, vp]),
+        "catcoc_mla_rows_workspace_bytes": (i64, [i32, i32, i32, i32]),
+        "catcoc_mla_rows": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, C.c_float, vp, u64, vp]),
         "catcoc_matmul_noalloc": (i32, [vp, i64, vp, i64, vp, i64, i32, i32, i32, i32, i32, i32, i32, vp]),
         "catcoc_matmul_noalloc_status": (i32, [P(u32)]),
     }

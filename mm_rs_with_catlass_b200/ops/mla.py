@@ -25,8 +25,6 @@ LATENT = 512
 ROPE = 64
 PAGE = 128
 
-_workspaces: dict = {}
-
 
 def _pick_splits(batch: int, rows_per_item: int, max_pages: int, sms: int = 148) -> int:
     """Slices per sequence. One CTA fits an SM, so the grid runs in waves of ``sms`` CTAs and a
@@ -92,23 +90,27 @@ def mla_decode(q_nope: torch.Tensor, q_rope: torch.Tensor, ckv_cache: torch.Tens
     if out.shape != q_nope.shape or out.dtype != dt or not out.is_contiguous():
         raise ValueError("out must be a contiguous tensor shaped like q_nope")
     max_pages = block_table.shape[1]
-    if splits is None:
-        splits = _pick_splits(batch, q_len * heads, max_pages)
     lib = N.lib()
-    need = int(lib.catcoc_mla_workspace_bytes(batch, q_len, heads, int(splits)))
-    ws = None
-    if need:
-        ws = _workspaces.get(dev.index)
-        if ws is None or ws.numel() < need:
-            ws = torch.empty(need, dtype=torch.uint8, device=dev)
-            _workspaces[dev.index] = ws          # kept: stream order makes the reuse by the next call safe
     with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        N.check(lib.catcoc_mla_decode(q_nope.data_ptr(), q_rope.data_ptr(), ckv_cache.data_ptr(), krope_cache.data_ptr(),
-                                      block_table.data_ptr(), kv_lens.data_ptr(), out.data_ptr(),
-                                      ws.data_ptr() if ws is not None else None, batch, q_len, heads,
+        stream = C.c_void_p(cm.stream_of(dev))
+        ptrs = (q_nope.data_ptr(), q_rope.data_ptr(), ckv_cache.data_ptr(), krope_cache.data_ptr(), block_table.data_ptr(),
+                kv_lens.data_ptr(), out.data_ptr())
+        need = int(lib.catcoc_mla_rows_workspace_bytes(batch, q_len, heads, max_pages)) if splits is None else -1
+        if need >= 0:
+            # few query rows per sequence: the keys are the M side, the pages of all sequences are dealt out over the SMs
+            ws = torch.empty(need, dtype=torch.uint8, device=dev)
+            N.check(lib.catcoc_mla_rows(*ptrs, ws.data_ptr(), batch, q_len, heads, ckv_cache.shape[0], max_pages,
+                                        cm.out_fmt(dt), int(causal), float(scale), cm.local_status(dev).data_ptr(),
+                                        cm.default_timeout_ns(), stream))
+            return out
+        if splits is None:
+            splits = _pick_splits(batch, q_len * heads, max_pages)
+        need = int(lib.catcoc_mla_workspace_bytes(batch, q_len, heads, int(splits)))
+        # scratch of the caching allocator: calls on several streams never share one
+        ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+        N.check(lib.catcoc_mla_decode(*ptrs, ws.data_ptr() if ws is not None else None, batch, q_len, heads,
                                       ckv_cache.shape[0], max_pages, cm.out_fmt(dt), int(causal), float(scale), int(splits),
-                                      cm.local_status(dev).data_ptr(), cm.default_timeout_ns(), C.c_void_p(stream)))
+                                      cm.local_status(dev).data_ptr(), cm.default_timeout_ns(), stream))
     return out
 
 
