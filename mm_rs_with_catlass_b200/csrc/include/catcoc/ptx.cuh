@@ -469,9 +469,11 @@ CATCOC_DEVICE uint32_t ld_shared_cluster_u32(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
   return v;
 }
+// Hands an accumulator back to the pair's leader. What it orders are TMEM reads (wait::ld + fence::before_thread_sync),
+// no memory: with .release.cluster the arrive waited for every store of the warp, its output windows included, and the
+// epilogue spent 2900 instead of 1150 cycles per 128 x 256 tile on converting.
 CATCOC_DEVICE void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
-               : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load issued by either CTA of a pair; completion bytes are credited to `bar_cluster_addr`,
 // which may live in the peer CTA (the pair's leader).
