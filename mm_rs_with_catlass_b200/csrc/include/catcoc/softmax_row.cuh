@@ -29,11 +29,29 @@ struct RowState {
   float m = -INFINITY, l = 0.0f;
 };
 
+// O *= alpha, one row of D fp32 columns in TMEM
+template <int D>
+CATCOC_DEVICE void rescale_o(uint32_t t_o, float alpha) {
+#pragma unroll
+  for (int c = 0; c < D / 16; ++c) {
+    uint32_t v[16];
+    ptx::tmem_ld_32x32b_x16(t_o + c * 16, v);
+    ptx::tcgen05_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * alpha);
+    ptx::tmem_st_32x32b_x16(t_o + c * 16, v);
+  }
+}
+
 // Reads 128 scores at TMEM address `t_s`, writes the packed probabilities over them (64 columns) and updates the
-// state. Returns the factor that O has to be multiplied by, and sets `move` (the same in all lanes) when that is not
-// 1 for some row of the warp. `vis_left`: keys of this block the row sees (used when `masked`).
-template <int FMT>
-CATCOC_DEVICE float softmax_row_block(uint32_t t_s, bool masked, int vis_left, float sc, RowState& st, bool& move) {
+// state. `rescale(alpha)` is called before the first probability when the reference maximum of some row of the warp
+// moved (all lanes together): O has to be multiplied by alpha. `half()` is called when the probabilities of the first
+// 64 keys have been issued. `vis_left`: keys of this block the row sees (used when `masked`).
+//
+// A quarter of the exponentials as a degree-5 polynomial on the FMA pipe was measured slower (causal 2 x 32 x 8192:
+// 1019 against 980 us): a chain of one row's steps, not the special-function unit, is what a tile waits for.
+template <int FMT, class Rescale, class Half>
+CATCOC_DEVICE void softmax_row_block(uint32_t t_s, bool masked, int vis_left, float sc, RowState& st, Rescale&& rescale, Half&& half) {
   uint32_t v[4][32];
 #pragma unroll
   for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32b_x32(t_s + c * 32, v[c]);
@@ -53,10 +71,11 @@ CATCOC_DEVICE float softmax_row_block(uint32_t t_s, bool masked, int vis_left, f
     for (int i = 2; i < 32; i += 2) mx[c] = ptx::max3(mx[c], __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
   }
   const float m_new = fmaxf(st.m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc);
-  move = __any_sync(0xffffffffu, m_new > st.m + kLazyRescale);   // -inf + 8 = -inf: the first block moves
+  const bool move = __any_sync(0xffffffffu, m_new > st.m + kLazyRescale);   // -inf + 8 = -inf: the first block moves
   const float m_use = move ? m_new : st.m;
   const float m_safe = (m_use == -INFINITY) ? 0.0f : m_use;      // a row that sees nothing yet
   const float alpha = !move ? 1.0f : ((st.m == -INFINITY) ? 0.0f : ptx::ex2_approx(st.m - m_safe));
+  if (move) rescale(alpha);
   const uint64_t sc2 = ptx::pack_f32x2(sc, sc), nm2 = ptx::pack_f32x2(-m_safe, -m_safe);
   uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
@@ -65,20 +84,20 @@ CATCOC_DEVICE float softmax_row_block(uint32_t t_s, bool masked, int vis_left, f
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       const int c = 2 * h + (i >> 4), e = (i & 15) * 2;
-      float x0, x1;
-      ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1])), sc2, nm2), x0, x1);
-      x0 = ptx::ex2_approx(x0);
-      x1 = ptx::ex2_approx(x1);
-      sum2[i & 1] = ptx::add_f32x2(sum2[i & 1], ptx::pack_f32x2(x0, x1));
-      w[i] = pack16<FMT>(x0, x1);
+      float e0, e1;
+      ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1])), sc2, nm2), e0, e1);
+      e0 = ptx::ex2_approx(e0);
+      e1 = ptx::ex2_approx(e1);
+      sum2[i & 1] = ptx::add_f32x2(sum2[i & 1], ptx::pack_f32x2(e0, e1));
+      w[i] = pack16<FMT>(e0, e1);
     }
     ptx::tmem_st_32x32b_x32(t_s + h * 32, w);
+    if (h == 0) half();
   }
   float s0, s1;
   ptx::unpack_f32x2(ptx::add_f32x2(sum2[0], sum2[1]), s0, s1);
   st.l = st.l * alpha + (s0 + s1);
   st.m = m_use;
-  return alpha;
 }
 
 }  // namespace attn

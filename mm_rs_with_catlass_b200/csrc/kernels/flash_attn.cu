@@ -9,7 +9,13 @@
 //
 // TMEM columns: S_0 [0, 128), S_1 [128, 256), O_0 [256, 256 + D), O_1 [256 + D, 256 + 2 D); P_t is 64 columns of
 // packed 16-bit pairs on top of S_t. While the softmax warps of one tile work, the tensor core runs the other
-// tile's two products, so neither waits for the other in the steady state.
+// tile's two products.
+//
+// Bound by the chain of one tile, scores -> maximum -> exponentials -> P V -> next scores (the tensor core is busy
+// 56 % of the time, the special-function unit as much). So the scores are read from TMEM once and stay in registers
+// (softmax_row.cuh; a split of the registers between the warpgroups makes room), and P V starts when the first 64
+// keys' probabilities are written. Causal, 2 x 32 / 8 heads x 8192, D = 128: 1118 -> 963 us (1.14 PFLOP/s), not
+// causal 1922 -> 1690 us; without the early half 981 us.
 //
 // The online-softmax recurrence (m: reference maximum, l: running sum, per row, in the log2 domain):
 //   P = exp2(scale S - m),  l' = l a + rowsum(P),  O' = O a + P V,  a = exp2(m - m')
@@ -28,6 +34,7 @@
 #include "catcoc/host_util.h"
 #include "catcoc/params.h"
 #include "catcoc/ptx.cuh"
+#include "catcoc/softmax_row.cuh"
 
 namespace catcoc {
 namespace attn {
@@ -35,11 +42,13 @@ namespace attn {
 constexpr int kBQ = 128;          // query rows per tile == TMEM lanes
 constexpr int kTiles = 2;         // query tiles per CTA
 constexpr int kBKV = 128;         // keys per block
-constexpr int kThreads = 320;     // 2 x 4 softmax warps, producer, issuer
+constexpr int kThreads = 384;     // 2 x 4 softmax warps, producer, issuer, two warps that only complete the warpgroup
+// Registers: a softmax thread keeps 128 scores and their probabilities. The block is launched with 168 a thread; the
+// third warpgroup gives up what the first two take: 2 x 216 + 72 = 3 x 168.
+constexpr int kSoftmaxRegs = 216, kOtherRegs = 72;
 constexpr int kProducerWarp = 8, kIssuerWarp = 9;
 constexpr int kBlockBytes = 128 * 128;   // one 128-row x 128-byte (64 element) swizzled block
 constexpr int kMaxSlots = 8;
-constexpr float kLazyRescale = 8.0f;     // log2 units the running maximum may exceed the reference by
 
 struct AttnParams {
   CUtensorMap tm_q, tm_k, tm_v;   // {D, S, B * H} with a {64, 128, 1} box, 128-byte swizzle
@@ -54,7 +63,7 @@ struct AttnParams {
 };
 
 struct Bars {
-  uint64_t q_full, kv_full[kMaxSlots], kv_empty[kMaxSlots], s_full[kTiles], p_full[kTiles], o_done[kTiles];
+  uint64_t q_full, kv_full[kMaxSlots], kv_empty[kMaxSlots], s_full[kTiles], p_half[kTiles], p_full[kTiles], o_done[kTiles];
   uint32_t tmem_base, abort_flag;
 };
 
@@ -64,12 +73,6 @@ CATCOC_DEVICE void fail(const AttnParams& p, uint32_t what, uint32_t a, uint32_t
     p.status[6] = blockIdx.x;
     __threadfence_system();
   }
-}
-
-template <int FMT>
-CATCOC_DEVICE uint32_t pack16(float lo, float hi) {
-  if constexpr (FMT == FMT_BF16) { __nv_bfloat162 hh = __floats2bfloat162_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&hh); }
-  else { __half2 hh = __floats2half2_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&hh); }
 }
 
 // D: head dimension; FMT: operand and output dtype (compile time: the softmax loop packs 64 pairs per row and block)
@@ -109,7 +112,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     for (int s = 0; s < kSlots; ++s) { ptx::mbar_init(&bars->kv_full[s], 1); ptx::mbar_init(&bars->kv_empty[s], 1); }
     for (int t = 0; t < kTiles; ++t) {
       ptx::mbar_init(&bars->s_full[t], 1);
-      ptx::mbar_init(&bars->p_full[t], 4);         // one arrival per softmax warp
+      ptx::mbar_init(&bars->p_half[t], 4);         // one arrival per softmax warp: P of the first 64 keys is in TMEM
+      ptx::mbar_init(&bars->p_full[t], 4);         // ... of all of them
       ptx::mbar_init(&bars->o_done[t], 1);
     }
     bars->abort_flag = 0;
@@ -122,6 +126,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   ptx::tcgen05_fence_after();
   const uint32_t tmem = bars->tmem_base;
 
+  if (warp >= kProducerWarp) ptx::reg_dec<kOtherRegs>();   // all four warps of the warpgroup at one place
   if (warp == kProducerWarp) {
     // ------------------------------ TMA producer ------------------------------
     if (ptx::elect_one()) {
@@ -163,14 +168,15 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       }
       ptx::tcgen05_commit(&bars->s_full[t]);
     };
-    auto issue_pv = [&](int t, int item, bool accumulate) {
+    auto issue_pv = [&](int t, int item, int half, bool accumulate) {
       // O_t[128, D] += P_t[128, 128 keys] V[128 keys, D]: P from TMEM (row = lane, two keys per 32-bit column, 8
       // columns per MMA), V MN-major (D contiguous): 16 key rows per MMA = 2048 bytes down a block, blocks of 64
       // head-dim columns 16 KiB apart
       const uint64_t dv = ptx::make_smem_desc_sw128(ptx::smem_u32(skv + (item % kSlots) * kSlotBytes),
                                                     static_cast<uint32_t>(kBlockBytes), 1024u);
 #pragma unroll
-      for (int kk = 0; kk < kBKV / 16; ++kk) {
+      for (int k2 = 0; k2 < kBKV / 32; ++k2) {
+        const int kk = half * (kBKV / 32) + k2;
         const uint64_t offb = static_cast<uint64_t>((kk * 16 * 128) >> 4);
         ptx::umma_f16_ts(tmem + kOCol + t * D, tmem + t * 128 + kk * 8, dv + offb, p.idesc_pv, (accumulate || kk != 0) ? 1u : 0u);
       }
@@ -191,13 +197,18 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       const bool next0 = j + 1 < nblk[0], next1 = j + 1 < nblk[1];
       bool v_here = false;
       if (j < nblk[0]) {
-        // P_0(j) is in TMEM and O_0 has been rescaled
-        ok = ptx::mbar_wait(&bars->p_full[0], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag) && wait_item(v_item);
+        // half of P_0(j) is in TMEM and O_0 has been rescaled: its product starts while the softmax finishes the other half
+        ok = ptx::mbar_wait(&bars->p_half[0], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag) && wait_item(v_item);
         if (!ok) break;
         v_here = true;
         ptx::tcgen05_fence_after();
+        if (ptx::elect_one()) issue_pv(0, v_item, 0, j > 0);
+        __syncwarp();
+        ok = ptx::mbar_wait(&bars->p_full[0], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
+        if (!ok) break;
+        ptx::tcgen05_fence_after();
         if (ptx::elect_one()) {
-          issue_pv(0, v_item, j > 0);
+          issue_pv(0, v_item, 1, true);
           if (!next0) ptx::tcgen05_commit(&bars->o_done[0]);
         }
         __syncwarp();
@@ -209,11 +220,16 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
           __syncwarp();
         }
       }
-      ok = ptx::mbar_wait(&bars->p_full[1], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag) && (v_here || wait_item(v_item));
+      ok = ptx::mbar_wait(&bars->p_half[1], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag) && (v_here || wait_item(v_item));
+      if (!ok) break;
+      ptx::tcgen05_fence_after();
+      if (ptx::elect_one()) issue_pv(1, v_item, 0, j > 0);
+      __syncwarp();
+      ok = ptx::mbar_wait(&bars->p_full[1], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
       if (!ok) break;
       ptx::tcgen05_fence_after();
       if (ptx::elect_one()) {
-        issue_pv(1, v_item, j > 0);
+        issue_pv(1, v_item, 1, true);
         ptx::tcgen05_commit(&bars->kv_empty[v_item % kSlots]);
         if (!next1) ptx::tcgen05_commit(&bars->o_done[1]);
       }
@@ -230,8 +246,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       }
     }
     if (!ok && lane == 0) { fail(p, 2u, 0u, 0u); *abort_flag = 1; }
-  } else {
+  } else if (warp < kProducerWarp) {
     // ------------------------------ softmax / correction / epilogue ------------------------------
+    ptx::reg_inc<kSoftmaxRegs>();
     const int t = warp >> 2;                         // query tile of this warp
     const int qd = warp & 3;                         // TMEM lane quarter of this warp
     const int row = qd * 32 + lane;                  // query row inside the tile
@@ -242,77 +259,22 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     const int vis = p.causal ? min(p.Sk, qi + shift + 1) : p.Sk;            // keys [0, vis) are visible to this row
     const int vis_tile = p.causal ? min(p.Sk, q0 + t * kBQ + shift + 1) : p.Sk;   // ... to every row of the tile
     const float sc = p.scale_log2;
-    float m_ref = -INFINITY, l = 0.0f;
+    RowState st;
     bool ok = true;
     for (int j = 0; j < n_mine; ++j) {
       if (!ptx::mbar_wait(&bars->s_full[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag)) { ok = false; break; }
       ptx::tcgen05_fence_after();
       const int key0 = j * kBKV;
-      const bool masked = key0 + kBKV > vis_tile;    // some row of the tile does not see all of this block
-      // pass 1: row maximum of the raw scores (the scale is positive)
-      float mx = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < kBKV / 64; ++c) {
-        uint32_t v0[32], v1[32];
-        ptx::tmem_ld_32x32b_x32(t_s + c * 64, v0);
-        ptx::tmem_ld_32x32b_x32(t_s + c * 64 + 32, v1);
-        ptx::tcgen05_wait_ld();
-        if (masked) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (key0 + c * 64 + i < vis) mx = fmaxf(mx, __uint_as_float(v0[i]));
-            if (key0 + c * 64 + 32 + i < vis) mx = fmaxf(mx, __uint_as_float(v1[i]));
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, fmaxf(__uint_as_float(v0[i]), __uint_as_float(v1[i])));
-        }
-      }
-      const float m_new = fmaxf(m_ref, mx * sc);
-      const bool move = __any_sync(0xffffffffu, m_new > m_ref + kLazyRescale);   // -inf + 8 = -inf: the first block moves
-      const float m_use = move ? m_new : m_ref;
-      const float m_safe = (m_use == -INFINITY) ? 0.0f : m_use;                   // a row that sees nothing yet
-      const float alpha = !move ? 1.0f : ((m_ref == -INFINITY) ? 0.0f : ptx::ex2_approx(m_ref - m_safe));
-      // pass 2: P = exp2(scale S - m), its row sum, P packed over the scores it came from
-      float sum = 0.0f;
-#pragma unroll
-      for (int c = 0; c < kBKV / 32; ++c) {
-        uint32_t v[32], w[16];
-        ptx::tmem_ld_32x32b_x32(t_s + c * 32, v);
-        ptx::tcgen05_wait_ld();
-        if (masked) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float e0 = (key0 + c * 32 + i < vis) ? ptx::ex2_approx(fmaf(__uint_as_float(v[i]), sc, -m_safe)) : 0.0f;
-            const float e1 = (key0 + c * 32 + i + 1 < vis) ? ptx::ex2_approx(fmaf(__uint_as_float(v[i + 1]), sc, -m_safe)) : 0.0f;
-            sum += e0 + e1;
-            w[i >> 1] = pack16<FMT>(e0, e1);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float e0 = ptx::ex2_approx(fmaf(__uint_as_float(v[i]), sc, -m_safe));
-            const float e1 = ptx::ex2_approx(fmaf(__uint_as_float(v[i + 1]), sc, -m_safe));
-            sum += e0 + e1;
-            w[i >> 1] = pack16<FMT>(e0, e1);
-          }
-        }
-        ptx::tmem_st_32x32b_x16(t_s + c * 16, w);
-      }
-      l = l * alpha + sum;
-      m_ref = m_use;
-      // O *= alpha where the reference maximum moved. s_full(j) was committed behind P V of block j - 1, so O is whole.
-      if (move && j > 0) {
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32b_x32(t_o + c * 32, v);
-          ptx::tcgen05_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-          ptx::tmem_st_32x32b_x32(t_o + c * 32, v);
-        }
-      }
+      // masked: some row of the tile does not see all of the block
+      softmax_row_block<FMT>(t_s, key0 + kBKV > vis_tile, vis - key0, sc, st, [&](float alpha) {
+        // s_full(j) was committed behind P V of block j - 1, so O is whole
+        if (j > 0) rescale_o<D>(t_o, alpha);
+      }, [&] {
+        ptx::tcgen05_wait_st();
+        ptx::tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->p_half[t]);
+      });
       ptx::tcgen05_wait_st();
       ptx::tcgen05_fence_before();
       __syncwarp();
@@ -323,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       if (lane == 0) { fail(p, 3u, t, 0u); *abort_flag = 1; }
     } else {
       ptx::tcgen05_fence_after();
-      const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
+      const float inv = (st.l > 0.0f) ? 1.0f / st.l : 0.0f;
       uint8_t* orow = static_cast<uint8_t*>(p.out) + (static_cast<int64_t>(bh) * p.Sq + qi) * D * 2;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {

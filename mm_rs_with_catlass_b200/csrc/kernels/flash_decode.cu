@@ -239,20 +239,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_decode_kernel(const __grid_
         if (!ptx::mbar_wait(&bars->s_full[t], static_cast<uint32_t>(i >> 1) & 1u, p.timeout_ns, abort_flag)) { ok = false; break; }
         ptx::tcgen05_fence_after();
         const int key0 = (blk0 + i - i0) * kBKV;
-        bool move;
-        const float alpha = attn::softmax_row_block<FMT>(t_s, key0 + kBKV > vis_all, vis - key0, p.scale_log2, st, move);
-        // s_full(i) was committed behind the second product of this parity's previous block, so O_t is whole
-        if (move && i > mine0) {
-#pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t v[32];
-            ptx::tmem_ld_32x32b_x32(t_o + c * 32, v);
-            ptx::tcgen05_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * alpha);
-            ptx::tmem_st_32x32b_x32(t_o + c * 32, v);
-          }
-        }
+        attn::softmax_row_block<FMT>(t_s, key0 + kBKV > vis_all, vis - key0, p.scale_log2, st, [&](float alpha) {
+          // s_full(i) was committed behind the second product of this parity's previous block, so O_t is whole
+          if (i > mine0) attn::rescale_o<D>(t_o, alpha);
+        }, [] {});
         ptx::tcgen05_wait_st();
         ptx::tcgen05_fence_before();
         __syncwarp();
@@ -323,38 +313,54 @@ __global__ void __launch_bounds__(kThreads, 1) flash_decode_kernel(const __grid_
   if (warp == kIssuerWarp) ptx::tmem_dealloc(tmem, kTmemCols);
 }
 
-// Merges the pieces of the sequences that were cut: out = sum_c 2^(m_c - m) O_c / sum_c 2^(m_c - m) l_c. Blocks of 128
-// threads, D / 4 threads per row; started early by the main kernel, whose results it waits for.
+// Merges the pieces of the sequences that were cut: out = sum_c 2^(m_c - m) O_c / sum_c 2^(m_c - m) l_c. One warp per row,
+// 32 pieces at a time: a lane takes the maximum and the weight of one piece, then all lanes add up its columns.
+// Started early by the main kernel, whose results it waits for.
 template <int D, int FMT>
 __global__ void __launch_bounds__(128) flash_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                            void* out, int BH, int rows, int nb, int per) {
-  constexpr int kRowThreads = D / 4;
-  const int64_t r_all = static_cast<int64_t>(blockIdx.x) * (128 / kRowThreads) + threadIdx.x / kRowThreads;
+                                                            void* out, int rows, int nb, int per) {
+  constexpr int kPer = D / 32;                     // columns per lane
+  const int bh = blockIdx.x, r = blockIdx.y * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
   ptx::grid_dependency_wait();
-  if (r_all >= static_cast<int64_t>(BH) * rows) return;
-  const int bh = static_cast<int>(r_all / rows), r = static_cast<int>(r_all - static_cast<int64_t>(bh) * rows);
-  const int c0 = static_cast<int>((static_cast<int64_t>(bh) * nb) / per);
-  const int c1 = static_cast<int>((static_cast<int64_t>(bh + 1) * nb - 1) / per);
+  const int c0 = bh * nb / per, c1 = ((bh + 1) * nb - 1) / per;
+  if (r >= rows) return;
   if (c0 == c1) return;                            // written by its CTA
-  const int col = (threadIdx.x % kRowThreads) * 4;
-  float m = -INFINITY;
-  for (int c = c0; c <= c1; ++c) m = fmaxf(m, part_ml[((static_cast<int64_t>(c) + bh) * rows + r) * 2]);
-  float l = 0.0f;
-  float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
-  for (int c = c0; c <= c1; ++c) {
-    const int64_t pr = (static_cast<int64_t>(c) + bh) * rows + r;
-    const float2 ml = *reinterpret_cast<const float2*>(part_ml + pr * 2);
-    const float4 o = *reinterpret_cast<const float4*>(part_o + pr * D + col);
-    const float w = ml.x == -INFINITY ? 0.0f : ptx::ex2_approx(ml.x - m);
-    l += w * ml.y;
-    acc.x += w * o.x; acc.y += w * o.y; acc.z += w * o.z; acc.w += w * o.w;
+  float m = -INFINITY, l = 0.0f, acc[kPer];
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) acc[e] = 0.0f;
+  for (int base = c0; base <= c1; base += 32) {
+    const int count = min(32, c1 + 1 - base);
+    const int64_t pr = (static_cast<int64_t>(base) + bh) * rows + r;        // piece c: + c * rows
+    const float2 ml = lane < count ? *reinterpret_cast<const float2*>(part_ml + (pr + static_cast<int64_t>(lane) * rows) * 2)
+                                   : make_float2(-INFINITY, 0.0f);
+    float mx = fmaxf(m, ml.x);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float old = m == -INFINITY ? 0.0f : ptx::ex2_approx(m - mx);
+    const float w = ml.x == -INFINITY ? 0.0f : ptx::ex2_approx(ml.x - mx);
+    float wl = w * ml.y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) wl += __shfl_xor_sync(0xffffffffu, wl, o);
+    m = mx;
+    l = l * old + wl;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) acc[e] *= old;
+#pragma unroll 8
+    for (int c = 0; c < count; ++c) {
+      const float wc = __shfl_sync(0xffffffffu, w, c);
+      const float* src = part_o + (pr + static_cast<int64_t>(c) * rows) * D + lane * kPer;
+      float o[kPer];
+      if constexpr (kPer == 4) *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(src);
+      else *reinterpret_cast<float2*>(o) = *reinterpret_cast<const float2*>(src);
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) acc[e] += wc * o[e];
+    }
   }
   const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-  uint2 packed;
-  packed.x = pack16<FMT>(acc.x * inv, acc.y * inv);
-  packed.y = pack16<FMT>(acc.z * inv, acc.w * inv);
-  *reinterpret_cast<uint2*>(static_cast<uint8_t*>(out) + (r_all * D + col) * 2) = packed;
+  uint32_t* dst = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(out) + ((static_cast<int64_t>(bh) * rows + r) * D + lane * kPer) * 2);
+#pragma unroll
+  for (int e = 0; e < kPer / 2; ++e) dst[e] = pack16<FMT>(acc[2 * e] * inv, acc[2 * e + 1] * inv);
 }
 
 }  // namespace decode
@@ -447,10 +453,9 @@ extern "C" int catcoc_flash_decode(const void* q, const void* k, const void* v, 
     main_kernel<<<d.ctas, decode::kThreads, smem, stream>>>(p);
     CATCOC_CUDA_OK(cudaGetLastError());
     if (!d.cut) return CATCOC_OK;
-    const int rows_per_block = 128 / (D / 4);
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(static_cast<unsigned>((bh * d.rows + rows_per_block - 1) / rows_per_block), 1, 1);
+    cfg.gridDim = dim3(static_cast<unsigned>(bh), static_cast<unsigned>((d.rows + 3) / 4), 1);
     cfg.blockDim = dim3(128, 1, 1);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -459,7 +464,7 @@ extern "C" int catcoc_flash_decode(const void* q, const void* k, const void* v, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     CATCOC_CUDA_OK(cudaLaunchKernelEx(&cfg, combine_kernel, static_cast<const float*>(p.part_o), static_cast<const float*>(p.part_ml),
-                                      out, p.BH, p.rows, p.nb, p.per));
+                                      out, p.rows, p.nb, p.per));
     return CATCOC_OK;
   };
   if (D == 128) {
