@@ -141,6 +141,13 @@ int catcoc_fused_launch(const CatcocOpArgs* args, void* stream);
 int64_t catcoc_slice_k_workspace_bytes(int groups);
 int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void* workspace, void* stream);
 
+/* A local product with few output tiles, its K range cut into `slices` slices of `k_slice` elements (a multiple of 256
+ * bytes): the slices run as the groups of one launch, each writing an fp32 (int8 operands: int32) plane to `workspace`
+ * (16-byte aligned, catcoc_splitk_workspace_bytes(M, N, slices) bytes); a second kernel sums the planes in slice order and
+ * applies everything that `args` says about the epilogue. args->tiling describes the tiles of the first launch. */
+int64_t catcoc_splitk_workspace_bytes(int M, int N, int slices);
+int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_slice, void* workspace, void* stream);
+
 /* Workspace sizes (bytes / words) for given problem + tiling, identical on every rank. */
 int64_t catcoc_stage_bytes(int M, int N, int W, int seg_dim, int bn, int cta_pair, int partial_fmt);
 int64_t catcoc_arrive_words(int M, int N, int W, int seg_dim, int bn, int cta_pair);

@@ -893,3 +893,165 @@ extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_
   p.gk_range = range;
   return catcoc_launch_params(p, kind, grid, pair, 0, stream);
 }
+
+// ---- split K: few output tiles, a long K ----
+namespace {
+struct FoldParams {
+  const uint8_t* parts;      // [slices][rows_pad][pitch] fp32 or int32
+  int64_t plane;             // elements per plane
+  int slices, rows, cols, pitch;
+  void* out;
+  int64_t ldc;
+  int out_fmt, vec_ok;       // vec_ok: four output elements can be stored at once
+  const float* scale_m; const float* scale_n; const int32_t* bias;
+  int affine;
+  float alpha, beta;
+  const void* c_src;
+  int64_t ldc_src;
+  const float* bias_f;
+  int act;
+};
+
+CATCOC_DEVICE void store1(void* out, int64_t i, int fmt, float v) {
+  if (fmt == FMT_F32) static_cast<float*>(out)[i] = v;
+  else if (fmt == FMT_BF16) static_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn(v);
+  else static_cast<__half*>(out)[i] = __float2half_rn(v);
+}
+CATCOC_DEVICE float load1(const void* p, int64_t i, int fmt) {
+  if (fmt == FMT_F32) return static_cast<const float*>(p)[i];
+  if (fmt == FMT_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
+  return __half2float(static_cast<const __half*>(p)[i]);
+}
+
+// Sums the planes in slice order and runs the epilogue of the product kernel on the sum, in the same order of operations.
+// Four columns a thread; the planes come from L2 (128 rows x 8192 columns x 4 slices: 17 MB).
+template <bool INT>
+__global__ void __launch_bounds__(256) splitk_fold_kernel(const FoldParams p) {
+  ptx::grid_dependency_wait();
+  const int units_row = (p.cols + 3) / 4;
+  const int64_t units = static_cast<int64_t>(p.rows) * units_row;
+  for (int64_t u = blockIdx.x * 256ll + threadIdx.x; u < units; u += gridDim.x * 256ll) {
+    const int r = static_cast<int>(u / units_row);
+    const int c0 = static_cast<int>(u - static_cast<int64_t>(r) * units_row) * 4;
+    const uint8_t* src = p.parts + (static_cast<int64_t>(r) * p.pitch + c0) * 4;
+    const int64_t step = p.plane * 4;
+    uint32_t a[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 4
+    for (int s = 0; s < p.slices; ++s) {
+      const uint4 v = __ldcg(reinterpret_cast<const uint4*>(src + s * step));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        a[e] = INT ? a[e] + w[e] : __float_as_uint(__uint_as_float(a[e]) + __uint_as_float(w[e]));
+    }
+    const int n = min(4, p.cols - c0);
+    const int64_t o = static_cast<int64_t>(r) * p.ldc + c0;
+    if (INT && p.bias != nullptr) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) if (e < n) a[e] += static_cast<uint32_t>(__ldg(p.bias + c0 + e));
+    }
+    if (INT && p.out_fmt == FMT_S32) {
+      uint32_t* dst = static_cast<uint32_t*>(p.out) + o;
+      if (p.vec_ok && n == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(a[0], a[1], a[2], a[3]);
+      else for (int e = 0; e < n; ++e) dst[e] = a[e];
+      continue;
+    }
+    float f[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = INT ? static_cast<float>(static_cast<int32_t>(a[e])) : __uint_as_float(a[e]);
+    if (p.scale_m != nullptr || p.scale_n != nullptr) {
+      const float sm = p.scale_m != nullptr ? __ldg(p.scale_m + r) : 1.0f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[e] = f[e] * ((p.scale_n != nullptr && e < n) ? __ldg(p.scale_n + c0 + e) : 1.0f) * sm;
+    }
+    if (p.affine) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (e < n) {
+          float x = p.alpha * f[e];
+          if (p.bias_f != nullptr) x += __ldg(p.bias_f + c0 + e);
+          if (p.c_src != nullptr) x += p.beta * load1(p.c_src, static_cast<int64_t>(r) * p.ldc_src + c0 + e, p.out_fmt);
+          f[e] = x;
+        }
+      }
+    }
+    if (p.act != ACT_NONE) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[e] = activate(f[e], p.act);
+    }
+    if (p.vec_ok && n == 4) {
+      if (p.out_fmt == FMT_F32) *reinterpret_cast<float4*>(static_cast<float*>(p.out) + o) = make_float4(f[0], f[1], f[2], f[3]);
+      else *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + o) = make_uint2(pack2(f[0], f[1], p.out_fmt), pack2(f[2], f[3], p.out_fmt));
+    } else {
+      for (int e = 0; e < n; ++e) store1(p.out, o + e, p.out_fmt, f[e]);
+    }
+  }
+}
+
+int splitk_rows(int M) { return round_up(M, 32); }    // whole 32-row windows leave the first launch by TMA
+int splitk_pitch(int N) { return round_up(N, 4); }
+}  // namespace
+
+extern "C" int64_t catcoc_splitk_workspace_bytes(int M, int N, int slices) {
+  if (M <= 0 || N <= 0 || slices <= 0) return 0;
+  return static_cast<int64_t>(slices) * splitk_rows(M) * splitk_pitch(N) * 4;
+}
+
+extern "C" int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_slice, void* workspace, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (args == nullptr || workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0 || slices < 2 || k_slice <= 0) {
+    set_error("splitk: bad arguments");
+    return CATCOC_E_BAD_ARG;
+  }
+  const CatcocOpArgs& a = *args;
+  Resolved rf;
+  int rc = resolve_format(a.in_fmt, &rf);
+  if (rc != 0) return rc;
+  if (a.mode != CATCOC_MODE_LOCAL || rf.kind == KIND_MX || a.num_groups != 0 || a.out == nullptr || a.ldc < a.N ||
+      (k_slice * rf.elt) % 256 != 0 || static_cast<int64_t>(k_slice) * (slices - 1) >= a.K || static_cast<int64_t>(k_slice) * slices < a.K) {
+    set_error("splitk: a local product whose K range is cut into whole stages (K=%d, %d slices of %d)", a.K, slices, k_slice);
+    return CATCOC_E_BAD_ARG;
+  }
+  const bool is_int = rf.kind == KIND_I8;
+  if (is_int ? (a.out_fmt == CATCOC_FMT_F32 && a.scale_m == nullptr && a.scale_n == nullptr) : (a.out_fmt == CATCOC_FMT_S32 || a.bias != nullptr)) {
+    set_error("splitk: output format or bias does not fit the operands");
+    return CATCOC_E_UNSUPPORTED;
+  }
+  const int rows = splitk_rows(a.M), pitch = splitk_pitch(a.N);
+  CatcocOpArgs g = a;
+  g.M = slices * rows; g.K = k_slice;
+  g.num_groups = slices; g.group_ends = nullptr; g.group_rows = rows;
+  g.a_rows_total = a.M; g.a_k_total = a.K; g.b_n_total = a.N; g.b_k_total = a.K;
+  g.g_a_row_back = rows; g.g_a_k = k_slice; g.g_b_row = 0; g.g_b_k = k_slice; g.g_nvec = 0;
+  g.out = workspace; g.ldc = pitch; g.out_fmt = is_int ? CATCOC_FMT_S32 : CATCOC_FMT_F32; g.partial_fmt = g.out_fmt;
+  g.scale_m = nullptr; g.scale_n = nullptr; g.bias = nullptr; g.bias_f = nullptr; g.c_src = nullptr; g.affine = 0; g.act = 0;
+  g.limit[LIM_OUT] = (static_cast<int64_t>(g.M - 1) * pitch + a.N) * 4;
+  rc = catcoc_fused_launch(&g, stream_);
+  if (rc != 0) return rc;
+  FoldParams f;
+  memset(&f, 0, sizeof(f));
+  f.parts = static_cast<const uint8_t*>(workspace);
+  f.plane = static_cast<int64_t>(rows) * pitch;
+  f.slices = slices; f.rows = a.M; f.cols = a.N; f.pitch = pitch;
+  f.out = a.out; f.ldc = a.ldc; f.out_fmt = a.out_fmt;
+  const int vec = 4 * fmt_bytes(a.out_fmt);
+  f.vec_ok = (reinterpret_cast<uintptr_t>(a.out) % vec) == 0 && (a.ldc % 4) == 0;
+  f.scale_m = a.scale_m; f.scale_n = a.scale_n; f.bias = a.bias;
+  f.affine = a.affine; f.alpha = a.alpha; f.beta = a.beta;
+  f.c_src = (a.affine && a.beta != 0.0f) ? a.c_src : nullptr;
+  f.ldc_src = a.ldc_src; f.bias_f = a.affine ? a.bias_f : nullptr; f.act = a.act;
+  const int64_t units = static_cast<int64_t>(a.M) * ((a.N + 3) / 4);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(static_cast<unsigned>(units > 148 * 8 * 256 ? 148 * 8 : (units + 255) / 256), 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CATCOC_CUDA_OK(is_int ? cudaLaunchKernelEx(&cfg, splitk_fold_kernel<true>, static_cast<const FoldParams&>(f))
+                        : cudaLaunchKernelEx(&cfg, splitk_fold_kernel<false>, static_cast<const FoldParams&>(f)));
+  return CATCOC_OK;
+}

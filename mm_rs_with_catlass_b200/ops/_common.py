@@ -210,6 +210,18 @@ def launch_slice_k(args: N.OpArgs, ranges, ws: torch.Tensor, device: torch.devic
     _launches += 1
 
 
+def launch_splitk(args: N.OpArgs, slices: int, k_slice: int, device: torch.device) -> None:
+    """Queues a product whose K range is cut into slices, and the kernel that sums them."""
+    args.timeout_ns = default_timeout_ns()
+    args.events, args.events_cap = _event_ring
+    lib = N.lib()
+    # scratch of the caching allocator: calls on several streams never share one
+    ws = torch.empty(int(lib.catcoc_splitk_workspace_bytes(args.M, args.N, slices)), dtype=torch.uint8, device=device)
+    N.check(lib.catcoc_splitk_launch(C.byref(args), slices, k_slice, ws.data_ptr(), C.c_void_p(stream_of(device))))
+    global _launches
+    _launches += 1
+
+
 _launches = 0
 _event_ring = (None, 0)
 

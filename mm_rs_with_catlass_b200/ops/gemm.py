@@ -70,8 +70,8 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
                cm.tkey(c), cm.tkey(bias_f32), activation)
         plan = _plans.get(key)
         if plan is not None and cm.on_device(a.device):
-            args, out_shape, plan_dtype, pad = plan
-            if out is None or pad is not None:
+            args, out_shape, plan_dtype, pad, split = plan
+            if out is None or pad is not None or split is not None:
                 args = N.OpArgs.from_buffer_copy(args)   # private copy: the plan itself stays immutable
             if pad is not None:
                 # a fresh buffer of the caching allocator per call: calls on several streams never share one
@@ -81,7 +81,10 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
             if out is None:
                 out = torch.empty(out_shape, dtype=plan_dtype, device=a.device)
                 args.out = out.data_ptr()
-            cm.launch(args, a.device)
+            if split is not None:
+                cm.launch_splitk(args, split[0], split[1], a.device)
+            else:
+                cm.launch(args, a.device)
             return out
     dev = cm.require_cuda(a, b, out, scale_m, scale_n, bias, c, bias_f32)
     if a.dtype != b.dtype:
@@ -115,9 +118,14 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
     if c is not None and beta != 0.0:
         if c.shape != (m, n) or c.dtype != out_dtype or c.stride(-1) != 1:
             raise ValueError("c must be a row-major [%d, %d] %s tensor" % (m, n, out_dtype))
+    split = None
     if tiling is None:
-        from ..tiling.chooser import choose
-        tiling = choose("matmul", m, n, k, 1, a.dtype)
+        from ..tiling import chooser
+        tiling = chooser.choose("matmul", m, n, k, 1, a.dtype)
+        if _group is None and trace is None:
+            split = chooser.split_k(m, n, k, a.element_size(), tiling)
+            if split is not None:
+                tiling = TilingConfig(bn=split[2], cta_pair=1)
     with torch.cuda.device(dev):
         # An operand whose base or row pitch TMA cannot take goes through the pad kernel first.
         oa = cm.as_operand(a, trans_a)
@@ -163,9 +171,12 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
         if _args_out is not None:
             # a caller that keeps its own plan of a group launch (ops/fused.py); None: the block points at a temporary copy
             _args_out.append(None if (oa.copied or ob.copied) else args)
-        cm.launch(args, dev)
+        if split is not None:
+            cm.launch_splitk(args, split[0], split[1], dev)
+        else:
+            cm.launch(args, dev)
         if key is not None and (not oa.copied or _wants_pad_prologue(a)) and not ob.copied:
             if len(_plans) >= _MAX_PLANS:
                 _plans.clear()
-            _plans[key] = (args, tuple(out.shape), out.dtype, oa.pad if oa.copied else None)
+            _plans[key] = (args, tuple(out.shape), out.dtype, oa.pad if oa.copied else None, split)
     return out

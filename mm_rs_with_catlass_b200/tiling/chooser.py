@@ -12,6 +12,7 @@ constant, examples/dynamic_tiling/dynamic_tiling.cpp:219-227).
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional
@@ -29,6 +30,16 @@ _NUM_SMS = 148
 # bound by the fill rate of shared memory, so halving the width costs far more than half.
 _TILE_EFF = {256: 1.0, 128: 0.56, 64: 0.43}
 _PAIR_GAIN = {256: 1.10, 128: 1.35}     # 2-CTA tiles: each CTA fills half of B
+
+
+# Cost model of split_k, in SM cycles, fitted to 84 shapes (bf16 and int8; 4 to 1024 rows, N of 992 to 28672, K of 3584 to
+# 28672): its choices lose 2 % on average against the best of all cuts that were measured, the direct kernel alone 28 %.
+_INTAKE = {1: 46.0, 2: 42.0}      # bytes per cycle that one CTA takes in while most of the others do the same (pair: per CTA)
+_HBM = 3600.0                     # bytes per cycle from HBM, all SMs
+_PLANES = 3500.0                  # bytes per cycle of the planes, written and read through L2
+_LAUNCH = 10000.0                 # start, fill and drain of a kernel
+_FOLD = 8000.0                    # the second kernel and the gap before it
+_INT8_EPILOGUE = 10000.0          # the dequantising epilogue of the direct kernel, which the second kernel spreads over all SMs
 
 
 def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bool = False) -> float:
@@ -90,6 +101,39 @@ def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype) -
     # 16 bytes reaches one peer either way)
     return TilingConfig(bn=bn, swizzle=swizzle, cta_pair=pair, rounds=rounds,
                         use_multicast=(op == "allgather_matmul" and world >= 4))
+
+
+@functools.lru_cache(maxsize=4096)
+def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
+    """``(slices, k_slice, bn)`` when a local product is faster with its K range cut into slices whose
+    planes a second kernel sums, else None.
+
+    With few output tiles the direct kernel runs a fraction of the SMs, or a last wave that is nearly
+    empty, and one CTA's intake bounds it: a 128-byte K block of a tile costs its MMAs (2 cycles per
+    column) or its bytes (all 128 rows of A are filled, whatever M is). Wide tiles cut into slices take
+    in fewer bytes per column; the price is the planes and a second kernel. bf16, M = 128, 8192 x 28672:
+    134 -> 94 us; M = 100, 3584 x 8192: 44 -> 29 us; int8, M = 128, 8192 x 28672: 106 -> 63 us."""
+    kb = -(-k * elt // 128)
+
+    def unit(bn, pair):
+        return max(2.0 * bn, (128 + bn // pair) * 128 / _INTAKE[pair])
+
+    hbm = (n * k + m * k) * elt / _HBM
+    pair, bn0 = (2 if direct.cta_pair == 2 else 1), direct.effective_bn
+    waves = -(-(-(-m // (128 * pair)) * -(-n // bn0)) // (_NUM_SMS // pair))
+    best, best_time = None, 0.95 * (max(hbm, waves * kb * unit(bn0, pair)) + _LAUNCH + (_INT8_EPILOGUE if elt == 1 else 0.0))
+    for bn in (256, 128):
+        if n < bn and bn > 128:
+            continue
+        tiles = -(-m // 128) * -(-n // bn)
+        for s in range(2, 33):
+            kbs = -(-(-(-kb // s)) // 2) * 2                  # K blocks per slice: whole 256-byte stages
+            if kbs < 8 or -(-kb // kbs) != s:
+                continue
+            t = max(hbm, -(-tiles * s // _NUM_SMS) * kbs * unit(bn, 1)) + s * m * n * 8 / _PLANES + _LAUNCH + _FOLD
+            if t < best_time:
+                best, best_time = (s, kbs * 128 // elt, bn), t
+    return best
 
 
 def choose(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype,
