@@ -371,17 +371,6 @@ CATCOC_DEVICE float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// ... and the forms that return a NaN when an operand is one
-CATCOC_DEVICE float max_nan(float a, float b) {
-  float d;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
-  return d;
-}
-CATCOC_DEVICE float max3_nan(float a, float b, float c) {
-  float d;
-  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
 // Register split between warpgroups (every warp of a warpgroup executes it); the shares must add up to no more than the
 // block was launched with
 template <int N> CATCOC_DEVICE void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -415,6 +404,22 @@ CATCOC_DEVICE uint64_t make_smem_desc_noswizzle(uint32_t smem_addr, uint32_t lbo
 // reaches the columns the block-scaled MMA reads.
 CATCOC_DEVICE void tmem_cp_32x128b_warpx4(uint32_t taddr, uint64_t sdesc) {
   asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
+// The same in both CTAs of a pair, each from its own shared memory at the leader's offset
+CATCOC_DEVICE void tmem_cp_32x128b_warpx4_pair(uint32_t taddr, uint64_t sdesc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
+// Pair form: 256 rows, the scales of A by CTA (its 128 rows), those of all N columns of B in both
+CATCOC_DEVICE void umma_mxf8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                  uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)
+      : "memory");
 }
 // D[tmem] (+)= (A * 2^(sfa-127)) (B * 2^(sfb-127)) with one UE8M0 scale per 32 K-elements.
 CATCOC_DEVICE void umma_mxf8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,

@@ -75,6 +75,20 @@ static int encode_2d(CUtensorMap* tm, const void* base, int elt_bytes, CUtensorM
   return CATCOC_OK;
 }
 
+// Packed scale factors: rows of 128 bytes, a box of four (one block of 128 rows x 4 K-blocks), not swizzled.
+static int encode_scales(CUtensorMap* tm, const void* base, int64_t rows) {
+  static EncodeTiledFn fn = driver_fn<EncodeTiledFn>("cuTensorMapEncodeTiled");
+  if (fn == nullptr) return CATCOC_E_DRIVER;
+  cuuint64_t gdim[2] = {128, static_cast<cuuint64_t>(rows)};
+  cuuint64_t gstride[1] = {128};
+  cuuint32_t box[2] = {128, 4};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (scales) failed: CUresult %d", static_cast<int>(r)); return CATCOC_E_DRIVER; }
+  return CATCOC_OK;
+}
+
 // CATCOC_OUT_TMA=0 keeps every output on plain vector stores (for A/B measurements).
 static bool out_tma_enabled() {
   static const bool on = [] {
@@ -318,9 +332,13 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   int rc = resolve_format(a.in_fmt, &rf);
   if (rc != 0) return rc;
   const bool mx = (rf.kind == KIND_MX);
-  const int bn = mx ? 128 : norm_bn(a.tiling.bn);   // block-scaled tiles are 128 wide (TMEM room for scales)
+  // Block-scaled tiles leave TMEM room for the scales: 128 x 128 on one CTA, or, for a local product of more than one row
+  // of tiles, 256 x 192 on a pair (two accumulators of 192 columns). A CTA's intake bounds the 128 x 128 tile (33 KiB per
+  // 256 cycles of MMAs; the pair: 29.5 KiB per 384): 4096 x 8192 x 7168 e4m3 with its quantisation 361 -> 258 us.
+  const bool mx_pair = mx && !fused && a.M > kBM && a.scale_m == nullptr && a.scale_n == nullptr && !a.affine && a.act == 0;
+  const int bn = mx ? (mx_pair ? 192 : 128) : norm_bn(a.tiling.bn);
   const int seg_dim = pick_seg_dim(a);
-  const bool pair = !mx && (a.tiling.cta_pair == 2);
+  const bool pair = mx ? mx_pair : (a.tiling.cta_pair == 2);
   if (mx) {
     if (a.trans_a || !a.trans_b) { set_error("block-scaled fp8 needs A stored [M, K] and B stored [N, K]"); return CATCOC_E_UNSUPPORTED; }
     if (a.sfa == nullptr || a.sfb == nullptr || a.sf_k_blocks < (a.K + 127) / 128) { set_error("block-scaled fp8 needs packed scale factors covering K"); return CATCOC_E_BAD_ARG; }
@@ -348,6 +366,14 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   p->sfa = static_cast<const uint8_t*>(a.sfa);
   p->sfb = static_cast<const uint8_t*>(a.sfb);
   p->sf_k_blocks = a.sf_k_blocks;
+  if (mx_pair) {
+    // 512-byte scale blocks as four 128-byte rows: the pair's copies are credited to the leader's barrier, which only
+    // tensor copies can do
+    const int rt_a = (a.M + 127) / 128, rt_b = (a.N + 127) / 128;
+    rc = encode_scales(&p->tm_a_gath[0], a.sfa, static_cast<int64_t>(rt_a) * a.sf_k_blocks * 4);
+    if (rc == 0) rc = encode_scales(&p->tm_a_gath[1], a.sfb, static_cast<int64_t>(rt_b) * a.sf_k_blocks * 4);
+    if (rc != 0) return rc;
+  }
   p->elt_bytes_a = rf.elt;
 
   if (fused && (a.mode == CATCOC_MODE_RS) && (a.M % a.W != 0)) {
@@ -698,7 +724,7 @@ static const inst::Unit* unit_for(int kind, bool pair) {
     case KIND_F16: return pair ? &inst::unit_f16_pair() : &inst::unit_f16_single();
     case KIND_I8: return pair ? &inst::unit_i8_pair() : &inst::unit_i8_single();
     case KIND_F8: return pair ? &inst::unit_f8_pair() : &inst::unit_f8_single();
-    case KIND_MX: return pair ? nullptr : &inst::unit_mx_single();
+    case KIND_MX: return pair ? &inst::unit_mx_pair() : &inst::unit_mx_single();
     default: return nullptr;
   }
 }
@@ -721,8 +747,8 @@ static cudaError_t prepare_kernels() {
 // How many 2-CTA clusters of the pair kernel can be resident at once (the persistent grid must
 // not exceed it: CTAs of different ranks wait on each other).
 int max_active_pairs(int kind) {
-  static int cached[3] = {-1, -1, -1};
-  if (kind < 0 || kind > 2) return 1;
+  static int cached[4] = {-1, -1, -1, -1};
+  if (kind < 0 || kind > KIND_MX) return 1;
   if (cached[kind] < 0) {
     if (prepare_kernels() != cudaSuccess) return 1;
     int n = unit_for(kind, true)->max_clusters();
