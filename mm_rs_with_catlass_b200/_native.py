@@ -111,8 +111,7 @@ def _declare(lib) -> None:
         "catcoc_is_checked_build": (i32, []),
         "catcoc_num_sms": (i32, [i32]),
         "catcoc_fused_launch": (i32, [P(OpArgs), vp]),
-        "catcoc_slice_k_workspace_bytes": (i64, [i32]),
-        "catcoc_slice_k_launch": (i32, [P(OpArgs), vp, vp, vp]),
+        "catcoc_slice_k_launch": (i32, [P(OpArgs), vp, vp]),
         "catcoc_splitk_workspace_bytes": (i64, [i32, i32, i32]),
         "catcoc_splitk_launch": (i32, [P(OpArgs), i32, i32, vp, vp]),
         "catcoc_stage_bytes": (i64, [i32, i32, i32, i32, i32, i32, i32]),

@@ -137,9 +137,8 @@ int catcoc_fused_launch(const CatcocOpArgs* args, void* stream);
 /* Products over ragged ranges of K in one launch (weight gradients of grouped products): group g of args->num_groups
  * multiplies the K rows [k_range[2 g], k_range[2 g + 1]) (host memory; an empty range leaves its output untouched) of
  * an A stored [K, M_g] and a B stored [K, N]; M_g = args->group_rows, args->K counts all K rows, the outputs are
- * stacked along rows. `workspace`: catcoc_slice_k_workspace_bytes(groups) bytes of device memory, 128-byte aligned. */
-int64_t catcoc_slice_k_workspace_bytes(int groups);
-int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void* workspace, void* stream);
+ * stacked along rows. fp16 / bf16. */
+int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void* stream);
 
 /* A local product with few output tiles, its K range cut into `slices` slices of `k_slice` elements (a multiple of 256
  * bytes): the slices run as the groups of one launch, each writing an fp32 (int8 operands: int32) plane to `workspace`

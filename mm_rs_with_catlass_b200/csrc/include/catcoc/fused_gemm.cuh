@@ -35,6 +35,7 @@
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <type_traits>
 #include "catcoc/params.h"
 #include "catcoc/ptx.cuh"
 
@@ -318,9 +319,10 @@ CATCOC_DEVICE TileInfo walk_tile(const FusedParams& p, int t, GroupWalk& w) {
 // ---------------------------------------------------------------------------------------
 // The kernel
 // ---------------------------------------------------------------------------------------
-template <int KIND, bool CTA2, int EPI>
+template <int KIND, bool CTA2, int EPI, class Params = FusedParams>
 __global__ void __launch_bounds__(threads_for(EPI), 1)
-fused_gemm_kernel(const __grid_constant__ FusedParams p) {
+fused_gemm_kernel(const __grid_constant__ Params p) {
+  constexpr bool kGk = std::is_same<Params, FusedParamsGk>::value;   // every group has a K range of its own
   // Epilogue variant (see EpiVariant in params.h): stages a launch cannot need are compiled out.
   constexpr bool kReduce = (EPI == EPI_REDUCE || EPI == EPI_FULL);   // push flavour of RS / AR: peers' partials, pushes, stamps
   constexpr bool kScale = (EPI == EPI_FULL);      // int32 bias, dequantisation, alpha / beta / C / fp32 bias
@@ -431,14 +433,14 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
         a_row -= ti.seg * p.g_a_row_back;
         a_k_off = ti.seg * p.g_a_k;
       }
-      int tile_kb = num_kb;
-      if (p.gk_range != nullptr) {
-        const int2 r = __ldg(p.gk_range + ti.seg);
+      int tile_k = p.K;
+      if constexpr (kGk) {
+        const int2 r = p.gk_range[ti.seg];
         a_k_off = r.x;
-        tile_kb = ceil_div(r.y - r.x, p.bk * kps);   // an empty range has no tile: every role skips it
-        tma = p.gk_maps + 2 * ti.seg;
-        if (tile_kb > 0) ptx::tmap_acquire(tma);
+        tile_k = r.y - r.x;                          // an empty range has no K block: every role skips the tile
+        tma = &p.gk_map[2 * ti.seg];
       }
+      const int tile_sub = ceil_div(tile_k, p.bk), tile_kb = ceil_div(tile_sub, kps);
       if (p.mode == MODE_AG && fused) {
         if (ti.seg == p.rank && p.ag_raw == 0) {
           a_row = ti.mi * sched.BM + sub * kBM;  // row inside the local shard
@@ -508,7 +510,8 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
           const uint32_t bar = CTA2 ? ptx::map_to_cta(ptx::smem_u32(&tail->full[stage]), 0u) : 0u;
           // Single flavour: this warp arms its own barrier with its bytes. Pair flavour: both
           // CTAs' copies are credited to the leader's barrier and only the leader arms it, with
-          // the bytes of the whole pair. K-blocks past the end of K are fetched as zeros.
+          // the bytes of the whole pair. K-blocks past the end of K are not fetched: no MMA reads them.
+          const int nsub = min(kps, tile_sub - kb * kps);
           if (KIND == KIND_MX && !CTA2) {
             // A block + the 512-byte scale-factor block of (this 128-row tile, this K-block)
             ptx::mbar_expect_tx(&tail->full[stage], kABytes + 512);
@@ -516,11 +519,11 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
             ptx::bulk_load_1d(smem + stage * kStageBytes + kSfSmemOff,
                               p.sfa + (static_cast<int64_t>(row_tile) * p.sf_k_blocks + kb) * 512, 512,
                               &tail->full[stage]);
-          } else if (!CTA2) ptx::mbar_expect_tx(&tail->full[stage], kps * kABytes);
-          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * kps * (kABytes + (KIND == KIND_MX ? 512 : 0)));
+          } else if (!CTA2) ptx::mbar_expect_tx(&tail->full[stage], nsub * kABytes);
+          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * nsub * (kABytes + (KIND == KIND_MX ? 512 : 0)));
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            if (j >= kps) break;
+            if (j >= nsub) break;
             uint8_t* sa = smem + stage * kStageBytes + j * sub_bytes;
             const int k0 = (kb * kps + j) * p.bk + a_k_off;
             // (a block past the last row or K-block only fills the stage: its MMAs are skipped or its rows not stored)
@@ -592,8 +595,8 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
       GroupWalk walk = group_walk_begin(p);
       for (int t = worker; ok && t < total_tiles; t += num_workers) {
         int tile_k = K, tile_kb = num_kb;
-        if (p.gk_range != nullptr) {
-          const int2 r = __ldg(p.gk_range + walk_tile(p, t, walk).seg);
+        if constexpr (kGk) {
+          const int2 r = p.gk_range[walk_tile(p, t, walk).seg];
           tile_k = r.y - r.x;
           tile_kb = ceil_div(tile_k, p.bk * kps);
           if (tile_kb <= 0) continue;
@@ -778,9 +781,8 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
     GroupWalk walk = group_walk_begin(p);
     for (int t = worker; ok && t < total_tiles; t += num_workers) {
       const TileInfo ti = walk_tile(p, t, walk);
-      if (p.gk_range != nullptr) {
-        const int2 r = __ldg(p.gk_range + ti.seg);
-        if (r.y <= r.x) continue;
+      if constexpr (kGk) {
+        if (p.gk_range[ti.seg].y <= p.gk_range[ti.seg].x) continue;
       }
       const bool own = !kReduce || !fused || (p.mode == MODE_AG) || (ti.seg == p.rank);
       const bool reduce_here = kReduce && fused && own && (p.mode == MODE_RS || p.mode == MODE_AR);
@@ -1283,14 +1285,14 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
         b_k_off = ti.seg * p.g_b_k;
       }
       const CUtensorMap* tmb = &p.tm_b;
-      int tile_kb = num_kb;
-      if (p.gk_range != nullptr) {
-        const int2 r = __ldg(p.gk_range + ti.seg);
+      int tile_k = p.K;
+      if constexpr (kGk) {
+        const int2 r = p.gk_range[ti.seg];
         b_k_off = r.x;
-        tile_kb = ceil_div(r.y - r.x, p.bk * kps);
-        tmb = p.gk_maps + 2 * ti.seg + 1;
-        if (tile_kb > 0) ptx::tmap_acquire(tmb);
+        tile_k = r.y - r.x;
+        tmb = &p.gk_map[2 * ti.seg + 1];
       }
+      const int tile_sub = ceil_div(tile_k, p.bk), tile_kb = ceil_div(tile_sub, kps);
       for (int kb = 0; kb < tile_kb; ++kb) {
         if (!ptx::mbar_wait(&tail->empty[stage], phase ^ 1u, p.timeout_ns, abort_flag)) {
           if (lane == 0) {
@@ -1302,6 +1304,7 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
         }
         if (ptx::elect_one()) {
           const int per_box = 128 / p.elt_bytes_a;
+          const int nsub = min(kps, tile_sub - kb * kps);
           const uint32_t bar = CTA2 ? ptx::map_to_cta(ptx::smem_u32(&tail->full[stage]), 0u) : 0u;
           if (KIND == KIND_MX && !CTA2) {
             const int nblk = BN / 128;
@@ -1310,11 +1313,11 @@ fused_gemm_kernel(const __grid_constant__ FusedParams p) {
               ptx::bulk_load_1d(smem + stage * kStageBytes + kSfSmemOff + 512 * (1 + j),
                                 p.sfb + (static_cast<int64_t>(b_col / 128 + j) * p.sf_k_blocks + kb) * 512, 512,
                                 &tail->full[stage]);
-          } else if (!CTA2) ptx::mbar_expect_tx(&tail->full[stage], kps * b_stage_bytes);
-          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * kps * (b_stage_bytes + (KIND == KIND_MX ? 1024 : 0)));
+          } else if (!CTA2) ptx::mbar_expect_tx(&tail->full[stage], nsub * b_stage_bytes);
+          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * nsub * (b_stage_bytes + (KIND == KIND_MX ? 1024 : 0)));
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            if (j >= kps) break;
+            if (j >= nsub) break;
             uint8_t* sb = smem + stage * kStageBytes + j * sub_bytes + kABytes;
             const int k0 = (kb * kps + j) * p.bk + b_k_off;
             if (KIND == KIND_MX && CTA2) {

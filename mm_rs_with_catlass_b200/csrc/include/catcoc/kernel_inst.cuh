@@ -22,14 +22,14 @@ struct Unit {
   int (*max_clusters)();                                                           // pair flavour: resident 2-CTA clusters
 };
 
-template <int KIND, bool CTA2, int EPI>
+template <int KIND, bool CTA2, int EPI, class Params = FusedParams>
 cudaError_t set_smem_attr() {
-  return cudaFuncSetAttribute(fused_gemm_kernel<KIND, CTA2, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(fused_gemm_kernel<KIND, CTA2, EPI, Params>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               Geo<CTA2>::kSmemBytes);
 }
 
-template <int KIND, bool CTA2, int EPI>
-cudaError_t launch_one(const FusedParams& p, int grid, int threads, cudaStream_t stream) {
+template <int KIND, bool CTA2, int EPI, class Params>
+cudaError_t launch_one(const Params& p, int grid, int threads, cudaStream_t stream) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(grid, 1, 1);
@@ -45,7 +45,7 @@ cudaError_t launch_one(const FusedParams& p, int grid, int threads, cudaStream_t
     cfg.attrs = attr;
     cfg.numAttrs = 1;
   }
-  return cudaLaunchKernelEx(&cfg, fused_gemm_kernel<KIND, CTA2, EPI>, p);
+  return cudaLaunchKernelEx(&cfg, fused_gemm_kernel<KIND, CTA2, EPI, Params>, p);
 }
 
 template <int KIND, int EPI>
@@ -77,6 +77,10 @@ const Unit& unit_f8_single();
 const Unit& unit_f8_pair();
 const Unit& unit_mx_single();
 const Unit& unit_mx_pair();
+
+// 16-bit products over ragged K ranges (kernels/inst/f16_slice_k.cu)
+cudaError_t prepare_slice_k();
+cudaError_t launch_slice_k(bool pair, const FusedParamsGk& p, int grid, cudaStream_t s);
 
 }  // namespace inst
 }  // namespace catcoc

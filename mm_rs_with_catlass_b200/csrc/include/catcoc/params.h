@@ -177,11 +177,6 @@ struct alignas(64) FusedParams {
   int g_b_row;                // N coordinate of B (stored [N, K]) starts at  g * g_b_row
   int g_b_k;                  // K coordinate of B starts at  g * g_b_k
   int g_nvec;                 // scale_n / bias / bias_f of group g start at  g * g_nvec
-  // Ragged K ranges (null: off): group g multiplies the K rows [gk_range[g].x, gk_range[g].y) of an A stored [K, M] and
-  // a B stored [K, N]. Its two tensor maps (A, B) end at the range's last row, so that the tail of the last K block
-  // reads as zeros and not as the next group's rows. Device memory, written ahead of the launch.
-  const CUtensorMap* gk_maps;
-  const int2* gk_range;
 
   // block-scaled fp8: scale factors packed in 512-byte blocks of 128 rows x 4 K-blocks
   // (row r, K-block s at (r % 32) * 16 + (r / 32) * 4 + s); block (row_tile, k128) at
@@ -211,6 +206,16 @@ struct alignas(64) FusedParams {
   // the host turns the ring into a Chrome trace (utils/trace.py).
   uint32_t* events;
   uint32_t events_cap;       // records the ring can hold
+};
+
+// Ragged K ranges (a kernel instantiation of its own): group g multiplies the K rows [range[g].x, range[g].y) of an A stored
+// [K, M] and a B stored [K, N]. Its two tensor maps (A, B) end at the range's last row, so that the tail of the last K block
+// reads as zeros and not as the next group's rows. They travel as kernel arguments: maps in global memory have to be
+// acquired by a proxy fence at every tile, which kept the producers busy 80 % of the time while the tensor core waited.
+constexpr int kMaxKGroups = 64;
+struct alignas(64) FusedParamsGk : FusedParams {
+  CUtensorMap gk_map[2 * kMaxKGroups];
+  int2 gk_range[kMaxKGroups];
 };
 
 enum EventRole : uint32_t { EV_PRODUCER = 0, EV_MMA = 1, EV_EPILOGUE = 2, EV_COMM = 3, EV_REDUCER = 4 };

@@ -126,11 +126,6 @@ CATCOC_DEVICE void prefetch_tmap(const void* tmap) {
 }
 
 // Innermost coordinate x (elements) times the element size must be a multiple of 16 bytes.
-// A tensor map in global memory that an earlier kernel wrote: its writer releases it, its reader acquires it
-CATCOC_DEVICE void tmap_release() { asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory"); }
-CATCOC_DEVICE void tmap_acquire(const void* tmap) {
-  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmap) : "memory");
-}
 CATCOC_DEVICE void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"

@@ -845,66 +845,43 @@ extern "C" int catcoc_fused_launch(const CatcocOpArgs* args, void* stream) {
   return catcoc_launch_params(p, kind, grid, pair, threads, static_cast<cudaStream_t>(stream));
 }
 
-// ---- ragged K ranges in one launch ----
-namespace {
-// The maps travel as a kernel argument (no host buffer has to outlive the call, and the launch can be captured).
-constexpr int kMapBatch = 48;
-struct alignas(64) MapBatch {
-  CUtensorMap map[2 * kMapBatch];
-  int2 range[kMapBatch];
-  int first, count;
-};
-
-__global__ void __launch_bounds__(128) store_maps_kernel(const __grid_constant__ MapBatch m, CUtensorMap* maps, int2* range) {
-  const uint4* src = reinterpret_cast<const uint4*>(m.map);
-  uint4* dst = reinterpret_cast<uint4*>(maps + 2 * m.first);
-  for (int i = threadIdx.x; i < m.count * 2 * static_cast<int>(sizeof(CUtensorMap) / 16); i += blockDim.x) dst[i] = src[i];
-  for (int i = threadIdx.x; i < m.count; i += blockDim.x) range[m.first + i] = m.range[i];
-  ptx::tmap_release();
-}
-}  // namespace
-
-extern "C" int64_t catcoc_slice_k_workspace_bytes(int groups) {
-  return groups > 0 ? static_cast<int64_t>(groups) * (2 * sizeof(CUtensorMap) + sizeof(int2)) : 0;
-}
-
-extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void* workspace, void* stream_) {
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  if (args == nullptr || k_range == nullptr || workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 127) != 0) {
-    set_error("slice_k: null argument, or a workspace that is not 128-byte aligned");
-    return CATCOC_E_BAD_ARG;
-  }
-  const CatcocOpArgs& a = *args;
-  if (a.num_groups <= 0 || a.group_ends != nullptr || !a.trans_a || a.trans_b || a.g_a_k != 0 || a.g_b_k != 0 || a.g_b_row != 0) {
-    set_error("slice_k takes uniform groups of an A stored [K, M] and a B stored [K, N]");
+// ---- ragged K ranges in one launch (of up to kMaxKGroups groups) ----
+extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void* stream_) {
+  if (args == nullptr || k_range == nullptr) { set_error("slice_k: null argument"); return CATCOC_E_BAD_ARG; }
+  Resolved rf;
+  int rc = resolve_format(args->in_fmt, &rf);
+  if (rc != 0) return rc;
+  if (rf.kind != KIND_F16 || args->num_groups <= 0 || args->group_ends != nullptr || !args->trans_a || args->trans_b ||
+      args->g_a_k != 0 || args->g_b_k != 0 || args->g_b_row != 0 || args->affine || args->act) {
+    set_error("slice_k takes uniform groups of a 16-bit A stored [K, M] and B stored [K, N], with the plain epilogue");
     return CATCOC_E_UNSUPPORTED;
   }
-  for (int g = 0; g < a.num_groups; ++g) {
-    if (k_range[2 * g] < 0 || k_range[2 * g + 1] < k_range[2 * g] || k_range[2 * g + 1] > a.K) {
-      set_error("slice_k: K range [%d, %d) of group %d lies outside [0, %d)", k_range[2 * g], k_range[2 * g + 1], g, a.K);
+  for (int g = 0; g < args->num_groups; ++g) {
+    if (k_range[2 * g] < 0 || k_range[2 * g + 1] < k_range[2 * g] || k_range[2 * g + 1] > args->K) {
+      set_error("slice_k: K range [%d, %d) of group %d lies outside [0, %d)", k_range[2 * g], k_range[2 * g + 1], g, args->K);
       return CATCOC_E_BAD_ARG;
     }
   }
-  FusedParams p;
-  int kind = 0, grid = 0, pair = 0;
-  int rc = catcoc_build_params(args, &p, &kind, &grid, &pair);
-  if (rc != 0) return rc;
-  Resolved rf;
-  rc = resolve_format(a.in_fmt, &rf);
-  if (rc != 0) return rc;
-  CUtensorMap* maps = static_cast<CUtensorMap*>(workspace);
-  int2* range = reinterpret_cast<int2*>(maps + 2 * a.num_groups);
+  static const cudaError_t ready = inst::prepare_slice_k();
+  CATCOC_CUDA_OK(ready);
   const int per128 = 128 / rf.elt;
-  const int b_cols = pair ? p.sched.BN / 2 : p.sched.BN;
-  MapBatch batch;
-  for (int g0 = 0; g0 < a.num_groups; g0 += kMapBatch) {
-    batch.first = g0;
-    batch.count = imin(kMapBatch, a.num_groups - g0);
-    for (int i = 0; i < batch.count; ++i) {
+  const int64_t group_bytes = static_cast<int64_t>(args->group_rows) * args->ldc * fmt_bytes(args->out_fmt);
+  FusedParamsGk p;
+  for (int g0 = 0; g0 < args->num_groups; g0 += kMaxKGroups) {
+    CatcocOpArgs a = *args;
+    a.num_groups = imin(kMaxKGroups, args->num_groups - g0);
+    a.M = a.num_groups * a.group_rows;
+    a.out = static_cast<uint8_t*>(args->out) + g0 * group_bytes;
+    if (a.limit[LIM_OUT] > 0) a.limit[LIM_OUT] -= g0 * group_bytes;
+    int kind = 0, grid = 0, pair = 0;
+    rc = catcoc_build_params(&a, &p, &kind, &grid, &pair);
+    if (rc != 0) return rc;
+    const int b_cols = pair ? p.sched.BN / 2 : p.sched.BN;
+    for (int i = 0; i < a.num_groups; ++i) {
       const int begin = k_range[2 * (g0 + i)], end = k_range[2 * (g0 + i) + 1];
-      batch.range[i] = make_int2(begin, end);
-      if (end <= begin) continue;                         // never read
-      CUtensorMap* ma = &batch.map[2 * i];
+      p.gk_range[i] = make_int2(begin, end);
+      if (end <= begin) continue;                         // its maps are never read
+      CUtensorMap* ma = &p.gk_map[2 * i];
       rc = p.a_3d ? encode_3d_blocks(ma, a.a, rf.elt, rf.dt, end, a.a_rows_total, a.lda, rf.bk, kBM / per128)
                   : encode_2d(ma, a.a, rf.elt, rf.dt, end, a.a_rows_total, a.lda, per128, rf.bk);
       if (rc == 0)
@@ -912,12 +889,9 @@ extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_
                     : encode_2d(ma + 1, a.b, rf.elt, rf.dt, end, a.b_n_total, a.ldb, per128, rf.bk);
       if (rc != 0) return rc;
     }
-    store_maps_kernel<<<1, 128, 0, stream>>>(batch, maps, range);
-    CATCOC_CUDA_OK(cudaGetLastError());
+    CATCOC_CUDA_OK(inst::launch_slice_k(pair != 0, p, grid, static_cast<cudaStream_t>(stream_)));
   }
-  p.gk_maps = maps;
-  p.gk_range = range;
-  return catcoc_launch_params(p, kind, grid, pair, 0, stream);
+  return CATCOC_OK;
 }
 
 // ---- split K: few output tiles, a long K ----

@@ -201,10 +201,10 @@ def launch(args: N.OpArgs, device: torch.device, timeout_ns: Optional[int] = Non
     _launches += 1
 
 
-def launch_slice_k(args: N.OpArgs, ranges, ws: torch.Tensor, device: torch.device) -> None:
+def launch_slice_k(args: N.OpArgs, ranges, device: torch.device) -> None:
     """Queues one launch over ragged K ranges (begin, end of every group, flat)."""
     args.events, args.events_cap = _event_ring
-    N.check(N.lib().catcoc_slice_k_launch(C.byref(args), (C.c_int32 * len(ranges))(*ranges), ws.data_ptr(),
+    N.check(N.lib().catcoc_slice_k_launch(C.byref(args), (C.c_int32 * len(ranges))(*ranges),
                                           C.c_void_p(stream_of(device))))
     global _launches
     _launches += 1
