@@ -292,6 +292,8 @@ def matmul_reduce_scatter(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = F
     partials instead (twice the bytes, no intermediate rounding at all).
     """
     ctx = _ctx(ctx)
+    if ctx.world == 1:      # the local product keeps plans of its own and makes the same checks
+        return _local_matmul(a, b, trans_a=trans_a, trans_b=trans_b, out=out, tiling=tiling)
     key = ("rs", cm.tkey(a), cm.tkey(b), trans_a, trans_b, cm.tkey(out), tiling)
     if tiling is None:
         small = _plan_hit(ctx, ("rs_small",) + key[1:])
@@ -310,8 +312,6 @@ def matmul_reduce_scatter(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = F
     dev = cm.require_cuda(a, b, out)
     _check_pair(a, b)
     m, n, k = cm.logical_shape(a, trans_a, b, trans_b)
-    if ctx.world == 1:
-        return _local_matmul(a, b, trans_a=trans_a, trans_b=trans_b, out=out, tiling=tiling)
     if m % ctx.world != 0:
         raise ValueError("matmul_reduce_scatter needs M %% world == 0 (M=%d, world=%d)" % (m, ctx.world))
     if a.dtype not in (torch.float16, torch.bfloat16):
@@ -462,6 +462,8 @@ def matmul_allreduce(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False,
     until the second-next fused call on the same context. Pass ``out`` to get a private copy.
     """
     ctx = _ctx(ctx)
+    if ctx.world == 1:      # the local product keeps plans of its own and makes the same checks
+        return _local_matmul(a, b, trans_a=trans_a, trans_b=trans_b, out=out, tiling=tiling)
     key = ("ar", cm.tkey(a), cm.tkey(b), trans_a, trans_b, tiling)
     if tiling is None:
         small = _plan_hit(ctx, ("ar_small",) + key[1:])
@@ -482,8 +484,6 @@ def matmul_allreduce(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False,
     dev = cm.require_cuda(a, b, out)
     _check_pair(a, b)
     m, n, k = cm.logical_shape(a, trans_a, b, trans_b)
-    if ctx.world == 1:
-        return _local_matmul(a, b, trans_a=trans_a, trans_b=trans_b, out=out, tiling=tiling)
     if a.dtype not in (torch.float16, torch.bfloat16):
         raise TypeError("matmul_allreduce takes fp16 / bf16 operands")
     if out is not None and (tuple(out.shape) != (m, n) or out.dtype != a.dtype):
@@ -642,6 +642,8 @@ def allgather_matmul(a_shard: torch.Tensor, b: torch.Tensor, *, trans_b: bool = 
     the shard travels by multicast stores.
     """
     ctx = _ctx(ctx)
+    if ctx.world == 1 and a_shard.dim() == 2:      # the local product keeps plans of its own and makes the same checks
+        return _local_matmul(a_shard, b, trans_b=trans_b, out=out, tiling=tiling, activation=activation), a_shard
     key = ("ag", cm.tkey(a_shard), cm.tkey(b), trans_b, cm.tkey(out), tiling, activation)
     if tiling is None and activation is None:
         small = _plan_hit(ctx, ("ag_small",) + key[1:])
@@ -664,9 +666,6 @@ def allgather_matmul(a_shard: torch.Tensor, b: torch.Tensor, *, trans_b: bool = 
     kb, n = (b.shape[1], b.shape[0]) if trans_b else (b.shape[0], b.shape[1])
     if k != kb:
         raise ValueError("inner dimensions differ: A gives K=%d, B gives K=%d" % (k, kb))
-    if ctx.world == 1:
-        o = _local_matmul(a_shard, b, trans_b=trans_b, out=out, tiling=tiling, activation=activation)
-        return o, a_shard
     if a_shard.dtype not in (torch.float16, torch.bfloat16):
         raise TypeError("allgather_matmul takes fp16 / bf16 operands")
     W = ctx.world
