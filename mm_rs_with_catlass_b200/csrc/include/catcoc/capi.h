@@ -39,7 +39,7 @@ enum { CATCOC_MODE_LOCAL = 0, CATCOC_MODE_RS = 1, CATCOC_MODE_AR = 2, CATCOC_MOD
 /* Communication tiling. Field-for-field superset of the reference's CocTilingParams
  * (examples/dynamic_tiling/include/info.h:29-42); see tiling/config.py for the mapping. */
 typedef struct CatcocTiling {
-  int bn;          /* tile columns: 64, 128 or 256 (0 = default 256)                    */
+  int bn;          /* tile columns: 64, 128 or 256 (0 = default 256); local products: 192 too, see launch.cu */
   int swizzle;     /* tiles per column group of the raster (0 = default)                */
   int num_ctas;    /* persistent CTAs (0 = one per SM)                                   */
   int seg_dim;     /* all-reduce ownership split: 0 rows, 1 cols, -1 auto                */

@@ -336,7 +336,10 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   // of tiles, 256 x 192 on a pair (two accumulators of 192 columns). A CTA's intake bounds the 128 x 128 tile (33 KiB per
   // 256 cycles of MMAs; the pair: 29.5 KiB per 384): 4096 x 8192 x 7168 e4m3 with its quantisation 361 -> 258 us.
   const bool mx_pair = mx && !fused && a.M > kBM && a.scale_m == nullptr && a.scale_n == nullptr && !a.affine && a.act == 0;
-  const int bn = mx ? (mx_pair ? 192 : 128) : norm_bn(a.tiling.bn);
+  // 192-column tiles: pairs of local products (no workspace geometry knows them) with a B stored [N, K]; a [K, N] one comes
+  // in 128-byte column blocks, of which a CTA's half would hold one and a half
+  const bool bn192 = a.tiling.bn == 192 && !fused && a.trans_b && a.tiling.cta_pair == 2;
+  const int bn = mx ? (mx_pair ? 192 : 128) : bn192 ? 192 : norm_bn(a.tiling.bn);
   const int seg_dim = pick_seg_dim(a);
   const bool pair = mx ? mx_pair : (a.tiling.cta_pair == 2);
   if (mx) {

@@ -121,7 +121,10 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
     split = None
     if tiling is None:
         from ..tiling import chooser
-        tiling = chooser.choose("matmul", m, n, k, 1, a.dtype)
+        # [N, K] storage, or a column-major view of [K, N], which as_operand folds into it
+        b_k_major = trans_b != (b.stride(-1) != 1 and b.stride(0) == 1 and min(b.shape) > 1)
+        tiling = chooser.choose("matmul", m, n, k, 1, a.dtype,
+                                b_k_major=b_k_major and _group is None)
         if _group is None and trace is None:
             split = chooser.split_k(m, n, k, a.element_size(), tiling)
             if split is not None:

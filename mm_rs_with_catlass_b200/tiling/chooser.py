@@ -28,8 +28,8 @@ _NUM_SMS = 148
 # Measured on B200 (bf16, CUDA-graph replay): time of one wave of tiles relative to the 128 x 256
 # single-CTA tile, per unit of output. Narrow tiles re-read A from L2 once per column tile and are
 # bound by the fill rate of shared memory, so halving the width costs far more than half.
-_TILE_EFF = {256: 1.0, 128: 0.56, 64: 0.43}
-_PAIR_GAIN = {256: 1.10, 128: 1.35}     # 2-CTA tiles: each CTA fills half of B
+_TILE_EFF = {256: 1.0, 192: 0.85, 128: 0.56, 64: 0.43}
+_PAIR_GAIN = {256: 1.18, 192: 1.18, 128: 1.35}     # 2-CTA tiles: each CTA fills half of B (192: pairs only)
 
 
 # Cost model of split_k, in SM cycles, fitted to 84 shapes (bf16 and int8; 4 to 1024 rows, N of 992 to 28672, K of 3584 to
@@ -57,7 +57,10 @@ def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bo
     return waves * bn / eff
 
 
-def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype) -> TilingConfig:
+def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b_k_major: bool = False) -> TilingConfig:
+    """``b_k_major``: the caller can launch 192-column pair tiles, i.e. a local product with a B stored
+    [N, K]. They fill waves that 256 columns leave nearly empty (8144 x 1696 x 5120: 124 -> 115 us;
+    1024 x 5120 x 6152: 93 -> 85 us); single 192-column tiles were never the best of 20 shapes."""
     rows = m
     fused = world > 1 and op in ("matmul_reduce_scatter", "quant_matmul_reduce_scatter", "matmul_allreduce",
                                  "allgather_matmul")
@@ -72,10 +75,14 @@ def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype) -
     for pair in (2, 1):
         if forced in ("1", "2") and pair != int(forced):
             continue
-        if pair == 2 and (seg_rows < 256 or seg_rows % 256 != 0):
-            continue   # ragged 256-row tiles are mostly padding
-        for bn in (256, 128, 64):
+        if pair == 2 and ((seg_rows < 256 or seg_rows % 256 != 0) if fused else seg_rows <= 128):
+            # ragged 256-row tiles of a segment are mostly padding; a local product has one ragged row of them
+            # (8144 x 1696 x 5120: 146 us on single tiles, 124 on pairs)
+            continue
+        for bn in (256, 192, 128, 64):
             if pair == 2 and bn < 128:
+                continue
+            if bn == 192 and (pair == 1 or not b_k_major or fused or n <= 192 or dtype == torch.int8):
                 continue
             if dtype == torch.int8 and (bn < 128 or (pair == 2 and bn < 256)):
                 continue   # 8-bit [K, N] operands need a full 128-byte run of N per TMA box and CTA
@@ -137,9 +144,9 @@ def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
 
 
 def choose(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype,
-           table: Optional["_table.TilingTable"] = None) -> TilingConfig:
+           table: Optional["_table.TilingTable"] = None, b_k_major: bool = False) -> TilingConfig:
     tbl = table if table is not None else _table.default_table()
     hit = tbl.lookup(op, m, n, k, world, dtype)
     if hit is not None:
         return hit
-    return heuristic(op, m, n, k, world, dtype)
+    return heuristic(op, m, n, k, world, dtype, b_k_major)
