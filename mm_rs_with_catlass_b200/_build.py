@@ -33,6 +33,7 @@ SOURCES = [
     "kernels/inst/f16_single.cu",
     "kernels/inst/f16_pair.cu",
     "kernels/inst/f16_slice_k.cu",
+    "kernels/inst/pair_tail.cu",
     "kernels/inst/i8_single.cu",
     "kernels/inst/i8_pair.cu",
     "kernels/inst/f8_single.cu",

@@ -114,6 +114,8 @@ def _declare(lib) -> None:
         "catcoc_slice_k_launch": (i32, [P(OpArgs), vp, vp]),
         "catcoc_splitk_workspace_bytes": (i64, [i32, i32, i32]),
         "catcoc_splitk_launch": (i32, [P(OpArgs), i32, i32, vp, vp]),
+        "catcoc_tail_workspace_bytes": (i64, [i32, i32, i32, i32, i32]),
+        "catcoc_tail_launch": (i32, [P(OpArgs), i32, i32, i32, vp, vp]),
         "catcoc_stage_bytes": (i64, [i32, i32, i32, i32, i32, i32, i32]),
         "catcoc_arrive_words": (i64, [i32, i32, i32, i32, i32, i32]),
         "catcoc_done_words": (i64, [i32, i32, i32, i32, i32, i32]),

@@ -147,6 +147,12 @@ int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_range, void
 int64_t catcoc_splitk_workspace_bytes(int M, int N, int slices);
 int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_slice, void* workspace, void* stream);
 
+/* A local product on pair tiles (args->tiling: cta_pair 2) whose last wave is nearly empty: the tiles from number `first` on
+ * are cut into `slices` slices of `k_slice` elements (a multiple of 512 bytes), so that they spread over all SMs; the planes go
+ * to `workspace` (128-byte aligned, catcoc_tail_workspace_bytes(...) bytes), a second kernel sums them and runs the epilogue. */
+int64_t catcoc_tail_workspace_bytes(int M, int N, int bn, int first, int slices);
+int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slices, int k_slice, void* workspace, void* stream);
+
 /* Workspace sizes (bytes / words) for given problem + tiling, identical on every rank. */
 int64_t catcoc_stage_bytes(int M, int N, int W, int seg_dim, int bn, int cta_pair, int partial_fmt);
 int64_t catcoc_arrive_words(int M, int N, int W, int seg_dim, int bn, int cta_pair);

@@ -316,6 +316,11 @@ CATCOC_DEVICE TileInfo walk_tile(const FusedParams& p, int t, GroupWalk& w) {
   return group_walk_tile(p.sched, p.num_groups, p.group_ends, p.group_rows, t, w);
 }
 
+CATCOC_DEVICE int sched_tail_first(const FusedParams&) { return 0; }
+CATCOC_DEVICE int sched_tail_first(const FusedParamsTail& p) { return p.tail_first; }
+CATCOC_DEVICE const CUtensorMap* push_map(const FusedParams& p, bool, int seg) { return &p.tm_stage[seg]; }
+CATCOC_DEVICE const CUtensorMap* push_map(const FusedParamsTail& p, bool tail, int seg) { return tail ? &p.tm_tail : &p.tm_stage[seg]; }
+
 // ---------------------------------------------------------------------------------------
 // The kernel
 // ---------------------------------------------------------------------------------------
@@ -323,6 +328,21 @@ template <int KIND, bool CTA2, int EPI, class Params = FusedParams>
 __global__ void __launch_bounds__(threads_for(EPI), 1)
 fused_gemm_kernel(const __grid_constant__ Params p) {
   constexpr bool kGk = std::is_same<Params, FusedParamsGk>::value;   // every group has a K range of its own
+  constexpr bool kTail = std::is_same<Params, FusedParamsTail>::value;   // the last tiles are cut along K
+  // work unit -> tile, and its K slice when it belongs to the tail (else -1)
+  auto unit_tile = [&](int t, GroupWalk& w, int& slice) {
+    slice = -1;
+    if constexpr (kTail) {
+      if (t >= p.tail_first) {
+        const int u = t - p.tail_first, q = u / p.tail_slices;
+        slice = u - q * p.tail_slices;
+        return get_tile(p.sched, p.tail_first + q);
+      }
+      return get_tile(p.sched, t);
+    } else {
+      return walk_tile(p, t, w);
+    }
+  };
   // Epilogue variant (see EpiVariant in params.h): stages a launch cannot need are compiled out.
   constexpr bool kReduce = (EPI == EPI_REDUCE || EPI == EPI_FULL);   // push flavour of RS / AR: peers' partials, pushes, stamps
   constexpr bool kScale = (EPI == EPI_FULL);      // int32 bias, dequantisation, alpha / beta / C / fp32 bias
@@ -366,7 +386,8 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
   // inside a K-block's part of the stage, after A and B: SFA, then one (pair: two) blocks of SFB
   constexpr int kSfSmemOff = kABytes + static_cast<int>(CTA2 ? kMxBN / 2 : kMxBN) * 128;
   const bool grouped = (p.num_groups > 0);
-  const int total_tiles = grouped ? grouped_total_tiles(p, lane) : sched.total_tiles;
+  int total_tiles = grouped ? grouped_total_tiles(p, lane) : sched.total_tiles;
+  if constexpr (kTail) total_tiles = p.tail_first + (total_tiles - p.tail_first) * p.tail_slices;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -425,7 +446,8 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
     int pre_tile = -1;
     GroupWalk walk = group_walk_begin(p);
     for (int t = worker; ok && t < total_tiles; t += num_workers) {
-      const TileInfo ti = walk_tile(p, t, walk);
+      int slice;
+      const TileInfo ti = unit_tile(t, walk, slice);
       const CUtensorMap* tma = &p.tm_a;
       int a_row = ti.m0 + sub * kBM;
       int a_k_off = 0;
@@ -439,6 +461,9 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
         a_k_off = r.x;
         tile_k = r.y - r.x;                          // an empty range has no K block: every role skips the tile
         tma = &p.gk_map[2 * ti.seg];
+      }
+      if constexpr (kTail) {
+        if (slice >= 0) { a_k_off = slice * p.tail_k; tile_k = min(p.tail_k, p.K - a_k_off); }
       }
       const int tile_sub = ceil_div(tile_k, p.bk), tile_kb = ceil_div(tile_sub, kps);
       if (p.mode == MODE_AG && fused) {
@@ -600,6 +625,12 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
           tile_k = r.y - r.x;
           tile_kb = ceil_div(tile_k, p.bk * kps);
           if (tile_kb <= 0) continue;
+        }
+        if constexpr (kTail) {
+          if (t >= p.tail_first) {
+            tile_k = min(p.tail_k, K - (t - p.tail_first) % p.tail_slices * p.tail_k);
+            tile_kb = ceil_div(tile_k, p.bk * kps);
+          }
         }
         const int mx_n0 = (KIND == KIND_MX && CTA2) ? walk_tile(p, t, walk).n0 : 0;
         tick.lap(c_issue);
@@ -765,7 +796,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
     // A partial tile pushed by TMA store is announced one tile late: the arrival stamp may only
     // follow the completion of the tile's bulk stores, and waiting for that right away would
     // stall the warp for a link round trip. `pending_stamp` is the stamp still owed (lane 0).
-    const bool any_tma = (p.out_tma != 0) || (kReduce && p.stage_tma != 0);
+    const bool any_tma = kTail || (p.out_tma != 0) || (kReduce && p.stage_tma != 0);
     uint32_t* pending_stamp = nullptr;
     bool prev_win_tma = false;   // the most recent window of this warp left by a TMA store
     auto settle_pending = [&]() {
@@ -780,15 +811,17 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
 
     GroupWalk walk = group_walk_begin(p);
     for (int t = worker; ok && t < total_tiles; t += num_workers) {
-      const TileInfo ti = walk_tile(p, t, walk);
+      int slice;
+      const TileInfo ti = unit_tile(t, walk, slice);
+      const bool tail_unit = kTail && slice >= 0;   // its raw accumulator goes to a plane
       if constexpr (kGk) {
         if (p.gk_range[ti.seg].y <= p.gk_range[ti.seg].x) continue;
       }
-      const bool own = !kReduce || !fused || (p.mode == MODE_AG) || (ti.seg == p.rank);
+      const bool own = !tail_unit && (!kReduce || !fused || (p.mode == MODE_AG) || (ti.seg == p.rank));
       const bool reduce_here = kReduce && fused && own && (p.mode == MODE_RS || p.mode == MODE_AR);
       const int st_fmt = (own && !pull) ? p.out_fmt : pfmt;   // format of what this tile's epilogue stores
       const int st_elt = fmt_bytes(st_fmt);
-      const int rows_valid = max(0, min(32, ti.rows - row_base));
+      const int rows_valid = tail_unit ? 32 : max(0, min(32, ti.rows - row_base));   // planes are written whole
       const int nvec_off = grouped ? ti.seg * p.g_nvec : 0;   // this group's per-column vectors
       const bool affine = kScale && (p.affine != 0) && own;
 
@@ -895,11 +928,11 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
                            (rows_valid == 32 || (!grouped && !fused));
       // A partial tile goes to its owner's slab the same way. Slabs are BM x BN whatever the
       // tile's valid extent, so whole windows are pushed and nothing needs clipping.
-      const bool tma_push = kReduce && !own && (p.stage_tma != 0);
+      const bool tma_push = tail_unit || (kReduce && !own && (p.stage_tma != 0));
       // pull flavour: the stamp of a tile stored by TMA follows the completion of its bulk stores
       const bool stamp_late = tma_push || (kPull && pull && tma_out && rows_valid > 0);
       const CUtensorMap* tm_o = (kPull && pull) ? &p.tm_part[parity] : &p.tm_out;
-      const int push_row0 = tma_push
+      const int push_row0 = tail_unit ? (t - sched_tail_first(p)) * sched.BM + row_base : tma_push
           ? static_cast<int>(stage_slot_offset(sched, st_elt, p.stage_parity_bytes, parity, p.rank, ti.tile_in_seg) /
                              (static_cast<int64_t>(BN) * st_elt)) + row_base
           : 0;
@@ -951,7 +984,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
             released = true;
           }
 
-          if (kScale && is_int && p.bias != nullptr) {
+          if (kScale && is_int && p.bias != nullptr && !tail_unit) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
               const int c = ti.n0 + col0 + j;
@@ -1023,7 +1056,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
           }
 
           // convert this row's 32 values to the stored format and stage them
-          if (st_fmt == FMT_S32 || (st_fmt == FMT_F32 && !is_int && !(dequant && own) && !affine && !(kScale && p.act != ACT_NONE))) {
+          if (st_fmt == FMT_S32 || (st_fmt == FMT_F32 && !is_int && !(dequant && own) && !affine && !(kScale && p.act != ACT_NONE && !tail_unit))) {
 #pragma unroll
             for (int u = 0; u < 8; ++u)
               stage_write(stg, lane, u,
@@ -1104,7 +1137,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
                 }
               }
             }
-            if (kScale && p.act != ACT_NONE) {
+            if (kScale && p.act != ACT_NONE && !tail_unit) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) f[j] = activate(f[j], p.act);
             }
@@ -1138,7 +1171,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
             ptx::fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              ptx::tma_store_2d(&p.tm_stage[ti.seg], stg, win * per_win, push_row0);
+              ptx::tma_store_2d(push_map(p, tail_unit, ti.seg), stg, win * per_win, push_row0);
               ptx::bulk_commit_group();
             }
             ++groups_sent;
@@ -1277,7 +1310,8 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
     bool ok = true;
     GroupWalk walk = group_walk_begin(p);
     for (int t = worker; ok && t < total_tiles; t += num_workers) {
-      const TileInfo ti = walk_tile(p, t, walk);
+      int slice;
+      const TileInfo ti = unit_tile(t, walk, slice);
       int b_col = ti.n0 + sub * b_cols_cta;
       int b_k_off = 0;
       if (grouped) {
@@ -1291,6 +1325,9 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
         b_k_off = r.x;
         tile_k = r.y - r.x;
         tmb = &p.gk_map[2 * ti.seg + 1];
+      }
+      if constexpr (kTail) {
+        if (slice >= 0) { b_k_off = slice * p.tail_k; tile_k = min(p.tail_k, p.K - b_k_off); }
       }
       const int tile_sub = ceil_div(tile_k, p.bk), tile_kb = ceil_div(tile_sub, kps);
       for (int kb = 0; kb < tile_kb; ++kb) {

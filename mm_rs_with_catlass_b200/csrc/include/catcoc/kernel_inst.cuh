@@ -82,6 +82,10 @@ const Unit& unit_mx_pair();
 cudaError_t prepare_slice_k();
 cudaError_t launch_slice_k(bool pair, const FusedParamsGk& p, int grid, cudaStream_t s);
 
+// Pair tiles of local products whose last tiles are cut along K (kernels/inst/pair_tail.cu)
+cudaError_t prepare_tail();
+cudaError_t launch_tail(int kind, bool full, const FusedParamsTail& p, int grid, cudaStream_t s);
+
 }  // namespace inst
 }  // namespace catcoc
 

@@ -218,6 +218,14 @@ struct alignas(64) FusedParamsGk : FusedParams {
   int2 gk_range[kMaxKGroups];
 };
 
+// A last wave that is nearly empty (a kernel instantiation of its own, local products): the tiles from `tail_first` on are cut
+// into `tail_slices` slices of `tail_k` K elements each, one work unit per slice, whose raw accumulators go to planes
+// [units * BM, BN] (partial_fmt: fp32 or int32); a second kernel sums them and runs the epilogue.
+struct alignas(64) FusedParamsTail : FusedParams {
+  CUtensorMap tm_tail;       // the planes, box of 32 rows x 128 bytes
+  int tail_first, tail_slices, tail_k;
+};
+
 enum EventRole : uint32_t { EV_PRODUCER = 0, EV_MMA = 1, EV_EPILOGUE = 2, EV_COMM = 3, EV_REDUCER = 4 };
 enum EventPhase : uint32_t { EV_BEGIN = 0, EV_END = 1, EV_WAIT_PEER = 2 };
 

@@ -926,7 +926,61 @@ CATCOC_DEVICE float load1(const void* p, int64_t i, int fmt) {
   return __half2float(static_cast<const __half*>(p)[i]);
 }
 
-// Sums the planes in slice order and runs the epilogue of the product kernel on the sum, in the same order of operations.
+// Four columns of one row: sums them over the planes in slice order and runs the epilogue of the product kernel on the sum,
+// in the same order of operations. `src`: the first plane's element (r, c0); `n`: columns that exist.
+template <bool INT>
+CATCOC_DEVICE void fold_store(const FoldParams& p, const uint8_t* src, int64_t step, int slices, int r, int c0, int n) {
+  uint32_t a[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 4
+  for (int s = 0; s < slices; ++s) {
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(src + s * step));
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      a[e] = INT ? a[e] + w[e] : __float_as_uint(__uint_as_float(a[e]) + __uint_as_float(w[e]));
+  }
+  const int64_t o = static_cast<int64_t>(r) * p.ldc + c0;
+  if (INT && p.bias != nullptr) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) if (e < n) a[e] += static_cast<uint32_t>(__ldg(p.bias + c0 + e));
+  }
+  if (INT && p.out_fmt == FMT_S32) {
+    uint32_t* dst = static_cast<uint32_t*>(p.out) + o;
+    if (p.vec_ok && n == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(a[0], a[1], a[2], a[3]);
+    else for (int e = 0; e < n; ++e) dst[e] = a[e];
+    return;
+  }
+  float f[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) f[e] = INT ? static_cast<float>(static_cast<int32_t>(a[e])) : __uint_as_float(a[e]);
+  if (p.scale_m != nullptr || p.scale_n != nullptr) {
+    const float sm = p.scale_m != nullptr ? __ldg(p.scale_m + r) : 1.0f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = f[e] * ((p.scale_n != nullptr && e < n) ? __ldg(p.scale_n + c0 + e) : 1.0f) * sm;
+  }
+  if (p.affine) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (e < n) {
+        float x = p.alpha * f[e];
+        if (p.bias_f != nullptr) x += __ldg(p.bias_f + c0 + e);
+        if (p.c_src != nullptr) x += p.beta * load1(p.c_src, static_cast<int64_t>(r) * p.ldc_src + c0 + e, p.out_fmt);
+        f[e] = x;
+      }
+    }
+  }
+  if (p.act != ACT_NONE) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = activate(f[e], p.act);
+  }
+  if (p.vec_ok && n == 4) {
+    if (p.out_fmt == FMT_F32) *reinterpret_cast<float4*>(static_cast<float*>(p.out) + o) = make_float4(f[0], f[1], f[2], f[3]);
+    else *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + o) = make_uint2(pack2(f[0], f[1], p.out_fmt), pack2(f[2], f[3], p.out_fmt));
+  } else {
+    for (int e = 0; e < n; ++e) store1(p.out, o + e, p.out_fmt, f[e]);
+  }
+}
+
 // Four columns a thread; the planes come from L2 (128 rows x 8192 columns x 4 slices: 17 MB).
 template <bool INT>
 __global__ void __launch_bounds__(256) splitk_fold_kernel(const FoldParams p) {
@@ -936,59 +990,59 @@ __global__ void __launch_bounds__(256) splitk_fold_kernel(const FoldParams p) {
   for (int64_t u = blockIdx.x * 256ll + threadIdx.x; u < units; u += gridDim.x * 256ll) {
     const int r = static_cast<int>(u / units_row);
     const int c0 = static_cast<int>(u - static_cast<int64_t>(r) * units_row) * 4;
-    const uint8_t* src = p.parts + (static_cast<int64_t>(r) * p.pitch + c0) * 4;
-    const int64_t step = p.plane * 4;
-    uint32_t a[4] = {0u, 0u, 0u, 0u};
-#pragma unroll 4
-    for (int s = 0; s < p.slices; ++s) {
-      const uint4 v = __ldcg(reinterpret_cast<const uint4*>(src + s * step));
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        a[e] = INT ? a[e] + w[e] : __float_as_uint(__uint_as_float(a[e]) + __uint_as_float(w[e]));
-    }
-    const int n = min(4, p.cols - c0);
-    const int64_t o = static_cast<int64_t>(r) * p.ldc + c0;
-    if (INT && p.bias != nullptr) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) if (e < n) a[e] += static_cast<uint32_t>(__ldg(p.bias + c0 + e));
-    }
-    if (INT && p.out_fmt == FMT_S32) {
-      uint32_t* dst = static_cast<uint32_t*>(p.out) + o;
-      if (p.vec_ok && n == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(a[0], a[1], a[2], a[3]);
-      else for (int e = 0; e < n; ++e) dst[e] = a[e];
-      continue;
-    }
-    float f[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = INT ? static_cast<float>(static_cast<int32_t>(a[e])) : __uint_as_float(a[e]);
-    if (p.scale_m != nullptr || p.scale_n != nullptr) {
-      const float sm = p.scale_m != nullptr ? __ldg(p.scale_m + r) : 1.0f;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) f[e] = f[e] * ((p.scale_n != nullptr && e < n) ? __ldg(p.scale_n + c0 + e) : 1.0f) * sm;
-    }
-    if (p.affine) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (e < n) {
-          float x = p.alpha * f[e];
-          if (p.bias_f != nullptr) x += __ldg(p.bias_f + c0 + e);
-          if (p.c_src != nullptr) x += p.beta * load1(p.c_src, static_cast<int64_t>(r) * p.ldc_src + c0 + e, p.out_fmt);
-          f[e] = x;
-        }
-      }
-    }
-    if (p.act != ACT_NONE) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) f[e] = activate(f[e], p.act);
-    }
-    if (p.vec_ok && n == 4) {
-      if (p.out_fmt == FMT_F32) *reinterpret_cast<float4*>(static_cast<float*>(p.out) + o) = make_float4(f[0], f[1], f[2], f[3]);
-      else *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + o) = make_uint2(pack2(f[0], f[1], p.out_fmt), pack2(f[2], f[3], p.out_fmt));
-    } else {
-      for (int e = 0; e < n; ++e) store1(p.out, o + e, p.out_fmt, f[e]);
-    }
+    fold_store<INT>(p, p.parts + (static_cast<int64_t>(r) * p.pitch + c0) * 4, p.plane * 4, p.slices, r, c0, min(4, p.cols - c0));
   }
+}
+
+// The same over the tiles from `first` on: blockIdx.y counts them, their planes are [slices][BM][BN].
+template <bool INT>
+__global__ void __launch_bounds__(256) tail_fold_kernel(const FoldParams p, const TileSched sched, int first) {
+  ptx::grid_dependency_wait();
+  const TileInfo ti = get_tile(sched, first + blockIdx.y);
+  const uint8_t* planes = p.parts + static_cast<int64_t>(blockIdx.y) * p.slices * p.plane * 4;
+  const int units_row = sched.BN / 4;
+  for (int u = blockIdx.x * 256 + threadIdx.x; u < ti.rows * units_row; u += gridDim.x * 256) {
+    const int r = u / units_row, c = (u - r * units_row) * 4;
+    if (c < ti.cols)
+      fold_store<INT>(p, planes + (static_cast<int64_t>(r) * sched.BN + c) * 4, p.plane * 4, p.slices, ti.m0 + r, ti.n0 + c, min(4, ti.cols - c));
+  }
+}
+
+// The epilogue that `a` describes
+FoldParams fold_params(const CatcocOpArgs& a) {
+  FoldParams f;
+  memset(&f, 0, sizeof(f));
+  f.rows = a.M; f.cols = a.N;
+  f.out = a.out; f.ldc = a.ldc; f.out_fmt = a.out_fmt;
+  f.vec_ok = (reinterpret_cast<uintptr_t>(a.out) % (4 * fmt_bytes(a.out_fmt))) == 0 && (a.ldc % 4) == 0;
+  f.scale_m = a.scale_m; f.scale_n = a.scale_n; f.bias = a.bias;
+  f.affine = a.affine; f.alpha = a.alpha; f.beta = a.beta;
+  f.c_src = (a.affine && a.beta != 0.0f) ? a.c_src : nullptr;
+  f.ldc_src = a.ldc_src; f.bias_f = a.affine ? a.bias_f : nullptr; f.act = a.act;
+  return f;
+}
+
+bool fold_fits(const CatcocOpArgs& a, bool is_int) {
+  if (is_int ? (a.out_fmt == CATCOC_FMT_F32 && a.scale_m == nullptr && a.scale_n == nullptr) : (a.out_fmt == CATCOC_FMT_S32 || a.bias != nullptr)) {
+    set_error("split K: output format or bias does not fit the operands");
+    return false;
+  }
+  return true;
+}
+
+template <class... Args>
+cudaError_t launch_dependent(dim3 grid, cudaStream_t stream, void (*kernel)(Args...), Args... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 int splitk_rows(int M) { return round_up(M, 32); }    // whole 32-row windows leave the first launch by TMA
@@ -1016,10 +1070,7 @@ extern "C" int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_
     return CATCOC_E_BAD_ARG;
   }
   const bool is_int = rf.kind == KIND_I8;
-  if (is_int ? (a.out_fmt == CATCOC_FMT_F32 && a.scale_m == nullptr && a.scale_n == nullptr) : (a.out_fmt == CATCOC_FMT_S32 || a.bias != nullptr)) {
-    set_error("splitk: output format or bias does not fit the operands");
-    return CATCOC_E_UNSUPPORTED;
-  }
+  if (!fold_fits(a, is_int)) return CATCOC_E_UNSUPPORTED;
   const int rows = splitk_rows(a.M), pitch = splitk_pitch(a.N);
   CatcocOpArgs g = a;
   g.M = slices * rows; g.K = k_slice;
@@ -1031,30 +1082,65 @@ extern "C" int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_
   g.limit[LIM_OUT] = (static_cast<int64_t>(g.M - 1) * pitch + a.N) * 4;
   rc = catcoc_fused_launch(&g, stream_);
   if (rc != 0) return rc;
-  FoldParams f;
-  memset(&f, 0, sizeof(f));
+  FoldParams f = fold_params(a);
   f.parts = static_cast<const uint8_t*>(workspace);
   f.plane = static_cast<int64_t>(rows) * pitch;
-  f.slices = slices; f.rows = a.M; f.cols = a.N; f.pitch = pitch;
-  f.out = a.out; f.ldc = a.ldc; f.out_fmt = a.out_fmt;
-  const int vec = 4 * fmt_bytes(a.out_fmt);
-  f.vec_ok = (reinterpret_cast<uintptr_t>(a.out) % vec) == 0 && (a.ldc % 4) == 0;
-  f.scale_m = a.scale_m; f.scale_n = a.scale_n; f.bias = a.bias;
-  f.affine = a.affine; f.alpha = a.alpha; f.beta = a.beta;
-  f.c_src = (a.affine && a.beta != 0.0f) ? a.c_src : nullptr;
-  f.ldc_src = a.ldc_src; f.bias_f = a.affine ? a.bias_f : nullptr; f.act = a.act;
+  f.slices = slices; f.pitch = pitch;
   const int64_t units = static_cast<int64_t>(a.M) * ((a.N + 3) / 4);
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(static_cast<unsigned>(units > 148 * 8 * 256 ? 148 * 8 : (units + 255) / 256), 1, 1);
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  CATCOC_CUDA_OK(is_int ? cudaLaunchKernelEx(&cfg, splitk_fold_kernel<true>, static_cast<const FoldParams&>(f))
-                        : cudaLaunchKernelEx(&cfg, splitk_fold_kernel<false>, static_cast<const FoldParams&>(f)));
+  const dim3 fold_grid(static_cast<unsigned>(units > 148 * 8 * 256 ? 148 * 8 : (units + 255) / 256));
+  CATCOC_CUDA_OK(launch_dependent(fold_grid, stream, is_int ? splitk_fold_kernel<true> : splitk_fold_kernel<false>, f));
+  return CATCOC_OK;
+}
+
+// ---- a nearly empty last wave: its tiles cut along K ----
+extern "C" int64_t catcoc_tail_workspace_bytes(int M, int N, int bn, int first, int slices) {
+  const TileSched s = make_sched(M, N, 2 * kBM, bn, 1, SEG_ROWS, 0, 1);
+  if (M <= 0 || N <= 0 || (bn != 128 && bn != 192 && bn != 256) || first < 0 || first >= s.total_tiles || slices < 2) return -1;
+  return static_cast<int64_t>(s.total_tiles - first) * slices * s.BM * s.BN * 4;
+}
+
+extern "C" int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slices, int k_slice, void* workspace, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (args == nullptr || workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 127) != 0 || slices < 2 || k_slice <= 0) {
+    set_error("tail: bad arguments");
+    return CATCOC_E_BAD_ARG;
+  }
+  CatcocOpArgs a = *args;
+  Resolved rf;
+  int rc = resolve_format(a.in_fmt, &rf);
+  if (rc != 0) return rc;
+  const bool is_int = rf.kind == KIND_I8;
+  if (a.mode != CATCOC_MODE_LOCAL || (rf.kind != KIND_F16 && !is_int) || a.num_groups != 0 || a.tiling.cta_pair != 2 ||
+      (k_slice * rf.elt) % 256 != 0 || static_cast<int64_t>(k_slice) * (slices - 1) >= a.K || static_cast<int64_t>(k_slice) * slices < a.K) {
+    set_error("tail: a local 16-bit or int8 product on pair tiles whose K range is cut into whole stages (K=%d, %d slices of %d)", a.K, slices, k_slice);
+    return CATCOC_E_BAD_ARG;
+  }
+  if (!fold_fits(a, is_int)) return CATCOC_E_UNSUPPORTED;
+  static const cudaError_t ready = inst::prepare_tail();
+  CATCOC_CUDA_OK(ready);
+  a.partial_fmt = is_int ? CATCOC_FMT_S32 : CATCOC_FMT_F32;
+  FusedParamsTail p;
+  int kind = 0, grid = 0, pair = 0;
+  rc = catcoc_build_params(&a, &p, &kind, &grid, &pair);
+  if (rc != 0) return rc;
+  if (first < 0 || first >= p.sched.total_tiles || pair == 0) { set_error("tail: tile %d of %d", first, p.sched.total_tiles); return CATCOC_E_BAD_ARG; }
+  const int tiles = p.sched.total_tiles - first;
+  p.tail_first = first; p.tail_slices = slices; p.tail_k = k_slice;
+  rc = encode_2d(&p.tm_tail, workspace, 4, is_int ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                 static_cast<int64_t>(tiles) * slices * p.sched.BM, p.sched.BN, p.sched.BN, 32, 32);
+  if (rc != 0) return rc;
+  int device = 0;
+  cudaGetDevice(&device);
+  grid = imin(sm_count(device), 2 * max_active_pairs(rf.kind)) & ~1;     // more units than tiles
+  if (a.tiling.num_ctas > 0) grid = imin(grid, a.tiling.num_ctas & ~1);
+  if (grid < 2) grid = 2;
+  const bool full = p.scale_m != nullptr || p.scale_n != nullptr || p.bias != nullptr || p.affine != 0 || p.act != 0;
+  CATCOC_CUDA_OK(inst::launch_tail(rf.kind, full, p, grid, stream));
+  FoldParams f = fold_params(a);
+  f.parts = static_cast<const uint8_t*>(workspace);
+  f.plane = static_cast<int64_t>(p.sched.BM) * p.sched.BN;
+  f.slices = slices; f.pitch = p.sched.BN;
+  const dim3 fold_grid(static_cast<unsigned>(p.sched.BM * p.sched.BN / 4 / 256), static_cast<unsigned>(tiles));
+  CATCOC_CUDA_OK(launch_dependent(fold_grid, stream, is_int ? tail_fold_kernel<true> : tail_fold_kernel<false>, f, p.sched, first));
   return CATCOC_OK;
 }

@@ -222,6 +222,18 @@ def launch_splitk(args: N.OpArgs, slices: int, k_slice: int, device: torch.devic
     _launches += 1
 
 
+def launch_tail(args: N.OpArgs, first: int, slices: int, k_slice: int, device: torch.device) -> None:
+    """Queues a product on pair tiles whose tiles from ``first`` on are cut along K, and the kernel that sums the slices."""
+    args.timeout_ns = default_timeout_ns()
+    args.events, args.events_cap = _event_ring
+    lib = N.lib()
+    ws = torch.empty(int(lib.catcoc_tail_workspace_bytes(args.M, args.N, args.tiling.bn or 256, first, slices)), dtype=torch.uint8,
+                     device=device)
+    N.check(lib.catcoc_tail_launch(C.byref(args), first, slices, k_slice, ws.data_ptr(), C.c_void_p(stream_of(device))))
+    global _launches
+    _launches += 1
+
+
 _launches = 0
 _event_ring = (None, 0)
 

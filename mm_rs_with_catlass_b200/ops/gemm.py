@@ -82,7 +82,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
                 out = torch.empty(out_shape, dtype=plan_dtype, device=a.device)
                 args.out = out.data_ptr()
             if split is not None:
-                cm.launch_splitk(args, split[0], split[1], a.device)
+                split[0](args, *split[1:], a.device)
             else:
                 cm.launch(args, a.device)
             return out
@@ -123,12 +123,18 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
         from ..tiling import chooser
         # [N, K] storage, or a column-major view of [K, N], which as_operand folds into it
         b_k_major = trans_b != (b.stride(-1) != 1 and b.stride(0) == 1 and min(b.shape) > 1)
+        tails = _group is None and trace is None and a.dtype in (torch.float16, torch.bfloat16, torch.int8)
         tiling = chooser.choose("matmul", m, n, k, 1, a.dtype,
-                                b_k_major=b_k_major and _group is None)
+                                b_k_major=b_k_major and _group is None, tails=tails)
         if _group is None and trace is None:
             split = chooser.split_k(m, n, k, a.element_size(), tiling)
             if split is not None:
                 tiling = TilingConfig(bn=split[2], cta_pair=1)
+                split = (cm.launch_splitk, split[0], split[1])
+        if split is None and tails and tiling.cta_pair == 2:
+            cut = chooser.tail_cut(m, n, k, a.element_size(), tiling.effective_bn)[1]
+            if cut is not None:
+                split = (cm.launch_tail, *cut)
     with torch.cuda.device(dev):
         # An operand whose base or row pitch TMA cannot take goes through the pad kernel first.
         oa = cm.as_operand(a, trans_a)
@@ -175,7 +181,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
             # a caller that keeps its own plan of a group launch (ops/fused.py); None: the block points at a temporary copy
             _args_out.append(None if (oa.copied or ob.copied) else args)
         if split is not None:
-            cm.launch_splitk(args, split[0], split[1], dev)
+            split[0](args, *split[1:], dev)
         else:
             cm.launch(args, dev)
         if key is not None and (not oa.copied or _wants_pad_prologue(a)) and not ob.copied:

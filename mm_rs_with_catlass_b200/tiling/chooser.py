@@ -34,6 +34,8 @@ _PAIR_GAIN = {256: 1.18, 192: 1.18, 128: 1.35}     # 2-CTA tiles: each CTA fills
 
 # Cost model of split_k, in SM cycles, fitted to 84 shapes (bf16 and int8; 4 to 1024 rows, N of 992 to 28672, K of 3584 to
 # 28672): its choices lose 2 % on average against the best of all cuts that were measured, the direct kernel alone 28 %.
+_TAIL_INT8 = 12000.0              # int8 products gain that much less from a cut tail than the model says (fitted)
+_TAIL_INTAKE = 52.0               # the same for a pair tile of a product that fills the GPU
 _INTAKE = {1: 46.0, 2: 42.0}      # bytes per cycle that one CTA takes in while most of the others do the same (pair: per CTA)
 _HBM = 3600.0                     # bytes per cycle from HBM, all SMs
 _PLANES = 3500.0                  # bytes per cycle of the planes, written and read through L2
@@ -57,8 +59,36 @@ def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bo
     return waves * bn / eff
 
 
-def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b_k_major: bool = False) -> TilingConfig:
-    """``b_k_major``: the caller can launch 192-column pair tiles, i.e. a local product with a B stored
+@functools.lru_cache(maxsize=4096)
+def tail_cut(m: int, n: int, k: int, elt: int, bn: int):
+    """A local product on pair tiles (256 x bn): ``(waves, cut)`` with ``cut = (first, slices, k_slice)``
+    when the tiles from ``first`` on, its last and nearly empty wave, are worth cutting along K so that
+    they spread over all SMs, else None; ``waves`` is what the product then costs, in waves of tiles.
+
+    The cut pays for its planes (written and read through L2) and for a second kernel, so it needs a long
+    K. bf16 1024 x 5120 x 6144 (80 tiles on 74 pairs): 81 -> 64 us; 600 x 8192 x 14336: 149 -> 134 us; int8
+    600 x 8192 x 14336: 101 -> 91 us; over 28 shapes the choice is within 5 % of the better form."""
+    units = _NUM_SMS // 2
+    tiles = -(-m // 256) * -(-n // bn)
+    first, rest = tiles // units * units, tiles % units
+    waves, kb = -(-tiles // units), -(-k * elt // 128)
+    wave_time = kb * max(2.0 * bn, (128 + bn // 2) * 128 / _TAIL_INTAKE)
+    best, best_time = None, 0.96 * (waves * wave_time + _LAUNCH)
+    for s in range(2, 25) if rest else ():
+        kbs = -(-(-(-kb // s)) // 2) * 2                      # K blocks per slice: whole pair stages
+        if kbs < 8 or -(-kb // kbs) != s:
+            continue
+        t = first // units * wave_time + -(-rest * s // units) * kbs * wave_time / kb
+        t += rest * s * 256.0 * bn * 8 / _PLANES + _LAUNCH + _FOLD + (_TAIL_INT8 if elt == 1 else 0.0)
+        if t < best_time:
+            best, best_time = (first, s, kbs * 128 // elt), t
+    return (waves, None) if best is None else ((best_time - _LAUNCH) / wave_time, best)
+
+
+def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b_k_major: bool = False,
+              tails: bool = False) -> TilingConfig:
+    """``tails``: the caller cuts the last wave along K where that pays (:func:`tail_cut`).
+    ``b_k_major``: the caller can launch 192-column pair tiles, i.e. a local product with a B stored
     [N, K]. They fill waves that 256 columns leave nearly empty (8144 x 1696 x 5120: 124 -> 115 us;
     1024 x 5120 x 6152: 93 -> 85 us); single 192-column tiles were never the best of 20 shapes."""
     rows = m
@@ -87,6 +117,8 @@ def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b
             if dtype == torch.int8 and (bn < 128 or (pair == 2 and bn < 256)):
                 continue   # 8-bit [K, N] operands need a full 128-byte run of N per TMA box and CTA
             cost = tile_cost(seg_rows, nseg, n, bn, pair, seg_cols=ar_cols)
+            if tails and pair == 2:
+                cost = tail_cut(rows, n, k, dtype.itemsize, bn)[0] * bn / (_TILE_EFF[bn] * _PAIR_GAIN[bn])
             if best is None or cost < best[0] - 1e-9:
                 best = (cost, bn, pair)
     if best is None:
@@ -128,6 +160,8 @@ def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
     hbm = (n * k + m * k) * elt / _HBM
     pair, bn0 = (2 if direct.cta_pair == 2 else 1), direct.effective_bn
     waves = -(-(-(-m // (128 * pair)) * -(-n // bn0)) // (_NUM_SMS // pair))
+    if pair == 2 and bn0 >= 128:
+        waves = tail_cut(m, n, k, elt, bn0)[0]
     best, best_time = None, 0.95 * (max(hbm, waves * kb * unit(bn0, pair)) + _LAUNCH + (_INT8_EPILOGUE if elt == 1 else 0.0))
     for bn in (256, 128):
         if n < bn and bn > 128:
@@ -144,9 +178,9 @@ def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
 
 
 def choose(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype,
-           table: Optional["_table.TilingTable"] = None, b_k_major: bool = False) -> TilingConfig:
+           table: Optional["_table.TilingTable"] = None, b_k_major: bool = False, tails: bool = False) -> TilingConfig:
     tbl = table if table is not None else _table.default_table()
     hit = tbl.lookup(op, m, n, k, world, dtype)
     if hit is not None:
         return hit
-    return heuristic(op, m, n, k, world, dtype, b_k_major)
+    return heuristic(op, m, n, k, world, dtype, b_k_major, tails)
