@@ -582,6 +582,12 @@ CATCOC_DEVICE void st_global_v4(void* p, uint4 v) {
                "r"(v.w)
                : "memory");
 }
+// 32 bytes at once (a whole sector; 32-byte aligned)
+CATCOC_DEVICE void st_global_v8(void* p, const uint32_t (&r)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+               "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
 CATCOC_DEVICE void st_shared_v4(uint32_t saddr, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y),
                "r"(v.z), "r"(v.w)

@@ -47,3 +47,10 @@ def test_more_groups_than_one_batch_of_maps():
 def test_neighbouring_rows_are_not_read():
     _check(256, 256, [100, 30, 77], torch.bfloat16, seed=4, poison=True)
     _check(136, 256, [100, 30, 77], torch.bfloat16, seed=5, poison=True)
+
+
+def test_short_and_long_ranges_store_by_different_paths():
+    # ranges of up to 256 rows store from registers, longer ones through the staging buffers; rows that do not start on a
+    # 32-byte sector (n = 328) never do
+    _check(256, 512, [256, 257, 40, 700, 256], torch.bfloat16, seed=6)
+    _check(256, 328, [256, 40, 700], torch.float16, seed=7)
