@@ -386,6 +386,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
   // inside a K-block's part of the stage, after A and B: SFA, then one (pair: two) blocks of SFB
   constexpr int kSfSmemOff = kABytes + static_cast<int>(CTA2 ? kMxBN / 2 : kMxBN) * 128;
   const bool grouped = (p.num_groups > 0);
+  if (grouped) ptx::grid_dependency_wait();   // the group list may be the predecessor's result
   int total_tiles = grouped ? grouped_total_tiles(p, lane) : sched.total_tiles;
   if constexpr (kTail) total_tiles = p.tail_first + (total_tiles - p.tail_first) * p.tail_slices;
 
@@ -421,6 +422,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
   if (CTA2) ptx::cluster_sync_all();   // the peer's barriers exist before anyone signals them
   ptx::tcgen05_fence_after();
   const uint32_t tmem_base = tail->tmem_base;
+  ptx::grid_dependency_wait();   // nothing above touches global memory; returns at once unless launched as a dependent
   // both CTAs of a pair must take the same decision (they meet again at cluster barriers)
   bool dead = tail->dead != 0u;
   if (CTA2) dead = dead || ptx::ld_shared_cluster_u32(ptx::map_to_cta(ptx::smem_u32(&tail->dead), static_cast<uint32_t>(sub ^ 1))) != 0u;

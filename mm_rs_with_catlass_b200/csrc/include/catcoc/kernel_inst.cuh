@@ -38,12 +38,18 @@ cudaError_t launch_one(const Params& p, int grid, int threads, cudaStream_t stre
   cfg.blockDim = dim3((threads >= kThreads && threads <= max_threads && threads % 32 == 0) ? threads : max_threads, 1, 1);
   cfg.dynamicSmemBytes = Geo<CTA2>::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
   if (CTA2) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = 2; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (p.W <= 1) {
+    // a local product is set up while its predecessor in the stream drains (see host::launch_overlapped)
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
   }
   return cudaLaunchKernelEx(&cfg, fused_gemm_kernel<KIND, CTA2, EPI, Params>, p);
 }

@@ -11,6 +11,7 @@
 #include "catcoc/capi.h"
 #include "catcoc/host_util.h"
 #include "catcoc/params.h"
+#include "catcoc/ptx.cuh"
 
 using namespace catcoc;
 
@@ -62,6 +63,7 @@ constexpr int kPadChunks = 4;   // chunks per thread: eight independent loads in
 __global__ void pad2d_kernel(uint8_t* dst, int64_t dst_pitch, const uint8_t* src, int64_t src_pitch, int64_t rows,
                              int64_t row_bytes) {
   const uint32_t cpr = static_cast<uint32_t>(dst_pitch >> 4);
+  ptx::grid_dependency_wait();
   const int64_t total = rows * cpr;
   const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x * kPadChunks;
   for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x * kPadChunks + threadIdx.x; base < total; base += step) {
@@ -283,9 +285,8 @@ extern "C" int catcoc_pad2d(void* dst, int64_t dst_pitch, const void* src, int64
   const int64_t chunks = rows * (dst_pitch >> 4);
   int64_t blocks = (chunks + 256 * kPadChunks - 1) / (256 * kPadChunks);
   if (blocks > 148 * 32) blocks = 148 * 32;
-  pad2d_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint8_t*>(dst), dst_pitch, static_cast<const uint8_t*>(src), src_pitch, rows, row_bytes);
-  CATCOC_CUDA_OK(cudaGetLastError());
+  CATCOC_CUDA_OK(host::launch_overlapped(pad2d_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                         static_cast<uint8_t*>(dst), dst_pitch, static_cast<const uint8_t*>(src), src_pitch, rows, row_bytes));
   return CATCOC_OK;
 }
 

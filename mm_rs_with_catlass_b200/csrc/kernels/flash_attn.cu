@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   __syncthreads();
   ptx::tcgen05_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  ptx::grid_dependency_wait();
 
   if (warp >= kProducerWarp) ptx::reg_dec<kOtherRegs>();   // all four warps of the warpgroup at one place
   if (warp == kProducerWarp) {
@@ -357,7 +358,8 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
     // (one attribute call per launch: it is cheap and keeps the four instantiations in one place)
     cudaError_t a = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (a != cudaSuccess) { set_error("cudaFuncSetAttribute failed: %s", cudaGetErrorString(a)); return -1000 - static_cast<int>(a); }
-    kernel<<<grid, attn::kThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
+    a = launch_overlapped(kernel, grid, dim3(attn::kThreads), smem, static_cast<cudaStream_t>(stream), p);
+    if (a != cudaSuccess) { set_error("flash_attention launch failed: %s", cudaGetErrorString(a)); return -1000 - static_cast<int>(a); }
     return 0;
   };
   int lrc;

@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_decode_kernel(const __grid_
   __syncthreads();
   ptx::tcgen05_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  ptx::grid_dependency_wait();
   ptx::launch_dependents();                      // the combine kernel waits for this grid's results by itself
 
   if (warp == kProducerWarp) {
@@ -450,21 +451,10 @@ extern "C" int catcoc_flash_decode(const void* q, const void* k, const void* v, 
   const size_t smem = static_cast<size_t>(2 + slots) * db * decode::kBlockBytes + sizeof(decode::Bars) + 1024;
   auto launch = [&](auto main_kernel, auto combine_kernel) -> int {
     CATCOC_CUDA_OK(cudaFuncSetAttribute(main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    main_kernel<<<d.ctas, decode::kThreads, smem, stream>>>(p);
-    CATCOC_CUDA_OK(cudaGetLastError());
+    CATCOC_CUDA_OK(launch_overlapped(main_kernel, dim3(static_cast<unsigned>(d.ctas)), dim3(decode::kThreads), smem, stream, p));
     if (!d.cut) return CATCOC_OK;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(static_cast<unsigned>(bh), static_cast<unsigned>((d.rows + 3) / 4), 1);
-    cfg.blockDim = dim3(128, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CATCOC_CUDA_OK(cudaLaunchKernelEx(&cfg, combine_kernel, static_cast<const float*>(p.part_o), static_cast<const float*>(p.part_ml),
-                                      out, p.rows, p.nb, p.per));
+    const dim3 grid(static_cast<unsigned>(bh), static_cast<unsigned>((d.rows + 3) / 4), 1);
+    CATCOC_CUDA_OK(launch_overlapped(combine_kernel, grid, dim3(128), 0, stream, p.part_o, p.part_ml, out, p.rows, p.nb, p.per));
     return CATCOC_OK;
   };
   if (D == 128) {

@@ -1030,21 +1030,6 @@ bool fold_fits(const CatcocOpArgs& a, bool is_int) {
   return true;
 }
 
-template <class... Args>
-cudaError_t launch_dependent(dim3 grid, cudaStream_t stream, void (*kernel)(Args...), Args... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 int splitk_rows(int M) { return round_up(M, 32); }    // whole 32-row windows leave the first launch by TMA
 int splitk_pitch(int N) { return round_up(N, 4); }
 }  // namespace
@@ -1088,7 +1073,7 @@ extern "C" int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_
   f.slices = slices; f.pitch = pitch;
   const int64_t units = static_cast<int64_t>(a.M) * ((a.N + 3) / 4);
   const dim3 fold_grid(static_cast<unsigned>(units > 148 * 8 * 256 ? 148 * 8 : (units + 255) / 256));
-  CATCOC_CUDA_OK(launch_dependent(fold_grid, stream, is_int ? splitk_fold_kernel<true> : splitk_fold_kernel<false>, f));
+  CATCOC_CUDA_OK(launch_overlapped(is_int ? splitk_fold_kernel<true> : splitk_fold_kernel<false>, fold_grid, dim3(256), 0, stream, f));
   return CATCOC_OK;
 }
 
@@ -1141,6 +1126,6 @@ extern "C" int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slice
   f.plane = static_cast<int64_t>(p.sched.BM) * p.sched.BN;
   f.slices = slices; f.pitch = p.sched.BN;
   const dim3 fold_grid(static_cast<unsigned>(p.sched.BM * p.sched.BN / 4 / 256), static_cast<unsigned>(tiles));
-  CATCOC_CUDA_OK(launch_dependent(fold_grid, stream, is_int ? tail_fold_kernel<true> : tail_fold_kernel<false>, f, p.sched, first));
+  CATCOC_CUDA_OK(launch_overlapped(is_int ? tail_fold_kernel<true> : tail_fold_kernel<false>, fold_grid, dim3(256), 0, stream, f, p.sched, first));
   return CATCOC_OK;
 }

@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1) mla_rows_kernel(const __grid_cons
   __syncthreads();
   ptx::tcgen05_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  ptx::grid_dependency_wait();
   ptx::launch_dependents();                         // the combine kernel waits for this grid's results by itself
   const Run run(p, lane);
 
@@ -616,20 +617,10 @@ extern "C" int catcoc_mla_rows(const void* q_nope, const void* q_rope, const voi
   auto launch = [&](auto main_kernel, auto combine_kernel, int tail) -> int {
     const int smem = tail + static_cast<int>(sizeof(mlar::Bars)) + 1024;
     CATCOC_CUDA_OK(cudaFuncSetAttribute(main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    main_kernel<<<dim3(static_cast<unsigned>(d.runs), static_cast<unsigned>(d.chunks)), mlar::kThreads, smem, stream>>>(p);
-    CATCOC_CUDA_OK(cudaGetLastError());
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(static_cast<unsigned>(rows_per_item), static_cast<unsigned>(B), 1);
-    cfg.blockDim = dim3(128, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CATCOC_CUDA_OK(cudaLaunchKernelEx(&cfg, combine_kernel, static_cast<const float*>(p.part_o), static_cast<const float*>(p.part_ml),
-                                      out, kv_lens, B, max_pages, rows_per_item, d.chunks, d.n, d.runs));
+    CATCOC_CUDA_OK(launch_overlapped(main_kernel, dim3(static_cast<unsigned>(d.runs), static_cast<unsigned>(d.chunks)), dim3(mlar::kThreads),
+                                     smem, stream, p));
+    CATCOC_CUDA_OK(launch_overlapped(combine_kernel, dim3(static_cast<unsigned>(rows_per_item), static_cast<unsigned>(B)), dim3(128), 0,
+                                     stream, p.part_o, p.part_ml, out, kv_lens, B, max_pages, rows_per_item, d.chunks, d.n, d.runs));
     return CATCOC_OK;
   };
   const bool bf = fmt == CATCOC_FMT_BF16;

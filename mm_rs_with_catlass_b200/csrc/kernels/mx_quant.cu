@@ -73,6 +73,7 @@ template <int FMT, bool E5M2>
 __global__ void __launch_bounds__(256) mx_quantize_kernel(const void* __restrict__ x, uint8_t* __restrict__ q,
                                                           uint8_t* __restrict__ scales, int64_t chunks) {
   const int64_t base = static_cast<int64_t>(blockIdx.x) * (blockDim.x * kQuantChunks) + threadIdx.x;
+  ptx::grid_dependency_wait();
   float f[kQuantChunks][8];
 #pragma unroll
   for (int j = 0; j < kQuantChunks; ++j) {
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(256) mx_quantize_kernel(const void* __restrict
 __global__ void __launch_bounds__(256) mx_pack_kernel(const uint8_t* __restrict__ scales, int rows, int kb,
                                                       uint32_t* __restrict__ out, int row_tiles, int k_tiles) {
   const int kt_groups = (k_tiles + 7) / 8;
+  ptx::grid_dependency_wait();
   const int64_t total = static_cast<int64_t>(row_tiles) * kt_groups * 1024;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -164,13 +166,15 @@ extern "C" int catcoc_mx_quantize(const void* x, int fmt, int64_t elems, int e5m
   const int64_t blocks = (chunks + per_block - 1) / per_block;
   if (blocks > 0x7fffffff) { host::set_error("mx_quantize: too many elements"); return CATCOC_E_TOO_LARGE; }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaSuccess;
   auto launch = [&](auto kernel) {
-    kernel<<<static_cast<int>(blocks), 256, 0, st>>>(x, static_cast<uint8_t*>(q), static_cast<uint8_t*>(scales), chunks);
+    e = host::launch_overlapped(kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, x, static_cast<uint8_t*>(q),
+                                static_cast<uint8_t*>(scales), chunks);
   };
   if (fmt == CATCOC_FMT_BF16) e5m2 ? launch(mx_quantize_kernel<FMT_BF16, true>) : launch(mx_quantize_kernel<FMT_BF16, false>);
   else if (fmt == CATCOC_FMT_F16) e5m2 ? launch(mx_quantize_kernel<FMT_F16, true>) : launch(mx_quantize_kernel<FMT_F16, false>);
   else e5m2 ? launch(mx_quantize_kernel<FMT_F32, true>) : launch(mx_quantize_kernel<FMT_F32, false>);
-  CATCOC_CUDA_OK(cudaGetLastError());
+  CATCOC_CUDA_OK(e);
   return CATCOC_OK;
 }
 
@@ -183,8 +187,7 @@ extern "C" int catcoc_mx_pack_scales(const void* scales, int rows, int kb, void*
   const int rt = (rows + 127) / 128, kt = (kb + 3) / 4;
   int64_t blocks = static_cast<int64_t>(rt) * ((kt + 7) / 8) * 4;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  mx_pack_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint8_t*>(scales), rows, kb, static_cast<uint32_t*>(out), rt, kt);
-  CATCOC_CUDA_OK(cudaGetLastError());
+  CATCOC_CUDA_OK(host::launch_overlapped(mx_pack_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                         static_cast<const uint8_t*>(scales), rows, kb, static_cast<uint32_t*>(out), rt, kt));
   return CATCOC_OK;
 }
