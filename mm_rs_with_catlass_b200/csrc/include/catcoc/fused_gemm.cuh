@@ -1357,6 +1357,8 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
         b_k_off = ti.seg * p.g_b_k;
       }
       const CUtensorMap* tmb = &p.tm_b;
+      bool b_3d = p.b_3d != 0;
+      if (p.b_3d == 2 && b_col + b_cols_cta > sched.N * p.elt_bytes_a / 128 * (128 / p.elt_bytes_a)) { b_3d = false; tmb = &p.tm_a_gath[1]; }
       int tile_k = p.K;
       if constexpr (kGk) {
         const int2 r = p.gk_range[ti.seg];
@@ -1404,7 +1406,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
             if (!CTA2) {
               if (!p.b_mn_major) {
                 ptx::tma_load_2d(sb, tmb, &tail->full[stage], k0, b_col);
-              } else if (p.b_3d) {
+              } else if (b_3d) {
                 ptx::tma_load_3d(sb, tmb, &tail->full[stage], 0, k0, b_col / per_box);
               } else {
                 for (int b = 0; b < b_cols_cta / per_box; ++b)
@@ -1413,7 +1415,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
             } else {
               if (!p.b_mn_major) {
                 ptx::tma_load_2d_pair(sb, tmb, bar, k0, b_col);
-              } else if (p.b_3d) {
+              } else if (b_3d) {
                 ptx::tma_load_3d_pair(sb, tmb, bar, 0, k0, b_col / per_box);
               } else {
                 for (int b = 0; b < b_cols_cta / per_box; ++b)

@@ -99,7 +99,9 @@ struct alignas(64) FusedParams {
   // operand staging: K elements per pipeline stage and per MMA instruction; smem majors
   int bk, umma_k;
   int a_mn_major, b_mn_major;
-  int a_3d, b_3d;   // M/N-contiguous operand fetched through a 3-D map {128 B, K, blocks}: one TMA per stage
+  int a_3d, b_3d;   // M/N-contiguous operand fetched through a 3-D map {128 B, K, blocks}: one TMA per stage. b_3d == 2: the
+                    // last, ragged column block is not in the 3-D map (its rows' ends may lie outside the operand); tiles that
+                    // touch it take 2-D boxes through tm_a_gath[1], which a local product has no other use for
   uint32_t idesc;
 
   // output (MODE_LOCAL / MODE_AG / RS own tiles): row-major [rows, ldc]

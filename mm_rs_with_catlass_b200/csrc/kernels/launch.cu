@@ -515,6 +515,11 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   } else if (b_n % per128 == 0 && b_blocks_ok) {
     rc = encode_3d_blocks(&p->tm_b, a.b, rf.elt, rf.dt, b_k, b_n, a.ldb, rf.bk, (pair ? bn / 2 : bn) / per128);
     p->b_3d = 1;
+  } else if (!fused && !mx && b_n > per128 && b_blocks_ok) {
+    // a ragged N in whole blocks but for the last column of tiles (8144 x 1696 x 5120 stored [K, N]: 161 -> 118 us)
+    rc = encode_3d_blocks(&p->tm_b, a.b, rf.elt, rf.dt, b_k, b_n / per128 * per128, a.ldb, rf.bk, (pair ? bn / 2 : bn) / per128);
+    if (rc == 0) rc = encode_2d(&p->tm_a_gath[1], a.b, rf.elt, rf.dt, b_k, b_n, a.ldb, per128, rf.bk);
+    p->b_3d = 2;
   } else {
     rc = encode_2d(&p->tm_b, a.b, rf.elt, rf.dt, b_k, b_n, a.ldb, per128, rf.bk);
   }
@@ -880,6 +885,7 @@ extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_
     rc = catcoc_build_params(&a, &p, &kind, &grid, &pair);
     if (rc != 0) return rc;
     const int b_cols = pair ? p.sched.BN / 2 : p.sched.BN;
+    if (p.b_3d == 2) p.b_3d = 0;                          // one map per group and operand
     for (int i = 0; i < a.num_groups; ++i) {
       const int begin = k_range[2 * (g0 + i)], end = k_range[2 * (g0 + i) + 1];
       p.gk_range[i] = make_int2(begin, end);
