@@ -14,7 +14,7 @@
 // Bound by the chain of one tile, scores -> maximum -> exponentials -> P V -> next scores (the tensor core is busy
 // 56 % of the time, the special-function unit as much). So the scores are read from TMEM once and stay in registers
 // (softmax_row.cuh; a split of the registers between the warpgroups makes room), and P V starts when the first 64
-// keys' probabilities are written. Causal, 2 x 32 / 8 heads x 8192, D = 128: 1118 -> 963 us (1.14 PFLOP/s), not
+// keys' probabilities are written. Causal, 2 x 32 / 8 heads x 8192, D = 128: 1118 -> 963 us (912 us, 1.21 PFLOP/s, in the CTA order below), not
 // causal 1922 -> 1690 us; without the early half 981 us.
 //
 // The online-softmax recurrence (m: reference maximum, l: running sum, per row, in the log2 domain):
@@ -28,6 +28,7 @@
 //   3rdparty/catlass/include/catlass/epilogue/block/block_epilogue_fa_softmax.hpp, ..._fa_rescale_o.hpp
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <algorithm>
 #include <cstring>
 #include "catcoc/attn_host.h"
 #include "catcoc/capi.h"
@@ -53,8 +54,10 @@ constexpr int kMaxSlots = 8;
 struct AttnParams {
   CUtensorMap tm_q, tm_k, tm_v;   // {D, S, B * H} with a {64, 128, 1} box, 128-byte swizzle
   void* out;                      // [B, Hq, Sq, D]
-  int B, Hq, Hk, Sq, Sk, D;
-  int causal;                     // key j is visible to query i when j <= i + (Sk - Sq)
+  int B, Hq, Hk, Sq, Sk, D;       // Sq: rows per (batch, query head), or per (batch, KV head) when its heads are packed
+  int pos;                        // query positions: row r stands at r % pos
+  int causal;                     // key j is visible to position i when j <= i + (Sk - pos)
+  int tiles, order_heads;         // CTAs per head; heads that are walked side by side (see the CTA order below)
   float scale_log2;               // softmax scale * log2(e), > 0
   int fmt;                        // FMT_F16 or FMT_BF16
   uint32_t idesc_qk, idesc_pv;
@@ -92,19 +95,28 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // late (long) causal tiles first
+  // CTA order: blocks of `order_heads` heads; inside a block the last (longest, when causal) tiles of all heads first, so
+  // that the launch ends with the shortest ones
+  const int per_block = p.order_heads * p.tiles;
+  const int blk = static_cast<int>(blockIdx.x) / per_block, in_blk = static_cast<int>(blockIdx.x) - blk * per_block;
+  const int heads = min(p.order_heads, p.B * p.Hq - blk * p.order_heads);
+  const int qt = p.tiles - 1 - in_blk / heads;
   const int q0 = qt * (kTiles * kBQ);
-  const int bh = blockIdx.y;                       // b * Hq + h
+  const int bh = blk * p.order_heads + in_blk % heads;   // b * Hq + h
   const int b = bh / p.Hq, h = bh - b * p.Hq;
   const int bhk = b * p.Hk + h / (p.Hq / p.Hk);    // grouped-query attention: several query heads share one KV head
-  const int shift = p.Sk - p.Sq;                   // causal diagonal offset
+  const int shift = p.Sk - p.pos;                  // causal diagonal offset
+  // positions of a tile's rows: [lo, hi], the whole range when the rows of two packed heads meet in it
+  auto tile_lo = [&](int t) { const int r = (q0 + t * kBQ) % p.pos; return r + kBQ > p.pos && p.pos < p.Sq ? 0 : r; };
+  auto tile_hi = [&](int t) { const int r = (q0 + t * kBQ) % p.pos; return r + kBQ > p.pos && p.pos < p.Sq ? p.pos - 1 : r + kBQ - 1; };
   // key blocks each tile walks (tile 1 never fewer than tile 0; rows past Sq are computed and not stored)
   int nblk[kTiles];
 #pragma unroll
   for (int t = 0; t < kTiles; ++t) {
-    const int kv_end = p.causal ? min(p.Sk, q0 + (t + 1) * kBQ + shift) : p.Sk;
+    const int kv_end = p.causal ? min(p.Sk, tile_hi(t) + 1 + shift) : p.Sk;
     nblk[t] = (kv_end + kBKV - 1) / kBKV;
   }
+  nblk[1] = max(nblk[0], nblk[1]);
   const int nmax = nblk[1];
 
   if (threadIdx.x == 0) {
@@ -257,8 +269,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     const uint32_t t_s = tmem + (static_cast<uint32_t>(qd * 32) << 16) + t * 128;   // scores, and P on top of them
     const uint32_t t_o = tmem + (static_cast<uint32_t>(qd * 32) << 16) + kOCol + t * D;
     const int n_mine = nblk[t];
-    const int vis = p.causal ? min(p.Sk, qi + shift + 1) : p.Sk;            // keys [0, vis) are visible to this row
-    const int vis_tile = p.causal ? min(p.Sk, q0 + t * kBQ + shift + 1) : p.Sk;   // ... to every row of the tile
+    const int vis = p.causal ? min(p.Sk, qi % p.pos + shift + 1) : p.Sk;    // keys [0, vis) are visible to this row
+    const int vis_tile = p.causal ? min(p.Sk, tile_lo(t) + shift + 1) : p.Sk;   // ... to every row of the tile
     const float sc = p.scale_log2;
     RowState st;
     bool ok = true;
@@ -331,6 +343,21 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
   if (fmt != CATCOC_FMT_F16 && fmt != CATCOC_FMT_BF16) { set_error("flash_attention takes fp16 / bf16"); return CATCOC_E_UNSUPPORTED; }
   if (causal && Sk < Sq) { set_error("causal attention needs Sk >= Sq"); return CATCOC_E_BAD_ARG; }
   if (!(scale > 0.0f)) { set_error("flash_attention: the softmax scale must be positive (the row maximum is taken before scaling)"); return CATCOC_E_UNSUPPORTED; }
+  // A call of few query positions: the query heads of a KV head are contiguous rows, so they can fill tiles together. It
+  // costs the keys that a head's early tiles would have skipped; in units of (CTA, 128-key block), a launch takes its
+  // total over the SMs or its longest CTA. 16 x 32 / 4 heads x 100 positions over 2000 keys: 154 -> 71 us,
+  // 16 x 32 / 8 x 64 over 1000 (D = 64): 78 -> 20 us.
+  const int group = Hq / Hk, rows_cta = attn::kTiles * attn::kBQ;
+  const int pos = Sq;
+  if (group > 1 && static_cast<int64_t>(group) * Sq <= (1 << 24)) {
+    auto blocks = [&](int hi) { return static_cast<double>((causal ? std::min<int64_t>(Sk, static_cast<int64_t>(hi) + Sk - pos) : Sk) + 127) / 128; };
+    double plain = 0.0;
+    const int plain_tiles = (Sq + rows_cta - 1) / rows_cta, packed_tiles = (group * Sq + rows_cta - 1) / rows_cta;
+    for (int i = 0; i < plain_tiles; ++i) plain += blocks(std::min((i + 1) * rows_cta, pos));
+    const double longest = blocks(pos), heads = static_cast<double>(B) * Hk;
+    const double t_plain = std::max(longest, heads * group * plain / 148.0), t_packed = std::max(longest, heads * packed_tiles * longest / 148.0);
+    if (t_packed < 0.95 * t_plain) { Sq = group * Sq; Hq = Hk; }
+  }
   attn::AttnParams p;
   memset(&p, 0, sizeof(p));
   const CUtensorMapDataType dt = fmt == CATCOC_FMT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -339,7 +366,14 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
   if (rc == 0) rc = encode_bsd(&p.tm_v, v, dt, static_cast<int64_t>(B) * Hk, Sk, D);
   if (rc != 0) return rc;
   p.out = out;
-  p.B = B; p.Hq = Hq; p.Hk = Hk; p.Sq = Sq; p.Sk = Sk; p.D = D;
+  p.B = B; p.Hq = Hq; p.Hk = Hk; p.Sq = Sq; p.Sk = Sk; p.D = D; p.pos = pos;
+  const int64_t ctas = static_cast<int64_t>(B) * Hq * ((Sq + rows_cta - 1) / rows_cta);
+  if (ctas > 0x7fffffff) { set_error("flash_attention: too many query tiles"); return CATCOC_E_TOO_LARGE; }
+  p.tiles = (Sq + rows_cta - 1) / rows_cta;
+  // Causal tiles differ in length, and with one head after the other the launch ended with the long tiles of its last
+  // heads (causal 2 x 32 x 8192: 952 -> 912 us in this order, 1 x 32 x 4096: 180 -> 151 us). Heads side by side share the L2, so their keys and values must fit it.
+  const int64_t kv_bytes = static_cast<int64_t>(Sk) * D * 4;
+  p.order_heads = causal ? static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(static_cast<int64_t>(B) * Hq, (72ll << 20) / kv_bytes * (Hq / Hk)))) : 1;
   p.causal = causal ? 1 : 0;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.fmt = fmt;
@@ -348,8 +382,7 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
   p.idesc_pv = ptx::make_instr_desc(1u, f, f, 0u, 1u, 128u, static_cast<uint32_t>(D));
   p.status = status;
   p.timeout_ns = timeout_ns ? timeout_ns : 10000000000ull;
-  const int rows = attn::kTiles * attn::kBQ;
-  const dim3 grid((Sq + rows - 1) / rows, B * Hq, 1);
+  const dim3 grid(static_cast<unsigned>(ctas));
   const int db = D / 64;
   const int slots = D == 128 ? 4 : 8;
   const size_t smem = static_cast<size_t>(attn::kTiles * db + slots * db) * attn::kBlockBytes + sizeof(attn::Bars) + 1024 + 64;
