@@ -43,19 +43,21 @@ CATCOC_DEVICE void rescale_o(uint32_t t_o, float alpha) {
   }
 }
 
-// Reads 128 scores at TMEM address `t_s`, writes the packed probabilities over them (64 columns) and updates the
-// state. `rescale(alpha)` is called before the first probability when the reference maximum of some row of the warp
-// moved (all lanes together): O has to be multiplied by alpha. `half()` is called when the probabilities of the first
-// 64 keys have been issued. `vis_left`: keys of this block the row sees (used when `masked`).
+// Reads 128 scores at TMEM address `t_s`, writes the packed probabilities (64 columns) to `t_p`, which may be the same
+// place, and updates the state. `loaded()` is called when the scores are in registers, `before(move, alpha)` ahead of the
+// first probability: with `move` (the same in all lanes) the reference maximum of some row of the warp moved and O has to
+// be multiplied by alpha. `half()` is called when the probabilities of the first 64 keys have been issued. `vis_left`: keys of this block the row sees (used when `masked`).
 //
 // A quarter of the exponentials as a degree-5 polynomial on the FMA pipe was measured slower (causal 2 x 32 x 8192:
 // 1019 against 980 us): a chain of one row's steps, not the special-function unit, is what a tile waits for.
-template <int FMT, class Rescale, class Half>
-CATCOC_DEVICE void softmax_row_block(uint32_t t_s, bool masked, int vis_left, float sc, RowState& st, Rescale&& rescale, Half&& half) {
+template <int FMT, class Loaded, class Before, class Half>
+CATCOC_DEVICE void softmax_row_block(uint32_t t_s, uint32_t t_p, bool masked, int vis_left, float sc, RowState& st, Loaded&& loaded,
+                                     Before&& before, Half&& half) {
   uint32_t v[4][32];
 #pragma unroll
   for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32b_x32(t_s + c * 32, v[c]);
   ptx::tcgen05_wait_ld();
+  loaded();
   if (masked) {
 #pragma unroll
     for (int c = 0; c < 4; ++c)
@@ -75,7 +77,7 @@ CATCOC_DEVICE void softmax_row_block(uint32_t t_s, bool masked, int vis_left, fl
   const float m_use = move ? m_new : st.m;
   const float m_safe = (m_use == -INFINITY) ? 0.0f : m_use;      // a row that sees nothing yet
   const float alpha = !move ? 1.0f : ((st.m == -INFINITY) ? 0.0f : ptx::ex2_approx(st.m - m_safe));
-  if (move) rescale(alpha);
+  before(move, alpha);
   const uint64_t sc2 = ptx::pack_f32x2(sc, sc), nm2 = ptx::pack_f32x2(-m_safe, -m_safe);
   uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
@@ -91,7 +93,7 @@ CATCOC_DEVICE void softmax_row_block(uint32_t t_s, bool masked, int vis_left, fl
       sum2[i & 1] = ptx::add_f32x2(sum2[i & 1], ptx::pack_f32x2(e0, e1));
       w[i] = pack16<FMT>(e0, e1);
     }
-    ptx::tmem_st_32x32b_x32(t_s + h * 32, w);
+    ptx::tmem_st_32x32b_x32(t_p + h * 32, w);
     if (h == 0) half();
   }
   float s0, s1;

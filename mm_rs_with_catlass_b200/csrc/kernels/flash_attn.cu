@@ -14,8 +14,9 @@
 // Bound by the chain of one tile, scores -> maximum -> exponentials -> P V -> next scores (the tensor core is busy
 // 56 % of the time, the special-function unit as much). So the scores are read from TMEM once and stay in registers
 // (softmax_row.cuh; a split of the registers between the warpgroups makes room), and P V starts when the first 64
-// keys' probabilities are written. Causal, 2 x 32 / 8 heads x 8192, D = 128: 1118 -> 963 us (912 us, 1.21 PFLOP/s, in the CTA order below), not
-// causal 1922 -> 1690 us; without the early half 981 us.
+// keys' probabilities are written. Causal, 2 x 32 / 8 heads x 8192, D = 128: 1118 -> 963 us (912 us, 1.21 PFLOP/s, in the
+// CTA order below), not causal 1922 -> 1690 us; without the early half 981 us. At D = 64 the probabilities have columns of their own
+// (O_0, O_1 at 256 and 320, P_0, P_1 at 384 and 448), which takes P V out of the chain: 771 -> 705 us.
 //
 // The online-softmax recurrence (m: reference maximum, l: running sum, per row, in the log2 domain):
 //   P = exp2(scale S - m),  l' = l a + rowsum(P),  O' = O a + P V,  a = exp2(m - m')
@@ -66,7 +67,7 @@ struct AttnParams {
 };
 
 struct Bars {
-  uint64_t q_full, kv_full[kMaxSlots], kv_empty[kMaxSlots], s_full[kTiles], p_half[kTiles], p_full[kTiles], o_done[kTiles];
+  uint64_t q_full, kv_full[kMaxSlots], kv_empty[kMaxSlots], s_full[kTiles], s_free[kTiles], p_half[kTiles], p_full[kTiles], pv_done[kTiles], o_done[kTiles];
   uint32_t tmem_base, abort_flag;
 };
 
@@ -87,6 +88,11 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   constexpr int kSlots = D == 128 ? 4 : 8;       // ring of K / V blocks (K_0 V_0 K_1 V_1 ...)
   constexpr uint32_t kTmemCols = 512;
   constexpr uint32_t kOCol = 256;
+  // D = 64 leaves 128 columns of TMEM: the probabilities get columns of their own, and the next scores are computed as soon
+  // as the softmax has read the present ones instead of behind the second product
+  constexpr bool kOwnP = D == 64;
+  constexpr uint32_t kPCol = kOwnP ? 384 : 0;      // P_t at kPCol + t * kPStride
+  constexpr uint32_t kPStride = kOwnP ? 64 : 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sq = smem;                            // two Q tiles
@@ -124,6 +130,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     for (int s = 0; s < kSlots; ++s) { ptx::mbar_init(&bars->kv_full[s], 1); ptx::mbar_init(&bars->kv_empty[s], 1); }
     for (int t = 0; t < kTiles; ++t) {
       ptx::mbar_init(&bars->s_full[t], 1);
+      ptx::mbar_init(&bars->s_free[t], 4);
+      ptx::mbar_init(&bars->pv_done[t], 1);
       ptx::mbar_init(&bars->p_half[t], 4);         // one arrival per softmax warp: P of the first 64 keys is in TMEM
       ptx::mbar_init(&bars->p_full[t], 4);         // ... of all of them
       ptx::mbar_init(&bars->o_done[t], 1);
@@ -191,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       for (int k2 = 0; k2 < kBKV / 32; ++k2) {
         const int kk = half * (kBKV / 32) + k2;
         const uint64_t offb = static_cast<uint64_t>((kk * 16 * 128) >> 4);
-        ptx::umma_f16_ts(tmem + kOCol + t * D, tmem + t * 128 + kk * 8, dv + offb, p.idesc_pv, (accumulate || kk != 0) ? 1u : 0u);
+        ptx::umma_f16_ts(tmem + kOCol + t * D, tmem + kPCol + t * kPStride + kk * 8, dv + offb, p.idesc_pv, (accumulate || kk != 0) ? 1u : 0u);
       }
     };
     bool ok = ptx::mbar_wait(&bars->q_full, 0u, p.timeout_ns, abort_flag);
@@ -205,7 +213,44 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       }
       __syncwarp();
     }
-    for (int j = 0; ok && j < nmax; ++j) {
+    for (int j = 0; kOwnP && ok && j < nmax; ++j) {
+      const int v_item = 2 * j + 1, k_next = 2 * j + 2;
+      if (j + 1 < nmax) {
+        ok = wait_item(k_next);
+#pragma unroll
+        for (int t = 0; t < kTiles; ++t) {
+          if (!ok || j + 1 >= nblk[t]) continue;
+          ok = ptx::mbar_wait(&bars->s_free[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
+          if (!ok) break;
+          ptx::tcgen05_fence_after();
+          if (ptx::elect_one()) {
+            issue_qk(t, k_next);
+            if (t == 1) ptx::tcgen05_commit(&bars->kv_empty[k_next % kSlots]);
+          }
+          __syncwarp();
+        }
+      }
+      ok = ok && wait_item(v_item);
+#pragma unroll
+      for (int t = 0; t < kTiles; ++t) {
+        if (!ok || j >= nblk[t]) continue;
+        ok = ptx::mbar_wait(&bars->p_half[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
+        if (!ok) break;
+        ptx::tcgen05_fence_after();
+        if (ptx::elect_one()) issue_pv(t, v_item, 0, j > 0);
+        __syncwarp();
+        ok = ptx::mbar_wait(&bars->p_full[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
+        if (!ok) break;
+        ptx::tcgen05_fence_after();
+        if (ptx::elect_one()) {
+          issue_pv(t, v_item, 1, true);
+          if (t == 1) ptx::tcgen05_commit(&bars->kv_empty[v_item % kSlots]);
+          ptx::tcgen05_commit(j + 1 < nblk[t] ? &bars->pv_done[t] : &bars->o_done[t]);
+        }
+        __syncwarp();
+      }
+    }
+    for (int j = 0; !kOwnP && ok && j < nmax; ++j) {
       const int v_item = 2 * j + 1, k_next = 2 * j + 2;
       const bool next0 = j + 1 < nblk[0], next1 = j + 1 < nblk[1];
       bool v_here = false;
@@ -267,6 +312,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     const int row = qd * 32 + lane;                  // query row inside the tile
     const int qi = q0 + t * kBQ + row;
     const uint32_t t_s = tmem + (static_cast<uint32_t>(qd * 32) << 16) + t * 128;   // scores, and P on top of them
+    const uint32_t t_p = kOwnP ? tmem + (static_cast<uint32_t>(qd * 32) << 16) + kPCol + t * kPStride : t_s;
     const uint32_t t_o = tmem + (static_cast<uint32_t>(qd * 32) << 16) + kOCol + t * D;
     const int n_mine = nblk[t];
     const int vis = p.causal ? min(p.Sk, qi % p.pos + shift + 1) : p.Sk;    // keys [0, vis) are visible to this row
@@ -279,15 +325,30 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       ptx::tcgen05_fence_after();
       const int key0 = j * kBKV;
       // masked: some row of the tile does not see all of the block
-      softmax_row_block<FMT>(t_s, key0 + kBKV > vis_tile, vis - key0, sc, st, [&](float alpha) {
-        // s_full(j) was committed behind P V of block j - 1, so O is whole
-        if (j > 0) rescale_o<D>(t_o, alpha);
+      softmax_row_block<FMT>(t_s, t_p, key0 + kBKV > vis_tile, vis - key0, sc, st, [&] {
+        if constexpr (kOwnP) {
+          ptx::tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->s_free[t]);
+        }
+      }, [&](bool move, float alpha) {
+        if constexpr (kOwnP) {
+          // P V of block j - 1 has read P, and O is whole
+          if (j > 0 && !ptx::mbar_wait(&bars->pv_done[t], static_cast<uint32_t>(j - 1) & 1u, p.timeout_ns, abort_flag)) ok = false;
+          ptx::tcgen05_fence_after();
+        }
+        // (else s_full(j) was committed behind P V of block j - 1, so O is whole)
+        if (move && j > 0) rescale_o<D>(t_o, alpha);
       }, [&] {
         ptx::tcgen05_wait_st();
         ptx::tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->p_half[t]);
       });
+      if constexpr (kOwnP) {
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+      }
       ptx::tcgen05_wait_st();
       ptx::tcgen05_fence_before();
       __syncwarp();

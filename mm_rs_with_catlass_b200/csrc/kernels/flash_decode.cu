@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_decode_kernel(const __grid_
         if (!ptx::mbar_wait(&bars->s_full[t], static_cast<uint32_t>(i >> 1) & 1u, p.timeout_ns, abort_flag)) { ok = false; break; }
         ptx::tcgen05_fence_after();
         const int key0 = (blk0 + i - i0) * kBKV;
-        attn::softmax_row_block<FMT>(t_s, key0 + kBKV > vis_all, vis - key0, p.scale_log2, st, [&](float alpha) {
+        attn::softmax_row_block<FMT>(t_s, t_s, key0 + kBKV > vis_all, vis - key0, p.scale_log2, st, [] {}, [&](bool move, float alpha) {
           // s_full(i) was committed behind the second product of this parity's previous block, so O_t is whole
-          if (i > mine0) attn::rescale_o<D>(t_o, alpha);
+          if (move && i > mine0) attn::rescale_o<D>(t_o, alpha);
         }, [] {});
         ptx::tcgen05_wait_st();
         ptx::tcgen05_fence_before();
