@@ -96,20 +96,8 @@ def _group_tiling(tiling: Optional[TilingConfig], rows_total: int, rows_per_grou
                   dtype: torch.dtype) -> TilingConfig:
     if tiling is not None:
         return tiling
-    from ..tiling.chooser import heuristic
-    t = heuristic("matmul", rows_total, n, k, 1, dtype)
-    if t.cta_pair == 2:
-        # waves of 256- and of 128-row tiles, over the groups' own row tiles where their extent is known, else with half a
-        # tile of padding per group. A 256-row tile is 1.18 times as fast per row in a call by itself; back to back its
-        # padding costs power as well (32 ragged groups of 440 rows on average: 230 -> 210 us from a cold start, 273 ->
-        # 282 us in a loop; 937 rows: 429 -> 388 us).
-        exact = isinstance(rows_per_group, int)
-        groups, nt = rows_total / rows_per_group, math.ceil(n / t.effective_bn)
-        pair, single = (math.ceil(groups * (math.ceil(rows_per_group / bm) if exact else rows_per_group / bm + 0.5) * nt
-                                  / (_NUM_SMS * 128 // bm)) for bm in (256, 128))
-        if pair > (1.18 if exact else 1.10) * single:
-            t = t.with_(cta_pair=1)
-    return t
+    from ..tiling.chooser import grouped
+    return grouped(rows_total, rows_per_group, n, dtype)
 
 
 def _ends_tensor(group_list: GroupList, device: torch.device) -> torch.Tensor:

@@ -1,0 +1,23 @@
+"""The tile choice for launches over groups of rows: legal for every dtype and size, pairs only where the groups' padding
+allows them, narrower tiles where wide ones leave most SMs idle."""
+import pytest
+import torch
+
+from mm_rs_with_catlass_b200.tiling.chooser import grouped
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.int8])
+@pytest.mark.parametrize("groups", [1, 8, 64])
+def test_choice_is_legal(dtype, groups):
+    for rows in (1, 3, 100, 129, 256, 300, 2000):
+        for n in (8, 64, 200, 1408, 4096):
+            for per in (rows, rows + 0.5):
+                t = grouped(int(groups * per), per, n, dtype).validate()
+                assert t.cta_pair == 1 or (per > 64 and t.effective_bn >= 128)
+                assert dtype != torch.int8 or t.effective_bn // (2 if t.cta_pair == 2 else 1) >= 128
+
+
+def test_choice_follows_the_waves():
+    assert grouped(8 * 1024, 1024, 8192, torch.bfloat16).cta_pair == 2          # whole 256-row tiles
+    assert grouped(14080, 440.0, 4096, torch.bfloat16).cta_pair == 1            # half a tile of padding in each of 32 groups
+    assert grouped(148, 18.5, 1408, torch.bfloat16).effective_bn < 256          # 48 wide tiles for 148 SMs
