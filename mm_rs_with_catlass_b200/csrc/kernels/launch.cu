@@ -1037,7 +1037,7 @@ bool fold_fits(const CatcocOpArgs& a, bool is_int) {
 }
 
 int splitk_rows(int M) { return round_up(M, 32); }    // whole 32-row windows leave the first launch by TMA
-int splitk_pitch(int N) { return round_up(N, 4); }
+int splitk_pitch(int N) { return round_up(N, 8); }    // rows start on 32-byte sectors
 }  // namespace
 
 extern "C" int64_t catcoc_splitk_workspace_bytes(int M, int N, int slices) {

@@ -80,3 +80,26 @@ def test_epilogues(monkeypatch):
     for kw in (dict(), dict(bias=ib), dict(scale_m=s1, scale_n=s2, bias=ib), dict(scale_m=s1, scale_n=s2, out_dtype=torch.float16), dict(scale_n=s2)):
         direct, cut = _both(monkeypatch, (3, 1024, 256), x1, x2, trans_b=True, **kw)
         assert torch.equal(direct, cut)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 32, 33, 64, 65])                      # planes up to 64 rows leave from the registers
+@pytest.mark.parametrize("n", [32, 136, 1001, 1024])                    # whole and partial 32-column pieces, padded pitch
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.int8])
+def test_planes_of_few_rows(monkeypatch, m, n, dtype):
+    k = 2048
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    if dtype == torch.int8:
+        a = torch.randint(-127, 128, (m, k), device="cuda", generator=g, dtype=dtype)
+        b = torch.randint(-127, 128, (n, k), device="cuda", generator=g, dtype=dtype)
+        kw = dict(scale_m=torch.rand(m, device="cuda", generator=g), scale_n=torch.rand(n, device="cuda", generator=g))
+    else:
+        a, b = (torch.randn(r, k, device="cuda", generator=g).to(dtype) for r in (m, n))
+        kw = dict(out_dtype=torch.float32)
+    for cut in ((4, 512, 128), (8, 256, 256)):
+        direct, sliced = _both(monkeypatch, cut, a, b, trans_b=True, **kw)
+        if dtype == torch.int8:
+            assert torch.equal(direct, sliced)                          # the planes hold whole numbers
+        else:
+            # fp32 sums of exact products in another order: k * 2^-24 relative to the sum of magnitudes (about sqrt(k))
+            assert (direct - sliced).abs().max().item() < k * 2.0 ** -24 * 4 * k ** 0.5
