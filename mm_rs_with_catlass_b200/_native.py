@@ -160,6 +160,7 @@ def _declare(lib) -> None:
         "catcoc_shmem_mc_reduce_bf16": (i32, [P(ShmemCtx), vp, i64, i64, vp]),
         "catcoc_shmem_put_blocks": (i32, []),
         "catcoc_pad2d": (i32, [vp, i64, vp, i64, i64, i64, vp]),
+        "catcoc_pad2d_pair": (i32, [vp, i64, vp, i64, i64, i64] * 2 + [vp]),
         "catcoc_mx_quantize": (i32, [vp, i32, i64, i32, vp, vp, vp]),
         "catcoc_mx_pack_scales": (i32, [vp, i32, i32, vp, vp]),
         "catcoc_splitk_reduce": (i32, [vp, i32, i64, i32, i32, vp, i64, i32, C.c_float, C.c_float, vp, i64, vp, vp]),

@@ -260,6 +260,10 @@ int catcoc_shmem_put_blocks(void);  /* blocks a put launches: each adds signal_v
 /* copy rows into a buffer whose pitch is TMA-legal, zero-filling the padding */
 int catcoc_pad2d(void* dst, int64_t dst_pitch, const void* src, int64_t src_pitch, int64_t rows,
                  int64_t row_bytes, void* stream);
+/* Two such copies (both operands of one product) in one launch. */
+int catcoc_pad2d_pair(void* dst0, int64_t dst_pitch0, const void* src0, int64_t src_pitch0, int64_t rows0, int64_t row_bytes0,
+                      void* dst1, int64_t dst_pitch1, const void* src1, int64_t src_pitch1, int64_t rows1, int64_t row_bytes1,
+                      void* stream);
 
 /* block-scaled fp8 (csrc/kernels/mx_quant.cu): x (fp16 / bf16 / fp32, `elems` contiguous elements, whole blocks of 32)
  * -> q = fp8(x / 2^e), scales = e + 127 per block with e = ceil(log2(amax / fp8_max)), 0 for an all-zero block; and the

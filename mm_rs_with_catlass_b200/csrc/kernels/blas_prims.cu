@@ -60,8 +60,14 @@ __device__ __forceinline__ int unpack_word(const uint4& w, int fmt, float* f) {
 // accesses. Only words that hold at least one byte of the row are touched. Measured: 8192 x 28671 fp16 in 219 us
 // (4.29 TB/s), 28672 x 8191 in 219 us.
 constexpr int kPadChunks = 4;   // chunks per thread: eight independent loads in flight
-__global__ void pad2d_kernel(uint8_t* dst, int64_t dst_pitch, const uint8_t* src, int64_t src_pitch, int64_t rows,
-                             int64_t row_bytes) {
+struct PadJob { uint8_t* dst; int64_t dst_pitch; const uint8_t* src; int64_t src_pitch, rows, row_bytes; };
+struct PadJobs { PadJob job[2]; };   // one per grid row: both operands of a product in one launch
+
+__global__ void pad2d_kernel(const __grid_constant__ PadJobs jobs) {
+  const PadJob& pj = jobs.job[blockIdx.y];
+  uint8_t* const dst = pj.dst;
+  const uint8_t* const src = pj.src;
+  const int64_t dst_pitch = pj.dst_pitch, src_pitch = pj.src_pitch, rows = pj.rows, row_bytes = pj.row_bytes;
   const uint32_t cpr = static_cast<uint32_t>(dst_pitch >> 4);
   ptx::grid_dependency_wait();
   const int64_t total = rows * cpr;
@@ -271,23 +277,46 @@ bool float_fmt(int fmt) { return fmt == CATCOC_FMT_F16 || fmt == CATCOC_FMT_BF16
 
 }  // namespace
 
+static int pad_launch(const PadJobs& jobs, int count, void* stream) {
+  int64_t blocks = 1;
+  for (int i = 0; i < count; ++i) {
+    const PadJob& j = jobs.job[i];
+    if (j.dst == nullptr || j.src == nullptr || j.row_bytes <= 0 || j.dst_pitch < j.row_bytes) {
+      host::set_error("pad2d: bad argument");
+      return CATCOC_E_BAD_ARG;
+    }
+    if ((reinterpret_cast<uintptr_t>(j.dst) & 15) != 0 || (j.dst_pitch & 15) != 0) {
+      host::set_error("pad2d: the destination needs a 16-byte aligned base and pitch");
+      return CATCOC_E_ALIGNMENT;
+    }
+    const int64_t need = (j.rows * (j.dst_pitch >> 4) + 256 * kPadChunks - 1) / (256 * kPadChunks);
+    if (need > blocks) blocks = need;
+  }
+  if (blocks > 148 * 32) blocks = 148 * 32;
+  CATCOC_CUDA_OK(host::launch_overlapped(pad2d_kernel, dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(count)), dim3(256), 0,
+                                         static_cast<cudaStream_t>(stream), jobs));
+  return CATCOC_OK;
+}
+
 extern "C" int catcoc_pad2d(void* dst, int64_t dst_pitch, const void* src, int64_t src_pitch, int64_t rows,
                             int64_t row_bytes, void* stream) {
   if (rows <= 0) return CATCOC_OK;
-  if (dst == nullptr || src == nullptr || row_bytes <= 0 || dst_pitch < row_bytes) {
-    host::set_error("pad2d: bad argument");
+  PadJobs jobs = {};
+  jobs.job[0] = {static_cast<uint8_t*>(dst), dst_pitch, static_cast<const uint8_t*>(src), src_pitch, rows, row_bytes};
+  return pad_launch(jobs, 1, stream);
+}
+
+extern "C" int catcoc_pad2d_pair(void* dst0, int64_t dst_pitch0, const void* src0, int64_t src_pitch0, int64_t rows0, int64_t row_bytes0,
+                                 void* dst1, int64_t dst_pitch1, const void* src1, int64_t src_pitch1, int64_t rows1, int64_t row_bytes1,
+                                 void* stream) {
+  if (rows0 <= 0 || rows1 <= 0) {
+    host::set_error("pad2d_pair: an empty matrix");
     return CATCOC_E_BAD_ARG;
   }
-  if ((reinterpret_cast<uintptr_t>(dst) & 15) != 0 || (dst_pitch & 15) != 0) {
-    host::set_error("pad2d: the destination needs a 16-byte aligned base and pitch");
-    return CATCOC_E_ALIGNMENT;
-  }
-  const int64_t chunks = rows * (dst_pitch >> 4);
-  int64_t blocks = (chunks + 256 * kPadChunks - 1) / (256 * kPadChunks);
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  CATCOC_CUDA_OK(host::launch_overlapped(pad2d_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                                         static_cast<uint8_t*>(dst), dst_pitch, static_cast<const uint8_t*>(src), src_pitch, rows, row_bytes));
-  return CATCOC_OK;
+  PadJobs jobs = {};
+  jobs.job[0] = {static_cast<uint8_t*>(dst0), dst_pitch0, static_cast<const uint8_t*>(src0), src_pitch0, rows0, row_bytes0};
+  jobs.job[1] = {static_cast<uint8_t*>(dst1), dst_pitch1, static_cast<const uint8_t*>(src1), src_pitch1, rows1, row_bytes1};
+  return pad_launch(jobs, 2, stream);
 }
 
 extern "C" int catcoc_splitk_reduce(const float* parts, int slices, int64_t slice_elems, int rows, int cols, void* out,

@@ -137,8 +137,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
                 split = (cm.launch_tail, *cut)
     with torch.cuda.device(dev):
         # An operand whose base or row pitch TMA cannot take goes through the pad kernel first.
-        oa = cm.as_operand(a, trans_a)
-        ob = cm.as_operand(b, trans_b)
+        oa, ob = cm.as_operands(a, trans_a, b, trans_b)
         args = N.OpArgs()
         args.mode = N.MODE_LOCAL
         args.in_fmt = cm.in_fmt(a.dtype)
