@@ -986,7 +986,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
       // per element made the epilogue longer than a short mainloop: int8, 32 ragged groups of
       // 440 rows, 4096 x 2048: 247 -> 174 us, 16 groups of 1875, 2048 x 2048: 187 -> 155 us).
       float row_scale = 1.0f;
-      if (kScale && dequant && own && p.scale_m != nullptr && ti.m0 + row_in_tile < sched.M) row_scale = __ldg(p.scale_m + ti.m0 + row_in_tile);
+      if (kScale && dequant && own && p.scale_m != nullptr && ti.m0 + row_in_tile < sched.M) row_scale = p.scale_m[ti.m0 + row_in_tile];
 
       // A group's last rows end inside the output, where TMA cannot clip: their 16-bit values leave from the registers, whole
       // 32-byte sectors of the lane's own row, where rows and the tile's columns allow it (64 groups of 31
@@ -1050,7 +1050,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
             if (vec_cols(bcol, ti.n0 + col0 + 32 <= sched.N)) {
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
-                const int4 b = __ldg(reinterpret_cast<const int4*>(bcol) + u);
+                const int4 b = reinterpret_cast<const int4*>(bcol)[u];
                 v[u * 4] += static_cast<uint32_t>(b.x); v[u * 4 + 1] += static_cast<uint32_t>(b.y);
                 v[u * 4 + 2] += static_cast<uint32_t>(b.z); v[u * 4 + 3] += static_cast<uint32_t>(b.w);
               }
@@ -1058,7 +1058,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 const int c = ti.n0 + col0 + j;
-                const int32_t b = (c < sched.N) ? __ldg(p.bias + nvec_off + c) : 0;
+                const int32_t b = (c < sched.N) ? p.bias[nvec_off + c] : 0;
                 v[j] = static_cast<uint32_t>(static_cast<int32_t>(v[j]) + b);
               }
             }
@@ -1156,7 +1156,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
               if (p.scale_n != nullptr && vec_cols(scol, ti.n0 + col0 + 32 <= sched.N)) {
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                  const float4 sn = __ldg(reinterpret_cast<const float4*>(scol) + u);
+                  const float4 sn = reinterpret_cast<const float4*>(scol)[u];
                   f[u * 4] = f[u * 4] * sn.x * row_scale; f[u * 4 + 1] = f[u * 4 + 1] * sn.y * row_scale;
                   f[u * 4 + 2] = f[u * 4 + 2] * sn.z * row_scale; f[u * 4 + 3] = f[u * 4 + 3] * sn.w * row_scale;
                 }
@@ -1165,7 +1165,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
                 for (int j = 0; j < 32; ++j) {
                   const int c = ti.n0 + col0 + j;
                   const float sn =
-                      (p.scale_n != nullptr && c < sched.N) ? __ldg(p.scale_n + nvec_off + c) : 1.0f;
+                      (p.scale_n != nullptr && c < sched.N) ? p.scale_n[nvec_off + c] : 1.0f;
                   f[j] = f[j] * sn * row_scale;
                 }
               }
@@ -1177,7 +1177,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 float x = alpha * f[j];
-                if (p.bias_f != nullptr && j < cvalid) x += __ldg(p.bias_f + nvec_off + ti.n0 + col0 + j);
+                if (p.bias_f != nullptr && j < cvalid) x += p.bias_f[nvec_off + ti.n0 + col0 + j];
                 f[j] = x;
               }
               if (p.c_src != nullptr && row_in_tile < ti.rows) {

@@ -569,6 +569,16 @@ CATCOC_DEVICE uint4 ld_global_v4(const void* p) {
                : "memory");
   return v;
 }
+// What an earlier grid of the stream wrote, read behind grid_dependency_wait() by a kernel that was resident while that grid
+// ran: in program order, and at L2.
+CATCOC_DEVICE uint4 ld_global_cg_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
 // Read-only streaming load of data this kernel never writes (operands being forwarded to peers).
 CATCOC_DEVICE uint4 ld_global_nc_v4(const void* p) {
   uint4 v;

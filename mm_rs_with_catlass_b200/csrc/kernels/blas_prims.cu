@@ -96,8 +96,8 @@ __global__ void pad2d_kernel(const __grid_constant__ PadJobs jobs) {
         sh[j] = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(s) & 15u);
         out[j] = dst + r * dst_pitch + o;
         const uint8_t* a = s - sh[j];
-        if (valid[j] > 0) w[j][0] = ldg_v4(a);
-        if (valid[j] > 0 && static_cast<int>(sh[j]) + valid[j] > 16) w[j][1] = ldg_v4(a + 16);
+        if (valid[j] > 0) w[j][0] = *reinterpret_cast<const uint4*>(a);
+        if (valid[j] > 0 && static_cast<int>(sh[j]) + valid[j] > 16) w[j][1] = *reinterpret_cast<const uint4*>(a + 16);
       }
     }
 #pragma unroll

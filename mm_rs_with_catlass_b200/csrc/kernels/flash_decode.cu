@@ -318,8 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_decode_kernel(const __grid_
 // 32 pieces at a time: a lane takes the maximum and the weight of one piece, then all lanes add up its columns.
 // Started early by the main kernel, whose results it waits for.
 template <int D, int FMT>
-__global__ void __launch_bounds__(128) flash_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                            void* out, int rows, int nb, int per) {
+__global__ void __launch_bounds__(128) flash_combine_kernel(const float* part_o, const float* part_ml, void* out, int rows, int nb, int per) {
   constexpr int kPer = D / 32;                     // columns per lane
   const int bh = blockIdx.x, r = blockIdx.y * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;

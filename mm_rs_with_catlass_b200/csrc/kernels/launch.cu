@@ -939,7 +939,7 @@ CATCOC_DEVICE void fold_store(const FoldParams& p, const uint8_t* src, int64_t s
   uint32_t a[4] = {0u, 0u, 0u, 0u};
 #pragma unroll 4
   for (int s = 0; s < slices; ++s) {
-    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(src + s * step));
+    const uint4 v = ptx::ld_global_cg_v4(src + s * step);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e)
@@ -948,7 +948,7 @@ CATCOC_DEVICE void fold_store(const FoldParams& p, const uint8_t* src, int64_t s
   const int64_t o = static_cast<int64_t>(r) * p.ldc + c0;
   if (INT && p.bias != nullptr) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) if (e < n) a[e] += static_cast<uint32_t>(__ldg(p.bias + c0 + e));
+    for (int e = 0; e < 4; ++e) if (e < n) a[e] += static_cast<uint32_t>(p.bias[c0 + e]);
   }
   if (INT && p.out_fmt == FMT_S32) {
     uint32_t* dst = static_cast<uint32_t*>(p.out) + o;
@@ -960,16 +960,16 @@ CATCOC_DEVICE void fold_store(const FoldParams& p, const uint8_t* src, int64_t s
 #pragma unroll
   for (int e = 0; e < 4; ++e) f[e] = INT ? static_cast<float>(static_cast<int32_t>(a[e])) : __uint_as_float(a[e]);
   if (p.scale_m != nullptr || p.scale_n != nullptr) {
-    const float sm = p.scale_m != nullptr ? __ldg(p.scale_m + r) : 1.0f;
+    const float sm = p.scale_m != nullptr ? p.scale_m[r] : 1.0f;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = f[e] * ((p.scale_n != nullptr && e < n) ? __ldg(p.scale_n + c0 + e) : 1.0f) * sm;
+    for (int e = 0; e < 4; ++e) f[e] = f[e] * ((p.scale_n != nullptr && e < n) ? p.scale_n[c0 + e] : 1.0f) * sm;
   }
   if (p.affine) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (e < n) {
         float x = p.alpha * f[e];
-        if (p.bias_f != nullptr) x += __ldg(p.bias_f + c0 + e);
+        if (p.bias_f != nullptr) x += p.bias_f[c0 + e];
         if (p.c_src != nullptr) x += p.beta * load1(p.c_src, static_cast<int64_t>(r) * p.ldc_src + c0 + e, p.out_fmt);
         f[e] = x;
       }
@@ -987,9 +987,10 @@ CATCOC_DEVICE void fold_store(const FoldParams& p, const uint8_t* src, int64_t s
   }
 }
 
-// Four columns a thread; the planes come from L2 (128 rows x 8192 columns x 4 slices: 17 MB).
+// Four columns a thread; the planes come from L2 (128 rows x 8192 columns x 4 slices: 17 MB). Bound by the loads in flight, so
+// the registers are held to eight blocks per SM (the fp32 form needs no more than 32 by itself).
 template <bool INT>
-__global__ void __launch_bounds__(256) splitk_fold_kernel(const FoldParams p) {
+__global__ void __launch_bounds__(256, INT ? 8 : 0) splitk_fold_kernel(const FoldParams p) {
   ptx::grid_dependency_wait();
   const int units_row = (p.cols + 3) / 4;
   const int64_t units = static_cast<int64_t>(p.rows) * units_row;
@@ -1002,7 +1003,7 @@ __global__ void __launch_bounds__(256) splitk_fold_kernel(const FoldParams p) {
 
 // The same over the tiles from `first` on: blockIdx.y counts them, their planes are [slices][BM][BN].
 template <bool INT>
-__global__ void __launch_bounds__(256) tail_fold_kernel(const FoldParams p, const TileSched sched, int first) {
+__global__ void __launch_bounds__(256, 6) tail_fold_kernel(const FoldParams p, const TileSched sched, int first) {
   ptx::grid_dependency_wait();
   const TileInfo ti = get_tile(sched, first + blockIdx.y);
   const uint8_t* planes = p.parts + static_cast<int64_t>(blockIdx.y) * p.slices * p.plane * 4;

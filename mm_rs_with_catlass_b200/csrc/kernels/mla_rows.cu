@@ -65,6 +65,7 @@ struct RowsParams {
   void* out;                      // [B * rows_per_item, 512]
   float* part_o;                  // [2 * run + (0: first piece of the run, 1: last)][chunk][N][512]
   float* part_ml;                 // the same without the columns, (m, l)
+  int2* place;                    // [B] of a sequence with pages: where its first page stands in the list, pages per run
   int B, q_len, H, max_pages, num_pages, rows_per_item, chunks;
   int causal;
   float scale_log2;
@@ -87,7 +88,7 @@ CATCOC_DEVICE void fail(const RowsParams& p, uint32_t what, uint32_t a) {
   }
 }
 
-CATCOC_DEVICE int item_len(const int* kv_lens, int max_pages, int item) { return min(max(0, __ldg(kv_lens + item)), max_pages * kPage); }
+CATCOC_DEVICE int item_len(const int* kv_lens, int max_pages, int item) { return min(max(0, kv_lens[item]), max_pages * kPage); }
 CATCOC_DEVICE int item_pages(const int* kv_lens, int max_pages, int item) { return (item_len(kv_lens, max_pages, item) + kPage - 1) / kPage; }
 
 // Equal runs; from 33 pages on at least two each (128 pieces of one page take longer to merge than a second page to read)
@@ -96,14 +97,15 @@ CATCOC_DEVICE int pages_per_run(int total, int runs) { return max(total > 32 ? 2
 // This CTA's run of the page list (computed by every warp for itself)
 struct Run {
   int n;            // pages of the run
+  int begin, per;   // where it starts in the page list, pages per run
   int item, page;   // where it starts
   CATCOC_DEVICE Run(const RowsParams& p, int lane) {
     int sum = 0;
     for (int i = lane; i < p.B; i += 32) sum += item_pages(p.kv_lens, p.max_pages, i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const int per = pages_per_run(sum, static_cast<int>(gridDim.x));
-    const int begin = static_cast<int>(blockIdx.x) * per;
+    per = pages_per_run(sum, static_cast<int>(gridDim.x));
+    begin = static_cast<int>(blockIdx.x) * per;
     n = min(sum, begin + per) - begin;
     item = 0; page = 0;
     if (n <= 0) { n = 0; return; }
@@ -216,11 +218,11 @@ __global__ void __launch_bounds__(kThreads, 1) mla_rows_kernel(const __grid_cons
     int seq = 0;
     for (Piece pc(p, run); ok && pc.i0 < run.n; pc.next(p, run), ++seq) {
       const int* table = p.block_table + static_cast<int64_t>(pc.item) * p.max_pages;
-      int page_next = __ldg(table + pc.page0);
+      int page_next = table[pc.page0];
       for (int i = pc.i0; ok && i < pc.i1; ++i) {
         // a bad entry reads a wrong page, never outside the cache
         const int page = min(max(page_next, 0), p.num_pages - 1);
-        if (i + 1 < pc.i1) page_next = __ldg(table + pc.page0 + (i + 1 - pc.i0));
+        if (i + 1 < pc.i1) page_next = table[pc.page0 + (i + 1 - pc.i0)];
         const int rs = i % G::kRopeSlots;
         ok = ptx::mbar_wait(&bars->rope_empty[rs], (static_cast<uint32_t>(i / G::kRopeSlots) & 1u) ^ 1u, p.timeout_ns, abort_flag);
         if (!ok) break;
@@ -328,6 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1) mla_rows_kernel(const __grid_cons
     const float sc = p.scale_log2;
     bool bad = false;
     for (Piece pc(p, run); !bad && pc.i0 < run.n; pc.next(p, run)) {
+      if (chunk == 0 && threadIdx.x == 0 && pc.page0 == 0) p.place[pc.item] = make_int2(run.begin + pc.i0, run.per);
       const int kv_len = item_len(p.kv_lens, p.max_pages, pc.item);
       const int vis_all = p.causal ? max(0, kv_len - (p.q_len - 1)) : kv_len;   // keys every row sees
       // lane r: the keys that row r of this chunk sees (with the causal mask a new token does not see those behind it)
@@ -458,31 +461,17 @@ __global__ void __launch_bounds__(kThreads, 1) mla_rows_kernel(const __grid_cons
 
 // Merges the pieces of the sequences that were cut, and zeroes the rows of empty sequences. One block per (row, sequence).
 template <int FMT>
-__global__ void __launch_bounds__(128) mla_rows_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                               void* out, const int* __restrict__ kv_lens, int B, int max_pages,
-                                                               int rows_per_item, int chunks, int n, int runs) {
-  __shared__ int s_before[4], s_total[4];
+__global__ void __launch_bounds__(128) mla_rows_combine_kernel(const float* part_o, const float* part_ml, const int2* place, void* out,
+                                                               const int* kv_lens, int max_pages, int rows_per_item, int chunks, int n, int runs) {
+  constexpr int kPieces = 8;                       // loads in flight per thread
   __shared__ float s_max[4], s_w[128], s_wl[128];
   const int item = blockIdx.y, row = blockIdx.x;
-  int before = 0, total = 0;
-  for (int i = threadIdx.x; i < B; i += 128) {
-    const int pg = item_pages(kv_lens, max_pages, i);
-    total += pg;
-    if (i < item) before += pg;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    before += __shfl_xor_sync(0xffffffffu, before, o);
-    total += __shfl_xor_sync(0xffffffffu, total, o);
-  }
-  if ((threadIdx.x & 31) == 0) { s_before[threadIdx.x >> 5] = before; s_total[threadIdx.x >> 5] = total; }
-  __syncthreads();
-  before = s_before[0] + s_before[1] + s_before[2] + s_before[3];
-  total = s_total[0] + s_total[1] + s_total[2] + s_total[3];
-  const int pages = item_pages(kv_lens, max_pages, item);
-  const int per = pages_per_run(total, runs);
-  const int c0 = before / per, c1 = pages > 0 ? (before + pages - 1) / per : c0;
   ptx::grid_dependency_wait();
+  const int pages = item_pages(kv_lens, max_pages, item);
+  // not written for a sequence without pages, nor behind a wait that ran out: whatever it holds, the pieces read are the workspace's
+  const int2 at = place[item];
+  const int before = min(max(0, at.x), 1 << 24), per = max(1, at.y);
+  const int c0 = min(before / per, runs - 1), c1 = min((before + pages - 1) / per, runs - 1);
   if (pages > 0 && c0 == c1) return;               // written by its CTA
   const int col = threadIdx.x * 4;
   const int chunk = row / n, r = row - chunk * n;
@@ -493,6 +482,14 @@ __global__ void __launch_bounds__(128) mla_rows_combine_kernel(const float* __re
   float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   for (int base = c0; pages > 0 && base <= c1; base += 128) {
     const int count = min(128, c1 + 1 - base);
+    // O of the first pieces is on its way while their weights are worked out
+    float4 o[kPieces];
+    auto fetch = [&](int c) {
+#pragma unroll
+      for (int e = 0; e < kPieces; ++e)
+        o[e] = c + e < count ? *reinterpret_cast<const float4*>(part_o + index(base + c + e) * kDV + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    fetch(0);
     const float2 ml = static_cast<int>(threadIdx.x) < count ? *reinterpret_cast<const float2*>(part_ml + index(base + threadIdx.x) * 2)
                                                             : make_float2(-INFINITY, 0.0f);
     float mx = warp_max(ml.x);
@@ -508,12 +505,14 @@ __global__ void __launch_bounds__(128) mla_rows_combine_kernel(const float* __re
     m = mx;
     l *= old;
     acc.x *= old; acc.y *= old; acc.z *= old; acc.w *= old;
-#pragma unroll 8
-    for (int c = 0; c < count; ++c) {
-      const float4 o = *reinterpret_cast<const float4*>(part_o + index(base + c) * kDV + col);
-      const float wc = s_w[c];
-      l += s_wl[c];
-      acc.x += wc * o.x; acc.y += wc * o.y; acc.z += wc * o.z; acc.w += wc * o.w;
+    for (int c = 0; c < count; c += kPieces) {
+      if (c > 0) fetch(c);
+#pragma unroll
+      for (int e = 0; e < kPieces; ++e) {          // (past the last piece: weights of zero)
+        const float wc = s_w[c + e];
+        l += s_wl[c + e];
+        acc.x += wc * o[e].x; acc.y += wc * o[e].y; acc.z += wc * o[e].z; acc.w += wc * o[e].w;
+      }
     }
   }
   const float inv = l > 0.0f ? 1.0f / l : 0.0f;
@@ -567,7 +566,7 @@ extern "C" int64_t catcoc_mla_rows_workspace_bytes(int B, int q_len, int H, int 
   if (rows > 128) return -1;
   if (B > 65535 || static_cast<int64_t>(B) * max_pages > (1 << 24)) return -1;
   const RowsPlan d = rows_plan(static_cast<int>(rows));
-  return static_cast<int64_t>(d.runs) * 2 * d.chunks * d.n * (mlar::kDV + 2) * static_cast<int64_t>(sizeof(float));
+  return static_cast<int64_t>(d.runs) * 2 * d.chunks * d.n * (mlar::kDV + 2) * static_cast<int64_t>(sizeof(float)) + B * static_cast<int64_t>(sizeof(int2));
 }
 
 extern "C" int catcoc_mla_rows(const void* q_nope, const void* q_rope, const void* ckv, const void* krope, const int* block_table,
@@ -605,6 +604,7 @@ extern "C" int catcoc_mla_rows(const void* q_nope, const void* q_rope, const voi
   p.block_table = block_table; p.kv_lens = kv_lens; p.out = out;
   p.part_o = static_cast<float*>(workspace);
   p.part_ml = p.part_o + static_cast<int64_t>(d.runs) * 2 * d.chunks * d.n * mlar::kDV;
+  p.place = reinterpret_cast<int2*>(p.part_ml + static_cast<int64_t>(d.runs) * 2 * d.chunks * d.n * 2);
   p.B = B; p.q_len = q_len; p.H = H; p.max_pages = max_pages; p.num_pages = num_pages;
   p.rows_per_item = rows_per_item; p.chunks = d.chunks;
   p.causal = causal ? 1 : 0;
@@ -620,7 +620,7 @@ extern "C" int catcoc_mla_rows(const void* q_nope, const void* q_rope, const voi
     CATCOC_CUDA_OK(launch_overlapped(main_kernel, dim3(static_cast<unsigned>(d.runs), static_cast<unsigned>(d.chunks)), dim3(mlar::kThreads),
                                      smem, stream, p));
     CATCOC_CUDA_OK(launch_overlapped(combine_kernel, dim3(static_cast<unsigned>(rows_per_item), static_cast<unsigned>(B)), dim3(128), 0,
-                                     stream, p.part_o, p.part_ml, out, kv_lens, B, max_pages, rows_per_item, d.chunks, d.n, d.runs));
+                                     stream, p.part_o, p.part_ml, p.place, out, kv_lens, max_pages, rows_per_item, d.chunks, d.n, d.runs));
     return CATCOC_OK;
   };
   const bool bf = fmt == CATCOC_FMT_BF16;

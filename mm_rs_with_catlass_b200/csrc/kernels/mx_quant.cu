@@ -23,12 +23,12 @@ template <int FMT>
 CATCOC_DEVICE void load8(const void* x, int64_t chunk, float (&f)[8]) {
   if constexpr (FMT == FMT_F32) {
     const uint4* p = static_cast<const uint4*>(x) + 2 * chunk;
-    const uint4 a = __ldg(p), b = __ldg(p + 1);
+    const uint4 a = p[0], b = p[1];
     const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(u[i]);
   } else {
-    const uint4 a = __ldg(static_cast<const uint4*>(x) + chunk);
+    const uint4 a = static_cast<const uint4*>(x)[chunk];
     const uint32_t u[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -70,8 +70,7 @@ CATCOC_DEVICE uint32_t cvt_fp8_special(float v) {
 // q = fp8(x / 2^e), scale = e + 127 with e = ceil(log2(amax / fp8_max)) per 32 elements. A thread converts 8
 // consecutive elements, four neighbouring lanes share a block.
 template <int FMT, bool E5M2>
-__global__ void __launch_bounds__(256) mx_quantize_kernel(const void* __restrict__ x, uint8_t* __restrict__ q,
-                                                          uint8_t* __restrict__ scales, int64_t chunks) {
+__global__ void __launch_bounds__(256) mx_quantize_kernel(const void* x, uint8_t* q, uint8_t* scales, int64_t chunks) {
   const int64_t base = static_cast<int64_t>(blockIdx.x) * (blockDim.x * kQuantChunks) + threadIdx.x;
   ptx::grid_dependency_wait();
   float f[kQuantChunks][8];
@@ -123,8 +122,7 @@ __global__ void __launch_bounds__(256) mx_quantize_kernel(const void* __restrict
 
 // out[rt][kt][l * 16 + j * 4 + s] = scales[rt * 128 + j * 32 + l][kt * 4 + s]; rows and K-blocks past the end read as
 // 127 (= 1.0). One thread per 4-byte word; eight neighbouring threads walk along K so that their reads share a sector.
-__global__ void __launch_bounds__(256) mx_pack_kernel(const uint8_t* __restrict__ scales, int rows, int kb,
-                                                      uint32_t* __restrict__ out, int row_tiles, int k_tiles) {
+__global__ void __launch_bounds__(256) mx_pack_kernel(const uint8_t* scales, int rows, int kb, uint32_t* out, int row_tiles, int k_tiles) {
   const int kt_groups = (k_tiles + 7) / 8;
   ptx::grid_dependency_wait();
   const int64_t total = static_cast<int64_t>(row_tiles) * kt_groups * 1024;
