@@ -264,6 +264,9 @@ def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: 
         else:
             ranges += [0, 0]
         begin = max(begin, end)
+    if not any(ranges):            # no group has a row: nothing to launch
+        out.zero_()
+        return True
     dev = a.device
     if tiling is None:
         from ..tiling.chooser import heuristic

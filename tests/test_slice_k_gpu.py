@@ -54,3 +54,16 @@ def test_short_and_long_ranges_store_by_different_paths():
     # 32-byte sector (n = 328) never do
     _check(256, 512, [256, 257, 40, 700, 256], torch.bfloat16, seed=6)
     _check(256, 328, [256, 40, 700], torch.float16, seed=7)
+
+
+@pytest.mark.parametrize("rows", [0, 40])
+def test_every_group_empty(rows):
+    # a rank of a mixture of experts that received no token in this step: zeros, whether or not rows are there
+    import mm_rs_with_catlass_b200 as catcoc
+    from mm_rs_with_catlass_b200.ops._common import local_status, raise_on_status
+    a, b = (torch.randn(rows, c, device="cuda").bfloat16() for c in (256, 128))
+    torch.full((4, 256, 128), float("nan"), device="cuda", dtype=torch.bfloat16)     # what the allocator hands out next
+    out = catcoc.grouped_matmul_slice_k(a, b, [0, 0, 0, 0])
+    assert tuple(out.shape) == (4, 256, 128) and bool((out == 0).all())
+    assert catcoc.grouped_matmul_slice_k(a, b, torch.zeros(3, dtype=torch.int64), out_dtype=torch.float32).abs().sum().item() == 0
+    raise_on_status(local_status(a.device), "slice_k")
