@@ -252,6 +252,8 @@ def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: 
     k_total, elt = a.shape[0], a.element_size()
     if a.dtype not in (torch.float16, torch.bfloat16) or a.dtype != b.dtype or g < 2 or m == 0 or n == 0:
         return False
+    if not out.dtype.is_floating_point:        # refused by the product of a group
+        return False
     if a.stride(-1) != 1 or b.stride(-1) != 1 or (m * elt) % 16 != 0:
         return False
     ranges, begin = [], 0

@@ -67,3 +67,11 @@ def test_every_group_empty(rows):
     assert tuple(out.shape) == (4, 256, 128) and bool((out == 0).all())
     assert catcoc.grouped_matmul_slice_k(a, b, torch.zeros(3, dtype=torch.int64), out_dtype=torch.float32).abs().sum().item() == 0
     raise_on_status(local_status(a.device), "slice_k")
+
+
+def test_an_integer_output_is_refused_however_many_groups():
+    import mm_rs_with_catlass_b200 as catcoc
+    a, b = (torch.randn(96, c, device="cuda").bfloat16() for c in (256, 128))
+    for ends in ([96], [40, 96]):
+        with pytest.raises(ValueError, match="int32"):
+            catcoc.grouped_matmul_slice_k(a, b, ends, out_dtype=torch.int32)
