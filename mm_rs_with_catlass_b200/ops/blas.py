@@ -34,6 +34,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import operator
 from typing import List, Optional, Sequence, Union
 
 import torch
@@ -258,7 +259,7 @@ def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: 
         return False
     ranges, begin = [], 0
     for end in ends:
-        end = int(end)
+        end = operator.index(end)
         if end > begin:
             if begin >= k_total:
                 return False

@@ -75,3 +75,13 @@ def test_an_integer_output_is_refused_however_many_groups():
     for ends in ([96], [40, 96]):
         with pytest.raises(ValueError, match="int32"):
             catcoc.grouped_matmul_slice_k(a, b, ends, out_dtype=torch.int32)
+
+
+def test_ends_are_whole_numbers():
+    import mm_rs_with_catlass_b200 as catcoc
+    a, b = (torch.randn(96, c, device="cuda").bfloat16() for c in (256, 128))
+    for ends in ([96.0], [40.5, 96.0], torch.tensor([40.5, 96.0])):
+        with pytest.raises(TypeError):
+            catcoc.grouped_matmul_slice_k(a, b, ends)
+    whole = catcoc.grouped_matmul_slice_k(a, b, torch.tensor([40, 96]))
+    assert torch.equal(whole, catcoc.grouped_matmul_slice_k(a, b, list(torch.tensor([40, 96], dtype=torch.int32))))
