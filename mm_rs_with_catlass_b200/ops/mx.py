@@ -25,6 +25,16 @@ BLOCK = 32
 _FP8_MAX = {"e4m3": 448.0, "e5m2": 57344.0}
 
 
+def _plain(x: torch.Tensor) -> bool:
+    """Whether a kernel may stand in for PyTorch's own operators on ``x``: values on a GPU that nobody differentiates,
+    batches, traces or intercepts. A pointer has none of that, so such inputs keep the operators."""
+    return (not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and (type(x) is torch.Tensor or type(x) is torch.nn.Parameter)
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch._C._functorch.is_functorch_wrapped_tensor(x)
+            and not (x.requires_grad and torch.is_grad_enabled()) and torch.autograd.forward_ad._current_level < 0
+            and x.is_cuda and x.numel() > 0)
+
+
 def quantize_mxf8(x: torch.Tensor, fmt: str = "e4m3") -> Tuple[torch.Tensor, torch.Tensor]:
     """``x [rows, K]`` (K % 32 == 0) -> (fp8 values ``[rows, K]``, UE8M0 scales ``uint8 [rows, K/32]``).
     The scale of a block is the smallest power of two that brings its largest magnitude into the
@@ -33,7 +43,7 @@ def quantize_mxf8(x: torch.Tensor, fmt: str = "e4m3") -> Tuple[torch.Tensor, tor
     if k % BLOCK:
         raise ValueError("K must be a multiple of 32 for block scaling (K=%d)" % k)
     dt = torch.float8_e4m3fn if fmt == "e4m3" else torch.float8_e5m2
-    if x.is_cuda and fmt in _FP8_MAX and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and x.numel():
+    if fmt in _FP8_MAX and x.dtype in (torch.float16, torch.bfloat16, torch.float32) and _plain(x):
         # one pass of the quantisation kernel: the same values as the passes below
         x = x.contiguous()
         if x.data_ptr() % 16:
@@ -64,7 +74,7 @@ def pack_scales(scales: torch.Tensor) -> torch.Tensor:
     layout; rows and K-blocks are padded with the neutral scale 127 (= 1.0)."""
     rows, kb = scales.shape
     rt, kt = (rows + 127) // 128, (kb + 3) // 4
-    if scales.is_cuda and scales.dtype == torch.uint8 and scales.numel():
+    if scales.dtype == torch.uint8 and _plain(scales):
         scales = scales.contiguous()
         if scales.data_ptr() % 4:
             scales = scales.clone()
