@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(kThreads, 1) mla_rows_kernel(const __grid_cons
     int seq = 0;
     for (Piece pc(p, run); ok && pc.i0 < run.n; pc.next(p, run), ++seq) {
       ok = ptx::mbar_wait(&bars->q_full, static_cast<uint32_t>(seq) & 1u, p.timeout_ns, abort_flag);
+      const int kv_len = item_len(p.kv_lens, p.max_pages, pc.item);
       for (int i = pc.i0; ok && i < pc.i1; ++i) {
         // S^T = K Q^T, 64 columns of the keys at a time: the rotary block, then the latent ones
         const int rs = i % G::kRopeSlots;
@@ -297,7 +298,9 @@ __global__ void __launch_bounds__(kThreads, 1) mla_rows_kernel(const __grid_cons
           __syncwarp();
         }
         if (!ok) break;
-        // O^T += V^T P^T, 128 output columns (one slot) at a time
+        // O^T += V^T P^T, 128 output columns (one slot) at a time. Only keys of the sequence, 16 at a time: what lies behind
+        // them in its last page has probability zero, but may hold anything, and zero times an infinity is a NaN
+        const int steps = min(kPage, kv_len - (pc.page0 + i - pc.i0) * kPage + 15) / 16;
         ok = ptx::mbar_wait(&bars->p_full, static_cast<uint32_t>(i) & 1u, p.timeout_ns, abort_flag);
         if (!ok) break;
         ptx::tcgen05_fence_after();
@@ -308,6 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) mla_rows_kernel(const __grid_cons
             const uint64_t dv = ptx::make_smem_desc_sw128(ptx::smem_u32(spair + slot * kPairBytes), static_cast<uint32_t>(kBlockBytes), 1024u);
 #pragma unroll
             for (int kk = 0; kk < kPage / 16; ++kk) {
+              if (kk >= steps) break;
               const uint64_t dp = ptx::make_smem_desc_sw128(ptx::smem_u32(sp + (kk >> 2) * N * 128), 16u, 1024u) + static_cast<uint64_t>((kk & 3) * 2);
               ptx::umma_f16(tmem + kOCol + c * N, dv + static_cast<uint64_t>((kk * 2048) >> 4), dp, p.idesc_pv,
                             (i > pc.i0 || kk != 0) ? 1u : 0u);

@@ -7,7 +7,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _case(q_len, heads, lens, dtype, causal=False, gain=None, seed=0, extra_pages=0):
+def _case(q_len, heads, lens, dtype, causal=False, gain=None, seed=0, extra_pages=0, stale=False):
     import mm_rs_with_catlass_b200 as catcoc
     from mm_rs_with_catlass_b200.ops.mla import mla_decode_reference
     from mm_rs_with_catlass_b200.ops._common import local_status, raise_on_status
@@ -25,6 +25,14 @@ def _case(q_len, heads, lens, dtype, causal=False, gain=None, seed=0, extra_page
         ramp = torch.linspace(gain[0], gain[1], max_pages, device=dev)
         for b in range(batch):
             kr[table[b].long()] = (kr[table[b].long()].abs().float() * ramp[:, None, None]).to(dtype)
+    if stale:
+        # slots of the last page that no token was written to yet hold whatever the memory held before (the kernel reads
+        # 16 keys at a time, so those up to the next multiple have to be finite)
+        for b, n in enumerate(lens):
+            page = table[b, (n - 1) // 128]
+            first = ((n - 1) % 128 + 16) // 16 * 16
+            for i, cache in enumerate((ckv, kr)):
+                cache[page, first:] = (float("nan"), float("inf"))[(b + i) % 2]
     kv = torch.tensor(lens, dtype=torch.int32, device=dev)
     out = catcoc.mla_decode(qn, qr, ckv, kr, table, kv, q_len=q_len, causal=causal)
     torch.cuda.synchronize()
@@ -59,3 +67,10 @@ def test_moving_reference_maximum(gain):
 
 def test_table_wider_than_the_sequences():
     _case(1, 16, [100, 300], torch.bfloat16, seed=3, extra_pages=5)
+
+
+@pytest.mark.parametrize("heads", [16, 32])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_stale_slots_of_the_last_page_do_not_matter(heads, dtype):
+    _case(1, heads, [1, 16, 17, 32, 96, 127, 128, 130, 300, 1000], dtype, seed=heads, stale=True)
+    _case(4, heads, [4, 32, 132, 260], dtype, seed=heads + 1, causal=True, stale=True)
