@@ -908,6 +908,9 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
         const int64_t span = static_cast<int64_t>(rows_valid - 1) * pitch + static_cast<int64_t>(ti.cols) * st_elt;
         if (kPull && pull) {
           dst_ok = CATCOC_BOUND(p, SITE_PART_STORE, (base - p.part_local) + span, LIM_PART);
+        } else if (tail_unit) {   // the planes of the cut tiles: rows of the map they are stored through
+          dst_ok = CATCOC_BOUND_ABS(p, SITE_PUSH_SLAB, static_cast<int64_t>(t - sched_tail_first(p)) * sched.BM + row_base + 32,
+                                    static_cast<int64_t>(total_tiles - sched_tail_first(p)) * sched.BM);
         } else if (!own) {   // slabs are stored whole
           dst_ok = CATCOC_BOUND(p, SITE_PUSH_SLAB, (base - p.stage[ti.seg]) + 31 * pitch + static_cast<int64_t>(BN) * st_elt,
                                 LIM_STAGE);
@@ -968,7 +971,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
               }
               released = true;
             }
-            if (lane < rows_valid) {
+            if (lane < rows_valid && dst_ok) {
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 uint32_t w[8];

@@ -86,6 +86,39 @@ def test_an_understated_output_extent_is_reported_and_nothing_is_written_past_it
     assert r["tail_untouched"] and r["head_written"], r
 
 
+def test_register_stores_of_short_k_ranges_respect_the_extent():
+    out = _child("""
+        import ctypes as C, json, torch
+        from mm_rs_with_catlass_b200 import _native as N
+        from mm_rs_with_catlass_b200.ops import _common as cm
+        dev = torch.device("cuda:0")
+        m, n, k = 256, 256, 128
+        a = torch.randn(k, m, device=dev).bfloat16()
+        b = torch.randn(k, n, device=dev).bfloat16()
+        out = torch.full((2, m, n), 7.0, device=dev, dtype=torch.bfloat16)
+        status = torch.zeros(8, dtype=torch.int32, device=dev)
+        args = N.OpArgs()
+        args.mode, args.in_fmt = N.MODE_LOCAL, N.IN_BF16
+        args.M, args.N, args.K = 2 * m, n, k
+        args.trans_a = 1
+        args.a, args.lda, args.b, args.ldb = a.data_ptr(), m, b.data_ptr(), n
+        args.out, args.ldc, args.out_fmt, args.partial_fmt = out.data_ptr(), n, N.FMT_BF16, N.FMT_BF16
+        args.tiling.bn = 128
+        args.rank, args.W = 0, 1
+        args.num_groups, args.group_rows, args.g_a_row_back = 2, m, m
+        args.a_rows_total, args.a_k_total, args.b_n_total, args.b_k_total = m, k, n, k
+        args.status = status.data_ptr()
+        args.limit[N.LIM_OUT] = m * n * 2              # the caller claims the first group's output alone
+        cm.launch_slice_k(args, [0, 64, 64, 128], dev)
+        torch.cuda.synchronize()
+        print(json.dumps({"status": status.cpu().tolist(), "second_untouched": bool((out[1] == 7.0).all().item()),
+                          "first_written": bool((out[0] != 7.0).any().item())}))
+    """, {"CATCOC_OUT_TMA": "0"})
+    r = out[-1]
+    assert r["status"][0] == 7 and r["status"][2] == 13 and r["status"][3] == 256 * 256 * 2, r
+    assert r["second_untouched"] and r["first_written"], r
+
+
 def test_the_launcher_refuses_a_tensor_map_over_an_understated_output():
     out = _child("""
         import json, torch
