@@ -1037,6 +1037,15 @@ bool fold_fits(const CatcocOpArgs& a, bool is_int) {
   return true;
 }
 
+// The second kernel writes the whole [M, N] output: it has to lie inside the extent that the caller states.
+bool fold_inside(const CatcocOpArgs& a) {
+  const int64_t need = (static_cast<int64_t>(a.M - 1) * a.ldc + a.N) * fmt_bytes(a.out_fmt);
+  if (a.limit[LIM_OUT] <= 0 || need <= a.limit[LIM_OUT]) return true;
+  set_error("the output buffer (%lld bytes) is smaller than [%d, %d] with pitch %lld", static_cast<long long>(a.limit[LIM_OUT]), a.M, a.N,
+            static_cast<long long>(a.ldc));
+  return false;
+}
+
 int splitk_rows(int M) { return round_up(M, 32); }    // whole 32-row windows leave the first launch by TMA
 int splitk_pitch(int N) { return round_up(N, 8); }    // rows start on 32-byte sectors
 }  // namespace
@@ -1063,6 +1072,7 @@ extern "C" int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_
   }
   const bool is_int = rf.kind == KIND_I8;
   if (!fold_fits(a, is_int)) return CATCOC_E_UNSUPPORTED;
+  if (!fold_inside(a)) return CATCOC_E_BAD_ARG;
   const int rows = splitk_rows(a.M), pitch = splitk_pitch(a.N);
   CatcocOpArgs g = a;
   g.M = slices * rows; g.K = k_slice;
@@ -1108,6 +1118,7 @@ extern "C" int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slice
     return CATCOC_E_BAD_ARG;
   }
   if (!fold_fits(a, is_int)) return CATCOC_E_UNSUPPORTED;
+  if (!fold_inside(a)) return CATCOC_E_BAD_ARG;
   static const cudaError_t ready = inst::prepare_tail();
   CATCOC_CUDA_OK(ready);
   a.partial_fmt = is_int ? CATCOC_FMT_S32 : CATCOC_FMT_F32;

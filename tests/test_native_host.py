@@ -169,3 +169,28 @@ def test_attention_entry_points_refuse_bad_arguments_without_a_gpu():
     assert mla(5, 1, None) == N.E_UNSUPPORTED                                                  # 1 to 4 new tokens
     assert mla(1, 3, None) == N.E_BAD_ARG                                                      # slices need the workspace
     assert mla(1, 100, dummy) == N.E_BAD_ARG
+
+
+def _cut_product(m=64, n=128, k=1024, **kw):
+    """Arguments of a local bf16 product; the pointers are never dereferenced."""
+    args = N.OpArgs()
+    args.mode, args.in_fmt = N.MODE_LOCAL, N.IN_BF16
+    args.M, args.N, args.K = m, n, k
+    args.a, args.lda, args.b, args.ldb = 4096, k, 4096, n
+    args.out, args.ldc, args.out_fmt, args.partial_fmt = 4096, n, N.FMT_BF16, N.FMT_BF16
+    args.rank, args.W = 0, 1
+    args.status = 4096
+    for key, v in kw.items():
+        setattr(args, key, v)
+    return args
+
+
+def test_products_cut_along_k_refuse_an_output_that_does_not_fit():
+    lib, ws = N.lib(), C.c_void_p(4096)
+    args = _cut_product()
+    args.limit[N.LIM_OUT] = 64 * 128 * 2 - 2
+    assert lib.catcoc_splitk_launch(C.byref(args), 2, 512, ws, None) == N.E_BAD_ARG and "smaller than" in N.last_error()
+    args = _cut_product(m=512)
+    args.tiling.cta_pair = 2
+    args.limit[N.LIM_OUT] = 512 * 128 * 2 - 2
+    assert lib.catcoc_tail_launch(C.byref(args), 0, 2, 512, ws, None) == N.E_BAD_ARG and "smaller than" in N.last_error()
