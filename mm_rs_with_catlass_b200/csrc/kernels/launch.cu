@@ -1096,8 +1096,9 @@ extern "C" int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_
 
 // ---- a nearly empty last wave: its tiles cut along K ----
 extern "C" int64_t catcoc_tail_workspace_bytes(int M, int N, int bn, int first, int slices) {
+  if (M <= 0 || N <= 0 || (bn != 128 && bn != 192 && bn != 256) || first < 0 || slices < 2) return -1;
   const TileSched s = make_sched(M, N, 2 * kBM, bn, 1, SEG_ROWS, 0, 1);
-  if (M <= 0 || N <= 0 || (bn != 128 && bn != 192 && bn != 256) || first < 0 || first >= s.total_tiles || slices < 2) return -1;
+  if (first >= s.total_tiles) return -1;
   return static_cast<int64_t>(s.total_tiles - first) * slices * s.BM * s.BN * 4;
 }
 

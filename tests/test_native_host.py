@@ -194,3 +194,15 @@ def test_products_cut_along_k_refuse_an_output_that_does_not_fit():
     args.tiling.cta_pair = 2
     args.limit[N.LIM_OUT] = 512 * 128 * 2 - 2
     assert lib.catcoc_tail_launch(C.byref(args), 0, 2, 512, ws, None) == N.E_BAD_ARG and "smaller than" in N.last_error()
+
+
+def test_workspace_sizes_of_impossible_cuts():
+    # asked in a child: an integer division by zero would end this process
+    code = ("import sys; sys.path.insert(0, %r)\n"
+            "from mm_rs_with_catlass_b200 import _native as N\n"
+            "f = N.lib().catcoc_tail_workspace_bytes\n"
+            "assert [f(512, 512, bn, 0, 2) for bn in (0, -256, 64, 100)] == [-1] * 4\n"
+            "assert [f(0, 512, 256, 0, 2), f(512, 0, 256, 0, 2), f(512, 512, 256, 4, 2), f(512, 512, 256, 0, 1)] == [-1] * 4\n"
+            "assert f(512, 512, 256, 3, 2) == 2 * 256 * 256 * 4\n") % REPO
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, (out.returncode, out.stderr[-500:])
