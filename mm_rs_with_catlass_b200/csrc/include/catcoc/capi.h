@@ -86,8 +86,8 @@ typedef struct CatcocOpArgs {
   int ag_m;                                /* all-gather: rows of one shard              */
   int ag_ld;                               /* all-gather: row pitch (elements) of the gathered buffer, >= K, 16-byte multiple */
   int ag_raw;                              /* all-gather: 1 = `a` may have any alignment and any pitch >= K (it is fetched by
-                                              the communication warps, never by TMA); then W == 1 is allowed too: the padding
-                                              prologue of a local GEMM (`gathered[0]` is the padded copy, an output)          */
+                                              the communication warps, never by TMA). W > 1 only: one rank has nothing to
+                                              gather, an unaligned `a` of a local product goes through catcoc_pad2d first     */
 
   /* block-scaled fp8 (CATCOC_IN_MX*): scale factors packed in 512-byte blocks of 128 rows x 4
    * K-blocks (row r, K-block s at (r % 32) * 16 + (r / 32) * 4 + s), block (row_tile, k128) at
@@ -148,7 +148,7 @@ int64_t catcoc_splitk_workspace_bytes(int M, int N, int slices);
 int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_slice, void* workspace, void* stream);
 
 /* A local product on pair tiles (args->tiling: cta_pair 2) whose last wave is nearly empty: the tiles from number `first` on
- * are cut into `slices` slices of `k_slice` elements (a multiple of 512 bytes), so that they spread over all SMs; the planes go
+ * are cut into `slices` slices of `k_slice` elements (a multiple of 256 bytes), so that they spread over all SMs; the planes go
  * to `workspace` (128-byte aligned, catcoc_tail_workspace_bytes(...) bytes), a second kernel sums them and runs the epilogue. */
 int64_t catcoc_tail_workspace_bytes(int M, int N, int bn, int first, int slices);
 int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slices, int k_slice, void* workspace, void* stream);

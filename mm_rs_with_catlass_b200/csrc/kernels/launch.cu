@@ -324,6 +324,10 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   }
   const bool ag_raw = (a.mode == CATCOC_MODE_AG) && (a.ag_raw != 0);
   const bool fused = a.mode != CATCOC_MODE_LOCAL && a.W > 1;
+  if (ag_raw && !fused) {
+    set_error("allgather: a raw shard needs W > 1 (W=%d); pad an unaligned operand of a local product first", a.W);
+    return CATCOC_E_UNSUPPORTED;
+  }
   if (fused && (a.W > kMaxWorld || a.W < 1 || a.rank < 0 || a.rank >= a.W)) {
     set_error("bad rank/world %d/%d", a.rank, a.W);
     return CATCOC_E_BAD_ARG;

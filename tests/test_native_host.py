@@ -206,3 +206,9 @@ def test_workspace_sizes_of_impossible_cuts():
             "assert f(512, 512, 256, 3, 2) == 2 * 256 * 256 * 4\n") % REPO
     out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, (out.returncode, out.stderr[-500:])
+
+
+def test_a_raw_shard_on_one_rank_is_refused():
+    args = _cut_product(mode=N.MODE_AG, ag_raw=1, ag_m=64, ag_ld=1024)
+    args.gathered[0], args.gflags[0] = 4096, 4096
+    assert N.lib().catcoc_fused_launch(C.byref(args), None) == N.E_UNSUPPORTED and "raw shard" in N.last_error()
