@@ -30,6 +30,7 @@ _NUM_SMS = 148
 # bound by the fill rate of shared memory, so halving the width costs far more than half.
 _TILE_EFF = {256: 1.0, 192: 0.85, 128: 0.56, 64: 0.43}
 _PAIR_GAIN = {256: 1.18, 192: 1.18, 128: 1.35}     # 2-CTA tiles: each CTA fills half of B (192: pairs only)
+_PAIR_GAIN_FUSED = {256: 1.10, 128: 1.35}          # ... of a launch that also communicates (measured on 2 to 8 GPUs)
 
 
 # Cost model of split_k, in SM cycles, fitted to 84 shapes (bf16 and int8; 4 to 1024 rows, N of 992 to 28672, K of 3584 to
@@ -44,7 +45,7 @@ _FOLD = 8000.0                    # the second kernel and the gap before it
 _INT8_EPILOGUE = 10000.0          # the dequantising epilogue of the direct kernel, which the second kernel spreads over all SMs
 
 
-def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bool = False) -> float:
+def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bool = False, fused: bool = False) -> float:
     """Relative time of a GEMM whose rows come in ``nseg`` segments of ``seg_rows`` rows (tiles never
     straddle segments): waves of tiles x time of one wave. With ``seg_cols`` the output is cut into
     ``nseg`` column segments instead and ``seg_rows`` is the full row count."""
@@ -55,7 +56,7 @@ def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bo
         tiles = nseg * math.ceil(seg_rows / bm) * math.ceil(n / bn)
     units = _NUM_SMS // pair
     waves = math.ceil(tiles / units)
-    eff = _TILE_EFF[bn] * (_PAIR_GAIN[bn] if pair == 2 else 1.0)
+    eff = _TILE_EFF[bn] * ((_PAIR_GAIN_FUSED if fused else _PAIR_GAIN)[bn] if pair == 2 else 1.0)
     return waves * bn / eff
 
 
@@ -116,7 +117,7 @@ def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b
                 continue
             if dtype == torch.int8 and (bn < 128 or (pair == 2 and bn < 256)):
                 continue   # 8-bit [K, N] operands need a full 128-byte run of N per TMA box and CTA
-            cost = tile_cost(seg_rows, nseg, n, bn, pair, seg_cols=ar_cols)
+            cost = tile_cost(seg_rows, nseg, n, bn, pair, seg_cols=ar_cols, fused=fused)
             if tails and pair == 2:
                 cost = tail_cut(rows, n, k, dtype.itemsize, bn)[0] * bn / (_TILE_EFF[bn] * _PAIR_GAIN[bn])
             if best is None or cost < best[0] - 1e-9:

@@ -107,6 +107,34 @@ def test_heuristic_follows_the_cost_model_and_is_deterministic():
     assert chooser.choose("matmul_reduce_scatter", 8192, 8192, 3584, 8, torch.bfloat16, table=tbl).bn == 128
 
 
+# Tiles of launches on several GPUs, as fitted there: M of 256, 512, 1024, 2048, 4096, 16384 (one word each) by N of 128, 512,
+# 1024, 1696, 2048, 4096, 8192, 28672 (one letter each: a 64, b 128, c 256 columns; d 128, e 256 on CTA pairs)
+_FUSED_TILES = {
+    ("matmul_reduce_scatter", 2): "aaaaaabc aaaaadee aaaddeee aadeeeee adeeeeee deeeeeee",
+    ("matmul_reduce_scatter", 4): "aaaaabcc aaaaabcc aaaddeee aadeeeee adeeeeee deeeeeee",
+    ("matmul_reduce_scatter", 8): "aaabbccc aaabbccc aaabbccc aadeeeee adeeeeee deeeeeee",
+    ("quant_matmul_reduce_scatter", 2): "bbbbbbbc bbbbbbee bbbbbeee bbbeeeee bbeeeeee beeeeeee",
+    ("quant_matmul_reduce_scatter", 4): "bbbbbbcc bbbbbbcc bbbbbeee bbbeeeee bbeeeeee beeeeeee",
+    ("quant_matmul_reduce_scatter", 8): "bbbbbccc bbbbbccc bbbbbccc bbbeeeee bbeeeeee beeeeeee",
+    ("matmul_allreduce", 2): "aaaaaade aaaaadee aaaddeee aadeeeee adeeeeee aeeeeeee",
+    ("matmul_allreduce", 4): "aaaaaade aaaaadee aaaddeee aadeeeee adeeeeee adeeeeee",
+    ("matmul_allreduce", 8): "aaabaade aaabadee aaabdeee aadeeeee aadeeeee aadeeeee",
+    ("allgather_matmul", 2): "aaaaaabc aaaaadee aaaddeee aadeeeee adeeeeee deeeeeee",
+    ("allgather_matmul", 4): "aaaaabcc aaaaabcc aaaddeee aadeeeee adeeeeee deeeeeee",
+    ("allgather_matmul", 8): "aaabbccc aaabbccc aaabbccc aadeeeee adeeeeee deeeeeee",
+}
+
+
+@pytest.mark.parametrize("op,world", sorted(_FUSED_TILES))
+def test_tiles_of_several_gpus_do_not_follow_what_was_fitted_on_one(op, world, monkeypatch):
+    monkeypatch.delenv("CATCOC_CTA_PAIR", raising=False)
+    dtype = torch.int8 if op.startswith("quant") else torch.bfloat16
+    letter = {(64, 1): "a", (128, 1): "b", (256, 1): "c", (128, 2): "d", (256, 2): "e"}
+    for m, word in zip((256, 512, 1024, 2048, 4096, 16384), _FUSED_TILES[op, world].split()):
+        tiles = [chooser.heuristic(op, m, n, 4096, world, dtype) for n in (128, 512, 1024, 1696, 2048, 4096, 8192, 28672)]
+        assert "".join(letter[t.bn, t.cta_pair] for t in tiles) == word, (op, world, m)
+
+
 def test_mx_scale_packing_matches_the_tensor_core_block_layout():
     from mm_rs_with_catlass_b200.ops import mx
     x = torch.randn(200, 160) * torch.exp2(torch.randint(-6, 6, (200, 5)).float()).repeat_interleave(32, 1)
