@@ -119,7 +119,7 @@ def _with_out(args, out_ptr: int):
 def _resolve_tiling(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype,
                     tiling: Optional[TilingConfig]) -> TilingConfig:
     if tiling is not None:
-        return tiling.validate()
+        return tiling.validate(local=False)
     from ..tiling.chooser import choose
     return choose(op, m, n, k, world, dtype)
 

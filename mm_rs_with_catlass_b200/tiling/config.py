@@ -29,7 +29,7 @@ from typing import Dict
 @dataclass(frozen=True)
 class TilingConfig:
     # --- knobs of this kernel ---
-    bn: int = 0            # tile columns: 64, 128, 256 (0 = 256)
+    bn: int = 0            # tile columns: 64, 128, 256 (0 = 256); 192 on CTA pairs of a local product with B stored [N, K]
     swizzle: int = 0       # tiles per column group of the raster (0 = 8)
     num_ctas: int = 0      # persistent CTAs (0 = one per SM)
     seg_dim: int = -1      # all-reduce ownership split: 0 rows, 1 cols, -1 auto
@@ -53,16 +53,17 @@ class TilingConfig:
     comm_npu_split: int = 1
     comm_data_split: int = 4
 
-    def validate(self) -> "TilingConfig":
-        if self.bn not in (0, 64, 128, 256):
-            raise ValueError("bn must be 0, 64, 128 or 256 (got %d)" % self.bn)
+    def validate(self, local: bool = True) -> "TilingConfig":
+        """Raises ValueError for a setting that no launch takes; ``local=False``: none that communicates."""
+        if self.bn not in (0, 64, 128, 256) and not (self.bn == 192 and self.cta_pair == 2 and local):
+            raise ValueError("bn must be 0, 64, 128 or 256, or 192 for a local product on CTA pairs (got %d)" % self.bn)
         if self.swizzle < 0 or self.swizzle > 64:
             raise ValueError("swizzle must be in [0, 64]")
         if self.num_ctas < 0:
             raise ValueError("num_ctas must be >= 0")
         if self.cta_pair not in (0, 1, 2):
             raise ValueError("cta_pair must be 0, 1 or 2")
-        if self.cta_pair == 2 and self.bn not in (0, 128, 256):
+        if self.cta_pair == 2 and self.bn not in (0, 128, 192, 256):
             raise ValueError("cta_pair=2 needs bn of 128 or 256")
         if self.rounds < 0 or self.rounds > 64:
             raise ValueError("rounds must be in [0, 64]")

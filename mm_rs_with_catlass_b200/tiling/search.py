@@ -86,7 +86,7 @@ def workspace_bytes(p: Problem, t: TilingConfig) -> int:
 def infeasible_reason(p: Problem, t: TilingConfig) -> Optional[str]:
     """None when the tiling can run this problem, otherwise the violated rule."""
     try:
-        t.validate()
+        t.validate(local=p.op == "matmul" and p.trans_b)
     except ValueError as e:
         return str(e)
     bn = t.effective_bn

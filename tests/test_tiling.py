@@ -14,6 +14,14 @@ def test_config_validation():
     for bad in (dict(bn=96), dict(cta_pair=3), dict(bn=64, cta_pair=2), dict(seg_dim=2), dict(num_ctas=-1)):
         with pytest.raises(ValueError):
             TilingConfig(**bad).validate()
+    # what the chooser returns for local products is a valid setting, and stays one for them alone
+    t = chooser.heuristic("matmul", 200, 576, 4096, 1, torch.bfloat16, b_k_major=True, tails=True)
+    assert (t.bn, t.cta_pair) == (192, 2) and t.validate() is t and t.with_(swizzle=2).bn == 192
+    for bad in (lambda: t.with_(cta_pair=1), lambda: t.validate(local=False)):
+        with pytest.raises(ValueError, match="192"):
+            bad()
+    for op, trans_b, ok in (("matmul", True, True), ("matmul", False, False), ("matmul_reduce_scatter", True, False)):
+        assert (search.infeasible_reason(search.Problem(op, 512, 576, 4096, 1, trans_b=trans_b), t) is None) == ok
     assert TilingConfig().effective_bn == 256
     assert set(["m0", "n0", "k0", "comm_interval", "comm_tile_m", "comm_block_m", "comm_npu_split",
                 "comm_data_split"]) <= set(TilingConfig().to_dict())      # the reference's CocTilingParams fields
