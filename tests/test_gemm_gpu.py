@@ -227,8 +227,8 @@ def test_launch_plans_follow_the_data_not_the_first_call(catcoc, device):
     assert catcoc.matmul(a, b, out=out) is out
     _check_status(device, "plan hit with out")
     assert_close(out, a.float() @ b.float(), k=192)
-    # an A whose base TMA cannot address is padded inside the launch (from the caller's memory, on every
-    # call): planned like any other operand, and still always current
+    # an A whose base TMA cannot address is padded by a kernel ahead of the product (from the caller's memory, on
+    # every call): planned with the geometry of its pad pass, and still always current
     big = torch.randn(256, 200, device=device).bfloat16()
     av = big[:, 3:195]
     before = len(G._plans)
@@ -268,10 +268,9 @@ def test_activation_in_the_epilogue(catcoc, act, pair):
         catcoc.matmul(a, b, activation="tanh")
 
 
-def test_unaligned_a_is_padded_inside_the_launch(catcoc):
-    """An A whose row pitch (or base) is not a multiple of 16 bytes is padded by the kernel's own
-    communication warps while the product already runs: no padded copy is made beforehand, the
-    call is planned, and repeated calls (alternating workspace halves) stay correct."""
+def test_unaligned_a_is_padded_ahead_of_the_product(catcoc):
+    """An A whose row pitch (or base) is not a multiple of 16 bytes is re-pitched by the pad kernel ahead of
+    the product, into a buffer of its own on every call: the call is planned, and repeated calls stay correct."""
     from mm_rs_with_catlass_b200.ops import gemm as G
     from mm_rs_with_catlass_b200.utils.verify import assert_close
     dev = torch.device("cuda:0")

@@ -48,7 +48,8 @@ def test_ragged_lengths_and_slices(kv_lens, splits):
 @pytest.mark.parametrize("q_len", [2, 3, 4])
 @pytest.mark.parametrize("causal", [False, True])
 def test_several_new_tokens_with_and_without_mask(q_len, causal):
-    _case(2, q_len, 16, [260, 75], torch.bfloat16, causal=causal, seed=q_len)        # 32 to 64 rows: the 64-row form
+    for splits in (1, 2, None):      # 32 to 64 rows: the 64-row form of this kernel, and (None) the kernel for few rows
+        _case(2, q_len, 16, [260, 75], torch.bfloat16, causal=causal, splits=splits, seed=q_len)
     _case(2, q_len, 128, [260, 75], torch.bfloat16, causal=causal, splits=2, seed=q_len + 10)   # several 128-row chunks
 
 

@@ -59,6 +59,16 @@ def test_new_tokens_and_the_causal_mask(q_len, heads, causal):
     _case(q_len, heads, [260, 4, 128, 129, 1000, 131], torch.bfloat16, causal=causal, seed=q_len)
 
 
+@pytest.mark.parametrize("heads", [16, 32])
+@pytest.mark.parametrize("lens", [[129, 130, 257, 1, 131, 128, 132, 258], [129, 130, 257, 3] * 20])
+def test_chunks_that_see_nothing_of_a_last_page(heads, lens):
+    # two and four chunks of rows; the first tokens' chunks see no key of a last page of one to three keys, which is a piece of
+    # its own in the short list (a page per CTA) and the start or end of a longer run in the other
+    for dtype in (torch.bfloat16, torch.float16):
+        _case(4, heads, lens, dtype, causal=True, seed=heads + len(lens))
+    _case(3, heads, lens, torch.bfloat16, causal=True, seed=heads)
+
+
 @pytest.mark.parametrize("gain", [(0.0, 40.0), (40.0, 0.0)])
 def test_moving_reference_maximum(gain):
     _case(1, 16, [3000, 900], torch.bfloat16, gain=gain, seed=1)

@@ -1,10 +1,7 @@
 """Local products whose last wave of pair tiles is cut along K: ragged last tiles among the cut ones, all tiles cut, a
-short last slice, every epilogue; results against the direct kernel."""
+short last slice, every epilogue; results against the direct kernel (GPU). The rule gives a valid cut for every shape (CPU)."""
 import pytest
 import torch
-
-
-pytestmark = pytest.mark.gpu
 
 
 def _both(monkeypatch, cut, bn, a, b, **kw):
