@@ -48,8 +48,8 @@ CATCOC_DEVICE void rescale_o(uint32_t t_o, float alpha) {
 // first probability: with `move` (the same in all lanes) the reference maximum of some row of the warp moved and O has to
 // be multiplied by alpha. `half()` is called when the probabilities of the first 64 keys have been issued. `vis_left`: keys of this block the row sees (used when `masked`).
 //
-// A quarter of the exponentials as a degree-5 polynomial on the FMA pipe was measured slower (causal 2 x 32 x 8192:
-// 1019 against 980 us): a chain of one row's steps, not the special-function unit, is what a tile waits for.
+// A quarter of the exponentials as a degree-5 polynomial on the FMA pipe gave no clear gain (4 % slower to 0.5 % faster in three
+// trials): a chain of one row's steps, not the special-function unit, is what a tile waits for.
 template <int FMT, class Loaded, class Before, class Half>
 CATCOC_DEVICE void softmax_row_block(uint32_t t_s, uint32_t t_p, bool masked, int vis_left, float sc, RowState& st, Loaded&& loaded,
                                      Before&& before, Half&& half) {

@@ -1,11 +1,15 @@
-"""Multi-head latent attention, decode step over a paged latent cache (``csrc/kernels/mla_decode.cu``).
+"""Multi-head latent attention, decode step over a paged latent cache (``csrc/kernels/mla_rows.cu`` and
+``mla_decode.cu``).
 
 All query heads share one key / value stream: a 512-wide latent that is key and value at once,
 plus a 64-wide rotary part that only the scores see. ``q_nope`` has already been multiplied by
 the key up-projection (the "absorbed" form), so the kernel is attention with 576-wide keys and
-512-wide values over a cache of 128-key pages. One CTA owns up to 128 query rows (new tokens x
-heads of one sequence), one half of the output columns and one slice of the sequence; the slices
-are merged by a second small kernel (flash decoding).
+512-wide values over a cache of 128-key pages. With at most 128 query rows per sequence (new tokens x
+heads) the keys are the M side of both products: a CTA holds 16 or 32 rows with all output columns, and
+the pages of all sequences, by their lengths on the device, are dealt out over the SMs. More rows, or an
+explicit number of slices, take the general kernel: a CTA owns up to 128 rows, one half of the output
+columns and one slice of a sequence. In both the pieces of a sequence are merged by a second small kernel
+(flash decoding).
 
 The reference carries the same computation as 3rdparty/catlass/examples/19_mla/mla_kernel.cpp;
 argument layouts and the golden follow its gen_data.py.
