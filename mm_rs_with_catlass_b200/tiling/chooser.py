@@ -30,6 +30,9 @@ _NUM_SMS = 148
 # bound by the fill rate of shared memory, so halving the width costs far more than half.
 _TILE_EFF = {256: 1.0, 192: 0.85, 128: 0.56, 64: 0.43}
 _PAIR_GAIN = {256: 1.18, 192: 1.18, 128: 1.35}     # 2-CTA tiles: each CTA fills half of B (192: pairs only)
+# int8: a pair of 256 columns in a single wave loses to 128-column tiles (256 x 8192 x 1024: 16.4 against 12.8 us, 205 x 8192 x
+# 3584: 21.8 against 19.9), and over several waves the choice is the same with either figure
+_PAIR_GAIN_INT8 = {256: 1.10, 128: 1.35}
 _PAIR_GAIN_FUSED = {256: 1.10, 128: 1.35}          # ... of a launch that also communicates (measured on 2 to 8 GPUs)
 
 
@@ -45,7 +48,8 @@ _FOLD = 8000.0                    # the second kernel and the gap before it
 _INT8_EPILOGUE = 10000.0          # the dequantising epilogue of the direct kernel, which the second kernel spreads over all SMs
 
 
-def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bool = False, fused: bool = False) -> float:
+def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bool = False,
+              gain: Optional[dict] = None) -> float:
     """Relative time of a GEMM whose rows come in ``nseg`` segments of ``seg_rows`` rows (tiles never
     straddle segments): waves of tiles x time of one wave. With ``seg_cols`` the output is cut into
     ``nseg`` column segments instead and ``seg_rows`` is the full row count."""
@@ -56,7 +60,7 @@ def tile_cost(seg_rows: int, nseg: int, n: int, bn: int, pair: int, seg_cols: bo
         tiles = nseg * math.ceil(seg_rows / bm) * math.ceil(n / bn)
     units = _NUM_SMS // pair
     waves = math.ceil(tiles / units)
-    eff = _TILE_EFF[bn] * ((_PAIR_GAIN_FUSED if fused else _PAIR_GAIN)[bn] if pair == 2 else 1.0)
+    eff = _TILE_EFF[bn] * ((gain or _PAIR_GAIN)[bn] if pair == 2 else 1.0)
     return waves * bn / eff
 
 
@@ -103,6 +107,7 @@ def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b
         seg_rows = rows
     forced = os.environ.get("CATCOC_CTA_PAIR")
     best = None
+    gain = _PAIR_GAIN_FUSED if fused else _PAIR_GAIN_INT8 if dtype == torch.int8 else _PAIR_GAIN
     for pair in (2, 1):
         if forced in ("1", "2") and pair != int(forced):
             continue
@@ -117,9 +122,9 @@ def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b
                 continue
             if dtype == torch.int8 and (bn < 128 or (pair == 2 and bn < 256)):
                 continue   # 8-bit [K, N] operands need a full 128-byte run of N per TMA box and CTA
-            cost = tile_cost(seg_rows, nseg, n, bn, pair, seg_cols=ar_cols, fused=fused)
+            cost = tile_cost(seg_rows, nseg, n, bn, pair, seg_cols=ar_cols, gain=gain)
             if tails and pair == 2:
-                cost = tail_cut(rows, n, k, dtype.itemsize, bn)[0] * bn / (_TILE_EFF[bn] * _PAIR_GAIN[bn])
+                cost = tail_cut(rows, n, k, dtype.itemsize, bn)[0] * bn / (_TILE_EFF[bn] * gain[bn])
             if best is None or cost < best[0] - 1e-9:
                 best = (cost, bn, pair)
     if best is None:
@@ -163,7 +168,8 @@ def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
     waves = -(-(-(-m // (128 * pair)) * -(-n // bn0)) // (_NUM_SMS // pair))
     if pair == 2 and bn0 >= 128:
         waves = tail_cut(m, n, k, elt, bn0)[0]
-    best, best_time = None, 0.95 * (max(hbm, waves * kb * unit(bn0, pair)) + _LAUNCH + (_INT8_EPILOGUE if elt == 1 else 0.0))
+    # (for 8-bit operands the model puts a cut rather high: 256 x 8192 x 7168 30.5 us direct, 25.7 cut)
+    best, best_time = None, (0.97 if elt == 1 else 0.95) * (max(hbm, waves * kb * unit(bn0, pair)) + _LAUNCH + (_INT8_EPILOGUE if elt == 1 else 0.0))
     for bn in (256, 128):
         if n < bn and bn > 128:
             continue

@@ -115,6 +115,16 @@ def test_heuristic_follows_the_cost_model_and_is_deterministic():
     assert chooser.choose("matmul_reduce_scatter", 8192, 8192, 3584, 8, torch.bfloat16, table=tbl).bn == 128
 
 
+def test_int8_products_of_one_wave_take_narrow_tiles():
+    for m, n, k in ((205, 8192, 3584), (256, 8192, 1024), (700, 2048, 2048), (2048, 1024, 1024)):
+        t = chooser.heuristic("matmul", m, n, k, 1, torch.int8, tails=True)
+        assert (t.bn, t.cta_pair) == (128, 1) and chooser.split_k(m, n, k, 1, t) is None
+    t = chooser.heuristic("matmul", 256, 8192, 7168, 1, torch.int8, tails=True)
+    assert chooser.split_k(256, 8192, 7168, 1, t) is not None                # long enough to cut
+    t = chooser.heuristic("matmul", 1024, 8192, 28672, 1, torch.int8, tails=True)
+    assert (t.bn, t.cta_pair) == (256, 2)
+
+
 # Tiles of launches on several GPUs, as fitted there: M of 256, 512, 1024, 2048, 4096, 16384 (one word each) by N of 128, 512,
 # 1024, 1696, 2048, 4096, 8192, 28672 (one letter each: a 64, b 128, c 256 columns; d 128, e 256 on CTA pairs)
 _FUSED_TILES = {
