@@ -192,7 +192,11 @@ def grouped(rows_total: int, rows_per_group: float, n: int, dtype: torch.dtype) 
     well (32 ragged groups of 440 rows on average: 230 -> 210 us from a cold start, 273 -> 282 us in a loop;
     937 rows: 429 -> 388 us), so ragged groups count 1.10. Few rows per group: 16 groups of 9 rows, 4096 x 2048:
     59 -> 50 us on wide tiles (the tiles used to be chosen for the rows of all groups as one product)"""
-    forced = os.environ.get("CATCOC_CTA_PAIR")
+    return _grouped(rows_total, rows_per_group, n, dtype, os.environ.get("CATCOC_CTA_PAIR"))
+
+
+@functools.lru_cache(maxsize=4096, typed=True)      # an exact row count and an equal mean are different questions
+def _grouped(rows_total: int, rows_per_group: float, n: int, dtype: torch.dtype, forced: Optional[str]) -> TilingConfig:
     exact = isinstance(rows_per_group, int)
     groups = rows_total / max(rows_per_group, 1e-9)
     best = (0.0, 256, 1)

@@ -21,3 +21,7 @@ def test_choice_follows_the_waves():
     assert grouped(8 * 1024, 1024, 8192, torch.bfloat16).cta_pair == 2          # whole 256-row tiles
     assert grouped(14080, 440.0, 4096, torch.bfloat16).cta_pair == 1            # half a tile of padding in each of 32 groups
     assert grouped(148, 18.5, 1408, torch.bfloat16).effective_bn < 256          # 48 wide tiles for 148 SMs
+    # an exact row count and an equal mean are different questions, in either order
+    assert [grouped(8 * 512, r, 8192, torch.bfloat16).cta_pair for r in (512.0, 512, 512.0)] == [
+        grouped(8 * 512, float(512), 8192, torch.bfloat16).cta_pair, 2, grouped(8 * 512, 512.0, 8192, torch.bfloat16).cta_pair]
+    assert grouped(14080, 440, 4096, torch.bfloat16) is not grouped(14080, 440.0, 4096, torch.bfloat16)
