@@ -212,3 +212,9 @@ def test_a_raw_shard_on_one_rank_is_refused():
     args = _cut_product(mode=N.MODE_AG, ag_raw=1, ag_m=64, ag_ld=1024)
     args.gathered[0], args.gflags[0] = 4096, 4096
     assert N.lib().catcoc_fused_launch(C.byref(args), None) == N.E_UNSUPPORTED and "raw shard" in N.last_error()
+
+
+def test_short_decode_runs_take_one_launch():
+    need = N.lib().catcoc_flash_decode_workspace_bytes
+    assert need(4, 32, 4, 1, 576, 128) == 0 and need(8, 32, 4, 2, 700, 128) == 0 and need(1, 32, 32, 4, 640, 64) == 0
+    assert need(1, 32, 4, 1, 800, 128) > 0 and need(16, 32, 8, 1, 4096, 128) > 0      # seven blocks and more are cut
