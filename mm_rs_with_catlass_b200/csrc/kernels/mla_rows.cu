@@ -21,7 +21,7 @@
 // four, and a slot is free again as soon as its quarter of the second product is done.
 //
 // Bound by HBM and the depth of the slots: batch 32, 16 heads, 2048 to 4096 keys (113 MB), in a loop: 82 us in mla_decode.cu,
-// 31 us here (3.6 TB/s); with 12288 keys on average 259 -> 99 us (4.6 TB/s). Straight-line code is kept short on purpose: a run is a few
+// 31 us here (3.7 TB/s); with 12288 keys on average 232 -> 81 us (5.6 TB/s). Straight-line code is kept short on purpose: a run is a few
 // pages, and with everything unrolled the instruction fetch of a cold launch cost up to 50 us.
 //
 // The reference carries this computation as 3rdparty/catlass/examples/19_mla/mla_kernel.cpp.
@@ -564,11 +564,14 @@ int encode_map(CUtensorMap* tm, const void* base, CUtensorMapDataType dt, int ra
 extern "C" int64_t catcoc_mla_rows_workspace_bytes(int B, int q_len, int H, int max_pages) {
   if (B <= 0 || q_len < 1 || q_len > 4 || H <= 0 || max_pages <= 0) return -1;
   const int64_t rows = static_cast<int64_t>(q_len) * H;
-  // Up to four chunks of 32 rows read a page side by side (from L2 but for the first). Measured against mla_decode.cu with
-  // the L2 flushed, batch 32, sequences of 2048 to 4096 keys, bf16: 16 rows 89 -> 42 us, 32 rows 89 -> 44, 64 rows 93 -> 58,
-  // 128 rows 151 -> 91; batch 1, one page: 17 -> 15 us. More rows have more chunks than that kernel has column halves.
+  // Up to four chunks of 32 rows read a page side by side (from L2 but for the first). Measured against mla_decode.cu in a
+  // loop, batch 32, sequences of 2048 to 4096 keys, bf16: 16 rows 83 -> 29 us, 32 rows 83 -> 33, 64 rows 87 -> 47, 128 rows
+  // 148 -> 79. More rows have more chunks than that kernel has column halves.
   if (rows > 128) return -1;
   if (B > 65535 || static_cast<int64_t>(B) * max_pages > (1 << 24)) return -1;
+  // One page a sequence: the general kernel is a single launch, which is what such a call waits for (batch 1 to 128, 16 to 128
+  // rows, back to back: 19 to 21 us against 24). Larger batches are several waves of its CTAs.
+  if (max_pages == 1 && B <= 128) return -1;
   const RowsPlan d = rows_plan(static_cast<int>(rows));
   return static_cast<int64_t>(d.runs) * 2 * d.chunks * d.n * (mlar::kDV + 2) * static_cast<int64_t>(sizeof(float)) + B * static_cast<int64_t>(sizeof(int2));
 }

@@ -46,7 +46,7 @@ def _case(q_len, heads, lens, dtype, causal=False, gain=None, seed=0, extra_page
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("lens", [[1], [128], [129], [0, 5, 0], [0, 0, 300], [4096, 0, 17, 2050, 128], [700] * 150,
+@pytest.mark.parametrize("lens", [[1], [128], [129], [0, 5, 0], [0, 0, 300], [4096, 0, 17, 2050, 128], [700] * 150, [100] * 140,
                                   [(37 * i) % 900 for i in range(70)], [20000]])
 @pytest.mark.parametrize("heads", [16, 5, 32, 17])
 def test_runs_of_pages(lens, dtype, heads):

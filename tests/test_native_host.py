@@ -214,7 +214,10 @@ def test_a_raw_shard_on_one_rank_is_refused():
     assert N.lib().catcoc_fused_launch(C.byref(args), None) == N.E_UNSUPPORTED and "raw shard" in N.last_error()
 
 
-def test_short_decode_runs_take_one_launch():
+def test_short_decode_runs_and_one_page_sequences_take_one_launch():
     need = N.lib().catcoc_flash_decode_workspace_bytes
     assert need(4, 32, 4, 1, 576, 128) == 0 and need(8, 32, 4, 2, 700, 128) == 0 and need(1, 32, 32, 4, 640, 64) == 0
     assert need(1, 32, 4, 1, 800, 128) > 0 and need(16, 32, 8, 1, 4096, 128) > 0      # seven blocks and more are cut
+    rows = N.lib().catcoc_mla_rows_workspace_bytes
+    assert rows(1, 1, 16, 1) == -1 and rows(128, 4, 32, 1) == -1
+    assert rows(129, 1, 16, 1) > 0 and rows(1, 1, 16, 2) > 0
