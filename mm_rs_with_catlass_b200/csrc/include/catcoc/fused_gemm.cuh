@@ -986,14 +986,14 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
       }
 
       // Dequantisation: the row's scale is read once per tile, the columns' scales and the int32 bias four at a time (one load
-      // per element made the epilogue longer than a short mainloop: int8, from a cold start, 32 ragged groups of 440 rows,
-      // 4096 x 2048: 247 -> 174 us, 16 groups of 1875, 2048 x 2048: 187 -> 155 us; a long K, 28672, gains nothing).
+      // per element made the epilogue longer than a short mainloop: int8, in a loop, 32 ragged groups of 440 rows,
+      // 4096 x 2048: 197 -> 170 us, 16 groups of 1875, 2048 x 2048: 189 -> 163 us; a long K, 28672, gains nothing).
       float row_scale = 1.0f;
       if (kScale && dequant && own && p.scale_m != nullptr && ti.m0 + row_in_tile < sched.M) row_scale = p.scale_m[ti.m0 + row_in_tile];
 
       // A group's last rows end inside the output, where TMA cannot clip: their 16-bit values leave from the registers, whole
       // 32-byte sectors of the lane's own row, where rows and the tile's columns allow it (64 groups of 31
-      // rows, 2048 x 1024, int8: 69 -> 61 us, bf16 56 -> 53; 32 groups of 440 rows, 4096 x 2048, bf16: no gain in a loop).
+      // rows, 2048 x 1024, int8: 75 -> 63 us, bf16 56 -> 55; 32 groups of 440 rows, 4096 x 2048, int8: 178 -> 170, bf16: no clear gain).
       const bool row_direct = !fused && own && !tma_out && dst_ok && st_elt == 2 && base != nullptr && (ti.cols & 31) == 0 &&
                               ((reinterpret_cast<uintptr_t>(base) | static_cast<uintptr_t>(pitch)) & 31) == 0;
 

@@ -15,8 +15,8 @@
 // 56 % of the time, the special-function unit as much). So the scores are read from TMEM once and stay in registers
 // (softmax_row.cuh; a split of the registers between the warpgroups makes room), and P V starts when the first 64
 // keys' probabilities are written. Causal, 2 x 32 / 8 heads x 8192, D = 128, in a loop (which holds the clocks at the power
-// limit): 1193 -> 1072 us, and 1038 us (1.06 PFLOP/s) in the CTA order below. At D = 64 the probabilities have columns of
-// their own (O_0, O_1 at 256 and 320, P_0, P_1 at 384 and 448), which takes P V out of the chain: 771 -> 705 us.
+// limit): 1196 -> 1065 us, and 1036 us (1.06 PFLOP/s) in the CTA order below. At D = 64 the probabilities have columns of
+// their own (O_0, O_1 at 256 and 320, P_0, P_1 at 384 and 448), which takes P V out of the chain: 776 -> 719 us.
 //
 // The online-softmax recurrence (m: reference maximum, l: running sum, per row, in the log2 domain):
 //   P = exp2(scale S - m),  l' = l a + rowsum(P),  O' = O a + P V,  a = exp2(m - m')
@@ -432,7 +432,7 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
   if (ctas > 0x7fffffff) { set_error("flash_attention: too many query tiles"); return CATCOC_E_TOO_LARGE; }
   p.tiles = (Sq + rows_cta - 1) / rows_cta;
   // Causal tiles differ in length, and with one head after the other the launch ended with the long tiles of its last
-  // heads (causal 2 x 32 x 8192 in a loop: 1075 -> 1038 us). Heads side by side share the L2, so their keys and values must fit it.
+  // heads (in a loop, causal 2 x 32 x 8192: 1065 -> 1036 us, 1 x 32 x 4096: 183 -> 150). Heads side by side share the L2, so their keys and values must fit it.
   const int64_t kv_bytes = static_cast<int64_t>(Sk) * D * 4;
   p.order_heads = causal ? static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(static_cast<int64_t>(B) * Hq, (72ll << 20) / kv_bytes * (Hq / Hk)))) : 1;
   p.causal = causal ? 1 : 0;
