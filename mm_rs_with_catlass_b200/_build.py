@@ -34,6 +34,9 @@ SOURCES = [
     "kernels/inst/f16_pair.cu",
     "kernels/inst/f16_slice_k.cu",
     "kernels/inst/pair_tail.cu",
+    "kernels/inst/double_f16.cu",
+    "kernels/inst/double_8bit.cu",
+    "kernels/inst/double_swapped.cu",
     "kernels/inst/i8_single.cu",
     "kernels/inst/i8_pair.cu",
     "kernels/inst/f8_single.cu",

@@ -37,7 +37,8 @@ LIM_STAGE, LIM_ARRIVE, LIM_DONE, LIM_AR_OUT, LIM_GATHERED, LIM_GFLAGS, LIM_PART,
 class Tiling(C.Structure):
     _fields_ = [("bn", C.c_int), ("swizzle", C.c_int), ("num_ctas", C.c_int), ("seg_dim", C.c_int),
                 ("use_multicast", C.c_int), ("rounds", C.c_int), ("cta_pair", C.c_int), ("pull", C.c_int),
-                ("comm_warps", C.c_int), ("push_tma", C.c_int)]
+                ("comm_warps", C.c_int), ("push_tma", C.c_int), ("twice", C.c_int), ("swap", C.c_int),
+                ("cut_slices", C.c_int), ("cut_k", C.c_int)]
 
 
 class OpArgs(C.Structure):
@@ -114,6 +115,9 @@ def _declare(lib) -> None:
         "catcoc_slice_k_launch": (i32, [P(OpArgs), vp, vp]),
         "catcoc_splitk_workspace_bytes": (i64, [i32, i32, i32]),
         "catcoc_splitk_launch": (i32, [P(OpArgs), i32, i32, vp, vp]),
+        "catcoc_double_workspace_bytes": (i64, [P(OpArgs)]),
+        "catcoc_double_launch": (i32, [P(OpArgs), vp, vp]),
+        "catcoc_double_plan_replay": (i32, [i32, i32, i32, i32, i32, i32, i32, i32, P(i32)]),
         "catcoc_tail_workspace_bytes": (i64, [i32, i32, i32, i32, i32]),
         "catcoc_tail_launch": (i32, [P(OpArgs), i32, i32, i32, vp, vp]),
         "catcoc_stage_bytes": (i64, [i32, i32, i32, i32, i32, i32, i32]),

@@ -51,6 +51,12 @@ typedef struct CatcocTiling {
   int comm_warps;  /* communication / reducer warps per CTA, 1..5 (0 = 5); all-gather and pull flavours */
   int push_tma;    /* push flavour: 1 = partial tiles go to their owners' slabs by TMA stores (stamps one tile
                       late), 0 = by 16-byte stores, -1 = CATCOC_PUSH_TMA decides (default off)            */
+  int twice;       /* local products with cta_pair 2: 1 = tiles of two accumulators, 256 x 2 bn, bn any multiple of
+                      32 from 64 to 256; 0 = one accumulator                                         */
+  int swap;        /* ... with the output's columns along the tiles' rows: 256 columns x 2 bn rows of the output; 16-bit
+                      and int8 operands, no C; over ragged groups the halves are made for each group (bn 256) */
+  int cut_slices;  /* ... and the units of 256 x bn past the last full wave cut along K into this many slices */
+  int cut_k;       /*     of cut_k elements (catcoc_double_launch); 0 = not cut                       */
 } CatcocTiling;
 
 typedef struct CatcocOpArgs {
@@ -152,6 +158,14 @@ int catcoc_splitk_launch(const CatcocOpArgs* args, int slices, int k_slice, void
  * to `workspace` (128-byte aligned, catcoc_tail_workspace_bytes(...) bytes), a second kernel sums them and runs the epilogue. */
 int64_t catcoc_tail_workspace_bytes(int M, int N, int bn, int first, int slices);
 int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slices, int k_slice, void* workspace, void* stream);
+
+/* A local product on double tiles (args->tiling: cta_pair 2, twice, cut_slices and cut_k): the units past the last full wave
+ * run as slices along K whose fp32 (int8: int32) planes go to `workspace` (128-byte aligned, catcoc_double_workspace_bytes); a
+ * second kernel sums them in slice order and runs the epilogue that `args` describes. */
+int catcoc_double_launch(const CatcocOpArgs* args, void* workspace, void* stream);
+int64_t catcoc_double_workspace_bytes(const CatcocOpArgs* args);
+/* Host replay of the double-tile plan: writes {kind, m0, n0, rows, cols, slice} of a worker's items, returns how many. */
+int catcoc_double_plan_replay(int M, int N, int bn, int swizzle, int workers, int slices, int worker, int max_items, int32_t* out);
 
 /* Workspace sizes (bytes / words) for given problem + tiling, identical on every rank. */
 int64_t catcoc_stage_bytes(int M, int N, int W, int seg_dim, int bn, int cta_pair, int partial_fmt);

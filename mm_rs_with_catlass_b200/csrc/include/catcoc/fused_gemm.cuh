@@ -88,6 +88,7 @@ struct SmemTail {
   uint64_t empty[kMaxStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+  uint64_t drain;      // double tiles: the MMAs of an aborted launch have retired
   uint32_t tmem_base;
   uint32_t abort_flag;
   uint32_t dead;   // the status block already held an error when this CTA started

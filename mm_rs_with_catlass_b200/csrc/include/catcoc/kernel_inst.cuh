@@ -92,6 +92,14 @@ cudaError_t launch_slice_k(bool pair, const FusedParamsGk& p, int grid, cudaStre
 cudaError_t prepare_tail();
 cudaError_t launch_tail(int kind, bool full, const FusedParamsTail& p, int grid, cudaStream_t s);
 
+// Double tiles of local products (kernels/inst/double_*.cu)
+cudaError_t prepare_double();
+cudaError_t launch_double(int kind, bool full, const FusedParams& p, int grid, cudaStream_t s);
+cudaError_t launch_double_f16(bool full, const FusedParams& p, int grid, cudaStream_t s);
+cudaError_t launch_double_8bit(int kind, bool full, const FusedParams& p, int grid, cudaStream_t s);
+cudaError_t launch_double_tokens(int kind, bool full, const FusedParamsTok& p, int grid, cudaStream_t s);
+cudaError_t launch_double_slice_k(const FusedParamsGk& p, int grid, cudaStream_t s);
+
 }  // namespace inst
 }  // namespace catcoc
 

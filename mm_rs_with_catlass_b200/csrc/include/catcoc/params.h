@@ -82,6 +82,17 @@ enum CheckSite : uint32_t {
 // [3] expected, [4] seen, [5] peer, [6] blockIdx, [7] reserved.
 constexpr int kStatusWords = 8;
 
+// Double tiles of local products (double_tile.cuh): a pair's two accumulators belong to one tile.
+struct DoubleTile {
+  int bn;            // columns of one accumulator, a multiple of 32; 0: off
+  int b_half;        // bytes of one half's B block in a stage (A is in front of the two), of a stage
+  int stage_bytes, sf_off;   // where a stage's scales start
+  int stages;
+  int lead;          // K blocks that half 0 runs ahead of half 1 at the ends of a tile
+  int swap;          // roles swapped: the tiles' rows are the output's columns (features) and their columns its rows (tokens)
+  DoublePlan plan;   // without groups; the planes of its cut units are described by tm_part[0]
+};
+
 struct alignas(64) FusedParams {
   CUtensorMap tm_a;          // A operand (AG: this rank's shard)
   CUtensorMap tm_a_gath[2];  // AG: gathered A, one map per parity buffer
@@ -208,6 +219,7 @@ struct alignas(64) FusedParams {
   // the host turns the ring into a Chrome trace (utils/trace.py).
   uint32_t* events;
   uint32_t events_cap;       // records the ring can hold
+  DoubleTile dt;
 };
 
 // Ragged K ranges (a kernel instantiation of its own): group g multiplies the K rows [range[g].x, range[g].y) of an A stored
@@ -218,6 +230,12 @@ constexpr int kMaxKGroups = 64;
 struct alignas(64) FusedParamsGk : FusedParams {
   CUtensorMap gk_map[2 * kMaxKGroups];
   int2 gk_range[kMaxKGroups];
+};
+
+// Ragged groups of tokens with swapped roles (a kernel instantiation of its own, double_tile.cuh): the tokens under one map for
+// each width that half a tile can have, map i for 32 (i + 1) tokens, 16 (i + 1) of them in each CTA of the pair.
+struct alignas(64) FusedParamsTok : FusedParams {
+  CUtensorMap tok_map[8];
 };
 
 // A last wave that is nearly empty (a kernel instantiation of its own, local products): the tiles from `tail_first` on are cut

@@ -225,6 +225,13 @@ CATCOC_DEVICE uint64_t make_smem_desc_sw128(uint32_t smem_addr, uint32_t lbo_byt
   return d;
 }
 
+// A descriptor from its low word (which holds the address) and its high word
+CATCOC_DEVICE uint64_t desc_of(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+
 // Instruction descriptor for kind::f16 / kind::i8 / kind::f8f6f4 (dense, no negate, no saturate).
 //   c_fmt: 0 f16, 1 f32, 2 s32.  a_fmt/b_fmt: f16 kinds 0 f16, 1 bf16; i8 kind 0 u8, 1 s8;
 //   f8f6f4 kind 0 e4m3, 1 e5m2.  *_mn_major: 1 when the operand is M/N-contiguous in smem.
@@ -404,18 +411,6 @@ CATCOC_DEVICE void tmem_cp_32x128b_warpx4(uint32_t taddr, uint64_t sdesc) {
 CATCOC_DEVICE void tmem_cp_32x128b_warpx4_pair(uint32_t taddr, uint64_t sdesc) {
   asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
-// Pair form: 256 rows, the scales of A by CTA (its 128 rows), those of all N columns of B in both
-CATCOC_DEVICE void umma_mxf8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                  uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], p;\n\t"
-      "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)
-      : "memory");
-}
 // D[tmem] (+)= (A * 2^(sfa-127)) (B * 2^(sfb-127)) with one UE8M0 scale per 32 K-elements.
 CATCOC_DEVICE void umma_mxf8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                              uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
@@ -531,7 +526,32 @@ CATCOC_DEVICE void tcgen05_commit_pair(uint64_t* bar, uint16_t cta_mask) {
 CATCOC_UMMA_PAIR(umma_f16_pair, "f16")
 CATCOC_UMMA_PAIR(umma_i8_pair, "i8")
 CATCOC_UMMA_PAIR(umma_f8f6f4_pair, "f8f6f4")
+// Two products of one A in a row: the first keeps A in the collector buffer, the second takes it from there.
+CATCOC_UMMA_PAIR(umma_f16_pair_fill, "f16.collector::a::fill")
+CATCOC_UMMA_PAIR(umma_i8_pair_fill, "i8.collector::a::fill")
+CATCOC_UMMA_PAIR(umma_f8f6f4_pair_fill, "f8f6f4.collector::a::fill")
+CATCOC_UMMA_PAIR(umma_f16_pair_use, "f16.collector::a::lastuse")
+CATCOC_UMMA_PAIR(umma_i8_pair_use, "i8.collector::a::lastuse")
+CATCOC_UMMA_PAIR(umma_f8f6f4_pair_use, "f8f6f4.collector::a::lastuse")
 #undef CATCOC_UMMA_PAIR
+// Block-scaled pair form: 256 rows, the scales of A by CTA (its 128 rows), those of all N columns of B in both
+#define CATCOC_UMMA_MX_PAIR(NAME, COLLECTOR)                                                     \
+  CATCOC_DEVICE void NAME(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,       \
+                          uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {             \
+    asm volatile(                                                                                  \
+        "{\n\t"                                                                                    \
+        ".reg .pred p;\n\t"                                                                        \
+        "setp.ne.b32 p, %6, 0;\n\t"                                                                \
+        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale" COLLECTOR                            \
+        " [%0], %1, %2, %3, [%4], [%5], p;\n\t"                                                    \
+        "}\n" ::"r"(tmem_d),                                                                       \
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)        \
+        : "memory");                                                                               \
+  }
+CATCOC_UMMA_MX_PAIR(umma_mxf8_pair, "")
+CATCOC_UMMA_MX_PAIR(umma_mxf8_pair_fill, ".collector::a::fill")
+CATCOC_UMMA_MX_PAIR(umma_mxf8_pair_use, ".collector::a::lastuse")
+#undef CATCOC_UMMA_MX_PAIR
 
 // ---------------------------------------------------------------------------------------
 // Scoped global loads / stores used for cross-GPU signalling and data movement
@@ -603,6 +623,7 @@ CATCOC_DEVICE void st_shared_v4(uint32_t saddr, uint4 v) {
                "r"(v.z), "r"(v.w)
                : "memory");
 }
+CATCOC_DEVICE void st_shared_u32(uint32_t saddr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(saddr), "r"(v) : "memory"); }
 CATCOC_DEVICE uint4 ld_shared_v4(uint32_t saddr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"

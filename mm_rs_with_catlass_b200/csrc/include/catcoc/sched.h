@@ -297,6 +297,139 @@ CATCOC_HD int group_walk_total(const TileSched& s, int num_groups, const int32_t
   return total;
 }
 
+// ---------------------------------------------------------------------------------------
+// Double tiles (double_tile.cuh): the output is cut into units of 256 rows x bn columns. Two neighbours run as one double
+// tile, which is the cheaper form; single units even out what whole double tiles leave to the last wave, and the units past
+// the last full wave may be cut along K, every slice an item of its own whose raw accumulator goes to a plane.
+//
+// The doubles come first (tile order of `sched`, whose BN is 2 bn and which leaves out an odd last column of units), then the
+// units of the double tiles that are not run as doubles, then the odd column's. The last `cut` units are the cut ones.
+// ---------------------------------------------------------------------------------------
+struct DoublePlan {
+  int workers;       // CTA pairs
+  int doubles;       // tiles run as doubles
+  int singles;       // units run whole
+  int cut, slices, slice_k;
+};
+
+CATCOC_HD TileSched make_double_sched(int M, int N, int bn, int swizzle) {
+  TileSched s = make_sched(M, N, 256, 2 * bn, 1, SEG_ROWS, 0, swizzle);
+  s.seg_nt = ceil_div(N, bn) / 2;
+  s.tiles_per_seg = s.total_tiles = s.seg_mt * s.seg_nt;
+  return s;
+}
+
+// slices < 2: no unit is cut
+CATCOC_HD DoublePlan make_double_plan(const TileSched& s, int bn, int workers, int slices, int slice_k) {
+  DoublePlan d;
+  const int units = s.seg_mt * ceil_div(s.N, bn);
+  d.workers = workers;
+  d.slices = slices < 2 ? 0 : slices;
+  d.slice_k = slice_k;
+  d.cut = slices < 2 ? 0 : units % workers;
+  const int waves = (units - d.cut + workers - 1) / workers;      // units of the busiest worker
+  d.doubles = imin(s.total_tiles, waves / 2 * workers);
+  if (2 * d.doubles > units - d.cut) d.doubles = (units - d.cut) / 2;   // the cut units are singles
+  d.singles = units - d.cut - 2 * d.doubles;
+  return d;
+}
+
+struct DoubleItem {
+  int kind;      // 0: none left, 1: double tile `index`, 2: unit `index`, 3: unit `index`, slice `slice`
+  int index, slice;
+};
+
+// The i-th item of a worker. Doubles go round; the workers that have one double less than the others take two singles each
+// first; then everything goes round again.
+CATCOC_HD DoubleItem double_item(const DoublePlan& d, int worker, int i) {
+  DoubleItem it = {0, 0, 0};
+  const int W = d.workers;
+  const int nd = d.doubles > worker ? (d.doubles - worker - 1) / W + 1 : 0;
+  if (i < nd) { it.kind = 1; it.index = worker + i * W; return it; }
+  i -= nd;
+  const int r = d.doubles % W;
+  const int level = r > 0 ? imin(d.singles, 2 * (W - r)) : 0;
+  if (worker >= r && r > 0) {
+    const int nl = (level > worker - r ? 1 : 0) + (level > worker - r + (W - r) ? 1 : 0);
+    if (i < nl) { it.kind = 2; it.index = worker - r + i * (W - r); return it; }
+    i -= nl;
+  }
+  const int rest = d.singles - level;
+  const int ns = rest > worker ? (rest - worker - 1) / W + 1 : 0;
+  if (i < ns) { it.kind = 2; it.index = level + worker + i * W; return it; }
+  i -= ns;
+  const int u = worker + i * W;
+  if (u < d.cut * d.slices) { it.kind = 3; it.index = d.singles + u / d.slices; it.slice = u % d.slices; }
+  return it;
+}
+
+// Extent of double tile `index`, or of unit `index` of those that are not part of one
+CATCOC_HD TileInfo double_tile_extent(const TileSched& s, int index) { return get_tile(s, index); }
+CATCOC_HD TileInfo double_unit_extent(const TileSched& s, const DoublePlan& d, int bn, int index) {
+  const int split = 2 * (s.total_tiles - d.doubles);
+  TileInfo ti;
+  if (index < split) {
+    ti = get_tile(s, d.doubles + index / 2);
+    ti.n0 += (index & 1) * bn;
+  } else {
+    ti.seg = 0;
+    ti.mi = index - split;
+    ti.ni = s.seg_nt;
+    ti.m0 = ti.mi * s.BM;
+    ti.n0 = s.seg_nt * s.BN;
+    ti.rows = imin(s.BM, s.M - ti.m0);
+    ti.tile_in_seg = 0;
+  }
+  ti.cols = imin(bn, s.N - ti.n0);
+  return ti;
+}
+
+// Ragged groups of tokens on double tiles whose columns are tokens (swapped roles): a group's tokens are spread evenly over as
+// few tiles as hold them, in halves of a multiple of 32, and every tile of tokens meets all blocks of 256 features.
+struct TokenWalk { int g, tile_base, begin, end; };
+CATCOC_HD int token_tiles(int rows) { return (rows + 511) / 512; }
+CATCOC_HD int token_half(int rows) {    // tokens of half a tile
+  const int t = token_tiles(rows);
+  return t > 0 ? round_up(ceil_div(ceil_div(rows, t), 2), 32) : 32;
+}
+CATCOC_HD TokenWalk token_walk_begin(int num_groups, const int32_t* ends, int group_rows, int M) {
+  TokenWalk w = {0, 0, 0, num_groups > 0 ? group_end_row(ends, group_rows, M, 0) : 0};
+  return w;
+}
+CATCOC_HD int token_walk_total(int feature_blocks, int num_groups, const int32_t* ends, int group_rows, int M) {
+  int total = 0, begin = 0;
+  for (int g = 0; g < num_groups; ++g) {
+    const int e = group_end_row(ends, group_rows, M, g);
+    if (e > begin) { total += token_tiles(e - begin) * feature_blocks; begin = e; }
+  }
+  return total;
+}
+// Tile `t` (not below an earlier call's): rows are features, columns tokens; `half` = tokens of each half
+CATCOC_HD TileInfo token_walk_tile(int features, int num_groups, const int32_t* ends, int group_rows, int M, int t, TokenWalk& w, int& half) {
+  const int fb = ceil_div(features, 256);
+  int rows = imin(w.end - w.begin, M);
+  while (t >= w.tile_base + token_tiles(rows > 0 ? rows : 0) * fb && w.g + 1 < num_groups) {
+    w.tile_base += token_tiles(rows > 0 ? rows : 0) * fb;
+    ++w.g;
+    if (w.end > w.begin) w.begin = w.end;
+    w.end = group_end_row(ends, group_rows, M, w.g);
+    rows = w.end - w.begin;
+  }
+  half = token_half(rows > 0 ? rows : 0);
+  TileInfo ti;
+  const int local = t - w.tile_base;
+  ti.seg = w.g;
+  ti.tile_in_seg = local;
+  ti.mi = local % fb;
+  ti.ni = local / fb;
+  ti.m0 = ti.mi * 256;
+  ti.n0 = w.begin + ti.ni * 2 * half;
+  ti.rows = imin(256, features - ti.m0);
+  ti.cols = imin(2 * half, w.end - ti.n0);
+  if (ti.cols < 0) ti.cols = 0;
+  return ti;
+}
+
 // Order in which a pusher visits its peers: the peer that consumes this rank's data earliest
 // comes first. For source-major consumers (allgather_matmul) rank r reads source q in phase
 // (q - r) mod W, so q serves q-1, q-2, ... For destination-major producers the order is

@@ -9,6 +9,7 @@
 #include "catcoc/capi.h"
 #include "catcoc/fused_gemm.cuh"
 #include "catcoc/kernel_inst.cuh"
+#include "catcoc/double_tile.cuh"
 #include "catcoc/host_util.h"
 
 namespace catcoc {
@@ -153,6 +154,31 @@ static int encode_3d_blocks(CUtensorMap* tm, const void* base, int elt_bytes, CU
     return CATCOC_E_DRIVER;
   }
   return CATCOC_OK;
+}
+
+// Plain (unswizzled) boxes of 32 columns x box_rows rows
+static int encode_plain(CUtensorMap* tm, const void* base, int elt_bytes, CUtensorMapDataType dt, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+  static EncodeTiledFn fn = driver_fn<EncodeTiledFn>("cuTensorMapEncodeTiled");
+  if (fn == nullptr) return CATCOC_E_DRIVER;
+  cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ld) * elt_bytes};
+  cuuint32_t box[2] = {32, static_cast<cuuint32_t>(box_rows)};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(tm, dt, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (plain) failed: CUresult %d", static_cast<int>(r)); return CATCOC_E_DRIVER; }
+  return CATCOC_OK;
+}
+
+// The product with its roles swapped: the tiles' rows run along the output's columns
+static CatcocOpArgs swap_roles(const CatcocOpArgs& o) {
+  CatcocOpArgs a = o;
+  a.M = o.N; a.N = o.M;
+  a.a = o.b; a.lda = o.ldb; a.trans_a = !o.trans_b;
+  a.b = o.a; a.ldb = o.lda; a.trans_b = !o.trans_a;
+  a.a_rows_total = o.b_n_total; a.b_n_total = o.a_rows_total;
+  a.a_k_total = o.b_k_total; a.b_k_total = o.a_k_total;
+  return a;
 }
 
 struct Resolved {
@@ -313,7 +339,9 @@ int max_active_pairs(int kind);
 // Fills the parameter block; shared by the normal and the allocation-free entry points.
 int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out, int* grid_out, int* pair_out) {
   if (args == nullptr) { set_error("null args"); return CATCOC_E_BAD_ARG; }
-  const CatcocOpArgs& a = *args;
+  const CatcocOpArgs& o = *args;        // the call as it came; `a`: with the tiles' rows under M
+  const bool swap = o.tiling.swap != 0;
+  const CatcocOpArgs a = swap ? swap_roles(o) : o;
   if (a.M <= 0 || a.N <= 0 || a.K <= 0) {
     set_error("bad problem size M=%d N=%d K=%d", a.M, a.N, a.K);
     return CATCOC_E_BAD_ARG;
@@ -343,7 +371,25 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   // 192-column tiles: pairs of local products (no workspace geometry knows them) with a B stored [N, K]; a [K, N] one comes
   // in 128-byte column blocks, of which a CTA's half would hold one and a half
   const bool bn192 = a.tiling.bn == 192 && !fused && a.trans_b && a.tiling.cta_pair == 2;
-  const int bn = mx ? (mx_pair ? 192 : 128) : bn192 ? 192 : norm_bn(a.tiling.bn);
+  // Double tiles (double_tile.cuh): 256 x 2 bn, local products on pairs
+  const bool twice = a.tiling.twice != 0;
+  const bool cut = a.tiling.cut_slices > 0;
+  if (cut && (!twice || a.num_groups > 0 || a.mode != CATCOC_MODE_LOCAL || a.part == nullptr || (reinterpret_cast<uintptr_t>(a.part) & 127) != 0 ||
+              a.tiling.cut_slices < 2 || a.tiling.cut_k <= 0 || (a.tiling.cut_k * rf.elt) % 128 != 0 ||
+              static_cast<int64_t>(a.tiling.cut_k) * (a.tiling.cut_slices - 1) >= a.K || static_cast<int64_t>(a.tiling.cut_k) * a.tiling.cut_slices < a.K)) {
+    set_error("double tiles: %d slices of %d elements do not cut K=%d into whole blocks of a local product", a.tiling.cut_slices, a.tiling.cut_k, a.K);
+    return CATCOC_E_BAD_ARG;
+  }
+  if (swap && (!twice || (rf.kind != KIND_F16 && rf.kind != KIND_I8) || a.c_src != nullptr ||
+               (a.num_groups > 0 && (a.tiling.bn != kMaxBN || o.trans_a || a.g_a_row_back != 0 || a.g_a_k != 0)))) {
+    set_error("swapped roles: 16-bit or int8 double tiles without C; over groups of rows of an A stored [M, K], with bn 256");
+    return CATCOC_E_UNSUPPORTED;
+  }
+  if (twice && (fused || a.tiling.cta_pair != 2 || a.tiling.bn < 64 || a.tiling.bn > kMaxBN || a.tiling.bn % 32 != 0 || (mx && (!mx_pair || a.tiling.bn != 192)))) {
+    set_error("double tiles (bn=%d) are pair tiles of local products, bn a multiple of 32 from 64 to 256 (block-scaled: 192)", a.tiling.bn);
+    return CATCOC_E_UNSUPPORTED;
+  }
+  const int bn = twice ? a.tiling.bn : mx ? (mx_pair ? 192 : 128) : bn192 ? 192 : norm_bn(a.tiling.bn);
   const int seg_dim = pick_seg_dim(a);
   const bool pair = mx ? mx_pair : (a.tiling.cta_pair == 2);
   if (mx) {
@@ -356,10 +402,11 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     if ((reinterpret_cast<uintptr_t>(a.sfa) & 15) || (reinterpret_cast<uintptr_t>(a.sfb) & 15)) { set_error("scale factor blocks must be 16-byte aligned"); return CATCOC_E_ALIGNMENT; }
   }
   const int bm = pair ? 2 * kBM : kBM;
-  if (pair && bn < 128) { set_error("cta_pair=2 needs bn >= 128"); return CATCOC_E_UNSUPPORTED; }
+  const int tile_n = twice ? 2 * bn : bn;   // of the tile walk
+  if (pair && bn < 128 && !twice) { set_error("cta_pair=2 needs bn >= 128"); return CATCOC_E_UNSUPPORTED; }
 
   memset(p, 0, sizeof(*p));
-  p->sched = build_sched(a, bm, bn, seg_dim);
+  p->sched = (twice && (swap || a.num_groups <= 0)) ? make_double_sched(a.M, a.N, bn, a.tiling.swizzle > 0 ? a.tiling.swizzle : 8) : build_sched(a, bm, tile_n, seg_dim);
   p->K = a.K;
   p->mode = a.mode;
   p->rank = fused ? a.rank : 0;
@@ -396,28 +443,28 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   const int b_k = (grouped && a.b_k_total > 0) ? a.b_k_total : a.K;
   if (grouped) {
     if (fused || a.mode != CATCOC_MODE_LOCAL || mx) { set_error("the group walk runs local, non block-scaled products only"); return CATCOC_E_UNSUPPORTED; }
-    if (a.group_ends == nullptr && (a.group_rows <= 0 || static_cast<int64_t>(a.group_rows) * a.num_groups != a.M)) {
-      set_error("uniform groups: M (%d) must be num_groups (%d) x group_rows (%d)", a.M, a.num_groups, a.group_rows);
+    if (a.group_ends == nullptr && (a.group_rows <= 0 || static_cast<int64_t>(a.group_rows) * a.num_groups != o.M)) {
+      set_error("uniform groups: M (%d) must be num_groups (%d) x group_rows (%d)", o.M, a.num_groups, a.group_rows);
       return CATCOC_E_BAD_ARG;
     }
     if (a.g_a_row_back < 0 || a.g_a_k < 0 || a.g_b_row < 0 || a.g_b_k < 0 || a.g_nvec < 0) { set_error("negative group stride"); return CATCOC_E_BAD_ARG; }
-    if (a.group_ends != nullptr && a.trans_a) {
+    if (a.group_ends != nullptr && o.trans_a) {
       // a ragged group origin would be the innermost TMA coordinate of an A stored [K, M]
       set_error("ragged groups need A stored [M, K]");
       return CATCOC_E_UNSUPPORTED;
     }
     // K origins of a group are innermost TMA coordinates of K-contiguous operands
-    if (!a.trans_a && (a.g_a_k * rf.elt) % 16 != 0) { set_error("group K stride of A must be a multiple of 16 bytes"); return CATCOC_E_ALIGNMENT; }
-    if (a.trans_b && (a.g_b_k * rf.elt) % 16 != 0) { set_error("group K stride of B must be a multiple of 16 bytes"); return CATCOC_E_ALIGNMENT; }
-    if (a.trans_a && (a.g_a_row_back * rf.elt) % 16 != 0) { set_error("group row stride of a transposed A must be a multiple of 16 bytes"); return CATCOC_E_ALIGNMENT; }
+    if (!o.trans_a && (a.g_a_k * rf.elt) % 16 != 0) { set_error("group K stride of A must be a multiple of 16 bytes"); return CATCOC_E_ALIGNMENT; }
+    if (o.trans_b && (a.g_b_k * rf.elt) % 16 != 0) { set_error("group K stride of B must be a multiple of 16 bytes"); return CATCOC_E_ALIGNMENT; }
+    if (o.trans_a && (a.g_a_row_back * rf.elt) % 16 != 0) { set_error("group row stride of a transposed A must be a multiple of 16 bytes"); return CATCOC_E_ALIGNMENT; }
     // a group whose K range is followed by another group's data must end on an MMA boundary,
     // or the last MMA would multiply into the neighbour's elements
     if ((a.g_a_k > 0 || a.g_b_k > 0) && (a.K % rf.umma_k) != 0) {
       set_error("K per group (%d) must be a multiple of %d when groups are stacked along K", a.K, rf.umma_k);
       return CATCOC_E_ALIGNMENT;
     }
-    if (static_cast<int64_t>(a.num_groups - 1) * a.g_a_k >= a_k ||
-        static_cast<int64_t>(a.num_groups - 1) * a.g_b_k >= b_k) {
+    if (static_cast<int64_t>(a.num_groups - 1) * a.g_a_k >= (swap ? b_k : a_k) ||
+        static_cast<int64_t>(a.num_groups - 1) * a.g_b_k >= (swap ? a_k : b_k)) {
       set_error("the last group's K origin lies outside the stored operands");
       return CATCOC_E_BAD_ARG;
     }
@@ -454,7 +501,7 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   const bool a_blocks_ok = !(p->sched.W > 1 && seg_dim == SEG_ROWS) || (p->sched.seg_len % per128) == 0;
   const bool b_blocks_ok = (!(p->sched.W > 1 && seg_dim == SEG_COLS) || (p->sched.seg_len % per128) == 0) &&
                            ((pair ? bn / 2 : bn) % per128) == 0;
-  if (!a.trans_b && (pair ? bn / 2 : bn) < per128) {
+  if (!a.trans_b && (pair ? bn / 2 : bn) < per128 && !twice) {
     set_error("8-bit operands stored [K, N] need bn >= 128 (one 128-byte run of N per TMA box)");
     return CATCOC_E_UNSUPPORTED;
   }
@@ -555,12 +602,17 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   // A local output leaves by TMA stores (32-row x 128-byte boxes, same swizzle as the staging
   // buffer) when its base and pitch allow a tensor map; the plain-store path covers the rest.
   if (!(fused && a.mode == CATCOC_MODE_AR) && p->out_vec_ok && out_tma_enabled()) {
-    const int64_t rows_out = (fused && a.mode == CATCOC_MODE_RS) ? p->sched.seg_len : a.M;
+    const int64_t rows_out = (fused && a.mode == CATCOC_MODE_RS) ? p->sched.seg_len : o.M;
     const CUtensorMapDataType odt = a.out_fmt == CATCOC_FMT_F16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                     : a.out_fmt == CATCOC_FMT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                     : a.out_fmt == CATCOC_FMT_F32  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                                                    : CU_TENSOR_MAP_DATA_TYPE_INT32;
-    if (encode_2d(&p->tm_out, a.out, oelt, odt, rows_out, a.N, a.ldc, 128 / oelt, 32) == CATCOC_OK) p->out_tma = 1;
+    if (swap) {
+      // windows of 32 columns x 64 (32-bit: 32) rows, and half ones
+      if (encode_plain(&p->tm_out, a.out, oelt, odt, rows_out, o.N, a.ldc, 128 / oelt) == CATCOC_OK &&
+          encode_plain(&p->tm_part[1], a.out, oelt, odt, rows_out, o.N, a.ldc, 32) == CATCOC_OK)
+        p->out_tma = 1;
+    } else if (encode_2d(&p->tm_out, a.out, oelt, odt, rows_out, a.N, a.ldc, 128 / oelt, 32) == CATCOC_OK) p->out_tma = 1;
   }
   const bool pull = wants_pull(a);
   if (pull) {
@@ -650,6 +702,16 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     }
     p->stage_tma = all ? 1 : 0;
   }
+  if (twice) {
+    DoubleTile& d = p->dt;
+    d.bn = bn;
+    d.swap = swap ? 1 : 0;
+    d.b_half = p->b_mn_major ? ceil_div(bn / 2, per128) * rf.bk * 128 : bn / 2 * 128;   // column blocks of 128 bytes are loaded whole
+    d.sf_off = kABytes + 2 * d.b_half;
+    d.stage_bytes = round_up(d.sf_off + (mx ? dtile::kMxSfBytes : 0), 1024);
+    d.stages = imin(kMaxStages, dtile::kRingBytes / d.stage_bytes);
+    d.lead = imin(dtile::kLead, d.stages - 1);
+  }
   p->scale_m = a.scale_m;
   p->scale_n = a.scale_n;
   p->bias = a.bias;
@@ -679,10 +741,10 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     return CATCOC_E_BAD_ARG;
   }
   if (p->out_tma && !p->pull && p->limit[LIM_OUT] > 0) {
-    const int64_t rows_out = (fused && a.mode == CATCOC_MODE_RS) ? p->sched.seg_len : a.M;
-    if (p->limit[LIM_OUT] < ((rows_out - 1) * a.ldc + a.N) * fmt_bytes(a.out_fmt)) {
+    const int64_t rows_out = (fused && a.mode == CATCOC_MODE_RS) ? p->sched.seg_len : o.M;
+    if (p->limit[LIM_OUT] < ((rows_out - 1) * a.ldc + o.N) * fmt_bytes(a.out_fmt)) {
       set_error("the output buffer (%lld bytes) is smaller than [%lld, %d] with pitch %lld",
-                static_cast<long long>(p->limit[LIM_OUT]), static_cast<long long>(rows_out), a.N, static_cast<long long>(a.ldc));
+                static_cast<long long>(p->limit[LIM_OUT]), static_cast<long long>(rows_out), o.N, static_cast<long long>(a.ldc));
       return CATCOC_E_BAD_ARG;
     }
   }
@@ -713,10 +775,11 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   int tiles_bound = p->sched.total_tiles;
   if (grouped) {
     // group extents are device data: bound the tile count by full tiles + one ragged tile per group
-    const int64_t mt = static_cast<int64_t>(a.M / bm) + a.num_groups;
-    const int64_t nt = (a.N + bn - 1) / bn;
+    const int64_t mt = swap ? p->sched.seg_mt : static_cast<int64_t>(a.M / bm) + a.num_groups;
+    const int64_t nt = swap ? static_cast<int64_t>(a.N / tile_n) + a.num_groups : (a.N + tile_n - 1) / tile_n;
     tiles_bound = static_cast<int>(mt * nt > (1 << 30) ? (1 << 30) : mt * nt);
   }
+  if (twice && !grouped) tiles_bound = p->sched.seg_mt * ceil_div(a.N, bn);   // units
   if (!(fused && a.mode == CATCOC_MODE_AG)) grid = imin(grid, tiles_bound * per_tile);
   // (an all-gather keeps every CTA: their communication warps share the copy of the shard)
   if (pair) {
@@ -725,6 +788,23 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     if (grid < 2) grid = 2;
   }
   if (grid < 1) grid = 1;
+  if (twice && !grouped) {
+    if (cut) grid = imin(imin(sms, a.tiling.num_ctas > 0 ? a.tiling.num_ctas : sms), 2 * max_active_pairs(rf.kind)) & ~1;   // more slices than units
+    p->dt.plan = make_double_plan(p->sched, bn, grid / 2, a.tiling.cut_slices, a.tiling.cut_k);
+    if (p->dt.plan.doubles == 0 && !mx) {
+      // one block of B per stage: more stages (what single units wait for is the latency of their loads)
+      p->dt.stage_bytes = round_up(kABytes + p->dt.b_half, 1024);
+      p->dt.stages = imin(kMaxStages, dtile::kRingBytes / p->dt.stage_bytes);
+    }
+    if (p->dt.plan.cut > 0) {
+      const bool is_int = rf.kind == KIND_I8;
+      const CUtensorMapDataType pdt = is_int ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+      const int64_t planes = static_cast<int64_t>(p->dt.plan.cut) * a.tiling.cut_slices;
+      rc = swap ? encode_plain(&p->tm_part[0], a.part, 4, pdt, planes * bn, 2 * kBM, 2 * kBM, 32)
+                : encode_2d(&p->tm_part[0], a.part, 4, pdt, planes * 2 * kBM, bn, bn, 32, 32);
+      if (rc != 0) return rc;
+    }
+  }
   *grid_out = grid;
   *kind_out = rf.kind;
   *pair_out = pair ? 1 : 0;
@@ -752,6 +832,8 @@ static cudaError_t prepare_kernels() {
         const cudaError_t e = u->prepare();
         if (e != cudaSuccess) err = e;
       }
+    const cudaError_t e = inst::prepare_double();
+    if (e != cudaSuccess) err = e;
   });
   return err;
 }
@@ -784,6 +866,12 @@ int catcoc_launch_params(const FusedParams& p, int kind, int grid, int pair, int
   cudaError_t e = prepare_kernels();
   if (e != cudaSuccess) {
     set_error("cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
+    return -1000 - static_cast<int>(e);
+  }
+  if (p.dt.bn != 0) {
+    e = inst::launch_double(kind, pick_epi(p) == EPI_FULL, p, grid, stream);
+    if (e == cudaSuccess) return CATCOC_OK;
+    set_error("kernel launch failed: %s", cudaGetErrorString(e));
     return -1000 - static_cast<int>(e);
   }
   const inst::Unit* u = unit_for(kind, pair != 0);
@@ -827,11 +915,56 @@ uint64_t hash_bytes(const void* data, size_t n) {
 }
 }  // namespace
 
+// Ragged groups with swapped roles: the same with a tensor map of the tokens for every width that half a tile can have
+namespace {
+struct TokPlan {
+  bool valid = false;
+  int device = -1, kind = 0, grid = 0;
+  CatcocOpArgs key;
+  FusedParamsTok params;
+};
+constexpr int kTokPlanSlots = 64;
+TokPlan g_tok_plans[kTokPlanSlots];
+}  // namespace
+
+static int launch_tokens(const CatcocOpArgs* args, int device, uint64_t h, cudaStream_t stream) {
+  TokPlan& slot = g_tok_plans[h % kTokPlanSlots];
+  FusedParamsTok p;
+  int kind = 0, grid = 0, pair = 0;
+  bool hit = false;
+  {
+    std::lock_guard<std::mutex> lock(g_plan_mu);
+    if (slot.valid && slot.device == device && memcmp(&slot.key, args, sizeof(CatcocOpArgs)) == 0) {
+      p = slot.params; kind = slot.kind; grid = slot.grid;
+      hit = true;
+    }
+  }
+  if (!hit) {
+    int rc = catcoc_build_params(args, &p, &kind, &grid, &pair);
+    if (rc != 0) return rc;
+    Resolved rf;
+    rc = resolve_format(args->in_fmt, &rf);
+    for (int i = 0; rc == 0 && i < 8; ++i)
+      rc = encode_2d(&p.tok_map[i], args->a, rf.elt, rf.dt, args->a_rows_total > 0 ? args->a_rows_total : args->M,
+                     args->a_k_total > 0 ? args->a_k_total : args->K, args->lda, rf.bk, 16 * (i + 1));
+    if (rc != 0) return rc;
+    std::lock_guard<std::mutex> lock(g_plan_mu);
+    slot.valid = true; slot.device = device; slot.kind = kind; slot.grid = grid;
+    memcpy(&slot.key, args, sizeof(CatcocOpArgs));
+    slot.params = p;
+  }
+  const cudaError_t e = inst::launch_double_tokens(kind, pick_epi(p) == EPI_FULL, p, grid, stream);
+  if (e == cudaSuccess) return CATCOC_OK;
+  set_error("kernel launch failed: %s", cudaGetErrorString(e));
+  return -1000 - static_cast<int>(e);
+}
+
 extern "C" int catcoc_fused_launch(const CatcocOpArgs* args, void* stream) {
   if (args == nullptr) { set_error("null args"); return CATCOC_E_BAD_ARG; }
   int device = 0;
   cudaGetDevice(&device);
   const uint64_t h = hash_bytes(args, sizeof(CatcocOpArgs)) ^ (static_cast<uint64_t>(device) * 0x9e3779b97f4a7c15ull);
+  if (args->tiling.swap != 0 && args->num_groups > 0) return launch_tokens(args, device, h, static_cast<cudaStream_t>(stream));
   Plan& slot = g_plans[h % kPlanSlots];
   FusedParams p;
   int kind = 0, grid = 0, pair = 0;
@@ -888,7 +1021,7 @@ extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_
     int kind = 0, grid = 0, pair = 0;
     rc = catcoc_build_params(&a, &p, &kind, &grid, &pair);
     if (rc != 0) return rc;
-    const int b_cols = pair ? p.sched.BN / 2 : p.sched.BN;
+    const int b_cols = p.dt.bn != 0 ? p.dt.bn / 2 : pair ? p.sched.BN / 2 : p.sched.BN;
     if (p.b_3d == 2) p.b_3d = 0;                          // one map per group and operand
     for (int i = 0; i < a.num_groups; ++i) {
       const int begin = k_range[2 * (g0 + i)], end = k_range[2 * (g0 + i) + 1];
@@ -902,7 +1035,8 @@ extern "C" int catcoc_slice_k_launch(const CatcocOpArgs* args, const int32_t* k_
                     : encode_2d(ma + 1, a.b, rf.elt, rf.dt, end, a.b_n_total, a.ldb, per128, rf.bk);
       if (rc != 0) return rc;
     }
-    CATCOC_CUDA_OK(inst::launch_slice_k(pair != 0, p, grid, static_cast<cudaStream_t>(stream_)));
+    if (p.dt.bn != 0) CATCOC_CUDA_OK(inst::launch_double_slice_k(p, grid, static_cast<cudaStream_t>(stream_)));
+    else CATCOC_CUDA_OK(inst::launch_slice_k(pair != 0, p, grid, static_cast<cudaStream_t>(stream_)));
   }
   return CATCOC_OK;
 }
@@ -1117,7 +1251,7 @@ extern "C" int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slice
   int rc = resolve_format(a.in_fmt, &rf);
   if (rc != 0) return rc;
   const bool is_int = rf.kind == KIND_I8;
-  if (a.mode != CATCOC_MODE_LOCAL || (rf.kind != KIND_F16 && !is_int) || a.num_groups != 0 || a.tiling.cta_pair != 2 ||
+  if (a.mode != CATCOC_MODE_LOCAL || (rf.kind != KIND_F16 && !is_int) || a.num_groups != 0 || a.tiling.cta_pair != 2 || a.tiling.twice != 0 ||
       (k_slice * rf.elt) % 256 != 0 || static_cast<int64_t>(k_slice) * (slices - 1) >= a.K || static_cast<int64_t>(k_slice) * slices < a.K) {
     set_error("tail: a local 16-bit or int8 product on pair tiles whose K range is cut into whole stages (K=%d, %d slices of %d)", a.K, slices, k_slice);
     return CATCOC_E_BAD_ARG;
@@ -1151,4 +1285,89 @@ extern "C" int catcoc_tail_launch(const CatcocOpArgs* args, int first, int slice
   const dim3 fold_grid(static_cast<unsigned>(p.sched.BM * p.sched.BN / 4 / 256), static_cast<unsigned>(tiles));
   CATCOC_CUDA_OK(launch_overlapped(is_int ? tail_fold_kernel<true> : tail_fold_kernel<false>, fold_grid, dim3(256), 0, stream, f, p.sched, first));
   return CATCOC_OK;
+}
+
+// ---- double tiles whose last units are cut along K ----
+namespace {
+// The units that were cut: blockIdx.y counts them, their planes are [slices][256][bn], with swapped roles [slices][bn][256].
+template <bool INT>
+__global__ void __launch_bounds__(256, 6) double_fold_kernel(const FoldParams p, const TileSched sched, const DoublePlan plan, int bn, int swap) {
+  ptx::grid_dependency_wait();
+  TileInfo ti = double_unit_extent(sched, plan, bn, plan.singles + blockIdx.y);
+  if (swap) {
+    const int m0 = ti.m0, rows = ti.rows;
+    ti.m0 = ti.n0; ti.rows = ti.cols;
+    ti.n0 = m0; ti.cols = rows;
+  }
+  const uint8_t* planes = p.parts + static_cast<int64_t>(blockIdx.y) * p.slices * p.plane * 4;
+  const int units_row = p.pitch / 4;
+  for (int u = blockIdx.x * 256 + threadIdx.x; u < ti.rows * units_row; u += gridDim.x * 256) {
+    const int r = u / units_row, c = (u - r * units_row) * 4;
+    if (c < ti.cols)
+      fold_store<INT>(p, planes + (static_cast<int64_t>(r) * p.pitch + c) * 4, p.plane * 4, p.slices, ti.m0 + r, ti.n0 + c, min(4, ti.cols - c));
+  }
+}
+
+int double_workers(const CatcocOpArgs& a, int kind) {
+  int device = 0;
+  cudaGetDevice(&device);
+  const int sms = sm_count(device);
+  return imin(a.tiling.num_ctas > 0 ? imin(a.tiling.num_ctas, sms) : sms, 2 * max_active_pairs(kind)) / 2;
+}
+}  // namespace
+
+extern "C" int64_t catcoc_double_workspace_bytes(const CatcocOpArgs* args) {
+  Resolved rf;
+  if (args == nullptr || args->M <= 0 || args->N <= 0 || args->tiling.cut_slices < 2 || args->tiling.bn < 64 || args->tiling.bn > kMaxBN ||
+      resolve_format(args->in_fmt, &rf) != 0)
+    return -1;
+  const int workers = double_workers(*args, rf.kind);
+  if (workers < 1) return -1;
+  const TileSched s = args->tiling.swap ? make_double_sched(args->N, args->M, args->tiling.bn, 1) : make_double_sched(args->M, args->N, args->tiling.bn, 1);
+  return static_cast<int64_t>(make_double_plan(s, args->tiling.bn, workers, args->tiling.cut_slices, 1).cut) * args->tiling.cut_slices * 2 * kBM * args->tiling.bn * 4;
+}
+
+extern "C" int catcoc_double_launch(const CatcocOpArgs* args, void* workspace, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (args == nullptr || workspace == nullptr || args->tiling.cut_slices < 2 || args->tiling.twice == 0 || args->M <= 0 || args->N <= 0 ||
+      args->tiling.bn < 64 || args->tiling.bn > kMaxBN) {
+    set_error("double_launch: bad arguments");
+    return CATCOC_E_BAD_ARG;
+  }
+  CatcocOpArgs a = *args;
+  Resolved rf;
+  int rc = resolve_format(a.in_fmt, &rf);
+  if (rc != 0) return rc;
+  const bool is_int = rf.kind == KIND_I8;
+  if (!fold_fits(a, is_int)) return CATCOC_E_UNSUPPORTED;
+  if (!fold_inside(a)) return CATCOC_E_BAD_ARG;
+  a.part = workspace;
+  rc = catcoc_fused_launch(&a, stream_);
+  if (rc != 0) return rc;
+  const bool swap = a.tiling.swap != 0;
+  const TileSched s = make_double_sched(swap ? a.N : a.M, swap ? a.M : a.N, a.tiling.bn, a.tiling.swizzle > 0 ? a.tiling.swizzle : 8);
+  const DoublePlan plan = make_double_plan(s, a.tiling.bn, double_workers(a, rf.kind), a.tiling.cut_slices, a.tiling.cut_k);
+  if (plan.cut == 0) return CATCOC_OK;
+  FoldParams f = fold_params(a);
+  f.parts = static_cast<const uint8_t*>(workspace);
+  f.plane = static_cast<int64_t>(2) * kBM * a.tiling.bn;
+  f.slices = a.tiling.cut_slices; f.pitch = swap ? 2 * kBM : a.tiling.bn;
+  const dim3 fold_grid(static_cast<unsigned>(2 * kBM * a.tiling.bn / 4 / 256), static_cast<unsigned>(plan.cut));
+  CATCOC_CUDA_OK(launch_overlapped(is_int ? double_fold_kernel<true> : double_fold_kernel<false>, fold_grid, dim3(256), 0, stream, f, s, plan, a.tiling.bn, swap ? 1 : 0));
+  return CATCOC_OK;
+}
+
+extern "C" int catcoc_double_plan_replay(int M, int N, int bn, int swizzle, int workers, int slices, int worker, int max_items, int32_t* out) {
+  if (M <= 0 || N <= 0 || bn < 64 || workers <= 0 || worker < 0 || worker >= workers || (max_items > 0 && out == nullptr)) return CATCOC_E_BAD_ARG;
+  const TileSched s = make_double_sched(M, N, bn, swizzle);
+  const DoublePlan d = make_double_plan(s, bn, workers, slices, 1);
+  int i = 0;
+  for (;; ++i) {
+    const DoubleItem it = double_item(d, worker, i);
+    if (it.kind == 0) return i;
+    if (i >= max_items) continue;
+    const TileInfo t = it.kind == 1 ? double_tile_extent(s, it.index) : double_unit_extent(s, d, bn, it.index);
+    const int32_t row[6] = {it.kind, t.m0, t.n0, t.rows, t.cols, it.slice};
+    memcpy(out + 6 * i, row, sizeof(row));
+  }
 }

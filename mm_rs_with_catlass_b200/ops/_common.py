@@ -189,6 +189,8 @@ def fill_tiling(args: N.OpArgs, tiling: Optional[TilingConfig]) -> None:
     args.tiling.pull = 0              # the fused ops switch it on once the buffers it needs are attached
     args.tiling.comm_warps = t.comm_warps
     args.tiling.push_tma = t.push_tma
+    args.tiling.twice, args.tiling.swap = int(t.twice), int(t.swap)
+    args.tiling.cut_slices, args.tiling.cut_k = t.cut_slices, t.cut_k
 
 
 def default_timeout_ns() -> int:
@@ -248,6 +250,17 @@ def launch_tail(args: N.OpArgs, first: int, slices: int, k_slice: int, device: t
     ws = torch.empty(int(lib.catcoc_tail_workspace_bytes(args.M, args.N, args.tiling.bn or 256, first, slices)), dtype=torch.uint8,
                      device=device)
     N.check(lib.catcoc_tail_launch(C.byref(args), first, slices, k_slice, ws.data_ptr(), C.c_void_p(stream_of(device))))
+    global _launches
+    _launches += 1
+
+
+def launch_double(args: N.OpArgs, device: torch.device) -> None:
+    """Queues a product on double tiles whose last units are cut along K, and the kernel that sums the slices."""
+    args.timeout_ns = default_timeout_ns()
+    args.events, args.events_cap = _event_ring
+    lib = N.lib()
+    ws = torch.empty(max(1, int(lib.catcoc_double_workspace_bytes(C.byref(args)))), dtype=torch.uint8, device=device)
+    N.check(lib.catcoc_double_launch(C.byref(args), ws.data_ptr(), C.c_void_p(stream_of(device))))
     global _launches
     _launches += 1
 

@@ -125,16 +125,19 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
         b_k_major = trans_b != (b.stride(-1) != 1 and b.stride(0) == 1 and min(b.shape) > 1)
         tails = _group is None and trace is None and a.dtype in (torch.float16, torch.bfloat16, torch.int8)
         tiling = chooser.choose("matmul", m, n, k, 1, a.dtype,
-                                b_k_major=b_k_major and _group is None, tails=tails)
-        if _group is None and trace is None:
+                                b_k_major=b_k_major and _group is None, tails=tails, doubles=tails,
+                                swap=c is None or beta == 0.0)
+        if _group is None and trace is None and not tiling.twice:
             split = chooser.split_k(m, n, k, a.element_size(), tiling)
             if split is not None:
                 tiling = TilingConfig(bn=split[2], cta_pair=1)
                 split = (cm.launch_splitk, split[0], split[1])
-        if split is None and tails and tiling.cta_pair == 2:
+        if split is None and tails and tiling.cta_pair == 2 and not tiling.twice:
             cut = chooser.tail_cut(m, n, k, a.element_size(), tiling.effective_bn)[1]
             if cut is not None:
                 split = (cm.launch_tail, *cut)
+    if tiling is not None and tiling.cut_slices and _group is None:
+        split = (cm.launch_double,)
     with torch.cuda.device(dev):
         # An operand whose base or row pitch TMA cannot take goes through the pad kernel first.
         oa, ob = cm.as_operands(a, trans_a, b, trans_b)

@@ -43,6 +43,7 @@ _TAIL_INTAKE = 52.0               # the same for a pair tile of a product that f
 _INTAKE = {1: 46.0, 2: 42.0}      # bytes per cycle that one CTA takes in while most of the others do the same (pair: per CTA)
 _HBM = 3600.0                     # bytes per cycle from HBM, all SMs
 _PLANES = 3500.0                  # bytes per cycle of the planes, written and read through L2
+_DOUBLE_EPILOGUE = 2500.0         # what a double tile's epilogue leaves uncovered
 _LAUNCH = 10000.0                 # start, fill and drain of a kernel
 _FOLD = 8000.0                    # the second kernel and the gap before it
 _INT8_EPILOGUE = 10000.0          # the dequantising epilogue of the direct kernel, which the second kernel spreads over all SMs
@@ -88,6 +89,70 @@ def tail_cut(m: int, n: int, k: int, elt: int, bn: int):
         if t < best_time:
             best, best_time = (first, s, kbs * 128 // elt), t
     return (waves, None) if best is None else ((best_time - _LAUNCH) / wave_time, best)
+
+
+@functools.lru_cache(maxsize=16384)
+def double_plan(rows: int, cols: int, k: int, elt: int, bn: int, rows_k_major: bool = True):
+    """A local product on double tiles, 256 ``rows`` x 2 bn ``cols``: ``(cycles, cut)`` with ``cut = (slices, k_slice)`` when the
+    units of 256 x bn past the last full wave are worth cutting along K, else None.
+
+    A K block of a double tile takes 122 + 3.8 bn cycles (bn 256: 1096, 192: 865; its MMAs: 4 bn), never less than the 610 of
+    its issue. One of a unit by itself takes what its loads' latency leaves: 780 above 160 columns, else 560, or 660 where the
+    operand under the rows is not K-contiguous (operands of zeros, K of 4096 to 8192)."""
+    workers = _NUM_SMS // 2
+    rt, ct, kb = -(-rows // 256), -(-cols // bn), -(-k * elt // 128)
+    total = rt * ct
+    twice, once = max(610.0, 122 + 3.8 * bn), 780.0 if bn > 160 else 560.0 if rows_k_major else 660.0
+
+    def whole(units):          # the busiest pair, as the units are dealt out (double_item in csrc/include/catcoc/sched.h)
+        waves = -(-units // workers)
+        doubles = min(rt * (ct // 2), waves // 2 * workers, units // 2)
+        singles, per, r = units - 2 * doubles, doubles // workers, doubles % workers
+        level = min(singles, 2 * (workers - r)) if r else 0
+        light = per * twice + -(-level // (workers - r)) * once
+        heavy = (per + (r > 0)) * twice
+        return kb * (max(heavy, light) + -(-(singles - level) // workers) * once) + (per + (r > 0)) * _DOUBLE_EPILOGUE
+
+    hbm = (rows + cols) * k * elt / _HBM
+    best, best_time = None, max(hbm, whole(total)) + _LAUNCH
+    rest = total % workers
+    full = whole(total - rest)
+    for s in range(2, 33) if rest else ():
+        kbs = -(-kb // s)
+        if kbs < 8 or -(-kb // kbs) != s:
+            continue
+        t = max(hbm, full + -(-rest * s // workers) * kbs * once) + rest * s * 256.0 * bn * 8 / _PLANES + _LAUNCH + 2 * _FOLD
+        if t < 0.94 * best_time:
+            best, best_time = (s, kbs * 128 // elt), t
+    return best_time, best
+
+
+def double(m: int, n: int, k: int, elt: int, b_k_major: bool, swap: bool, limit: float) -> Optional[TilingConfig]:
+    """The best tiling on double tiles whose predicted cycles are below ``limit``, else None. With B stored [K, N] the halves must
+    be whole 128-byte blocks of columns for every CTA (192 columns: 3890 us where 256 take 3250, bf16 8192 x 28672 x 8192); with
+    ``swap`` the output's rows may run along the tiles' columns, whose width then fits them: int8 614 x 8192 x 7168: 48 -> 32 us,
+    bf16 302 x 14336 x 8192: 116 -> 74 us, 106 x 14336 x 8192 with B [N, K]: 58 -> 49 us.
+
+    Over 120 shapes that this rule sends here (129 to 16384 rows, bf16 and int8, both storages of B) the product is 12 % faster
+    on average than on the other tiles, in a loop; the worst lost 3 %."""
+    best = None
+    for turned in (False, True):
+        if (turned and not swap) or (m <= 128 and not (turned and b_k_major)):
+            continue           # few rows on the tiles' rows are mostly padding, and a [K, N] weight under them is slower to load
+        rows, cols = (n, m) if turned else (m, n)
+        for bn in ((256, 224, 192, 160, 128, 96, 64) if b_k_major or turned else (256,)):
+            if bn > 64 and bn >= cols + 32:
+                continue
+            t, cut = double_plan(rows, cols, k, elt, bn, b_k_major if turned else True)
+            # the cluster's start, an epilogue that nothing covers; turning the tile
+            t += (5500.0 if turned else 4500.0) + (_INT8_EPILOGUE if elt == 1 else 0.0)
+            if t < limit:
+                limit, best = t, (bn, turned, cut)
+    if best is None:
+        return None
+    bn, turned, cut = best
+    return TilingConfig(bn=bn, swizzle=4, cta_pair=2, twice=True, swap=turned, cut_slices=cut[0] if cut else 0,
+                        cut_k=cut[1] if cut else 0)
 
 
 def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b_k_major: bool = False,
@@ -148,7 +213,6 @@ def heuristic(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b
                         use_multicast=(op == "allgather_matmul" and world >= 4))
 
 
-@functools.lru_cache(maxsize=4096)
 def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
     """``(slices, k_slice, bn)`` when a local product is faster with its K range cut into slices whose
     planes a second kernel sums, else None.
@@ -158,6 +222,12 @@ def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
     column) or its bytes (all 128 rows of A are filled, whatever M is). Wide tiles cut into slices take
     in fewer bytes per column; the price is the planes and a second kernel. bf16, M = 128, 8192 x 28672:
     134 -> 94 us; M = 100, 3584 x 8192: 44 -> 29 us; int8, M = 128, 8192 x 28672: 106 -> 63 us."""
+    return _split_k(m, n, k, elt, direct)[0]
+
+
+@functools.lru_cache(maxsize=4096)
+def _split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
+    """``split_k``'s answer and the cycles that the product then takes."""
     kb = -(-k * elt // 128)
 
     def unit(bn, pair):
@@ -169,7 +239,8 @@ def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
     if pair == 2 and bn0 >= 128:
         waves = tail_cut(m, n, k, elt, bn0)[0]
     # (for 8-bit operands the model puts a cut rather high: 256 x 8192 x 7168 30.5 us direct, 25.7 cut)
-    best, best_time = None, (0.97 if elt == 1 else 0.95) * (max(hbm, waves * kb * unit(bn0, pair)) + _LAUNCH + (_INT8_EPILOGUE if elt == 1 else 0.0))
+    whole = max(hbm, waves * kb * unit(bn0, pair)) + _LAUNCH + (_INT8_EPILOGUE if elt == 1 else 0.0)
+    best, best_time = None, (0.97 if elt == 1 else 0.95) * whole
     for bn in (256, 128):
         if n < bn and bn > 128:
             continue
@@ -181,7 +252,7 @@ def split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
             t = max(hbm, -(-tiles * s // _NUM_SMS) * kbs * unit(bn, 1)) + s * m * n * 8 / _PLANES + _LAUNCH + _FOLD
             if t < best_time:
                 best, best_time = (s, kbs * 128 // elt, bn), t
-    return best
+    return best, whole if best is None else best_time
 
 
 def grouped(rows_total: int, rows_per_group: float, n: int, dtype: torch.dtype) -> TilingConfig:
@@ -217,9 +288,24 @@ def _grouped(rows_total: int, rows_per_group: float, n: int, dtype: torch.dtype,
 
 
 def choose(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype,
-           table: Optional["_table.TilingTable"] = None, b_k_major: bool = False, tails: bool = False) -> TilingConfig:
+           table: Optional["_table.TilingTable"] = None, b_k_major: bool = False, tails: bool = False,
+           doubles: bool = False, swap: bool = False) -> TilingConfig:
+    """``doubles``: the caller can launch double tiles (local products), ``swap``: with swapped roles too."""
     tbl = table if table is not None else _table.default_table()
     hit = tbl.lookup(op, m, n, k, world, dtype)
     if hit is not None:
         return hit
-    return heuristic(op, m, n, k, world, dtype, b_k_major, tails)
+    t = heuristic(op, m, n, k, world, dtype, b_k_major, tails)
+    if doubles and os.environ.get("CATCOC_CTA_PAIR") != "1":
+        return _with_doubles(m, n, k, dtype.itemsize, b_k_major, swap, t)
+    return t
+
+
+@functools.lru_cache(maxsize=4096)
+def _with_doubles(m: int, n: int, k: int, elt: int, b_k_major: bool, swap: bool, t: TilingConfig) -> TilingConfig:
+    cut, cycles = _split_k(m, n, k, elt, t)
+    if cut is None and t.cta_pair == 2:
+        bn = t.effective_bn
+        cycles = tail_cut(m, n, k, elt, bn)[0] * -(-k * elt // 128) * max(2.0 * bn, (128 + bn // 2) * 128 / _TAIL_INTAKE) + _LAUNCH + (
+            _INT8_EPILOGUE if elt == 1 else 0.0)
+    return double(m, n, k, elt, b_k_major, swap, 0.99 * cycles) or t

@@ -43,6 +43,11 @@ class TilingConfig:
     comm_warps: int = 0    # communication / reducer warps per CTA, 1..5 (0 = 5): all-gather and pull flavours
     push_tma: int = -1     # push flavour: partial tiles travel by TMA stores (1) or 16-byte stores (0); -1: the
                            # CATCOC_PUSH_TMA environment variable decides (default: 16-byte stores)
+    twice: bool = False    # local products, cta_pair=2: tiles of two accumulators, 256 x 2 bn; bn is then any multiple of 32
+                           # from 64 to 256 (block-scaled fp8: 192)
+    swap: bool = False     # ... with the output's columns along the tiles' rows: 256 columns x 2 bn rows of the output
+    cut_slices: int = 0    # ... whose units of 256 x bn past the last full wave are cut along K into this many slices
+    cut_k: int = 0         # of cut_k elements (whole K blocks of 128 bytes); 0 = not cut
     # --- reference-compatible fields (carried, reported, not steering the kernel) ---
     m0: int = 128
     n0: int = 256
@@ -55,7 +60,16 @@ class TilingConfig:
 
     def validate(self, local: bool = True) -> "TilingConfig":
         """Raises ValueError for a setting that no launch takes; ``local=False``: none that communicates."""
-        if self.bn not in (0, 64, 128, 256) and not (self.bn == 192 and self.cta_pair == 2 and local):
+        if self.twice:
+            if self.cta_pair != 2 or not local:
+                raise ValueError("twice needs a local product on CTA pairs (cta_pair=2)")
+            if not 64 <= self.bn <= 256 or self.bn % 32:
+                raise ValueError("twice needs bn to be a multiple of 32 from 64 to 256 (got %d)" % self.bn)
+        if self.swap and not self.twice:
+            raise ValueError("swap goes with twice")
+        if (self.cut_slices or self.cut_k) and not (self.twice and self.cut_slices >= 2 and self.cut_k > 0):
+            raise ValueError("cut_slices (at least 2) and cut_k go with twice")
+        if not self.twice and self.bn not in (0, 64, 128, 256) and not (self.bn == 192 and self.cta_pair == 2 and local):
             raise ValueError("bn must be 0, 64, 128 or 256, or 192 for a local product on CTA pairs (got %d)" % self.bn)
         if self.swizzle < 0 or self.swizzle > 64:
             raise ValueError("swizzle must be in [0, 64]")
@@ -63,7 +77,7 @@ class TilingConfig:
             raise ValueError("num_ctas must be >= 0")
         if self.cta_pair not in (0, 1, 2):
             raise ValueError("cta_pair must be 0, 1 or 2")
-        if self.cta_pair == 2 and self.bn not in (0, 128, 192, 256):
+        if self.cta_pair == 2 and not self.twice and self.bn not in (0, 128, 192, 256):
             raise ValueError("cta_pair=2 needs bn of 128 or 256")
         if self.rounds < 0 or self.rounds > 64:
             raise ValueError("rounds must be in [0, 64]")

@@ -1,0 +1,149 @@
+"""Double tiles (256 x 2 bn on a CTA pair): the plan covers the output once and deals it out evenly, the rule's choices are
+legal (CPU); results are the bits of the one-accumulator kernel, whose products run in the same order along K (GPU)."""
+import ctypes as C
+
+import pytest
+import torch
+
+from mm_rs_with_catlass_b200 import _native as N
+from mm_rs_with_catlass_b200.tiling import chooser
+from mm_rs_with_catlass_b200.tiling.config import TilingConfig
+
+
+@pytest.mark.parametrize("workers", [1, 7, 74])
+@pytest.mark.parametrize("slices", [0, 3])
+def test_plan_covers_the_output_once_and_evenly(workers, slices):
+    buf = (C.c_int32 * (6 * 4096))()
+    for m in (1, 257, 600, 2365, 8192):
+        for n in (64, 200, 300, 700, 1696, 5120):
+            for bn in (64, 192, 256):
+                rt, ct = -(-m // 256), -(-n // bn)
+                seen, cut, loads = {}, {}, []
+                for w in range(workers):
+                    cnt = N.lib().catcoc_double_plan_replay(m, n, bn, 4, workers, slices, w, 4096, buf)
+                    load = 0
+                    for kind, m0, n0, rows, cols, s in (buf[6 * i:6 * i + 6] for i in range(cnt)):
+                        assert m0 % 256 == 0 and n0 % bn == 0 and rows == min(256, m - m0) and cols == min(bn * (2 if kind == 1 else 1), n - n0)
+                        units = [(m0, n0)] + ([(m0, n0 + bn)] if kind == 1 else [])
+                        assert kind != 1 or cols > bn                      # no half of a double tile is empty
+                        for u in units:
+                            if kind == 3:
+                                cut.setdefault(u, []).append(s)
+                            else:
+                                seen[u] = seen.get(u, 0) + 1
+                        load += 0 if kind == 3 else len(units)
+                    loads.append(load)
+                assert all(v == 1 for v in seen.values()) and all(sorted(v) == list(range(slices)) for v in cut.values())
+                assert len(seen) + len(cut) == rt * ct and not (set(seen) & set(cut))
+                assert len(cut) == (rt * ct % workers if slices else 0)
+                assert max(loads) == -(-len(seen) // workers)              # no worker has more than its share
+
+
+def test_choices_are_legal():
+    hits = 0
+    for m in (1, 64, 129, 300, 1024, 2365, 8144):
+        for n in (8, 200, 1696, 8192, 28672):
+            for k in (64, 520, 5120, 28672):
+                for dt in (torch.bfloat16, torch.int8):
+                    for major in (False, True):
+                        for swap in (False, True):
+                            t = chooser.choose("matmul", m, n, k, 1, dt, b_k_major=major, tails=True, doubles=True, swap=swap).validate()
+                            assert swap or not t.swap
+                            if t.twice:
+                                hits += 1
+                                assert major or t.swap or t.bn == 256
+                                if t.cut_slices:
+                                    assert t.cut_k * dt.itemsize % 128 == 0 and t.cut_k * (t.cut_slices - 1) < k <= t.cut_k * t.cut_slices
+                            # a caller that does not ask for them gets what it got
+                            old = chooser.choose("matmul", m, n, k, 1, dt, b_k_major=major, tails=True)
+                            assert not old.twice and old == chooser.heuristic("matmul", m, n, k, 1, dt, major, True)
+    assert hits > 100
+    for bad in (dict(twice=True, bn=256), dict(twice=True, bn=100, cta_pair=2), dict(swap=True), dict(cut_slices=2, cut_k=64),
+                dict(twice=True, bn=256, cta_pair=2, cut_slices=1, cut_k=64)):
+        with pytest.raises(ValueError):
+            TilingConfig(**bad).validate()
+    with pytest.raises(ValueError):
+        TilingConfig(twice=True, bn=256, cta_pair=2).validate(local=False)
+
+
+def _check(what):
+    from mm_rs_with_catlass_b200.ops._common import local_status, raise_on_status
+    torch.cuda.synchronize()
+    raise_on_status(local_status(torch.device("cuda", 0)), what)
+
+
+def _operand(g, dtype, *shape):
+    if dtype == torch.int8:
+        return torch.randint(-127, 128, shape, device="cuda", dtype=dtype, generator=g)
+    return torch.randn(*shape, device="cuda", generator=g).to(dtype)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.int8])
+@pytest.mark.parametrize("m,n,k,bn", [
+    (1, 64, 64, 64),            # one unit, one K block
+    (256, 512, 128, 256),       # one whole double tile, two K blocks: no block between the two ends of the tile
+    (300, 1000, 72, 224),       # ragged everywhere; half a window behind the last whole one of a half
+    (513, 336, 1296, 160), (1040, 2064, 520, 96), (2000, 40, 640, 128)])
+def test_matches_the_single_accumulator_kernel(dtype, m, n, k, bn):
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    if dtype == torch.int8:
+        m, n, k = (-(-x // 16) * 16 for x in (m, n, k))
+    for ta in (False, True):
+        for tb in (False, True):
+            a, b = _operand(g, dtype, *((k, m) if ta else (m, k))), _operand(g, dtype, *((n, k) if tb else (k, n)))
+            for out_dtype in ((torch.int32,) if dtype == torch.int8 else (dtype, torch.float32)):
+                want = catcoc.matmul(a, b, trans_a=ta, trans_b=tb, out_dtype=out_dtype, tiling=TilingConfig(bn=256, cta_pair=1))
+                for swap in (False, True):
+                    out = torch.full_like(want, 7)
+                    catcoc.matmul(a, b, trans_a=ta, trans_b=tb, out=out, tiling=TilingConfig(bn=bn, cta_pair=2, twice=True, swap=swap, swizzle=2))
+                    _check("double tiles")
+                    assert torch.equal(out, want), (ta, tb, out_dtype, swap)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("swap", [False, True])
+def test_epilogues(swap):
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(3)
+    m, n, k = 600, 1216, 768
+    t, ref = TilingConfig(bn=224, cta_pair=2, twice=True, swap=swap), TilingConfig(bn=256, cta_pair=1)
+    a, b = _operand(g, torch.bfloat16, m, k), _operand(g, torch.bfloat16, k, n) * 0.05
+    c, bias = _operand(g, torch.bfloat16, m, n), torch.randn(n, device="cuda", generator=g)
+    for kw in (dict(activation="gelu"), dict(alpha=0.5, bias_f32=bias), dict(alpha=-2.0, bias_f32=bias, activation="silu"), dict(alpha=0.5, beta=2.0, c=c)):
+        if swap and "c" in kw:
+            with pytest.raises(RuntimeError, match="without C"):
+                catcoc.matmul(a, b, tiling=t, **kw)
+            continue
+        got, want = catcoc.matmul(a, b, tiling=t, **kw), catcoc.matmul(a, b, tiling=ref, **kw)
+        _check("epilogues")
+        # the same operations on the same sums, which the compiler may contract differently: one bf16 rounding apart at most
+        assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 1e-3).all(), kw
+    x, w = _operand(g, torch.int8, m, k), _operand(g, torch.int8, k, n)
+    s1, s2 = torch.rand(m, device="cuda", generator=g) * 0.02, torch.rand(n, device="cuda", generator=g) * 0.01
+    ib = torch.randint(-1000, 1000, (n,), device="cuda", dtype=torch.int32, generator=g)
+    for kw in (dict(bias=ib), dict(scale_m=s1, scale_n=s2, bias=ib), dict(scale_n=s2, out_dtype=torch.float16), dict(scale_m=s1, out_dtype=torch.float32)):
+        got, want = catcoc.matmul(x, w, tiling=t, **kw), catcoc.matmul(x, w, tiling=ref, **kw)
+        _check("dequantisation")
+        assert torch.equal(got, want), kw
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,bn,slices,cut_k", [(300, 700, 1104, 160, 3, 384), (1024, 2368, 2048, 128, 4, 512), (4000, 5008, 1024, 224, 2, 512)])
+@pytest.mark.parametrize("swap", [False, True])
+def test_cut_units(m, n, k, bn, slices, cut_k, swap):
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(m)
+    t = TilingConfig(bn=bn, cta_pair=2, twice=True, swap=swap, cut_slices=slices, cut_k=cut_k)
+    for tb in (True, False):
+        a, b = _operand(g, torch.bfloat16, m, k), _operand(g, torch.bfloat16, *((n, k) if tb else (k, n)))
+        got = catcoc.matmul(a, b, trans_b=tb, out_dtype=torch.float32, tiling=t)
+        assert torch.equal(got, catcoc.matmul(a, b, trans_b=tb, out_dtype=torch.float32, tiling=t))      # the planned call
+        want = catcoc.matmul(a, b, trans_b=tb, out_dtype=torch.float32, tiling=TilingConfig(bn=256, cta_pair=1))
+        _check("cut units")
+        # both are fp32 sums of exact products, in another order: k * 2^-24 relative to the sum of magnitudes (about sqrt(k))
+        assert (got - want).abs().max().item() < k * 2.0 ** -24 * 4 * k ** 0.5
+        x, w = _operand(g, torch.int8, m // 16 * 16, k), _operand(g, torch.int8, *((n, k) if tb else (k, n)))
+        assert torch.equal(catcoc.matmul(x, w, trans_b=tb, tiling=t), catcoc.matmul(x, w, trans_b=tb, tiling=TilingConfig(bn=256, cta_pair=1)))
+        _check("cut units")
