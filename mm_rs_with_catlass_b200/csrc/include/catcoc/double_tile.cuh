@@ -332,11 +332,9 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
           uint8_t* base = smem + stage * dt.stage_bytes;
           const int k0 = kb * p.bk + k_off;
           if (kMx) {
-            // 512-byte blocks of scales: of this CTA's 128 rows, or of all of the tile's columns
-            for (int b = 0; b < (is_a ? 1 : 3); ++b) {
-              const int blk = is_a ? mn0 / kBM : ti.n0 / 128 + b;
-              ptx::tma_load_2d_pair(base + dt.sf_off + (is_a ? 0 : 512 * (1 + b)), &p.tm_a_gath[is_a ? 0 : 1], bar, 0, (blk * p.sf_k_blocks + kb) * 4);
-            }
+            // 512-byte blocks of scales: of this CTA's 128 rows, or of all of the tile's columns (three blocks, wherever it starts)
+            ptx::tma_load_3d_pair(base + dt.sf_off + (is_a ? 0 : 512), &p.tm_a_gath[is_a ? 0 : 1], bar, 0, (it.k_off / p.bk + kb) * 4,
+                                  is_a ? mn0 / kBM : ti.n0 / 128);
           }
           for (int h = 0; h < parts; ++h) {
             uint8_t* dst = base + smem_off + h * dt.b_half;

@@ -76,15 +76,16 @@ static int encode_2d(CUtensorMap* tm, const void* base, int elt_bytes, CUtensorM
   return CATCOC_OK;
 }
 
-// Packed scale factors: rows of 128 bytes, a box of four (one block of 128 rows x 4 K-blocks), not swizzled.
-static int encode_scales(CUtensorMap* tm, const void* base, int64_t rows) {
+// Packed scale factors, blocks of 512 bytes (128 rows x 4 K-blocks) as four lines of 128, not swizzled: {line, lines of a row tile,
+// row tiles}; a box is the block of one K-block of 128 and `tiles` row tiles in a row.
+static int encode_scales(CUtensorMap* tm, const void* base, int row_tiles, int k_blocks, int tiles) {
   static EncodeTiledFn fn = driver_fn<EncodeTiledFn>("cuTensorMapEncodeTiled");
   if (fn == nullptr) return CATCOC_E_DRIVER;
-  cuuint64_t gdim[2] = {128, static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstride[1] = {128};
-  cuuint32_t box[2] = {128, 4};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t gdim[3] = {128, static_cast<cuuint64_t>(k_blocks) * 4, static_cast<cuuint64_t>(row_tiles)};
+  cuuint64_t gstride[2] = {128, static_cast<cuuint64_t>(k_blocks) * 512};
+  cuuint32_t box[3] = {128, 4, static_cast<cuuint32_t>(tiles)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (scales) failed: CUresult %d", static_cast<int>(r)); return CATCOC_E_DRIVER; }
   return CATCOC_OK;
@@ -365,14 +366,15 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   if (rc != 0) return rc;
   const bool mx = (rf.kind == KIND_MX);
   // Block-scaled tiles leave TMEM room for the scales: 128 x 128 on one CTA, or, for a local product of more than one row
-  // of tiles, 256 x 192 on a pair (two accumulators of 192 columns). A CTA's intake bounds the 128 x 128 tile (33 KiB per
-  // 256 cycles of MMAs; the pair: 29.5 KiB per 384): 4096 x 8192 x 7168 e4m3 with its quantisation 361 -> 258 us.
+  // of tiles, double tiles of 2 x 192 columns (double_tile.cuh). A CTA's intake bounds the 128 x 128 tile (33 KiB per 256 cycles of
+  // MMAs; 256 x 192 on a pair: 29.5 KiB per 384, the double tile: 42 KiB per 768): 4096 x 8192 x 7168 e4m3 with its quantisation
+  // 361, 256 and 222 us.
   const bool mx_pair = mx && !fused && a.M > kBM && a.scale_m == nullptr && a.scale_n == nullptr && !a.affine && a.act == 0;
   // 192-column tiles: pairs of local products (no workspace geometry knows them) with a B stored [N, K]; a [K, N] one comes
   // in 128-byte column blocks, of which a CTA's half would hold one and a half
   const bool bn192 = a.tiling.bn == 192 && !fused && a.trans_b && a.tiling.cta_pair == 2;
   // Double tiles (double_tile.cuh): 256 x 2 bn, local products on pairs
-  const bool twice = a.tiling.twice != 0;
+  const bool twice = a.tiling.twice != 0 || mx_pair;
   const bool cut = a.tiling.cut_slices > 0;
   if (cut && (!twice || a.num_groups > 0 || a.mode != CATCOC_MODE_LOCAL || a.part == nullptr || (reinterpret_cast<uintptr_t>(a.part) & 127) != 0 ||
               a.tiling.cut_slices < 2 || a.tiling.cut_k <= 0 || (a.tiling.cut_k * rf.elt) % 128 != 0 ||
@@ -385,11 +387,11 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     set_error("swapped roles: 16-bit or int8 double tiles without C; over groups of rows of an A stored [M, K], with bn 256");
     return CATCOC_E_UNSUPPORTED;
   }
-  if (twice && (fused || a.tiling.cta_pair != 2 || a.tiling.bn < 64 || a.tiling.bn > kMaxBN || a.tiling.bn % 32 != 0 || (mx && (!mx_pair || a.tiling.bn != 192)))) {
-    set_error("double tiles (bn=%d) are pair tiles of local products, bn a multiple of 32 from 64 to 256 (block-scaled: 192)", a.tiling.bn);
+  if (twice && !mx_pair && (fused || mx || a.tiling.cta_pair != 2 || a.tiling.bn < 64 || a.tiling.bn > kMaxBN || a.tiling.bn % 32 != 0)) {
+    set_error("double tiles (bn=%d) are pair tiles of local products, bn a multiple of 32 from 64 to 256", a.tiling.bn);
     return CATCOC_E_UNSUPPORTED;
   }
-  const int bn = twice ? a.tiling.bn : mx ? (mx_pair ? 192 : 128) : bn192 ? 192 : norm_bn(a.tiling.bn);
+  const int bn = mx ? (mx_pair ? static_cast<int>(dtile::kMxBN) : 128) : twice ? a.tiling.bn : bn192 ? 192 : norm_bn(a.tiling.bn);
   const int seg_dim = pick_seg_dim(a);
   const bool pair = mx ? mx_pair : (a.tiling.cta_pair == 2);
   if (mx) {
@@ -424,8 +426,8 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     // 512-byte scale blocks as four 128-byte rows: the pair's copies are credited to the leader's barrier, which only
     // tensor copies can do
     const int rt_a = (a.M + 127) / 128, rt_b = (a.N + 127) / 128;
-    rc = encode_scales(&p->tm_a_gath[0], a.sfa, static_cast<int64_t>(rt_a) * a.sf_k_blocks * 4);
-    if (rc == 0) rc = encode_scales(&p->tm_a_gath[1], a.sfb, static_cast<int64_t>(rt_b) * a.sf_k_blocks * 4);
+    rc = encode_scales(&p->tm_a_gath[0], a.sfa, rt_a, a.sf_k_blocks, 1);
+    if (rc == 0) rc = encode_scales(&p->tm_a_gath[1], a.sfb, rt_b, a.sf_k_blocks, 3);
     if (rc != 0) return rc;
   }
   p->elt_bytes_a = rf.elt;
@@ -791,9 +793,10 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   if (twice && !grouped) {
     if (cut) grid = imin(imin(sms, a.tiling.num_ctas > 0 ? a.tiling.num_ctas : sms), 2 * max_active_pairs(rf.kind)) & ~1;   // more slices than units
     p->dt.plan = make_double_plan(p->sched, bn, grid / 2, a.tiling.cut_slices, a.tiling.cut_k);
-    if (p->dt.plan.doubles == 0 && !mx) {
+    if (p->dt.plan.doubles == 0) {
       // one block of B per stage: more stages (what single units wait for is the latency of their loads)
-      p->dt.stage_bytes = round_up(kABytes + p->dt.b_half, 1024);
+      p->dt.sf_off = kABytes + p->dt.b_half;
+      p->dt.stage_bytes = round_up(p->dt.sf_off + (mx ? dtile::kMxSfBytes : 0), 1024);
       p->dt.stages = imin(kMaxStages, dtile::kRingBytes / p->dt.stage_bytes);
     }
     if (p->dt.plan.cut > 0) {
@@ -816,7 +819,7 @@ static const inst::Unit* unit_for(int kind, bool pair) {
     case KIND_F16: return pair ? &inst::unit_f16_pair() : &inst::unit_f16_single();
     case KIND_I8: return pair ? &inst::unit_i8_pair() : &inst::unit_i8_single();
     case KIND_F8: return pair ? &inst::unit_f8_pair() : &inst::unit_f8_single();
-    case KIND_MX: return pair ? &inst::unit_mx_pair() : &inst::unit_mx_single();
+    case KIND_MX: return pair ? nullptr : &inst::unit_mx_single();   // (pairs: double tiles)
     default: return nullptr;
   }
 }
@@ -845,7 +848,7 @@ int max_active_pairs(int kind) {
   if (kind < 0 || kind > KIND_MX) return 1;
   if (cached[kind] < 0) {
     if (prepare_kernels() != cudaSuccess) return 1;
-    int n = unit_for(kind, true)->max_clusters();
+    int n = unit_for(kind == KIND_MX ? KIND_F8 : kind, true)->max_clusters();
     int device = 0;
     cudaGetDevice(&device);
     if (n <= 0) n = sm_count(device) / 2;

@@ -17,6 +17,7 @@ import torch
 
 from .. import _native as N
 from ..parallel.shmem import ShmemContext
+from ..tiling.chooser import double_plan
 from ..tiling.config import TilingConfig
 from . import _common as cm
 from . import fused as _fused
@@ -140,7 +141,12 @@ def mxf8_matmul(a_q: torch.Tensor, sfa_packed: torch.Tensor, b_q: torch.Tensor, 
         args.partial_fmt = args.out_fmt
         args.rank, args.W = 0, 1
         args.status = cm.local_status(dev).data_ptr()
-        cm.launch(args, dev)
+        cut = double_plan(m, n, k, 1, 192)[1] if m > 128 else None
+        if cut is None:
+            cm.launch(args, dev)
+        else:
+            cm.fill_tiling(args, TilingConfig(bn=192, cta_pair=2, twice=True, swizzle=4, cut_slices=cut[0], cut_k=cut[1]))
+            cm.launch_double(args, dev)
     return out
 
 

@@ -147,3 +147,35 @@ def test_cut_units(m, n, k, bn, slices, cut_k, swap):
         x, w = _operand(g, torch.int8, m // 16 * 16, k), _operand(g, torch.int8, *((n, k) if tb else (k, n)))
         assert torch.equal(catcoc.matmul(x, w, trans_b=tb, tiling=t), catcoc.matmul(x, w, trans_b=tb, tiling=TilingConfig(bn=256, cta_pair=1)))
         _check("cut units")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(130, 200, 128), (300, 584, 1056), (1024, 1536, 640)])
+def test_block_scaled_cut_units(monkeypatch, m, n, k):
+    import mm_rs_with_catlass_b200 as catcoc
+    from mm_rs_with_catlass_b200.ops import mx
+    g = torch.Generator(device="cuda").manual_seed(k)
+    ops = []
+    for rows in (m, n):
+        q, s = catcoc.quantize_mxf8(torch.randn(rows, k, device="cuda", generator=g), "e4m3")
+        ops += [q, catcoc.pack_scales(s)]
+    res = []
+    for cut in (None, (2, -(-k // 256) * 128)) if k > 128 else (None,):
+        monkeypatch.setattr(mx, "double_plan", lambda *a: (0.0, cut))
+        res.append(catcoc.mxf8_matmul(*ops, out_dtype=torch.float32))
+        _check("block-scaled")
+    # fp32 sums in another order, as above; the operands' magnitudes are about one
+    assert (res[0] - res[-1]).abs().max().item() < k * 2.0 ** -24 * 4 * k ** 0.5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ends", [[0, 1, 70, 70, 333, 900], [900], [64, 128, 900]])
+def test_weight_gradients(ends):
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(9)
+    for m, n in ((256, 512), (264, 520), (520, 1408)):
+        a, b = _operand(g, torch.bfloat16, 900, m), _operand(g, torch.bfloat16, 900, n)
+        want = catcoc.grouped_matmul_slice_k(a, b, ends, tiling=TilingConfig(bn=256, cta_pair=1))
+        got = catcoc.grouped_matmul_slice_k(a, b, ends, tiling=TilingConfig(bn=256, cta_pair=2, twice=True))
+        _check("weight gradients")
+        assert torch.equal(got, want)
