@@ -272,10 +272,8 @@ def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: 
         return True
     dev = a.device
     if tiling is None:
-        from ..tiling.chooser import heuristic
-        tiling = heuristic("matmul", g * m, n, k_total, 1, a.dtype)
-        if tiling.cta_pair == 2 and math.ceil(m / 256) * 256 > 1.18 * math.ceil(m / 128) * 128:
-            tiling = tiling.with_(cta_pair=1)
+        from ..tiling.chooser import slice_k_groups
+        tiling = slice_k_groups(g, m, n, k_total, a.dtype)
     with torch.cuda.device(dev):
         oa, ob = cm.as_operand(a, True), cm.as_operand(b, False)
         if not oa.trans or ob.trans:
