@@ -27,7 +27,8 @@ constexpr int kRingBytes = 192 * 1024;
 #define CATCOC_DT_LEAD 2
 #endif
 constexpr int kLead = CATCOC_DT_LEAD;
-constexpr int kSmemBytes = kRingBytes + 2 * kEpiWarps * kEpiWinBytes + 256 /*barriers*/ + 1024 /*align slack*/;
+constexpr int kSmemBytes = kRingBytes + 2 * kEpiWarps * kEpiWinBytes + 256 /*barriers*/ + 8 * kMaxTokenGroups + 1024 /*align slack*/;
+static_assert(sizeof(SmemTail) <= 256 && kSmemBytes <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t kMxBN = 192;                  // block-scaled: two accumulators of 192 columns, the scales behind them
 constexpr uint32_t kMxSfCol = 2 * kMxBN;         // + slot * 16: SFA (4 columns), SFB of the tile's 384 columns (12)
 constexpr int kMxSfBytes = 4 * 512;              // in a stage: one block of SFA, three of SFB
@@ -41,10 +42,10 @@ CATCOC_DEVICE void umma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
 
 // The same A for both halves of a tile of two column halves: read from shared memory once
 template <int KIND>
-CATCOC_DEVICE void umma_pair_both(uint32_t d0, uint32_t d1, uint64_t a, uint64_t b0, uint64_t b1, uint32_t idesc, uint32_t accum) {
-  if (KIND == KIND_F16) { ptx::umma_f16_pair_fill(d0, a, b0, idesc, accum); ptx::umma_f16_pair_use(d1, a, b1, idesc, accum); }
-  else if (KIND == KIND_I8) { ptx::umma_i8_pair_fill(d0, a, b0, idesc, accum); ptx::umma_i8_pair_use(d1, a, b1, idesc, accum); }
-  else { ptx::umma_f8f6f4_pair_fill(d0, a, b0, idesc, accum); ptx::umma_f8f6f4_pair_use(d1, a, b1, idesc, accum); }
+CATCOC_DEVICE void umma_pair_both(uint32_t d0, uint32_t d1, uint64_t a, uint64_t b0, uint64_t b1, uint32_t idesc, uint32_t idesc1, uint32_t accum) {
+  if (KIND == KIND_F16) { ptx::umma_f16_pair_fill(d0, a, b0, idesc, accum); ptx::umma_f16_pair_use(d1, a, b1, idesc1, accum); }
+  else if (KIND == KIND_I8) { ptx::umma_i8_pair_fill(d0, a, b0, idesc, accum); ptx::umma_i8_pair_use(d1, a, b1, idesc1, accum); }
+  else { ptx::umma_f8f6f4_pair_fill(d0, a, b0, idesc, accum); ptx::umma_f8f6f4_pair_use(d1, a, b1, idesc1, accum); }
 }
 
 // Scales, int32 bias, alpha / beta / C / fp32 bias and activation on 32 columns of one row, in the order of the fused kernel:
@@ -194,11 +195,40 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
   const bool grouped = p.num_groups > 0;
   if (grouped) ptx::grid_dependency_wait();   // the group list may be the predecessor's result
   int total_tiles = 0;
+  TokenGroup* tok_groups = reinterpret_cast<TokenGroup*>(reinterpret_cast<uint8_t*>(tail) + 256);
   if constexpr (kTok) {
-    for (int g = lane; g < p.num_groups; g += 32) {
-      const int b = g == 0 ? 0 : group_end_row(p.group_ends, p.group_rows, sched.N, g - 1);
-      total_tiles += token_tiles(max(0, group_end_row(p.group_ends, p.group_rows, sched.N, g) - b)) * sched.seg_mt;
+    // the groups by falling width of their tiles: extents as in group_walk_tile (clamped, never decreasing) by a scan of one warp,
+    // then every group counts those in front of it
+    TokenGroup* found = reinterpret_cast<TokenGroup*>(epi_stage);
+    if (warp == 0) {
+      int before = 0;
+      for (int g0 = 0; g0 < p.num_groups; g0 += 32) {
+        const int g = g0 + lane;
+        int e = g < p.num_groups ? group_end_row(p.group_ends, p.group_rows, sched.N, g) : 0;
+        int most = e;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int x = __shfl_up_sync(0xffffffffu, most, o);
+          if (lane >= o) most = max(most, x);
+        }
+        const int prev = __shfl_up_sync(0xffffffffu, most, 1);
+        const int begin = lane == 0 ? before : max(before, prev);
+        if (g < p.num_groups) found[g] = TokenGroup{begin, max(0, e - begin) << 7 | g};
+        before = max(before, __shfl_sync(0xffffffffu, most, 31));
+      }
     }
+    __syncthreads();
+    if (threadIdx.x < p.num_groups) {
+      const int g = threadIdx.x, mine = token_width(found[g].rows_g >> 7);
+      int rank = 0;
+      for (int o = 0; o < p.num_groups; ++o) {
+        const int w = token_width(found[o].rows_g >> 7);
+        rank += w > mine || (w == mine && o < g) ? 1 : 0;
+      }
+      tok_groups[rank] = found[g];
+    }
+    __syncthreads();
+    for (int g = lane; g < p.num_groups; g += 32) total_tiles += token_tiles(tok_groups[g].rows_g >> 7) * sched.seg_mt;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) total_tiles += __shfl_xor_sync(0xffffffffu, total_tiles, o);
   } else if (grouped) {
@@ -233,21 +263,36 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
   ptx::grid_dependency_wait();   // nothing above touches global memory
   const long long cta_t0 = (p.trace != nullptr) ? ptx::clock_cycles() : 0;
 
-  // The i-th item of this pair: a tile, its number of halves (a single unit takes one accumulator, in turn), its K range and,
-  // for a slice of a cut unit, its plane (else -1)
-  struct Item { TileInfo ti; int bn, parts, half, k_off, k_len, plane; };
+  // The i-th item of this pair: a tile, its number of halves (a single unit takes one accumulator, in turn) and their columns,
+  // its K range and, for a slice of a cut unit, its plane (else -1)
+  struct Item { TileInfo ti; int bn, bn1, parts, half, k_off, k_len, plane; };
+  struct TokenWalk { int g, tile_base; };
   using Walk = typename std::conditional<kTok, TokenWalk, GroupWalk>::type;
   auto walk_begin = [&]() {
-    if constexpr (kTok) return token_walk_begin(p.num_groups, p.group_ends, p.group_rows, sched.N);
+    if constexpr (kTok) return TokenWalk{0, 0};
     else return group_walk_begin(p);
   };
   auto get_item = [&](int i, Walk& walk, Item& it) {
-    it.bn = dt.bn; it.parts = 2; it.half = 0; it.k_off = 0; it.k_len = p.K; it.plane = -1;
+    it.bn = it.bn1 = dt.bn; it.parts = 2; it.half = 0; it.k_off = 0; it.k_len = p.K; it.plane = -1;
     if constexpr (kTok) {
-      const int t = worker + i * num_workers;
+      const int t = i * num_workers + ((i & 1) ? num_workers - 1 - worker : worker);
       if (t >= total_tiles) return false;
-      it.ti = token_walk_tile(sched.M, p.num_groups, p.group_ends, p.group_rows, sched.N, t, walk, it.bn);
-      if (it.ti.cols <= it.bn) { it.parts = 1; it.half = i & 1; }
+      int tiles = token_tiles(tok_groups[walk.g].rows_g >> 7) * sched.seg_mt;
+      while (t >= walk.tile_base + tiles) {
+        walk.tile_base += tiles;
+        tiles = token_tiles(tok_groups[++walk.g].rows_g >> 7) * sched.seg_mt;
+      }
+      const int local = t - walk.tile_base;
+      const TokenTile tt = token_tile(tok_groups[walk.g], local / sched.seg_mt);
+      it.ti.seg = tt.group;
+      it.ti.mi = local % sched.seg_mt;
+      it.ti.m0 = it.ti.mi * 2 * kBM;
+      it.ti.rows = min(2 * kBM, sched.M - it.ti.m0);
+      it.ti.n0 = tt.n0;
+      it.ti.cols = tt.valid;
+      it.bn = token_half0(tt.width);
+      it.bn1 = tt.width - it.bn;
+      if (it.bn1 == 0) { it.parts = 1; it.half = i & 1; }
       return true;
     } else if (grouped) {
       const int t = worker + i * num_workers;
@@ -298,9 +343,8 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
       const TileInfo& ti = it.ti;
       const int parts = is_a ? 1 : it.parts;                        // each half has a block of B of its own
       int k_off = it.k_off;
-      const int bn = it.bn, cta_cols = is_a ? kBM : bn / 2, boxes = ceil_div(cta_cols, per_box);
-      const int part_bytes = is_a ? kABytes : kTok ? bn * 64 : dt.b_half;
-      int mn0 = (is_a ? ti.m0 + sub * kBM : ti.n0 + sub * cta_cols);
+      const int bytes = is_a ? kABytes : kTok ? (it.bn + (parts == 2 ? it.bn1 : 0)) * 64 : parts * dt.b_half;
+      int mn0 = is_a ? ti.m0 + sub * kBM : ti.n0;
       if (grouped) {
         // (with swapped roles the operand under A is the groups' weights)
         const bool weights = is_a == SWAP;
@@ -309,8 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
       }
       const CUtensorMap* tm = is_a ? &p.tm_a : &p.tm_b;
       bool map_3d = is_a ? p.a_3d != 0 : p.b_3d != 0;
-      if (!is_a && p.b_3d == 2 && mn0 + (parts - 1) * bn + cta_cols > sched.N / per_box * per_box) { map_3d = false; tm = &p.tm_a_gath[1]; }
-      if constexpr (kTok) { if (!is_a) tm = &p.tok_map[bn / 32 - 1]; }
+      if (!is_a && p.b_3d == 2 && mn0 + (parts - 1) * it.bn + sub * it.bn / 2 + it.bn / 2 > sched.N / per_box * per_box) { map_3d = false; tm = &p.tm_a_gath[1]; }
       if constexpr (kGk) tm = &p.gk_map[2 * ti.seg + (is_a ? 0 : 1)];
       const int tile_kb = ceil_div(it.k_len, p.bk);
       for (int kb = 0; kb < tile_kb; ++kb) {
@@ -328,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
         if (ptx::elect_one()) {
           // both CTAs' copies are credited to the leader's barrier; only the leader arms it, with the bytes of the pair
           const uint32_t bar = ptx::map_to_cta(ptx::smem_u32(&tail->full[stage]), 0u);
-          if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * (parts * part_bytes + (!kMx ? 0 : is_a ? 512 : 1536)));
+          if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * (bytes + (!kMx ? 0 : is_a ? 512 : 1536)));
           uint8_t* base = smem + stage * dt.stage_bytes;
           const int k0 = kb * p.bk + k_off;
           if (kMx) {
@@ -338,13 +381,15 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
           }
           for (int h = 0; h < parts; ++h) {
             uint8_t* dst = base + smem_off + h * dt.b_half;
-            const int c0 = mn0 + h * bn;
+            const int bn = h == 0 ? it.bn : it.bn1;
+            const int c0 = is_a ? mn0 : mn0 + h * it.bn + sub * (bn / 2);
+            if constexpr (kTok) { if (!is_a) tm = &p.tok_map[bn / 32 - 1]; }
             if (!mn) {
               ptx::tma_load_2d_pair(dst, tm, bar, k0, c0);
             } else if (map_3d) {
               ptx::tma_load_3d_pair(dst, tm, bar, 0, k0, c0 / per_box);
             } else {
-              for (int b = 0; b < boxes; ++b) ptx::tma_load_2d_pair(dst + b * (p.bk * 128), tm, bar, c0 + b * per_box, k0);
+              for (int b = 0; b * per_box < (is_a ? kBM : bn / 2); ++b) ptx::tma_load_2d_pair(dst + b * (p.bk * 128), tm, bar, c0 + b * per_box, k0);
             }
           }
         }
@@ -378,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
       const uint32_t a_lo = static_cast<uint32_t>(da0), a_hi = static_cast<uint32_t>(da0 >> 32);
       const uint32_t b_lo = static_cast<uint32_t>(db0), b_hi = static_cast<uint32_t>(db0 >> 32);
       const uint32_t b_half = static_cast<uint32_t>(dt.b_half) >> 4;
-      uint32_t idesc = p.idesc;
+      uint32_t idesc = p.idesc, idesc1 = p.idesc;
       const bool tr = (p.trace != nullptr) && lane == 0;
       unsigned long long c_full = 0, c_acc = 0, c_issue = 0;
       Tick tick(tr);
@@ -388,7 +433,10 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
       for (int i = 0; ok && get_item(i, walk, it); ++i) {
         const int tile_kb = ceil_div(it.k_len, p.bk), k_mmas = ceil_div(it.k_len, p.umma_k);
         if (tile_kb <= 0) continue;
-        if constexpr (kTok) idesc = (p.idesc & ~(0x3Fu << 17)) | static_cast<uint32_t>(it.bn >> 3) << 17;   // the tile's own width
+        if constexpr (kTok) {   // the halves' own widths
+          idesc = (p.idesc & ~(0x3Fu << 17)) | static_cast<uint32_t>(it.bn >> 3) << 17;
+          idesc1 = (p.idesc & ~(0x3Fu << 17)) | static_cast<uint32_t>(it.bn1 >> 3) << 17;
+        }
         const uint32_t sfb0 = 4u + (static_cast<uint32_t>(it.ti.n0 & 127) >> 5);   // block-scaled: a tile may start inside a block
         // Waits for the stage under half 0's cursor. `probed` is the answer of a probe made before the previous stage's products
         // were issued: a stage that was ready by then costs nothing here.
@@ -440,9 +488,9 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
                 ptx::umma_mxf8_pair(d, da, db, id, sf | sel, sfb | sel, accum);
               }
             } else if (m == 2) {
-              umma_pair_both<KIND>(d, d + acc_stride, da, db, ptx::desc_of(bl + b_half + k * b_kinc, b_hi), idesc, accum);
+              umma_pair_both<KIND>(d, d + acc_stride, da, db, ptx::desc_of(bl + b_half + k * b_kinc, b_hi), idesc, idesc1, accum);
             } else {
-              umma_pair<KIND>(d, da, db, idesc, accum);
+              umma_pair<KIND>(d, da, db, m == 1 ? idesc1 : idesc, accum);
             }
           };
           const int left = k_mmas - kb * 4;
@@ -546,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
       const TileInfo& ti = it.ti;
       const bool raw = it.plane >= 0;         // a slice's accumulator goes to its plane whole, as it is
       const int st_fmt = raw ? (KIND == KIND_I8 ? FMT_S32 : FMT_F32) : p.out_fmt, st_elt = fmt_bytes(st_fmt);
-      const int bn = it.bn, col_base = it.parts == 2 ? h * bn : 0;
+      const int bn = it.parts == 2 && h == 1 ? it.bn1 : it.bn, col_base = it.parts == 2 ? h * it.bn : 0;
       const int rows_valid = raw ? 32 : max(0, min(32, ti.rows - row_base));   // (swapped roles: features, and tokens below)
       const int cols = raw ? bn : max(0, min(bn, ti.cols - col_base));
       const int n0 = ti.n0 + col_base;

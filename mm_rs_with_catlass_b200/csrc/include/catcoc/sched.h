@@ -384,51 +384,28 @@ CATCOC_HD TileInfo double_unit_extent(const TileSched& s, const DoublePlan& d, i
   return ti;
 }
 
-// Ragged groups of tokens on double tiles whose columns are tokens (swapped roles): a group's tokens are spread evenly over as
-// few tiles as hold them, in halves of a multiple of 32, and every tile of tokens meets all blocks of 256 features.
-struct TokenWalk { int g, tile_base, begin, end; };
+// Ragged groups of tokens on tiles whose columns are tokens (swapped roles). A group's tokens are spread evenly over as few tiles
+// of up to 512 as hold them, every one a multiple of 32 wide, and every tile of tokens meets all blocks of 256 features. Up to
+// 160 tokens are a single unit: its MMAs then take no longer to issue than to run, and the pair's accumulators alternate.
+// Groups are visited by falling width and dealt out forwards and backwards in turn, which evens out what the workers get: the
+// widest tiles go first and the narrowest fill up (32 groups of 110 to 770 tokens, 16 feature blocks, 74 workers: the busiest
+// has 4 % more than the mean, in the order of the groups 12 %).
+constexpr int kMaxTokenGroups = 128;
+struct TokenGroup { int begin, rows_g; };   // first token; tokens << 7 | group
+struct TokenTile { int group, n0, width, valid; };
 CATCOC_HD int token_tiles(int rows) { return (rows + 511) / 512; }
-CATCOC_HD int token_half(int rows) {    // tokens of half a tile
-  const int t = token_tiles(rows);
-  return t > 0 ? round_up(ceil_div(ceil_div(rows, t), 2), 32) : 32;
+CATCOC_HD int token_width(int rows) { return rows > 0 ? round_up(ceil_div(rows, token_tiles(rows)), 32) : 0; }
+// j-th tile of tokens of a group
+CATCOC_HD TokenTile token_tile(const TokenGroup& g, int j) {
+  const int rows = g.rows_g >> 7, w = token_width(rows);
+  TokenTile t;
+  t.group = g.rows_g & (kMaxTokenGroups - 1);
+  t.n0 = g.begin + j * w;
+  t.valid = imin(w, rows - j * w);
+  t.width = round_up(t.valid, 32);
+  return t;
 }
-CATCOC_HD TokenWalk token_walk_begin(int num_groups, const int32_t* ends, int group_rows, int M) {
-  TokenWalk w = {0, 0, 0, num_groups > 0 ? group_end_row(ends, group_rows, M, 0) : 0};
-  return w;
-}
-CATCOC_HD int token_walk_total(int feature_blocks, int num_groups, const int32_t* ends, int group_rows, int M) {
-  int total = 0, begin = 0;
-  for (int g = 0; g < num_groups; ++g) {
-    const int e = group_end_row(ends, group_rows, M, g);
-    if (e > begin) { total += token_tiles(e - begin) * feature_blocks; begin = e; }
-  }
-  return total;
-}
-// Tile `t` (not below an earlier call's): rows are features, columns tokens; `half` = tokens of each half
-CATCOC_HD TileInfo token_walk_tile(int features, int num_groups, const int32_t* ends, int group_rows, int M, int t, TokenWalk& w, int& half) {
-  const int fb = ceil_div(features, 256);
-  int rows = imin(w.end - w.begin, M);
-  while (t >= w.tile_base + token_tiles(rows > 0 ? rows : 0) * fb && w.g + 1 < num_groups) {
-    w.tile_base += token_tiles(rows > 0 ? rows : 0) * fb;
-    ++w.g;
-    if (w.end > w.begin) w.begin = w.end;
-    w.end = group_end_row(ends, group_rows, M, w.g);
-    rows = w.end - w.begin;
-  }
-  half = token_half(rows > 0 ? rows : 0);
-  TileInfo ti;
-  const int local = t - w.tile_base;
-  ti.seg = w.g;
-  ti.tile_in_seg = local;
-  ti.mi = local % fb;
-  ti.ni = local / fb;
-  ti.m0 = ti.mi * 256;
-  ti.n0 = w.begin + ti.ni * 2 * half;
-  ti.rows = imin(256, features - ti.m0);
-  ti.cols = imin(2 * half, w.end - ti.n0);
-  if (ti.cols < 0) ti.cols = 0;
-  return ti;
-}
+CATCOC_HD int token_half0(int width) { return width <= 160 ? width : round_up(ceil_div(width, 2), 32); }
 
 // Order in which a pusher visits its peers: the peer that consumes this rank's data earliest
 // comes first. For source-major consumers (allgather_matmul) rank r reads source q in phase

@@ -383,8 +383,8 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     return CATCOC_E_BAD_ARG;
   }
   if (swap && (!twice || (rf.kind != KIND_F16 && rf.kind != KIND_I8) || a.c_src != nullptr ||
-               (a.num_groups > 0 && (a.tiling.bn != kMaxBN || o.trans_a || a.g_a_row_back != 0 || a.g_a_k != 0)))) {
-    set_error("swapped roles: 16-bit or int8 double tiles without C; over groups of rows of an A stored [M, K], with bn 256");
+               (a.num_groups > 0 && (a.tiling.bn != kMaxBN || a.num_groups > kMaxTokenGroups || o.M >= (1 << 24) || o.trans_a || a.g_a_row_back != 0 || a.g_a_k != 0)))) {
+    set_error("swapped roles: 16-bit or int8 double tiles without C; over up to %d groups of rows of an A stored [M, K], with bn 256", kMaxTokenGroups);
     return CATCOC_E_UNSUPPORTED;
   }
   if (twice && !mx_pair && (fused || mx || a.tiling.cta_pair != 2 || a.tiling.bn < 64 || a.tiling.bn > kMaxBN || a.tiling.bn % 32 != 0)) {

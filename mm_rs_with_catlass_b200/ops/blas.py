@@ -40,6 +40,7 @@ from typing import List, Optional, Sequence, Union
 import torch
 
 from .. import _native as N
+from ..tiling.chooser import token_groups
 from ..tiling.config import TilingConfig
 from . import _common as cm
 from .gemm import matmul
@@ -179,7 +180,7 @@ def _grouped_launch(a, b, ends, trans_b, out, out_dtype, tiling, **epilogue):
     b2 = b.contiguous().reshape(g * b.shape[1], b.shape[2])
     a2 = a if a.is_contiguous() else a.contiguous()
     return matmul(a2, b2, trans_b=trans_b, out=out, out_dtype=out_dtype,
-                  tiling=_group_tiling(tiling, m_total, m_total / max(1, g), n, k, a.dtype), _group=group, **epilogue)
+                  tiling=tiling if tiling is not None else token_groups(m_total, g, n, k, a.dtype), _group=group, **epilogue)
 
 
 def grouped_matmul(a: torch.Tensor, b: torch.Tensor, group_list: GroupList, *, trans_b: bool = False,

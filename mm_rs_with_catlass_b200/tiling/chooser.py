@@ -303,6 +303,43 @@ def _grouped(rows_total: int, rows_per_group: float, n: int, dtype: torch.dtype,
     return TilingConfig(bn=best[1], swizzle=4, cta_pair=best[2])
 
 
+def token_groups(rows_total: int, groups: int, n: int, k: int, dtype: torch.dtype) -> TilingConfig:
+    """Tiling of a product over ragged groups of rows of an A stored [M, K] (their extents are on the device): :func:`grouped`'s,
+    or double tiles with swapped roles, whose columns fit each group's rows to 32 where the other tiles pad them to 128 or 256.
+
+    Groups of 110 to 770 rows, 32 of them, 4096 x 2048: 256 -> 227 us; 16 of 539 on average, 4096 x 4096: 321 -> 278; int8, 8 of
+    451, 4096 x 2048: 55 -> 49. Few rows per group are bound by the weights' bytes, and the narrow pairs stream them more slowly
+    (64 groups of 18, 1408 x 2048: 74 against 88 us), as does a short K, whose epilogues nothing covers."""
+    return _token_groups(rows_total, groups, n, k, dtype, os.environ.get("CATCOC_CTA_PAIR"))
+
+
+@functools.lru_cache(maxsize=4096)
+def _token_groups(rows_total: int, groups: int, n: int, k: int, dtype: torch.dtype, forced: Optional[str]) -> TilingConfig:
+    rows = rows_total / max(1, groups)
+    old = _grouped(rows_total, rows, n, dtype, forced)
+    if forced == "1" or rows < 128 or groups > 128 or rows_total >= 1 << 24 or dtype not in (torch.float16, torch.bfloat16, torch.int8):
+        return old
+    if dtype == torch.int8 and old.cta_pair == 2:      # 32 groups of 837, 4096 x 4096: 445 us, 499 with swapped roles
+        return old
+    kb, fb, hbm = -(-k * dtype.itemsize // 128), -(-n // 256), groups * n * k * dtype.itemsize / _HBM
+    total = count = 0.0
+    for f in (0.375, 0.625, 0.875, 1.125, 1.375, 1.625):       # a spread of sizes around the mean
+        t = math.ceil(rows * f / 512)
+        w = min(512, math.ceil(rows * f / t / 32) * 32)
+        total += t * (kb * (560 if w <= 128 else max(610.0, 122 + 1.9 * w)) + 6000) / 6
+        count += t / 6
+    waves = count * groups * fb / (_NUM_SMS // 2)
+    uneven = min(math.ceil(waves) - waves, 0.5 if waves > 1 else 1.0) if waves < 4 else 0.35
+    new = max(total * groups * fb / (_NUM_SMS // 2) + total / count * uneven, hbm)
+    bm = 128 * old.cta_pair
+    unit = {(256, 1): 900, (128, 1): 620, (64, 1): 500, (256, 2): 640, (128, 2): 430}[(old.effective_bn, old.cta_pair)]
+    tiles = groups * max(1.0, rows / bm + 0.5) * -(-n // old.effective_bn)
+    cycles = max(math.ceil(tiles / (_NUM_SMS // old.cta_pair)) * kb * unit, hbm)
+    if new + _LAUNCH < (cycles + _LAUNCH) / (0.985 if dtype != torch.int8 else 1.02):
+        return TilingConfig(bn=256, swizzle=4, cta_pair=2, twice=True, swap=True)
+    return old
+
+
 def choose(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype,
            table: Optional["_table.TilingTable"] = None, b_k_major: bool = False, tails: bool = False,
            doubles: bool = False, swap: bool = False) -> TilingConfig:

@@ -179,3 +179,50 @@ def test_weight_gradients(ends):
         got = catcoc.grouped_matmul_slice_k(a, b, ends, tiling=TilingConfig(bn=256, cta_pair=2, twice=True))
         _check("weight gradients")
         assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.int8])
+@pytest.mark.parametrize("sizes", [
+    [0, 1, 31, 32, 33, 160, 161, 192, 0], [512, 513, 0, 1025, 300], [777], [3] * 128, [0, 0, 256, 0]])
+def test_token_groups(dtype, sizes):
+    # groups at the edges of the widths (32, the single unit of 160, one tile of 512), empty ones, the most groups; their order
+    # by width is the kernel's own affair
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    total, n, k = sum(sizes), 336, 256
+    ends = torch.tensor(sizes).cumsum(0).to(torch.int32).cuda()
+    t, ref = TilingConfig(bn=256, cta_pair=2, twice=True, swap=True), TilingConfig(bn=256, cta_pair=1)
+    for tb in (False, True):
+        a, b = _operand(g, dtype, total, k), _operand(g, dtype, *((len(sizes), n, k) if tb else (len(sizes), k, n)))
+        if dtype == torch.int8:
+            s1, s2 = torch.rand(total, device="cuda", generator=g), torch.rand(len(sizes), n, device="cuda", generator=g)
+            res = [catcoc.grouped_quant_matmul(a, b, s1, s2, ends, trans_b=tb, tiling=x) for x in (t, ref)]
+        else:
+            res = [catcoc.grouped_matmul(a, b, ends, trans_b=tb, tiling=x) for x in (t, ref)]
+            res += [catcoc.grouped_matmul(a, b, ends, trans_b=tb, out_dtype=torch.float32, tiling=x) for x in (t, ref)]
+        _check("token groups")
+        assert all(torch.equal(x, y) for x, y in zip(res[::2], res[1::2])), tb
+
+
+@pytest.mark.gpu
+def test_malformed_group_lists_stay_inside_the_output():
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(2)
+    a, b = _operand(g, torch.bfloat16, 300, 128), _operand(g, torch.bfloat16, 4, 128, 256)
+    ends = torch.tensor([200, 100, 1000, -5], dtype=torch.int32, device="cuda")      # decreasing, past the end, negative
+    out = [catcoc.grouped_matmul(a, b, ends, out=torch.zeros(300, 256, device="cuda", dtype=torch.bfloat16), tiling=t)
+           for t in (TilingConfig(bn=256, cta_pair=2, twice=True, swap=True), TilingConfig(bn=256, cta_pair=1))]
+    _check("group lists")
+    assert torch.equal(out[0], out[1])
+
+
+def test_token_group_choice():
+    for groups in (1, 8, 64, 200):
+        for rows in (1, 100, 440, 3000):
+            for n, k in ((1408, 1024), (4096, 4096), (8, 64)):
+                for dt in (torch.bfloat16, torch.int8):
+                    t = chooser.token_groups(groups * rows, groups, n, k, dt).validate()
+                    assert not t.twice or (t.swap and t.bn == 256 and groups <= 128 and rows >= 128)
+    assert chooser.token_groups(14080, 32, 4096, 2048, torch.bfloat16).swap
+    assert not chooser.token_groups(1158, 64, 1408, 2048, torch.bfloat16).twice
