@@ -46,13 +46,14 @@ CATCOC_DEVICE void rescale_o(uint32_t t_o, float alpha) {
 // Reads 128 scores at TMEM address `t_s`, writes the packed probabilities (64 columns) to `t_p`, which may be the same
 // place, and updates the state. `loaded()` is called when the scores are in registers, `before(move, alpha)` ahead of the
 // first probability: with `move` (the same in all lanes) the reference maximum of some row of the warp moved and O has to
-// be multiplied by alpha. `half()` is called when the probabilities of the first 64 keys have been issued. `vis_left`: keys of this block the row sees (used when `masked`).
+// be multiplied by alpha; `ready()` ahead of the first store of probabilities, `half()` behind
+// it (those of the first 64 keys). `vis_left`: keys of this block the row sees (used when `masked`).
 //
-// A quarter of the exponentials as a degree-5 polynomial on the FMA pipe gave no clear gain (4 % slower to 0.5 % faster in three
-// trials): a chain of one row's steps, not the special-function unit, is what a tile waits for.
-template <int FMT, class Loaded, class Before, class Half>
+// Tried and not kept: a quarter of the exponentials as a degree-5 polynomial on the FMA pipe (D = 128, causal 4 % faster, not causal 2
+// to 6 % slower, D = 64 slower), the two warps of a scheduler taking their exponentials strictly in turn (4 % slower).
+template <int FMT, class Loaded, class Before, class Ready, class Half>
 CATCOC_DEVICE void softmax_row_block(uint32_t t_s, uint32_t t_p, bool masked, int vis_left, float sc, RowState& st, Loaded&& loaded,
-                                     Before&& before, Half&& half) {
+                                     Before&& before, Ready&& ready, Half&& half) {
   uint32_t v[4][32];
 #pragma unroll
   for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32b_x32(t_s + c * 32, v[c]);
@@ -93,6 +94,7 @@ CATCOC_DEVICE void softmax_row_block(uint32_t t_s, uint32_t t_p, bool masked, in
       sum2[i & 1] = ptx::add_f32x2(sum2[i & 1], ptx::pack_f32x2(e0, e1));
       w[i] = pack16<FMT>(e0, e1);
     }
+    if (h == 0) ready();
     ptx::tmem_st_32x32b_x32(t_p + h * 32, w);
     if (h == 0) half();
   }

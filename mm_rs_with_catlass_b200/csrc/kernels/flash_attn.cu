@@ -5,18 +5,18 @@
 //                                   TMEM when the running maximum moved by more than 2^8, final O / l and the store
 //   warp 8      TMA producer      : both Q tiles once, then K and V blocks of 128 keys through one ring of slots
 //   warp 9      MMA issuer        : S_t = Q_t K^T into TMEM, O_t += P_t V with P read from TMEM (the A operand of
-//                                   tcgen05.mma may live there), alternating between the two tiles
+//                                   tcgen05.mma may live there); at D = 128 for tile 0, and warp 10 for tile 1
 //
-// TMEM columns: S_0 [0, 128), S_1 [128, 256), O_0 [256, 256 + D), O_1 [256 + D, 256 + 2 D); P_t is 64 columns of
-// packed 16-bit pairs on top of S_t. While the softmax warps of one tile work, the tensor core runs the other
-// tile's two products.
+// TMEM columns, D = 128: one buffer of scores for both tiles [0, 128), P_0 and P_1 (64 columns of packed 16-bit pairs each) at
+// 128 and 192, O_0 and O_1 at 256 and 384. D = 64: S_0, S_1 at 0 and 128, O_0, O_1 at 256 and 320, P_0, P_1 at 384 and 448. The
+// scores are read from TMEM once and stay in registers (softmax_row.cuh; a split of the registers between the warpgroups makes
+// room), so that a tile's next scores are computed while its softmax works on the present ones.
 //
-// Bound by the chain of one tile, scores -> maximum -> exponentials -> P V -> next scores (the tensor core is busy
-// 56 % of the time, the special-function unit as much). So the scores are read from TMEM once and stay in registers
-// (softmax_row.cuh; a split of the registers between the warpgroups makes room), and P V starts when the first 64
-// keys' probabilities are written. Causal, 2 x 32 / 8 heads x 8192, D = 128, in a loop (which holds the clocks at the power
-// limit): 1196 -> 1065 us, and 1036 us (1.06 PFLOP/s) in the CTA order below. At D = 64 the probabilities have columns of
-// their own (O_0, O_1 at 256 and 320, P_0, P_1 at 384 and 448), which takes P V out of the chain: 776 -> 719 us.
+// Bound by the steps of one row: of 2930 cycles a block (D = 128, per tile, cycle counters) 260 go to reading the scores, 300 to
+// the maximum, 1840 to the exponentials beside the other tile's (the special-function unit alone: 1024), 400 to waiting for
+// the next scores; tensor cores and special-function unit are 70 % busy. With P on top of S_t and one issuer for both tiles, whose
+// products waited behind the other tile's softmax, a block took 3490. Causal, 2 x 32 / 8 heads x 8192, D = 128: 855 -> 770 us
+// at full clock (operands of zeros), 1040 -> 980 us in a loop, which the power limit holds.
 //
 // The online-softmax recurrence (m: reference maximum, l: running sum, per row, in the log2 domain):
 //   P = exp2(scale S - m),  l' = l a + rowsum(P),  O' = O a + P V,  a = exp2(m - m')
@@ -48,7 +48,7 @@ constexpr int kThreads = 384;     // 2 x 4 softmax warps, producer, issuer, two 
 // Registers: a softmax thread keeps 128 scores and their probabilities. The block is launched with 168 a thread; the
 // third warpgroup gives up what the first two take: 2 x 216 + 72 = 3 x 168.
 constexpr int kSoftmaxRegs = 216, kOtherRegs = 72;
-constexpr int kProducerWarp = 8, kIssuerWarp = 9;
+constexpr int kProducerWarp = 8, kIssuerWarp = 9;   // + t: a tile's issuer
 constexpr int kBlockBytes = 128 * 128;   // one 128-row x 128-byte (64 element) swizzled block
 constexpr int kMaxSlots = 8;
 
@@ -88,11 +88,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   constexpr int kSlots = D == 128 ? 4 : 8;       // ring of K / V blocks (K_0 V_0 K_1 V_1 ...)
   constexpr uint32_t kTmemCols = 512;
   constexpr uint32_t kOCol = 256;
-  // D = 64 leaves 128 columns of TMEM: the probabilities get columns of their own, and the next scores are computed as soon
-  // as the softmax has read the present ones instead of behind the second product
-  constexpr bool kOwnP = D == 64;
-  constexpr uint32_t kPCol = kOwnP ? 384 : 0;      // P_t at kPCol + t * kPStride
-  constexpr uint32_t kPStride = kOwnP ? 64 : 128;
+  // The probabilities have columns of their own, so that the next scores are computed as soon as the softmax has read the
+  // present ones and not behind the second product. At D = 128 that leaves one buffer of scores, which the tiles take in turn.
+  // Each tile then has an issuer of its own, so that no tile's products wait behind the other's softmax (one issuer for both: 864
+  // us where two take 772, causal 2 x 32 / 8 x 8192 of zeros). At D = 64 one warp issues both tiles' scores, then both products with V,
+  // which start on the first half of the keys (two issuers, whole blocks: 728 -> 764 us, 2 x 32 x 8192 of zeros).
+  constexpr bool kOneS = D == 128;
+  constexpr int kIssuers = kOneS ? 2 : 1;
+  constexpr uint32_t kPCol = kOneS ? 128 : 384;    // P_t at kPCol + t * 64
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sq = smem;                            // two Q tiles
@@ -127,7 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
 
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bars->q_full, 1);
-    for (int s = 0; s < kSlots; ++s) { ptx::mbar_init(&bars->kv_full[s], 1); ptx::mbar_init(&bars->kv_empty[s], 1); }
+    for (int s = 0; s < kSlots; ++s) { ptx::mbar_init(&bars->kv_full[s], 1); ptx::mbar_init(&bars->kv_empty[s], kIssuers); }
     for (int t = 0; t < kTiles; ++t) {
       ptx::mbar_init(&bars->s_full[t], 1);
       ptx::mbar_init(&bars->s_free[t], 4);
@@ -173,134 +176,90 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       }
       __syncwarp();
     }
-  } else if (warp == kIssuerWarp) {
-    // ------------------------------ MMA issuer ------------------------------
+  } else if (warp >= kIssuerWarp && warp < kIssuerWarp + kIssuers) {
+    // ------------------------------ MMA issuers ------------------------------
+    const uint64_t dq0 = ptx::make_smem_desc_sw128(ptx::smem_u32(sq), 16u, 1024u);
+    const uint64_t dk0 = ptx::make_smem_desc_sw128(ptx::smem_u32(skv), 16u, 1024u);
+    const uint64_t dv0 = ptx::make_smem_desc_sw128(ptx::smem_u32(skv), static_cast<uint32_t>(kBlockBytes), 1024u);
+    // (addresses are in the low words, which no tile or slot carries over into the high ones)
+    const uint32_t q_lo = static_cast<uint32_t>(dq0), q_hi = static_cast<uint32_t>(dq0 >> 32);
+    const uint32_t k_lo = static_cast<uint32_t>(dk0), k_hi = static_cast<uint32_t>(dk0 >> 32);
+    const uint32_t v_lo = static_cast<uint32_t>(dv0), v_hi = static_cast<uint32_t>(dv0 >> 32);
     auto wait_item = [&](int item) {
       return ptx::mbar_wait(&bars->kv_full[item % kSlots], static_cast<uint32_t>(item / kSlots) & 1u, p.timeout_ns, abort_flag);
     };
-    auto issue_qk = [&](int t, int item) {
-      // S_t[128, 128 keys] = Q_t[128, D] K^T: both operands K-major (D contiguous), 16 elements of D per MMA
-      const uint64_t dq = ptx::make_smem_desc_sw128(ptx::smem_u32(sq + t * kQBytes), 16u, 1024u);
-      const uint64_t dk = ptx::make_smem_desc_sw128(ptx::smem_u32(skv + (item % kSlots) * kSlotBytes), 16u, 1024u);
+    // (one warp for both tiles has waited for tile 0's block when it comes to tile 1)
+    auto first_use = [&](int t, int j) { return kOneS || t == 0 || j >= nblk[0]; };
+    // S_t[128, 128 keys] = Q_t[128, D] K^T of block j, behind the softmax's read of what is in the buffer: both operands
+    // K-major (D contiguous), 16 elements of D per MMA
+    auto scores = [&](int t, int j) {
+      if (first_use(t, j) && !wait_item(2 * j)) return false;
+      const int before = !kOneS || t == 0 || j >= nblk[0] ? j - 1 : j;             // the block and the tile that were there
+      const int tile = !kOneS ? t : (t == 1 && j < nblk[0] ? 0 : 1);
+      if (before >= 0 && !ptx::mbar_wait(&bars->s_free[tile], static_cast<uint32_t>(before & 1), p.timeout_ns, abort_flag)) return false;
+      ptx::tcgen05_fence_after();
+      const int slot = (2 * j) % kSlots;
+      if (ptx::elect_one()) {
+        const uint32_t ql = q_lo + static_cast<uint32_t>(t * (kQBytes >> 4)), kl = k_lo + static_cast<uint32_t>(slot * (kSlotBytes >> 4));
 #pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        const uint64_t off = static_cast<uint64_t>(((kk >> 2) * kBlockBytes + (kk & 3) * 32) >> 4);
-        ptx::umma_f16(tmem + t * 128, dq + off, dk + off, p.idesc_qk, kk != 0 ? 1u : 0u);
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint32_t off = static_cast<uint32_t>(((kk >> 2) * kBlockBytes + (kk & 3) * 32) >> 4);
+          ptx::umma_f16(tmem + (kOneS ? 0 : t * 128), ptx::desc_of(ql + off, q_hi), ptx::desc_of(kl + off, k_hi), p.idesc_qk, kk != 0 ? 1u : 0u);
+        }
+        ptx::tcgen05_commit(&bars->s_full[t]);
+        if (kOneS || t == 1) ptx::tcgen05_commit(&bars->kv_empty[slot]);     // (tile 1 walks no fewer blocks than tile 0)
       }
-      ptx::tcgen05_commit(&bars->s_full[t]);
+      __syncwarp();
+      return true;
     };
-    auto issue_pv = [&](int t, int item, int half, bool accumulate) {
-      // O_t[128, D] += P_t[128, 128 keys] V[128 keys, D]: P from TMEM (row = lane, two keys per 32-bit column, 8
-      // columns per MMA), V MN-major (D contiguous): 16 key rows per MMA = 2048 bytes down a block, blocks of 64
-      // head-dim columns 16 KiB apart
-      const uint64_t dv = ptx::make_smem_desc_sw128(ptx::smem_u32(skv + (item % kSlots) * kSlotBytes),
-                                                    static_cast<uint32_t>(kBlockBytes), 1024u);
+    // O_t[128, D] += P_t[128, 128 keys] V[128 keys, D] of block j: P from TMEM (row = lane, two keys per 32-bit column, 8 columns
+    // per MMA), V MN-major (D contiguous): 16 key rows per MMA = 2048 bytes down a block, blocks of 64 head-dim columns 16 KiB
+    // apart
+    auto values = [&](int t, int j) {
+      const int v_item = 2 * j + 1, slot = v_item % kSlots;
+      const uint32_t vl = v_lo + static_cast<uint32_t>(slot * (kSlotBytes >> 4));
+      if (first_use(t, j) && !wait_item(v_item)) return false;
+      constexpr int kParts = kOneS ? 1 : 2, kPerPart = kBKV / 16 / kParts;
 #pragma unroll
-      for (int k2 = 0; k2 < kBKV / 32; ++k2) {
-        const int kk = half * (kBKV / 32) + k2;
-        const uint64_t offb = static_cast<uint64_t>((kk * 16 * 128) >> 4);
-        ptx::umma_f16_ts(tmem + kOCol + t * D, tmem + kPCol + t * kPStride + kk * 8, dv + offb, p.idesc_pv, (accumulate || kk != 0) ? 1u : 0u);
+      for (int part = 0; part < kParts; ++part) {
+        if (!ptx::mbar_wait(part + 1 < kParts ? &bars->p_half[t] : &bars->p_full[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag)) return false;
+        ptx::tcgen05_fence_after();
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (int kk = part * kPerPart; kk < (part + 1) * kPerPart; ++kk)
+            ptx::umma_f16_ts(tmem + kOCol + t * D, tmem + kPCol + t * 64 + kk * 8, ptx::desc_of(vl + static_cast<uint32_t>((kk * 16 * 128) >> 4), v_hi),
+                             p.idesc_pv, (j > 0 || kk != 0) ? 1u : 0u);
+          if (part + 1 == kParts) {
+            ptx::tcgen05_commit(j + 1 < nblk[t] ? &bars->pv_done[t] : &bars->o_done[t]);
+            if (kOneS || t == 1) ptx::tcgen05_commit(&bars->kv_empty[slot]);
+          }
+        }
+        __syncwarp();
       }
+      return true;
     };
     bool ok = ptx::mbar_wait(&bars->q_full, 0u, p.timeout_ns, abort_flag);
-    if (ok) ok = wait_item(0);
-    if (ok) {
-      ptx::tcgen05_fence_after();
-      if (ptx::elect_one()) {
-        issue_qk(0, 0);
-        issue_qk(1, 0);
-        ptx::tcgen05_commit(&bars->kv_empty[0]);
+    if constexpr (kOneS) {
+      const int t = warp - kIssuerWarp, nt = nblk[t];
+      ok = ok && scores(t, 0);
+      for (int j = 0; ok && j < nt; ++j) {
+        if (j + 1 < nt) ok = scores(t, j + 1);      // ahead of the product with V, which waits for this block's softmax
+        ok = ok && values(t, j);
       }
-      __syncwarp();
-    }
-    for (int j = 0; kOwnP && ok && j < nmax; ++j) {
-      const int v_item = 2 * j + 1, k_next = 2 * j + 2;
-      if (j + 1 < nmax) {
-        ok = wait_item(k_next);
+      // the other tile walks on: its blocks are released for this one too, each when it has arrived
+      for (int item = 2 * nt; ok && item < 2 * nmax; ++item) {
+        ok = wait_item(item);
+        if (ok && lane == 0) ptx::mbar_arrive(&bars->kv_empty[item % kSlots]);
+      }
+    } else {
+      ok = ok && scores(0, 0) && scores(1, 0);
+      for (int j = 0; ok && j < nmax; ++j) {
 #pragma unroll
-        for (int t = 0; t < kTiles; ++t) {
-          if (!ok || j + 1 >= nblk[t]) continue;
-          ok = ptx::mbar_wait(&bars->s_free[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
-          if (!ok) break;
-          ptx::tcgen05_fence_after();
-          if (ptx::elect_one()) {
-            issue_qk(t, k_next);
-            if (t == 1) ptx::tcgen05_commit(&bars->kv_empty[k_next % kSlots]);
-          }
-          __syncwarp();
-        }
-      }
-      ok = ok && wait_item(v_item);
+        for (int t = 0; t < kTiles; ++t)
+          if (j + 1 < nblk[t]) ok = ok && scores(t, j + 1);
 #pragma unroll
-      for (int t = 0; t < kTiles; ++t) {
-        if (!ok || j >= nblk[t]) continue;
-        ok = ptx::mbar_wait(&bars->p_half[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
-        if (!ok) break;
-        ptx::tcgen05_fence_after();
-        if (ptx::elect_one()) issue_pv(t, v_item, 0, j > 0);
-        __syncwarp();
-        ok = ptx::mbar_wait(&bars->p_full[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
-        if (!ok) break;
-        ptx::tcgen05_fence_after();
-        if (ptx::elect_one()) {
-          issue_pv(t, v_item, 1, true);
-          if (t == 1) ptx::tcgen05_commit(&bars->kv_empty[v_item % kSlots]);
-          ptx::tcgen05_commit(j + 1 < nblk[t] ? &bars->pv_done[t] : &bars->o_done[t]);
-        }
-        __syncwarp();
-      }
-    }
-    for (int j = 0; !kOwnP && ok && j < nmax; ++j) {
-      const int v_item = 2 * j + 1, k_next = 2 * j + 2;
-      const bool next0 = j + 1 < nblk[0], next1 = j + 1 < nblk[1];
-      bool v_here = false;
-      if (j < nblk[0]) {
-        // half of P_0(j) is in TMEM and O_0 has been rescaled: its product starts while the softmax finishes the other half
-        ok = ptx::mbar_wait(&bars->p_half[0], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag) && wait_item(v_item);
-        if (!ok) break;
-        v_here = true;
-        ptx::tcgen05_fence_after();
-        if (ptx::elect_one()) issue_pv(0, v_item, 0, j > 0);
-        __syncwarp();
-        ok = ptx::mbar_wait(&bars->p_full[0], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
-        if (!ok) break;
-        ptx::tcgen05_fence_after();
-        if (ptx::elect_one()) {
-          issue_pv(0, v_item, 1, true);
-          if (!next0) ptx::tcgen05_commit(&bars->o_done[0]);
-        }
-        __syncwarp();
-        if (next0) {
-          ok = wait_item(k_next);
-          if (!ok) break;
-          ptx::tcgen05_fence_after();
-          if (ptx::elect_one()) issue_qk(0, k_next);      // the scores of block j + 1 land on P_0(j): in issue order
-          __syncwarp();
-        }
-      }
-      ok = ptx::mbar_wait(&bars->p_half[1], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag) && (v_here || wait_item(v_item));
-      if (!ok) break;
-      ptx::tcgen05_fence_after();
-      if (ptx::elect_one()) issue_pv(1, v_item, 0, j > 0);
-      __syncwarp();
-      ok = ptx::mbar_wait(&bars->p_full[1], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag);
-      if (!ok) break;
-      ptx::tcgen05_fence_after();
-      if (ptx::elect_one()) {
-        issue_pv(1, v_item, 1, true);
-        ptx::tcgen05_commit(&bars->kv_empty[v_item % kSlots]);
-        if (!next1) ptx::tcgen05_commit(&bars->o_done[1]);
-      }
-      __syncwarp();
-      if (next1) {
-        ok = wait_item(k_next);
-        if (!ok) break;
-        ptx::tcgen05_fence_after();
-        if (ptx::elect_one()) {
-          issue_qk(1, k_next);
-          ptx::tcgen05_commit(&bars->kv_empty[k_next % kSlots]);
-        }
-        __syncwarp();
+        for (int t = 0; t < kTiles; ++t)
+          if (j < nblk[t]) ok = ok && values(t, j);
       }
     }
     if (!ok && lane == 0) { fail(p, 2u, 0u, 0u); *abort_flag = 1; }
@@ -311,8 +270,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     const int qd = warp & 3;                         // TMEM lane quarter of this warp
     const int row = qd * 32 + lane;                  // query row inside the tile
     const int qi = q0 + t * kBQ + row;
-    const uint32_t t_s = tmem + (static_cast<uint32_t>(qd * 32) << 16) + t * 128;   // scores, and P on top of them
-    const uint32_t t_p = kOwnP ? tmem + (static_cast<uint32_t>(qd * 32) << 16) + kPCol + t * kPStride : t_s;
+    const uint32_t t_s = tmem + (static_cast<uint32_t>(qd * 32) << 16) + (kOneS ? 0 : t * 128);
+    const uint32_t t_p = tmem + (static_cast<uint32_t>(qd * 32) << 16) + kPCol + t * 64;
     const uint32_t t_o = tmem + (static_cast<uint32_t>(qd * 32) << 16) + kOCol + t * D;
     const int n_mine = nblk[t];
     const int vis = p.causal ? min(p.Sk, qi % p.pos + shift + 1) : p.Sk;    // keys [0, vis) are visible to this row
@@ -325,30 +284,28 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
       ptx::tcgen05_fence_after();
       const int key0 = j * kBKV;
       // masked: some row of the tile does not see all of the block
+      // P V of block j - 1 has read P, and O is whole
+      auto previous = [&] {
+        if (j > 0 && !ptx::mbar_wait(&bars->pv_done[t], static_cast<uint32_t>(j - 1) & 1u, p.timeout_ns, abort_flag)) ok = false;
+        ptx::tcgen05_fence_after();
+      };
       softmax_row_block<FMT>(t_s, t_p, key0 + kBKV > vis_tile, vis - key0, sc, st, [&] {
-        if constexpr (kOwnP) {
-          ptx::tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&bars->s_free[t]);
-        }
-      }, [&](bool move, float alpha) {
-        if constexpr (kOwnP) {
-          // P V of block j - 1 has read P, and O is whole
-          if (j > 0 && !ptx::mbar_wait(&bars->pv_done[t], static_cast<uint32_t>(j - 1) & 1u, p.timeout_ns, abort_flag)) ok = false;
-          ptx::tcgen05_fence_after();
-        }
-        // (else s_full(j) was committed behind P V of block j - 1, so O is whole)
-        if (move && j > 0) rescale_o<D>(t_o, alpha);
-      }, [&] {
-        ptx::tcgen05_wait_st();
         ptx::tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->p_half[t]);
+        if (lane == 0) ptx::mbar_arrive(&bars->s_free[t]);
+      }, [&](bool move, float alpha) {
+        if (!kOneS || move) previous();
+        if (move && j > 0) rescale_o<D>(t_o, alpha);
+      }, [&] { if constexpr (kOneS) previous(); }, [&] {
+        if constexpr (!kOneS) {
+          ptx::tcgen05_wait_st();
+          ptx::tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->p_half[t]);
+        }
       });
-      if constexpr (kOwnP) {
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
       ptx::tcgen05_wait_st();
       ptx::tcgen05_fence_before();
       __syncwarp();

@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_decode_kernel(const __grid_
         attn::softmax_row_block<FMT>(t_s, t_s, key0 + kBKV > vis_all, vis - key0, p.scale_log2, st, [] {}, [&](bool move, float alpha) {
           // s_full(i) was committed behind the second product of this parity's previous block, so O_t is whole
           if (move && i > mine0) attn::rescale_o<D>(t_o, alpha);
-        }, [] {});
+        }, [] {}, [] {});
         ptx::tcgen05_wait_st();
         ptx::tcgen05_fence_before();
         __syncwarp();
