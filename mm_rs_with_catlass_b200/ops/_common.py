@@ -1,6 +1,7 @@
 """Shared plumbing of the op layer: dtype tables, operand normalisation and native launches."""
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
 from dataclasses import dataclass
@@ -175,6 +176,20 @@ def tkey(t: Optional[torch.Tensor]):
 
 def on_device(device: torch.device) -> bool:
     return torch.cuda.current_device() == (device.index if device.index is not None else 0)
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def guard(device: torch.device):
+    """Makes ``device`` current for a block; nothing to do, and nothing paid for it, where it is already."""
+    return _NO_GUARD if on_device(device) else torch.cuda.device(device)
+
+
+def layout(t: Optional[torch.Tensor]):
+    """What an argument block says about a tensor besides its address. Blocks that are kept by the layouts of a call's tensors
+    serve any buffers so laid out: the caller writes the addresses into a copy and checks what depends on them."""
+    return None if t is None else (t.shape, t.stride(), t.dtype, t.device)
 
 
 def fill_tiling(args: N.OpArgs, tiling: Optional[TilingConfig]) -> None:

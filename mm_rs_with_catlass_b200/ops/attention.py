@@ -62,7 +62,7 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal
         scale = 1.0 / math.sqrt(d)
     if not scale > 0.0:
         raise ValueError("the softmax scale must be positive")
-    with torch.cuda.device(dev):
+    with cm.guard(dev):
         lib, stream = N.lib(), C.c_void_p(cm.stream_of(dev))
         tail = (b, hq, hk, sq, sk, d, cm.out_fmt(q.dtype), int(causal), float(scale), cm.local_status(dev).data_ptr(),
                 cm.default_timeout_ns(), stream)

@@ -35,6 +35,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import operator
+import os
 from typing import List, Optional, Sequence, Union
 
 import torch
@@ -159,7 +160,27 @@ def batched_matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, t
     return out
 
 
-def _grouped_launch(a, b, ends, trans_b, out, out_dtype, tiling, **epilogue):
+# Argument blocks of grouped products by the layouts of their tensors (cm.layout), without addresses: a call whose operands TMA
+# can address as they are copies the block and writes its own addresses into it.
+_group_blocks: dict = {}
+_MAX_BLOCKS = 1024
+
+
+def _grouped_launch(a, b, ends, trans_b, out, out_dtype, tiling, scale_m=None, scale_n=None):
+    key = (cm.layout(a), cm.layout(b), cm.layout(ends), trans_b, cm.layout(out), out_dtype, tiling, cm.layout(scale_m), cm.layout(scale_n),
+           os.environ.get("CATCOC_CTA_PAIR"))
+    kept = _group_blocks.get(key)
+    pa, pb = a.data_ptr(), b.data_ptr()
+    if kept is not None and (pa | pb) & 15 == 0:
+        args = N.OpArgs.from_buffer_copy(kept[0])
+        if out is None:
+            out = torch.empty(kept[1], dtype=kept[2], device=a.device)
+        args.a, args.b, args.out, args.group_ends = pa, pb, out.data_ptr(), ends.data_ptr()
+        if scale_m is not None:
+            args.scale_m, args.scale_n = scale_m.data_ptr(), scale_n.data_ptr()
+        with cm.guard(a.device):
+            cm.launch(args, a.device)
+        return out
     g = b.shape[0]
     m_total, k = a.shape
     kb, n = (b.shape[2], b.shape[1]) if trans_b else (b.shape[1], b.shape[2])
@@ -175,12 +196,18 @@ def _grouped_launch(a, b, ends, trans_b, out, out_dtype, tiling, **epilogue):
         group.update(b_n_total=g * n, b_k_total=k, g_b_row=n)
     else:
         group.update(b_n_total=n, b_k_total=g * k, g_b_k=k)
-    if epilogue.get("scale_n") is not None or epilogue.get("bias_f32") is not None or epilogue.get("bias") is not None:
+    if scale_n is not None:
         group["g_nvec"] = n
     b2 = b.contiguous().reshape(g * b.shape[1], b.shape[2])
     a2 = a if a.is_contiguous() else a.contiguous()
-    return matmul(a2, b2, trans_b=trans_b, out=out, out_dtype=out_dtype,
-                  tiling=tiling if tiling is not None else token_groups(m_total, g, n, k, a.dtype), _group=group, **epilogue)
+    built = []
+    res = matmul(a2, b2, trans_b=trans_b, out=out, out_dtype=out_dtype, scale_m=scale_m, scale_n=scale_n,
+                 tiling=tiling if tiling is not None else token_groups(m_total, g, n, k, a.dtype), _group=group, _args_out=built)
+    if built[0] is not None and a.is_contiguous() and b.is_contiguous():     # (else it points at copies)
+        if len(_group_blocks) >= _MAX_BLOCKS:
+            _group_blocks.clear()
+        _group_blocks[key] = (bytes(built[0]), tuple(res.shape), res.dtype)
+    return res
 
 
 def grouped_matmul(a: torch.Tensor, b: torch.Tensor, group_list: GroupList, *, trans_b: bool = False,
@@ -241,6 +268,9 @@ def grouped_matmul_slice_k(a: torch.Tensor, b: torch.Tensor, group_list: Sequenc
     return out
 
 
+_slice_k_blocks: dict = {}      # as _group_blocks
+
+
 def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: torch.Tensor,
                     tiling: Optional[TilingConfig]) -> bool:
     """All groups of a K-sliced product in one launch. Every group has tensor maps of its own that end
@@ -259,8 +289,7 @@ def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: 
     if a.stride(-1) != 1 or b.stride(-1) != 1 or (m * elt) % 16 != 0:
         return False
     ranges, begin = [], 0
-    for end in ends:
-        end = operator.index(end)
+    for end in map(operator.index, ends):
         if end > begin:
             if begin >= k_total:
                 return False
@@ -272,6 +301,15 @@ def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: 
         out.zero_()
         return True
     dev = a.device
+    key = (cm.layout(a), cm.layout(b), cm.layout(out), tiling, os.environ.get("CATCOC_CTA_PAIR"))
+    kept = _slice_k_blocks.get(key)
+    pa, pb = a.data_ptr(), b.data_ptr()
+    if kept is not None and (pa | pb) & 15 == 0:
+        args = N.OpArgs.from_buffer_copy(kept)
+        args.a, args.b, args.out, args.timeout_ns = pa, pb, out.data_ptr(), cm.default_timeout_ns()
+        with cm.guard(dev):
+            _slice_k_queue(args, ranges, out, dev)
+        return True
     if tiling is None:
         from ..tiling.chooser import slice_k_groups
         tiling = slice_k_groups(g, m, n, k_total, a.dtype)
@@ -293,11 +331,19 @@ def _slice_k_launch(a: torch.Tensor, b: torch.Tensor, ends: Sequence[int], out: 
         args.a_rows_total, args.a_k_total, args.b_n_total, args.b_k_total = m, k_total, n, k_total
         args.status = cm.local_status(dev).data_ptr()
         args.timeout_ns = cm.default_timeout_ns()
-        for i in range(g):
-            if ranges[2 * i + 1] <= ranges[2 * i]:
-                out[i].zero_()
-        cm.launch_slice_k(args, ranges, dev)
+        _slice_k_queue(args, ranges, out, dev)
+        if not oa.copied and not ob.copied:
+            if len(_slice_k_blocks) >= _MAX_BLOCKS:
+                _slice_k_blocks.clear()
+            _slice_k_blocks[key] = bytes(args)
     return True
+
+
+def _slice_k_queue(args, ranges, out: torch.Tensor, dev: torch.device) -> None:
+    for i in range(len(ranges) // 2):
+        if ranges[2 * i + 1] <= ranges[2 * i]:
+            out[i].zero_()
+    cm.launch_slice_k(args, ranges, dev)
 
 
 def group_gemm(problems: Sequence[dict], *, tiling: Optional[TilingConfig] = None) -> List[torch.Tensor]:

@@ -95,7 +95,7 @@ def mla_decode(q_nope: torch.Tensor, q_rope: torch.Tensor, ckv_cache: torch.Tens
         raise ValueError("out must be a contiguous tensor shaped like q_nope")
     max_pages = block_table.shape[1]
     lib = N.lib()
-    with torch.cuda.device(dev):
+    with cm.guard(dev):
         stream = C.c_void_p(cm.stream_of(dev))
         ptrs = (q_nope.data_ptr(), q_rope.data_ptr(), ckv_cache.data_ptr(), krope_cache.data_ptr(), block_table.data_ptr(),
                 kv_lens.data_ptr(), out.data_ptr())

@@ -162,6 +162,7 @@ def test_block_scaled_cut_units(monkeypatch, m, n, k):
     res = []
     for cut in (None, (2, -(-k // 256) * 128)) if k > 128 else (None,):
         monkeypatch.setattr(mx, "double_plan", lambda *a: (0.0, cut))
+        mx._blocks.clear()
         res.append(catcoc.mxf8_matmul(*ops, out_dtype=torch.float32))
         _check("block-scaled")
     # fp32 sums in another order, as above; the operands' magnitudes are about one
@@ -226,3 +227,35 @@ def test_token_group_choice():
                     assert not t.twice or (t.swap and t.bn == 256 and groups <= 128 and rows >= 128)
     assert chooser.token_groups(14080, 32, 4096, 2048, torch.bfloat16).swap
     assert not chooser.token_groups(1158, 64, 1408, 2048, torch.bfloat16).twice
+
+
+@pytest.mark.gpu
+def test_kept_argument_blocks_serve_other_buffers():
+    # the same layouts at other addresses, at an address TMA cannot take, and back; contents of their own each time
+    import mm_rs_with_catlass_b200 as catcoc
+    from mm_rs_with_catlass_b200.ops import blas, mx
+    g = torch.Generator(device="cuda").manual_seed(12)
+    ends = torch.tensor([100, 130, 300], dtype=torch.int32, device="cuda")
+    for kept in (blas._group_blocks, blas._slice_k_blocks, mx._blocks):
+        kept.clear()
+    for shift in (0, 0, 4, 0):
+        a = torch.randn(300 * 256 + shift, device="cuda", generator=g).bfloat16()[shift:].view(300, 256)
+        b = torch.randn(3, 256, 384, device="cuda", generator=g).bfloat16()
+        want = torch.cat([a[x:y].float() @ b[i].float() for i, (x, y) in enumerate(((0, 100), (100, 130), (130, 300)))])
+        got = catcoc.grouped_matmul(a, b, ends)
+        assert (got.float() - want).abs().max().item() < 2.0 ** -7 * want.abs().max().item()
+        x1, x2 = _operand(g, torch.int8, 300, 256), _operand(g, torch.int8, 3, 256, 384)
+        s1, s2 = torch.rand(300, device="cuda", generator=g), torch.rand(3, 384, device="cuda", generator=g)
+        deq = torch.cat([(x1[x:y].double() @ x2[i].double()) * s2[i] * s1[x:y, None] for i, (x, y) in enumerate(((0, 100), (100, 130), (130, 300)))])
+        got = catcoc.grouped_quant_matmul(x1, x2, s1, s2, ends)
+        assert (got.double() - deq).abs().max().item() < 2.0 ** -7 * deq.abs().max().item()
+        c = torch.randn(300, 128, device="cuda", generator=g).bfloat16()
+        want = torch.stack([a[x:y].float().t() @ c[x:y].float() for x, y in ((0, 10), (10, 10), (10, 300))])
+        got = catcoc.grouped_matmul_slice_k(a, c, [10, 10, 300])
+        assert (got.float() - want).abs().max().item() < 2.0 ** -7 * want.abs().max().item()
+        qs = [catcoc.quantize_mxf8(torch.randn(r, 256, device="cuda", generator=g)) for r in (200, 96)]
+        want = catcoc.ops.mx.dequantize_mxf8(*qs[0]) @ catcoc.ops.mx.dequantize_mxf8(*qs[1]).t()
+        got = catcoc.mxf8_matmul(qs[0][0], catcoc.pack_scales(qs[0][1]), qs[1][0], catcoc.pack_scales(qs[1][1]))
+        assert (got.float() - want).abs().max().item() < 2.0 ** -7 * want.abs().max().item()
+        _check("kept blocks")
+    assert blas._group_blocks and blas._slice_k_blocks and mx._blocks
