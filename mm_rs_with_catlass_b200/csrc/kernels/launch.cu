@@ -602,8 +602,9 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     p->out_vec_ok = (((a.ldc * oelt) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) ? 1 : 0;
   }
   // A local output leaves by TMA stores (32-row x 128-byte boxes, same swizzle as the staging
-  // buffer) when its base and pitch allow a tensor map; the plain-store path covers the rest.
-  if (!(fused && a.mode == CATCOC_MODE_AR) && p->out_vec_ok && out_tma_enabled()) {
+  // buffer) when its base and pitch allow a tensor map; the plain-store path covers the rest. A TMA store clips at whole
+  // 16-byte units: rows that end inside one (a view into a wider buffer) would overwrite what lies beside them.
+  if (!(fused && a.mode == CATCOC_MODE_AR) && p->out_vec_ok && o.N * oelt % 16 == 0 && out_tma_enabled()) {
     const int64_t rows_out = (fused && a.mode == CATCOC_MODE_RS) ? p->sched.seg_len : o.M;
     const CUtensorMapDataType odt = a.out_fmt == CATCOC_FMT_F16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                     : a.out_fmt == CATCOC_FMT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
