@@ -151,26 +151,17 @@ CATCOC_DEVICE void finish_tokens(const FusedParams& p, uint32_t (&v)[32], float 
   }
 }
 
-// Rows of a staged window (unswizzled, `row_bytes` each) to global memory: `rows` rows, `bytes` of each
-CATCOC_DEVICE void flush_rows(uint32_t stg, int lane, int row_bytes, uint8_t* base, int64_t pitch, int rows, int bytes, int elt, bool vec_ok) {
-  const int units = row_bytes / 16;
-  for (int r = lane / units; r < rows; r += 32 / units) {
-    const int b0 = (lane % units) * 16;
-    if (b0 >= bytes) continue;
-    const uint4 v = ptx::ld_shared_v4(stg + r * row_bytes + b0);
-    uint8_t* ptr = base + r * pitch + b0;
-    if (vec_ok && b0 + 16 <= bytes) {
-      ptx::st_global_v4(ptr, v);
-    } else {
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      const int n = min(16, bytes - b0) / elt;
-      if (elt == 2) {
-        for (int e = 0; e < n; ++e) *reinterpret_cast<uint16_t*>(ptr + e * 2) = static_cast<uint16_t>(w[e >> 1] >> ((e & 1) * 16));
-      } else {
-        for (int e = 0; e < n; ++e) *reinterpret_cast<uint32_t*>(ptr + e * 4) = w[e];
-      }
-    }
+// Rows of a staged window (unswizzled, `row_bytes` each: 64 or 128) to global memory: `rows` rows, `n` values of each. A word a
+// lane where the output's pitch or the row's end is no multiple of 16 bytes, as in flush_staged.
+CATCOC_DEVICE void flush_rows(uint32_t stg, int lane, int row_bytes, uint8_t* base, int64_t pitch, int rows, int n, int elt, bool vec_ok) {
+  if (vec_ok && n * elt % 16 == 0) {
+    const int units = row_bytes / 16, b0 = (lane % units) * 16;
+    for (int r = lane / units; r < rows; r += 32 / units)
+      if (b0 < n * elt) ptx::st_global_v4(base + r * pitch + b0, ptx::ld_shared_v4(stg + r * row_bytes + b0));
+    return;
   }
+  const int width = row_bytes / 4;
+  store_rows_by_word(lane, width, base, pitch, rows, n, elt, [&](int r) { return ptx::ld_shared_u32(stg + r * row_bytes + (lane & (width - 1)) * 4); });
 }
 
 template <int KIND, bool FULL, bool SWAP, class Params>
@@ -695,8 +686,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
             prev_tma = true;
           } else {
             __syncwarp();
-            flush_rows(stg, lane, row_bytes, base + static_cast<int64_t>(c0) * pitch, pitch, tokens, rows_valid * st_elt, st_elt,
-                       p.out_vec_ok != 0);
+            flush_rows(stg, lane, row_bytes, base + static_cast<int64_t>(c0) * pitch, pitch, tokens, rows_valid, st_elt, p.out_vec_ok != 0);
           }
           __syncwarp();
         }

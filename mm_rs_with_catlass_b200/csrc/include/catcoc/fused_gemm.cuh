@@ -240,12 +240,57 @@ CATCOC_DEVICE void stage_write(uint32_t stg, int lane, int unit, uint4 v) {
   ptx::st_shared_v4(stg + lane * 128 + ((unit ^ (lane & 7)) << 4), v);
 }
 
-// Writes the staged 32 x 128 B block out. Lanes cooperate so that 8 lanes cover one 128-byte
-// row segment. `cols_valid` counts elements of `elt` bytes inside the matrix within this
+// Staged rows of `n` values each to rows that begin at any address of the value's alignment, a word a lane: `width` lanes hold
+// a row, `word(r)` is the lane's word of row r (callable for 8 rows from any multiple of 8 on). Where a row of 16-bit values
+// begins inside a word, the words written are the staged ones moved by half a word, and the row's first and last value leave by
+// themselves. Eight rows are read before the first is written: one at a time, the reads' latencies add up.
+template <class Word>
+CATCOC_DEVICE void store_rows_by_word(int lane, int width, uint8_t* dst, int64_t pitch, int rows, int n, int elt, Word word) {
+  const int sub = lane & (width - 1), mine = lane / width, step = 32 / width;
+  dst += mine * pitch + sub * 4;
+  const bool whole = elt == 4 ? sub < n : 2 * sub + 1 < n, low = elt == 2 && 2 * sub + 1 == n;   // rows that begin at a word
+  const bool moved = sub > 0 && 2 * sub < n, first = sub == 0, last = 2 * sub + 2 == n;          // rows that begin inside one
+  if (((reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>(pitch)) & 3) == 0) {
+    for (int r0 = 0; r0 < rows; r0 += 8 * step) {
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = word(r0 + i * step + mine);
+#pragma unroll
+      for (int i = 0; i < 8; ++i, dst += step * pitch) {
+        const bool in = r0 + i * step + mine < rows;
+        if (in && whole) *reinterpret_cast<uint32_t*>(dst) = w[i];
+        if (in && low) *reinterpret_cast<uint16_t*>(dst) = static_cast<uint16_t>(w[i]);
+      }
+    }
+    return;
+  }
+  for (int r0 = 0; r0 < rows; r0 += 8 * step) {
+    uint32_t w[8], prev[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = word(r0 + i * step + mine);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) prev[i] = __shfl_up_sync(0xffffffffu, w[i], 1, width);
+#pragma unroll
+    for (int i = 0; i < 8; ++i, dst += step * pitch) {
+      const bool in = r0 + i * step + mine < rows;
+      const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(dst)) & 2u;
+      if (in && (off ? moved : whole)) *reinterpret_cast<uint32_t*>(dst - off) = off ? __funnelshift_l(prev[i], w[i], 16) : w[i];
+      if (in && (off ? first : low)) *reinterpret_cast<uint16_t*>(dst) = static_cast<uint16_t>(w[i]);
+      if (in && off && last) *reinterpret_cast<uint16_t*>(dst + 2) = static_cast<uint16_t>(w[i] >> 16);
+    }
+  }
+}
+
+// Writes the staged 32 x 128 B block out. `cols_valid` counts elements of `elt` bytes inside the matrix within this
 // 128-byte window; `rows_valid` in [0, 32]. Destinations:
 //   mc != nullptr          : one multimem.st per unit reaches every rank (aligned tiles only)
 //   peer_bases != nullptr  : the same block goes to peer_bases[rank], [rank+1], ... (+ off)
 //   otherwise              : `base` only
+// Aligned windows of whole units: 8 lanes cover a row's 128 bytes, 16 bytes each. Others (a pitch that is no multiple of 16
+// bytes, the last columns): a row at a time, a word a lane, so that a store instruction still covers whole sectors. Storing
+// each value by itself, four rows and eight distant pieces of a row to an instruction, held the kernel up. bf16, K = 3712,
+// 4096 rows: 5706 columns 174 -> 116 us, 5705 (every other row begins inside a word) 172 -> 120 us, 5704 by TMA 113 us; 1085
+// rows (swapped double tiles) 69 -> 41, 70 -> 46, 40 us; 9676 x 194 x 192, one tile a CTA: 22.6 -> 11.9 us, 192 columns 9.0 us.
 CATCOC_DEVICE void flush_staged(uint32_t stg, int lane, uint8_t* base, int64_t pitch,
                                 int rows_valid, int cols_valid, int elt, bool vec_ok,
                                 uint8_t* mc, uint8_t* const* peer_bases, int64_t off, int rank,
@@ -254,34 +299,26 @@ CATCOC_DEVICE void flush_staged(uint32_t stg, int lane, uint8_t* base, int64_t p
   const int per_unit = 16 / elt;
   const int c0 = unit * per_unit;
   const int ndst = (peer_bases != nullptr) ? W : 1;
+  if (mc == nullptr && (!vec_ok || cols_valid % per_unit != 0)) {
+    for (int d = 0; d < ndst; ++d) {
+      uint8_t* dst = (peer_bases != nullptr) ? peer_bases[peer_for_push_rs(rank, d, W)] + off : base;
+      store_rows_by_word(lane, 32, dst, pitch, rows_valid, cols_valid, elt, [&](int row) {
+        return ptx::ld_shared_u32(stg + row * 128 + (((lane >> 2) ^ (row & 7)) << 4) + (lane & 3) * 4);
+      });
+    }
+    return;
+  }
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
     const int row = it * 4 + (lane >> 3);
     const uint4 v = ptx::ld_shared_v4(stg + row * 128 + ((unit ^ (row & 7)) << 4));
     if (row < rows_valid && c0 < cols_valid) {
       const int64_t rel = row * pitch + unit * 16;
-      const bool full = vec_ok && (c0 + per_unit <= cols_valid);
       if (mc != nullptr) {
         ptx::multimem_st_v4(mc + rel, v);
       } else {
-        for (int d = 0; d < ndst; ++d) {
-          uint8_t* ptr = (peer_bases != nullptr)
-                             ? peer_bases[peer_for_push_rs(rank, d, W)] + off + rel
-                             : base + rel;
-          if (full) {
-            ptx::st_global_v4(ptr, v);
-          } else {
-            const int n = min(per_unit, cols_valid - c0);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-            if (elt == 2) {
-              for (int e = 0; e < n; ++e)
-                *reinterpret_cast<uint16_t*>(ptr + e * 2) =
-                    static_cast<uint16_t>(w[e >> 1] >> ((e & 1) * 16));
-            } else {
-              for (int e = 0; e < n; ++e) *reinterpret_cast<uint32_t*>(ptr + e * 4) = w[e];
-            }
-          }
-        }
+        for (int d = 0; d < ndst; ++d)
+          ptx::st_global_v4((peer_bases != nullptr) ? peer_bases[peer_for_push_rs(rank, d, W)] + off + rel : base + rel, v);
       }
     }
   }

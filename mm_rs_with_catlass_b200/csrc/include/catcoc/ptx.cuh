@@ -624,6 +624,11 @@ CATCOC_DEVICE void st_shared_v4(uint32_t saddr, uint4 v) {
                : "memory");
 }
 CATCOC_DEVICE void st_shared_u32(uint32_t saddr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(saddr), "r"(v) : "memory"); }
+CATCOC_DEVICE uint32_t ld_shared_u32(uint32_t saddr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
+  return v;
+}
 CATCOC_DEVICE uint4 ld_shared_v4(uint32_t saddr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"

@@ -1,4 +1,4 @@
-"""Views into a wider buffer: the same bits as in an aligned buffer, nothing written beside them."""
+"""Outputs whose rows begin at any element: the same bits as in an aligned buffer, nothing written beside them."""
 import pytest
 import torch
 
@@ -23,7 +23,7 @@ def test_rows_at_any_element(tiling, kind):
     t = TilingConfig(swizzle=2, **TILINGS[tiling])
     for m, n in ((1, 1), (7, 2), (33, 63), (255, 64), (64, 65), (301, 97), (300, 127), (257, 128), (31, 129), (129, 250), (301, 323)):
         want = catcoc.matmul(a[:m], b[:n], trans_b=True, tiling=t, out=torch.empty(m, 336, device="cuda", dtype=dt)[:, :n])
-        for pitch, first in ((336, 0), (336, 4)):
+        for pitch, first in ((336, 0), (336, 1), (335, 0), (335, 3), (334, 0), (334, 1), (332, 2), (336, 4)):
             first = min(first, pitch - n)
             whole = torch.full((m, pitch), 77, device="cuda", dtype=dt)
             catcoc.matmul(a[:m], b[:n], trans_b=True, tiling=t, out=whole[:, first:first + n])
