@@ -5,6 +5,7 @@
 // Counterparts in the reference's GEMM template library: the ReduceAdd stage of
 // 3rdparty/catlass/include/catlass/gemm/kernel/splitk_matmul.hpp:30-160 and the vector-core GEMV
 // 3rdparty/catlass/include/catlass/gemv/kernel/kernel_gemv_aiv.hpp (z = alpha * A x + beta * y).
+#include <algorithm>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -55,55 +56,82 @@ __device__ __forceinline__ int unpack_word(const uint4& w, int fmt, float* f) {
 
 // 2-D copy with independent pitches and zero fill of the padding columns: makes a TMA-legal (16-byte pitch, 16-byte
 // base) copy of a matrix that is not. Bound by HBM (bytes read + written). A destination chunk of 16 bytes straddles
-// two ALIGNED 16-byte words of the source whatever the row's alignment is; both are fetched as such (the second one is
-// the next thread's first: an L1 hit) and shifted into place, so a row of any byte alignment moves in 16-byte
-// accesses. Only words that hold at least one byte of the row are touched. Measured: 8192 x 28671 fp16 in 219 us
-// (4.29 TB/s), 28672 x 8191 in 219 us.
-constexpr int kPadChunks = 4;   // chunks per thread: eight independent loads in flight
+// two ALIGNED 16-byte words of the source whatever the row's alignment is; both are fetched as such and shifted into place, so a
+// row of any byte alignment moves in 16-byte accesses. Only words that hold at least one byte of the row are touched.
+//   By stretches: a warp takes 128 chunks of one row, so that the shift is the same for all its lanes, each lane reads one word of
+// every chunk and takes the next one from its neighbour.
+//   Flat (`kFlat`): a thread takes any four chunks of the list and reads both words of each (the second one is the next thread's
+// first: an L1 hit).
+// Stretches need fewer instructions a byte as long as they are filled; flat, no lane idles at a row's end. 100 MB (8 MB) of rows
+// of 34, 1000, 1800, 2400, 5000, 8000, 12296 bytes, us: stretches 1674, 60, 35.2, 48.4, 36.7, 32.0, 34.4 (136, 6.7, 4.7, 6.1,
+// 5.5, 4.6, 4.7), flat 58, 39, 37.8, 36.2, 37.0, 36.2, 36.6 (6.7, 5.5, 5.3, 5.1, 5.2, 5.1, 5.2), so stretches from five sixths
+// full on. One unit of work a thread: flat with at most 32 blocks an SM, each on several units, 62, 44.5, 42.9, 41.3, 42.3, 41.3,
+// 42.0. 8192 x 28671 fp16 179 -> 138 us (6.8 TB/s), 5210 x 7015 32.3 -> 24.1, 3710 x 5705 20.0 -> 15.3, 1024 x 6148 7.6 -> 6.5.
+constexpr int kPadChunks = 4;   // chunks per lane, all read before the first is written
 struct PadJob { uint8_t* dst; int64_t dst_pitch; const uint8_t* src; int64_t src_pitch, rows, row_bytes; };
 struct PadJobs { PadJob job[2]; };   // one per grid row: both operands of a product in one launch
 
+// 32-lane units of work of a job: stretches of a row, or pieces of the flat list
+__host__ __device__ constexpr int64_t pad_units(int64_t rows, int64_t cpr, bool flat) {
+  return flat ? (rows * cpr + 32 * kPadChunks - 1) / (32 * kPadChunks) : rows * ((cpr + 32 * kPadChunks - 1) / (32 * kPadChunks));
+}
+
 // kJobs = 1: the one matrix's sizes stay operands in the constant bank; picked by the block's row they cost 1 to 2 % of a
 // large copy (8192 x 28671 x 1023 with both operands padded: 1067 -> 1078 us).
-template <int kJobs>
-__global__ void pad2d_kernel(const __grid_constant__ PadJobs jobs) {
+template <int kJobs, bool kFlat>
+__global__ void __launch_bounds__(256) pad2d_kernel(const __grid_constant__ PadJobs jobs) {
   const PadJob& pj = jobs.job[kJobs == 1 ? 0 : blockIdx.y];
   uint8_t* const dst = pj.dst;
   const uint8_t* const src = pj.src;
   const int64_t dst_pitch = pj.dst_pitch, src_pitch = pj.src_pitch, rows = pj.rows, row_bytes = pj.row_bytes;
-  const uint32_t cpr = static_cast<uint32_t>(dst_pitch >> 4);
+  const int64_t cpr = dst_pitch >> 4, chunks = rows * cpr, total = pad_units(rows, cpr, kFlat);
+  const uint32_t segs = static_cast<uint32_t>((cpr + 32 * kPadChunks - 1) / (32 * kPadChunks));
+  const int lane = static_cast<int>(threadIdx.x & 31);
   ptx::grid_dependency_wait();
-  const int64_t total = rows * cpr;
-  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x * kPadChunks;
-  for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x * kPadChunks + threadIdx.x; base < total; base += step) {
-    uint4 w[kPadChunks][2];
+  const int64_t step = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
+  // (32-bit division when the index allows it: the 64-bit one is a long instruction sequence)
+  auto quotient = [](int64_t x, int64_t limit, uint32_t d) { return (limit >> 32) == 0 ? static_cast<int64_t>(static_cast<uint32_t>(x) / d) : x / d; };
+  for (int64_t u = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5); u < total; u += step) {
+    uint4 w[kPadChunks + 1], next[kFlat ? kPadChunks : 1];
     uint32_t sh[kPadChunks];
-    int valid[kPadChunks];
-    uint8_t* out[kPadChunks];
+    int64_t row[kPadChunks + 1], off[kPadChunks + 1];   // chunk j: bytes from `off` on of `row` (off < 0: none)
+    const int64_t r0 = kFlat ? 0 : quotient(u, total, segs);
 #pragma unroll
-    for (int j = 0; j < kPadChunks; ++j) {
-      const int64_t i = base + static_cast<int64_t>(j) * blockDim.x;
-      w[j][0] = w[j][1] = make_uint4(0u, 0u, 0u, 0u);
-      out[j] = nullptr;
-      sh[j] = 0; valid[j] = 0;
-      if (i < total) {
-        // (32-bit division when the index allows it: the 64-bit one is a long instruction sequence)
-        const int64_t r = (total >> 32) == 0 ? static_cast<int64_t>(static_cast<uint32_t>(i) / cpr) : i / cpr;
-        const int64_t o = (i - r * cpr) << 4;
-        const uint8_t* s = src + r * src_pitch + o;
-        const int64_t left = row_bytes - o;
-        valid[j] = left >= 16 ? 16 : static_cast<int>(left);
-        sh[j] = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(s) & 15u);
-        out[j] = dst + r * dst_pitch + o;
-        const uint8_t* a = s - sh[j];
-        if (valid[j] > 0) w[j][0] = *reinterpret_cast<const uint4*>(a);
-        if (valid[j] > 0 && static_cast<int>(sh[j]) + valid[j] > 16) w[j][1] = *reinterpret_cast<const uint4*>(a + 16);
+    for (int j = 0; j < kPadChunks + (kFlat ? 0 : 1); ++j) {
+      int64_t c;
+      if (kFlat) {
+        const int64_t i = u * (32 * kPadChunks) + j * 32 + lane;
+        row[j] = i < chunks ? quotient(i, chunks, static_cast<uint32_t>(cpr)) : 0;
+        c = i < chunks ? i - row[j] * cpr : -1;
+      } else {
+        row[j] = r0;
+        c = (u - r0 * segs) * (32 * kPadChunks) + j * 32 + lane;
+      }
+      off[j] = c * 16;
+      const uint8_t* s = src + row[j] * src_pitch;
+      const uint32_t shift = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(s) & 15u);
+      const int64_t end = row_bytes + shift;
+      const uint4* a = reinterpret_cast<const uint4*>(s - shift + off[j]);
+      if (j < kPadChunks) sh[j] = shift;
+      w[j] = make_uint4(0u, 0u, 0u, 0u);
+      // (the word behind the stretch: read by lane 0 for lane 31)
+      if (c >= 0 && off[j] < end && (j < kPadChunks || lane == 0)) w[j] = a[0];
+      if (kFlat) {
+        next[kFlat ? j : 0] = make_uint4(0u, 0u, 0u, 0u);
+        if (c >= 0 && off[j] + 16 < end) next[kFlat ? j : 0] = a[1];
       }
     }
 #pragma unroll
     for (int j = 0; j < kPadChunks; ++j) {
-      if (out[j] == nullptr) continue;
-      uint32_t x[8] = {w[j][0].x, w[j][0].y, w[j][0].z, w[j][0].w, w[j][1].x, w[j][1].y, w[j][1].z, w[j][1].w};
+      uint4 n;
+      if (kFlat) {
+        n = next[kFlat ? j : 0];
+      } else {
+        const uint4 give = lane == 0 ? w[j + 1] : w[j];   // lane 31's next word is lane 0's of the next chunk
+        n = make_uint4(__shfl_sync(0xffffffffu, give.x, lane + 1), __shfl_sync(0xffffffffu, give.y, lane + 1),
+                       __shfl_sync(0xffffffffu, give.z, lane + 1), __shfl_sync(0xffffffffu, give.w, lane + 1));
+      }
+      uint32_t x[8] = {w[j].x, w[j].y, w[j].z, w[j].w, n.x, n.y, n.z, n.w};
       if (sh[j] & 8u) {
 #pragma unroll
         for (int k = 0; k < 6; ++k) x[k] = x[k + 2];
@@ -112,15 +140,18 @@ __global__ void pad2d_kernel(const __grid_constant__ PadJobs jobs) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) x[k] = x[k + 1];
       }
-      const uint32_t bits = (sh[j] & 3u) * 8u;
+      const int64_t left = row_bytes - off[j];
       uint32_t y[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        y[k] = __funnelshift_r(x[k], x[k + 1], bits);
-        const int keep = valid[j] - 4 * k;   // bytes of this word that belong to the row
-        if (keep < 4) y[k] = keep <= 0 ? 0u : (y[k] & ((1u << (8 * keep)) - 1u));
+      for (int k = 0; k < 4; ++k) y[k] = __funnelshift_r(x[k], x[k + 1], (sh[j] & 3u) * 8u);
+      if (left < 16) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int64_t keep = left - 4 * k;   // bytes of this word that belong to the row
+          if (keep < 4) y[k] = keep <= 0 ? 0u : (y[k] & ((1u << (8 * keep)) - 1u));
+        }
       }
-      *reinterpret_cast<uint4*>(out[j]) = make_uint4(y[0], y[1], y[2], y[3]);
+      if (off[j] >= 0 && off[j] < dst_pitch) *reinterpret_cast<uint4*>(dst + row[j] * dst_pitch + off[j]) = make_uint4(y[0], y[1], y[2], y[3]);
     }
   }
 }
@@ -281,7 +312,8 @@ bool float_fmt(int fmt) { return fmt == CATCOC_FMT_F16 || fmt == CATCOC_FMT_BF16
 }  // namespace
 
 static int pad_launch(const PadJobs& jobs, int count, void* stream) {
-  int64_t blocks = 1;
+  int64_t most = 0;     // the larger job decides
+  bool flat = true;
   for (int i = 0; i < count; ++i) {
     const PadJob& j = jobs.job[i];
     if (j.dst == nullptr || j.src == nullptr || j.row_bytes <= 0 || j.dst_pitch < j.row_bytes) {
@@ -292,11 +324,18 @@ static int pad_launch(const PadJobs& jobs, int count, void* stream) {
       host::set_error("pad2d: the destination needs a 16-byte aligned base and pitch");
       return CATCOC_E_ALIGNMENT;
     }
-    const int64_t need = (j.rows * (j.dst_pitch >> 4) + 256 * kPadChunks - 1) / (256 * kPadChunks);
-    if (need > blocks) blocks = need;
+    const int64_t cpr = j.dst_pitch >> 4;
+    if (j.rows * cpr > most) {
+      most = j.rows * cpr;
+      flat = 6 * cpr < 5 * (32 * kPadChunks) * pad_units(1, cpr, false);
+    }
   }
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  CATCOC_CUDA_OK(host::launch_overlapped(count == 1 ? pad2d_kernel<1> : pad2d_kernel<2>, dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(count)), dim3(256), 0,
+  int64_t blocks = 1;
+  for (int i = 0; i < count; ++i)
+    blocks = std::max(blocks, (pad_units(jobs.job[i].rows, jobs.job[i].dst_pitch >> 4, flat) + 7) / 8);
+  blocks = std::min<int64_t>(blocks, 1 << 20);
+  auto* kernel = flat ? (count == 1 ? pad2d_kernel<1, true> : pad2d_kernel<2, true>) : (count == 1 ? pad2d_kernel<1, false> : pad2d_kernel<2, false>);
+  CATCOC_CUDA_OK(host::launch_overlapped(kernel, dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(count)), dim3(256), 0,
                                          static_cast<cudaStream_t>(stream), jobs));
   return CATCOC_OK;
 }
