@@ -348,7 +348,7 @@ int catcoc_mla_decode(const void* q_nope, const void* q_rope, const void* ckv, c
                       int max_pages, int fmt, int causal, float scale, int splits, uint32_t* status,
                       uint64_t timeout_ns, void* stream);
 
-/* The same step for few query rows per sequence (csrc/kernels/mla_rows.cu): the pages of all sequences are dealt out over
+/* The same step with the query rows on the N side (csrc/kernels/mla_rows.cu): the pages of all sequences are dealt out over
  * the SMs by the lengths on the device. catcoc_mla_rows_workspace_bytes: scratch bytes, or -1 when it does not take the call. */
 int64_t catcoc_mla_rows_workspace_bytes(int B, int q_len, int H, int max_pages);
 int catcoc_mla_rows(const void* q_nope, const void* q_rope, const void* ckv, const void* krope, const int* block_table,

@@ -4,8 +4,8 @@
 All query heads share one key / value stream: a 512-wide latent that is key and value at once,
 plus a 64-wide rotary part that only the scores see. ``q_nope`` has already been multiplied by
 the key up-projection (the "absorbed" form), so the kernel is attention with 576-wide keys and
-512-wide values over a cache of 128-key pages. With at most 128 query rows per sequence (new tokens x
-heads) the keys are the M side of both products: a CTA holds 16 or 32 rows with all output columns, and
+512-wide values over a cache of 128-key pages. With at most 1024 query rows per sequence (new tokens x
+heads) the keys are the M side of both products: a CTA holds 16, 32 or 64 rows with all output columns, and
 the pages of all sequences, by their lengths on the device, are dealt out over the SMs. More rows, or an
 explicit number of slices, take the general kernel: a CTA owns up to 128 rows, one half of the output
 columns and one slice of a sequence. In both the pieces of a sequence are merged by a second small kernel
@@ -101,7 +101,7 @@ def mla_decode(q_nope: torch.Tensor, q_rope: torch.Tensor, ckv_cache: torch.Tens
                 kv_lens.data_ptr(), out.data_ptr())
         need = int(lib.catcoc_mla_rows_workspace_bytes(batch, q_len, heads, max_pages)) if splits is None else -1
         if need >= 0:
-            # few query rows per sequence: the keys are the M side, the pages of all sequences are dealt out over the SMs
+            # the keys are the M side, the pages of all sequences are dealt out over the SMs
             ws = torch.empty(need, dtype=torch.uint8, device=dev)
             N.check(lib.catcoc_mla_rows(*ptrs, ws.data_ptr(), batch, q_len, heads, ckv_cache.shape[0], max_pages,
                                         cm.out_fmt(dt), int(causal), float(scale), cm.local_status(dev).data_ptr(),
