@@ -23,10 +23,7 @@ namespace dtile {
 
 constexpr int kThreads = 384;
 constexpr int kRingBytes = 192 * 1024;
-#ifndef CATCOC_DT_LEAD
-#define CATCOC_DT_LEAD 2
-#endif
-constexpr int kLead = CATCOC_DT_LEAD;
+constexpr int kLead = 2;
 constexpr int kSmemBytes = kRingBytes + 2 * kEpiWarps * kEpiWinBytes + 256 /*barriers*/ + 8 * kMaxTokenGroups + 1024 /*align slack*/;
 static_assert(sizeof(SmemTail) <= 256 && kSmemBytes <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t kMxBN = 192;                  // block-scaled: two accumulators of 192 columns, the scales behind them
