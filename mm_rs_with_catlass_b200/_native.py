@@ -175,6 +175,9 @@ def _declare(lib) -> None:
         "catcoc_gemv_workspace_floats": (i64, [i32, i32, i32]),
         "catcoc_gemv": (i32, [vp, i64, i32, i32, i32, i32, vp, vp, vp, C.c_float, C.c_float, vp, vp]),
         "catcoc_flash_attention": (i32, [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, vp, u64, vp]),
+        "catcoc_flash_attention_workspace_bytes": (i64, [i32, i32, i32, i32, i32, i32, i32]),
+        "catcoc_attention_route": (i64, [i32, i32, i32, i32, i32, i32, i32]),
+        "catcoc_flash_attention_cut": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, vp, u64, vp]),
         "catcoc_flash_decode_workspace_bytes": (i64, [i32, i32, i32, i32, i32, i32]),
         "catcoc_flash_decode": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, vp, u64, vp]),
         "catcoc_mla_workspace_bytes": (i64, [i32, i32, i32, i32]),

@@ -329,12 +329,21 @@ int catcoc_flash_attention(const void* q, const void* k, const void* v, void* ou
                            int Sk, int D, int fmt, int causal, float scale, uint32_t* status, uint64_t timeout_ns,
                            void* stream);
 
+/* The same with scratch for keys cut into slices (few query tiles over many keys). catcoc_flash_attention_workspace_bytes: its size, 0
+ * when a call is not cut; without scratch no call is. */
+int64_t catcoc_flash_attention_workspace_bytes(int B, int Hq, int Hk, int Sq, int Sk, int D, int causal);
+int catcoc_flash_attention_cut(const void* q, const void* k, const void* v, void* out, void* workspace, int B, int Hq, int Hk, int Sq,
+                               int Sk, int D, int fmt, int causal, float scale, uint32_t* status, uint64_t timeout_ns, void* stream);
 /* The same function for few query rows per key / value head (csrc/kernels/flash_decode.cu): the keys are cut over the SMs.
  * catcoc_flash_decode_workspace_bytes says whether the kernel takes a call (-1: no) and how much scratch it needs. */
 int64_t catcoc_flash_decode_workspace_bytes(int B, int Hq, int Hk, int Sq, int Sk, int D);
 int catcoc_flash_decode(const void* q, const void* k, const void* v, void* out, void* workspace, int B, int Hq, int Hk,
                         int Sq, int Sk, int D, int fmt, int causal, float scale, uint32_t* status, uint64_t timeout_ns,
                         void* stream);
+
+/* Which of the two takes a call, and its scratch: n >= 0: catcoc_flash_decode with n bytes, else catcoc_flash_attention_cut with
+ * -1 - n bytes. */
+int64_t catcoc_attention_route(int B, int Hq, int Hk, int Sq, int Sk, int D, int causal);
 
 /* ---- multi-head latent attention, decode step over a paged cache (csrc/kernels/mla_decode.cu) ----
  * q_nope [T, H, 512], q_rope [T, H, 64] (T = B * q_len new tokens, q_len 1..4), latent cache [num_pages, 128, 512],

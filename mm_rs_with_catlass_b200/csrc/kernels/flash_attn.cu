@@ -64,6 +64,9 @@ struct AttnParams {
   uint32_t idesc_qk, idesc_pv;
   uint32_t* status;
   uint64_t timeout_ns;
+  float* part_o;                  // keys cut into slices: [slice][B * Hq * Sq][D] unnormalised pieces
+  float* part_ml;                 // [slice][B * Hq * Sq][2]
+  int per;                        // key blocks of a slice
 };
 
 struct Bars {
@@ -79,8 +82,9 @@ CATCOC_DEVICE void fail(const AttnParams& p, uint32_t what, uint32_t a, uint32_t
   }
 }
 
-// D: head dimension; FMT: operand and output dtype (compile time: the softmax loop packs 64 pairs per row and block)
-template <int D, int FMT>
+// D: head dimension; FMT: operand and output dtype (compile time: the softmax loop packs 64 pairs per row and block);
+// CUT: a CTA takes the key blocks of slice blockIdx.y only and leaves a piece
+template <int D, int FMT, bool CUT>
 __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_constant__ AttnParams p) {
   constexpr int kDB = D / 64;                    // 128-byte blocks along the head dimension
   constexpr int kQBytes = kDB * kBlockBytes;     // one Q tile
@@ -125,6 +129,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     const int kv_end = p.causal ? min(p.Sk, tile_hi(t) + 1 + shift) : p.Sk;
     nblk[t] = (kv_end + kBKV - 1) / kBKV;
   }
+  // (a slice that some tile sees nothing of is a masked block there: a maximum of -inf, a sum of zero)
+  const int j0 = CUT ? static_cast<int>(blockIdx.y) * p.per : 0;
+  if constexpr (CUT) {
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) nblk[t] = max(1, min(p.per, nblk[t] - j0));
+  }
   nblk[1] = max(nblk[0], nblk[1]);
   const int nmax = nblk[1];
 
@@ -149,6 +159,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   ptx::tcgen05_fence_after();
   const uint32_t tmem = bars->tmem_base;
   ptx::grid_dependency_wait();
+  if constexpr (CUT) ptx::launch_dependents();                       // the combine kernel waits for this grid's results by itself
 
   if (warp >= kProducerWarp) ptx::reg_dec<kOtherRegs>();   // all four warps of the warpgroup at one place
   if (warp == kProducerWarp) {
@@ -172,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
         ptx::mbar_expect_tx(&bars->kv_full[slot], kSlotBytes);
         const CUtensorMap* tm = (item & 1) ? &p.tm_v : &p.tm_k;
         for (int d = 0; d < kDB; ++d)
-          ptx::tma_load_3d(skv + slot * kSlotBytes + d * kBlockBytes, tm, &bars->kv_full[slot], d * 64, (item >> 1) * kBKV, bhk);
+          ptx::tma_load_3d(skv + slot * kSlotBytes + d * kBlockBytes, tm, &bars->kv_full[slot], d * 64, (j0 + (item >> 1)) * kBKV, bhk);
       }
       __syncwarp();
     }
@@ -282,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
     for (int j = 0; j < n_mine; ++j) {
       if (!ptx::mbar_wait(&bars->s_full[t], static_cast<uint32_t>(j & 1), p.timeout_ns, abort_flag)) { ok = false; break; }
       ptx::tcgen05_fence_after();
-      const int key0 = j * kBKV;
+      const int key0 = (j0 + j) * kBKV;
       // masked: some row of the tile does not see all of the block
       // P V of block j - 1 has read P, and O is whole
       auto previous = [&] {
@@ -323,7 +334,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
         uint32_t v[32];
         ptx::tmem_ld_32x32b_x32(t_o + c * 32, v);
         ptx::tcgen05_wait_ld();
-        if (qi < p.Sq) {
+        if (CUT && qi < p.Sq) {
+          const int64_t prow = (static_cast<int64_t>(blockIdx.y) * p.B * p.Hq + bh) * p.Sq + qi;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) ptx::st_global_v4(p.part_o + prow * D + c * 32 + u * 4, make_uint4(v[u * 4], v[u * 4 + 1], v[u * 4 + 2], v[u * 4 + 3]));
+          if (c == 0) *reinterpret_cast<float2*>(p.part_ml + prow * 2) = make_float2(st.m, st.l);
+        } else if (qi < p.Sq) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             uint32_t w[4];
@@ -343,15 +359,116 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   if (warp == kIssuerWarp) ptx::tmem_dealloc(tmem, kTmemCols);
 }
 
+// The slices of a row, a warp each; every row has a slice that it sees something of unless it sees nothing at all
+template <int D, int FMT>
+__global__ void __launch_bounds__(128) flash_slices_kernel(const float* part_o, const float* part_ml, void* out, int64_t rows, int slices) {
+  constexpr int kPer = D / 32;                     // columns per lane
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  ptx::grid_dependency_wait();
+  if (r >= rows) return;
+  const float2 ml = lane < slices ? *reinterpret_cast<const float2*>(part_ml + (lane * rows + r) * 2) : make_float2(-INFINITY, 0.0f);
+  float mx = ml.x;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const float w = ml.x == -INFINITY ? 0.0f : ptx::ex2_approx(ml.x - mx);
+  float l = w * ml.y, acc[kPer];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) acc[e] = 0.0f;
+#pragma unroll 4
+  for (int c = 0; c < slices; ++c) {
+    const float wc = __shfl_sync(0xffffffffu, w, c);
+    const float* src = part_o + (c * rows + r) * D + lane * kPer;
+    float o[kPer];
+    if constexpr (kPer == 4) *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(src);
+    else *reinterpret_cast<float2*>(o) = *reinterpret_cast<const float2*>(src);
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) acc[e] += wc * o[e];
+  }
+  const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+  uint32_t* dst = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(out) + (r * D + lane * kPer) * 2);
+#pragma unroll
+  for (int e = 0; e < kPer / 2; ++e) dst[e] = pack16<FMT>(acc[2 * e] * inv, acc[2 * e + 1] * inv);
+}
+
 }  // namespace attn
 }  // namespace catcoc
 
 using namespace catcoc;
 using namespace catcoc::host;
 
+namespace {
+struct AttnPlan {
+  int Hq, Sq;          // as the kernel sees them (the query heads of a KV head may be packed)
+  int tiles;
+  int slices, per;     // keys cut into slices of `per` blocks
+};
+
+AttnPlan attn_plan(int B, int Hq, int Hk, int Sq, int Sk, int causal, bool cut) {
+  const int group = Hq / Hk, rows_cta = attn::kTiles * attn::kBQ, pos = Sq;
+  auto blocks = [&](int hi) { return static_cast<double>((causal ? std::min<int64_t>(Sk, static_cast<int64_t>(hi) + Sk - pos) : Sk) + 127) / 128; };
+  const double longest = blocks(pos);
+  AttnPlan d{Hq, Sq, (Sq + rows_cta - 1) / rows_cta, 1, 0}, packed = d;
+  bool pack = false;
+  // A call of few query positions: the query heads of a KV head are contiguous rows, so they can fill tiles together. It
+  // costs the keys that a head's early tiles would have skipped; in units of (CTA, 128-key block), a launch takes its
+  // total over the SMs or its longest CTA. 16 x 32 / 4 heads x 100 positions over 2000 keys: 154 -> 71 us,
+  // 16 x 32 / 8 x 64 over 1000 (D = 64): 78 -> 20 us.
+  if (group > 1 && static_cast<int64_t>(group) * Sq <= (1 << 24)) {
+    double plain = 0.0;
+    packed.Sq = group * Sq;
+    packed.Hq = Hk;
+    packed.tiles = (packed.Sq + rows_cta - 1) / rows_cta;
+    pack = true;
+    for (int i = 0; i < d.tiles; ++i) plain += blocks(std::min((i + 1) * rows_cta, pos));
+    const double heads = static_cast<double>(B) * Hk;
+    const double t_plain = std::max(longest, heads * group * plain / 148.0), t_packed = std::max(longest, heads * packed.tiles * longest / 148.0);
+    if (t_packed < 0.95 * t_plain) d = packed;
+  }
+  // Few tiles over many keys leave SMs idle: the keys are then cut into slices, which a second kernel merges. In us, a CTA takes 5
+  // and 1.55 a block of keys, the merge 4 and its bytes at 3 TB/s. In a loop, D = 128: 32 heads x 131 positions over 3404 keys 46 ->
+  // 26 us, 256 over 4096 54 -> 26, 8 heads x 512 over 16384 199 -> 40, 4 x 4096 causal 54 -> 39. Below 14 blocks a call waits
+  // for its host work, which the second launch makes longer (8 blocks 17.0 -> 20.0 us, 12 blocks 22.9 -> 24.0).
+  const int nblk = (Sk + 127) / 128;
+  if (!cut || longest < 14.0) return d;
+  double best = 0.85 * (5.0 + 1.55 * longest);
+  const AttnPlan forms[2] = {d, packed};
+  for (int f = 0; f < (pack ? 2 : 1); ++f) {
+    const AttnPlan& x = forms[f];
+    const int64_t ctas = static_cast<int64_t>(B) * x.Hq * x.tiles, rows = static_cast<int64_t>(B) * x.Hq * x.Sq;
+    for (int n = 2; n <= 16 && ctas * n <= 148 && 2 * n <= nblk; ++n) {
+      const int per = (nblk + n - 1) / n, slices = (nblk + per - 1) / per;
+      const double t = 9.0 + 1.55 * per + static_cast<double>(slices) * rows * 128 * 8 / 3e6;
+      if (t < best) { best = t; d = x; d.slices = slices; d.per = per; }
+    }
+  }
+  return d;
+}
+}  // namespace
+
+// Scratch of a call whose keys are cut into slices, else 0
+extern "C" int64_t catcoc_flash_attention_workspace_bytes(int B, int Hq, int Hk, int Sq, int Sk, int D, int causal) {
+  if (B <= 0 || Hq <= 0 || Hk <= 0 || Sq <= 0 || Sk <= 0 || Hq % Hk != 0 || (D != 64 && D != 128)) return 0;
+  const AttnPlan d = attn_plan(B, Hq, Hk, Sq, Sk, causal, true);
+  return d.slices > 1 ? static_cast<int64_t>(d.slices) * B * Hq * Sq * (D + 2) * static_cast<int64_t>(sizeof(float)) : 0;
+}
+
+extern "C" int64_t catcoc_attention_route(int B, int Hq, int Hk, int Sq, int Sk, int D, int causal) {
+  const int64_t decode = catcoc_flash_decode_workspace_bytes(B, Hq, Hk, Sq, Sk, D);
+  return decode >= 0 ? decode : -1 - catcoc_flash_attention_workspace_bytes(B, Hq, Hk, Sq, Sk, D, causal);
+}
+
 extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* v, void* out, int B, int Hq, int Hk,
                                       int Sq, int Sk, int D, int fmt, int causal, float scale, uint32_t* status,
                                       uint64_t timeout_ns, void* stream) {
+  return catcoc_flash_attention_cut(q, k, v, out, nullptr, B, Hq, Hk, Sq, Sk, D, fmt, causal, scale, status, timeout_ns, stream);
+}
+
+extern "C" int catcoc_flash_attention_cut(const void* q, const void* k, const void* v, void* out, void* workspace, int B, int Hq, int Hk,
+                                          int Sq, int Sk, int D, int fmt, int causal, float scale, uint32_t* status,
+                                          uint64_t timeout_ns, void* stream) {
   if (!q || !k || !v || !out || !status || B <= 0 || Hq <= 0 || Hk <= 0 || Sq <= 0 || Sk <= 0) {
     set_error("flash_attention: bad arguments");
     return CATCOC_E_BAD_ARG;
@@ -361,21 +478,10 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
   if (fmt != CATCOC_FMT_F16 && fmt != CATCOC_FMT_BF16) { set_error("flash_attention takes fp16 / bf16"); return CATCOC_E_UNSUPPORTED; }
   if (causal && Sk < Sq) { set_error("causal attention needs Sk >= Sq"); return CATCOC_E_BAD_ARG; }
   if (!(scale > 0.0f)) { set_error("flash_attention: the softmax scale must be positive (the row maximum is taken before scaling)"); return CATCOC_E_UNSUPPORTED; }
-  // A call of few query positions: the query heads of a KV head are contiguous rows, so they can fill tiles together. It
-  // costs the keys that a head's early tiles would have skipped; in units of (CTA, 128-key block), a launch takes its
-  // total over the SMs or its longest CTA. 16 x 32 / 4 heads x 100 positions over 2000 keys: 154 -> 71 us,
-  // 16 x 32 / 8 x 64 over 1000 (D = 64): 78 -> 20 us.
-  const int group = Hq / Hk, rows_cta = attn::kTiles * attn::kBQ;
-  const int pos = Sq;
-  if (group > 1 && static_cast<int64_t>(group) * Sq <= (1 << 24)) {
-    auto blocks = [&](int hi) { return static_cast<double>((causal ? std::min<int64_t>(Sk, static_cast<int64_t>(hi) + Sk - pos) : Sk) + 127) / 128; };
-    double plain = 0.0;
-    const int plain_tiles = (Sq + rows_cta - 1) / rows_cta, packed_tiles = (group * Sq + rows_cta - 1) / rows_cta;
-    for (int i = 0; i < plain_tiles; ++i) plain += blocks(std::min((i + 1) * rows_cta, pos));
-    const double longest = blocks(pos), heads = static_cast<double>(B) * Hk;
-    const double t_plain = std::max(longest, heads * group * plain / 148.0), t_packed = std::max(longest, heads * packed_tiles * longest / 148.0);
-    if (t_packed < 0.95 * t_plain) { Sq = group * Sq; Hq = Hk; }
-  }
+  const int rows_cta = attn::kTiles * attn::kBQ, pos = Sq;
+  const AttnPlan d = attn_plan(B, Hq, Hk, Sq, Sk, causal, workspace != nullptr);
+  Hq = d.Hq;
+  Sq = d.Sq;
   attn::AttnParams p;
   memset(&p, 0, sizeof(p));
   const CUtensorMapDataType dt = fmt == CATCOC_FMT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -384,10 +490,14 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
   if (rc == 0) rc = encode_bsd(&p.tm_v, v, dt, static_cast<int64_t>(B) * Hk, Sk, D);
   if (rc != 0) return rc;
   p.out = out;
+  const int64_t rows = static_cast<int64_t>(B) * Hq * Sq;
+  p.part_o = static_cast<float*>(workspace);
+  p.part_ml = workspace != nullptr ? p.part_o + d.slices * rows * D : nullptr;
+  p.per = d.per;
   p.B = B; p.Hq = Hq; p.Hk = Hk; p.Sq = Sq; p.Sk = Sk; p.D = D; p.pos = pos;
   const int64_t ctas = static_cast<int64_t>(B) * Hq * ((Sq + rows_cta - 1) / rows_cta);
   if (ctas > 0x7fffffff) { set_error("flash_attention: too many query tiles"); return CATCOC_E_TOO_LARGE; }
-  p.tiles = (Sq + rows_cta - 1) / rows_cta;
+  p.tiles = d.tiles;
   // Causal tiles differ in length, and with one head after the other the launch ended with the long tiles of its last
   // heads (in a loop, causal 2 x 32 x 8192: 1065 -> 1036 us, 1 x 32 x 4096: 183 -> 150). Heads side by side share the L2, so their keys and values must fit it.
   const int64_t kv_bytes = static_cast<int64_t>(Sk) * D * 4;
@@ -400,7 +510,7 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
   p.idesc_pv = ptx::make_instr_desc(1u, f, f, 0u, 1u, 128u, static_cast<uint32_t>(D));
   p.status = status;
   p.timeout_ns = timeout_ns ? timeout_ns : 10000000000ull;
-  const dim3 grid(static_cast<unsigned>(ctas));
+  const dim3 grid(static_cast<unsigned>(ctas), static_cast<unsigned>(d.slices));
   const int db = D / 64;
   const int slots = D == 128 ? 4 : 8;
   const size_t smem = static_cast<size_t>(attn::kTiles * db + slots * db) * attn::kBlockBytes + sizeof(attn::Bars) + 1024 + 64;
@@ -413,9 +523,23 @@ extern "C" int catcoc_flash_attention(const void* q, const void* k, const void* 
     if (a != cudaSuccess) { set_error("flash_attention launch failed: %s", cudaGetErrorString(a)); return -1000 - static_cast<int>(a); }
     return 0;
   };
+  auto merge = [&](auto kernel) -> int {
+    CATCOC_CUDA_OK(launch_overlapped(kernel, dim3(static_cast<unsigned>((rows + 3) / 4)), dim3(128), 0, static_cast<cudaStream_t>(stream), p.part_o, p.part_ml, out,
+                                     rows, d.slices));
+    return 0;
+  };
+  const bool bf = fmt == CATCOC_FMT_BF16;
   int lrc;
-  if (D == 128) lrc = fmt == CATCOC_FMT_BF16 ? launch(attn::flash_attn_kernel<128, FMT_BF16>) : launch(attn::flash_attn_kernel<128, FMT_F16>);
-  else lrc = fmt == CATCOC_FMT_BF16 ? launch(attn::flash_attn_kernel<64, FMT_BF16>) : launch(attn::flash_attn_kernel<64, FMT_F16>);
+  if (d.slices > 1) {
+    if (D == 128) lrc = bf ? launch(attn::flash_attn_kernel<128, FMT_BF16, true>) : launch(attn::flash_attn_kernel<128, FMT_F16, true>);
+    else lrc = bf ? launch(attn::flash_attn_kernel<64, FMT_BF16, true>) : launch(attn::flash_attn_kernel<64, FMT_F16, true>);
+    if (lrc == 0 && D == 128) lrc = bf ? merge(attn::flash_slices_kernel<128, FMT_BF16>) : merge(attn::flash_slices_kernel<128, FMT_F16>);
+    else if (lrc == 0) lrc = bf ? merge(attn::flash_slices_kernel<64, FMT_BF16>) : merge(attn::flash_slices_kernel<64, FMT_F16>);
+  } else if (D == 128) {
+    lrc = bf ? launch(attn::flash_attn_kernel<128, FMT_BF16, false>) : launch(attn::flash_attn_kernel<128, FMT_F16, false>);
+  } else {
+    lrc = bf ? launch(attn::flash_attn_kernel<64, FMT_BF16, false>) : launch(attn::flash_attn_kernel<64, FMT_F16, false>);
+  }
   if (lrc != 0) return lrc;
   e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("flash_attention launch failed: %s", cudaGetErrorString(e)); return -1000 - static_cast<int>(e); }

@@ -66,14 +66,12 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal
         lib, stream = N.lib(), C.c_void_p(cm.stream_of(dev))
         tail = (b, hq, hk, sq, sk, d, cm.out_fmt(q.dtype), int(causal), float(scale), cm.local_status(dev).data_ptr(),
                 cm.default_timeout_ns(), stream)
-        # few query rows per key / value head (decode steps): the keys are cut over the SMs instead of the queries
-        need = int(lib.catcoc_flash_decode_workspace_bytes(b, hq, hk, sq, sk, d))
-        if need >= 0:
-            ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
-            N.check(lib.catcoc_flash_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                            ws.data_ptr() if need else None, *tail))
-        else:
-            N.check(lib.catcoc_flash_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), *tail))
+        # few query rows per key / value head (decode steps): the keys are cut over the SMs instead of the queries; few tiles of
+        # query rows over many keys: the keys are cut into slices
+        need = int(lib.catcoc_attention_route(b, hq, hk, sq, sk, d, int(causal)))
+        kernel, need = (lib.catcoc_flash_decode, need) if need >= 0 else (lib.catcoc_flash_attention_cut, -1 - need)
+        ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+        N.check(kernel(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), ws.data_ptr() if need else None, *tail))
     return out
 
 
