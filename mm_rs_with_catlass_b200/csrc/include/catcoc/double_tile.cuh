@@ -112,10 +112,7 @@ CATCOC_DEVICE void finish_columns(const FusedParams& p, uint32_t (&v)[32], float
       }
     }
   }
-  if (p.act != ACT_NONE) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) f[j] = activate(f[j], p.act);
-  }
+  if (p.act != ACT_NONE) activate32(f, p.act);
 }
 
 // The same for swapped roles: 32 tokens of one feature. `feature` is the lane's own (nv: its place in the per-feature vectors).
@@ -142,10 +139,7 @@ CATCOC_DEVICE void finish_tokens(const FusedParams& p, uint32_t (&v)[32], float 
       f[j] = p.bias_f != nullptr ? x + b : x;
     }
   }
-  if (p.act != ACT_NONE) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) f[j] = activate(f[j], p.act);
-  }
+  if (p.act != ACT_NONE) activate32(f, p.act);
 }
 
 // Rows of a staged window (unswizzled, `row_bytes` each: 64 or 128) to global memory: `rows` rows, `n` values of each. A word a

@@ -212,6 +212,53 @@ CATCOC_DEVICE float activate(float x, int act) {
   return x;
 }
 
+// x / (1 + exp(-x)) without a branch: the approximate quotient is corrected by its own residual (one step of Newton's method), after
+// which it is as near as a rounded division. `plain` is set where that does not hold: no finite x, or a divisor beyond 2^125.
+CATCOC_DEVICE float silu_corrected(float x, bool& plain) {
+  const float d = 1.0f + __expf(-x), r = ptx::rcp_approx(d);
+  const float q = x * r;
+  plain = plain || !(d <= 0x1p125f) || !(fabsf(x) <= 0x1p125f);
+  return fmaf(fmaf(-q, d, x), r, q);
+}
+
+// The same for 32 values. What a tile's first pass costs is the fetch of its instructions: the choice is made once and not per value, and
+// the two long ones run as a loop over eight values whose registers move up. The division of silu, with its branch, took a value at a
+// time. bf16, K = 4096, relu / gelu / silu (none): 287 x 7168 54 / 56 / 94 -> 33 / 36 / 41 us (30), 92 x 14336 50 / 51 / 68 -> 35 / 37 /
+// 39 (33), 1024 x 7168 on double tiles 80 / 80 / 89 -> 54 / 58 / 60 (51). Errors of silu against fp64: the same to three digits.
+CATCOC_DEVICE void activate32(float (&f)[32], int act) {
+  if (act == ACT_RELU) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) f[j] = activate(f[j], ACT_RELU);
+    return;
+  }
+#pragma unroll 1
+  for (int pass = 0; pass < 4; ++pass) {
+    float done[8];
+    if (act == ACT_GELU_TANH) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) done[j] = activate(f[j], ACT_GELU_TANH);
+    } else {
+      bool plain = false;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) done[j] = silu_corrected(f[j], plain);
+      if (plain) {
+#pragma unroll 1
+        for (int pass8 = 0; pass8 < 8; ++pass8) {
+          const float x = activate(f[0], ACT_SILU), y = f[0];
+#pragma unroll
+          for (int j = 0; j < 7; ++j) { done[j] = done[j + 1]; f[j] = f[j + 1]; }
+          done[7] = x;
+          f[7] = y;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 24; ++j) f[j] = f[j + 8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[24 + j] = done[j];
+  }
+}
+
 // 16 bytes from an address that is only `vec`-byte aligned (vec = 8, 4 or 2), of which the first
 // `valid` (even, possibly <= 0) hold data; the rest reads as zero and is never touched in memory.
 CATCOC_DEVICE uint4 load16_pieces(const uint8_t* src, int vec, int valid) {
@@ -1236,10 +1283,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
                 }
               }
             }
-            if (kScale && p.act != ACT_NONE && !tail_unit) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) f[j] = activate(f[j], p.act);
-            }
+            if (kScale && p.act != ACT_NONE && !tail_unit) activate32(f, p.act);
             if (st_fmt == FMT_F32) {
 #pragma unroll
               for (int u = 0; u < 8; ++u)
