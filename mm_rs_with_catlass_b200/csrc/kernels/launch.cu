@@ -368,8 +368,8 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   // Block-scaled tiles leave TMEM room for the scales: 128 x 128 on one CTA, or, for a local product of more than one row
   // of tiles, double tiles of 2 x 192 columns (double_tile.cuh). A CTA's intake bounds the 128 x 128 tile (33 KiB per 256 cycles of
   // MMAs; 256 x 192 on a pair: 29.5 KiB per 384, the double tile: 42 KiB per 768): 4096 x 8192 x 7168 e4m3 with its quantisation
-  // 361, 256 and 222 us.
-  const bool mx_pair = mx && !fused && a.M > kBM && a.scale_m == nullptr && a.scale_n == nullptr && !a.affine && a.act == 0;
+  // 361, 256 and 222 us. Up to 128 rows: where the caller wants the units cut along K.
+  const bool mx_pair = mx && !fused && (a.M > kBM || a.tiling.cut_slices > 0) && a.scale_m == nullptr && a.scale_n == nullptr && !a.affine && a.act == 0;
   // 192-column tiles: pairs of local products (no workspace geometry knows them) with a B stored [N, K]; a [K, N] one comes
   // in 128-byte column blocks, of which a CTA's half would hold one and a half
   const bool bn192 = a.tiling.bn == 192 && !fused && a.trans_b && a.tiling.cta_pair == 2;

@@ -129,6 +129,17 @@ def _fill(args, a_q, sfa_packed, b_q, sfb_packed, m, n, k, kt):
 _blocks: dict = {}
 
 
+def _cut(m: int, n: int, k: int):
+    """``(slices, elements)`` along K for the units of 256 x 192 past the last full wave, or None. Up to 128 rows fill half of such
+    a unit and otherwise take tiles of 128 x 128, one per SM, at 820 cycles a K block: cut units where they are predicted to take
+    less (8192 columns, K = 28672: 16 rows 100 -> 77 us, 128 rows 104 -> 83; 1024 columns 93 -> 40; K = 7168, not cut: 28 against 31
+    for three slices). Below 75000 cycles the host work of the second launch would show (256 columns, K = 8192: 35 -> 40 us)."""
+    time, cut = double_plan(m, n, k, 1, 192)
+    if m <= 128 and max(time, 75000.0) > -(-n // 128 // 148) * -(-k // 128) * 820.0:
+        return None
+    return cut
+
+
 def mxf8_matmul(a_q: torch.Tensor, sfa_packed: torch.Tensor, b_q: torch.Tensor, sfb_packed: torch.Tensor, *,
                 out_dtype: torch.dtype = torch.bfloat16, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[M, N] = dequant(A) @ dequant(B).T`` with fp32 accumulation on one GPU."""
@@ -158,7 +169,7 @@ def mxf8_matmul(a_q: torch.Tensor, sfa_packed: torch.Tensor, b_q: torch.Tensor, 
         args.partial_fmt = args.out_fmt
         args.rank, args.W = 0, 1
         args.status = cm.local_status(dev).data_ptr()
-        cut = double_plan(m, n, k, 1, 192)[1] if m > 128 else None
+        cut = _cut(m, n, k)
         if cut is not None:
             cm.fill_tiling(args, TilingConfig(bn=192, cta_pair=2, twice=True, swizzle=4, cut_slices=cut[0], cut_k=cut[1]))
         block = bytes(args)
