@@ -348,14 +348,17 @@ def choose(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype,
     hit = tbl.lookup(op, m, n, k, world, dtype)
     if hit is not None:
         return hit
-    t = heuristic(op, m, n, k, world, dtype, b_k_major, tails)
-    if doubles and os.environ.get("CATCOC_CTA_PAIR") != "1":
-        return _with_doubles(m, n, k, dtype.itemsize, b_k_major, swap, t)
-    return t
+    forced = os.environ.get("CATCOC_CTA_PAIR")
+    if doubles and forced != "1":
+        return _with_doubles(op, m, n, k, world, dtype, b_k_major, tails, swap, forced)
+    return heuristic(op, m, n, k, world, dtype, b_k_major, tails)
 
 
 @functools.lru_cache(maxsize=4096)
-def _with_doubles(m: int, n: int, k: int, elt: int, b_k_major: bool, swap: bool, t: TilingConfig) -> TilingConfig:
+def _with_doubles(op: str, m: int, n: int, k: int, world: int, dtype: torch.dtype, b_k_major: bool, tails: bool, swap: bool,
+                  forced: Optional[str]) -> TilingConfig:
+    # (kept by the sizes: a call without a plan, such as one whose weight needs a padded copy, comes here each time)
+    t, elt = heuristic(op, m, n, k, world, dtype, b_k_major, tails), dtype.itemsize
     cut, cycles = _split_k(m, n, k, elt, t)
     if cut is None and t.cta_pair == 2:
         bn = t.effective_bn
