@@ -311,19 +311,39 @@ CATCOC_DEVICE void store_rows_by_word(int lane, int width, uint8_t* dst, int64_t
     }
     return;
   }
+  // the end values by one store: the lane of the first one, and that of the last, which is the upper half of its word
+  const bool upper = last && !first, ends = first || last;
+  const int up_bits = upper ? 16 : 0, up_bytes = upper ? 2 : 0;
   for (int r0 = 0; r0 < rows; r0 += 8 * step) {
     uint32_t w[8], prev[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) w[i] = word(r0 + i * step + mine);
 #pragma unroll
     for (int i = 0; i < 8; ++i) prev[i] = __shfl_up_sync(0xffffffffu, w[i], 1, width);
+    if (width == 32 && (pitch & 2) != 0) {
+      // every other row begins inside a word: pairs of rows, one of each kind, without a choice per row
+      const bool odd = (reinterpret_cast<uintptr_t>(dst) & 2) != 0;
+      uint8_t *da = dst + (odd ? pitch : 0), *dm = dst + (odd ? 0 : pitch);
+#pragma unroll
+      for (int i = 0; i < 8; i += 2, da += 2 * pitch, dm += 2 * pitch) {
+        const uint32_t wa = odd ? w[i + 1] : w[i], wm = odd ? w[i] : w[i + 1];
+        const bool ina = r0 + i + (odd ? 1 : 0) < rows, inm = r0 + i + (odd ? 0 : 1) < rows;
+        if (ina && whole) *reinterpret_cast<uint32_t*>(da) = wa;
+        if (inm && moved) *reinterpret_cast<uint32_t*>(dm - 2) = __funnelshift_l(odd ? prev[i] : prev[i + 1], wm, 16);
+        if (inm && ends) *reinterpret_cast<uint16_t*>(dm + up_bytes) = static_cast<uint16_t>(wm >> up_bits);
+        if ((n & 1) != 0 && ina && low) *reinterpret_cast<uint16_t*>(da) = static_cast<uint16_t>(wa);
+        if (n == 2 && inm && first) *reinterpret_cast<uint16_t*>(dm + 2) = static_cast<uint16_t>(wm >> 16);
+      }
+      dst += 8 * pitch;
+      continue;
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i, dst += step * pitch) {
       const bool in = r0 + i * step + mine < rows;
       const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(dst)) & 2u;
       if (in && (off ? moved : whole)) *reinterpret_cast<uint32_t*>(dst - off) = off ? __funnelshift_l(prev[i], w[i], 16) : w[i];
-      if (in && (off ? first : low)) *reinterpret_cast<uint16_t*>(dst) = static_cast<uint16_t>(w[i]);
-      if (in && off && last) *reinterpret_cast<uint16_t*>(dst + 2) = static_cast<uint16_t>(w[i] >> 16);
+      if (in && (off ? ends : low)) *reinterpret_cast<uint16_t*>(dst + up_bytes) = static_cast<uint16_t>(w[i] >> up_bits);
+      if (n == 2 && in && off && first) *reinterpret_cast<uint16_t*>(dst + 2) = static_cast<uint16_t>(w[i] >> 16);
     }
   }
 }
@@ -337,7 +357,8 @@ CATCOC_DEVICE void store_rows_by_word(int lane, int width, uint8_t* dst, int64_t
 // bytes, the last columns): a row at a time, a word a lane, so that a store instruction still covers whole sectors. Storing
 // each value by itself, four rows and eight distant pieces of a row to an instruction, held the kernel up. bf16, K = 3712,
 // 4096 rows: 5706 columns 174 -> 116 us, 5705 (every other row begins inside a word) 172 -> 120 us, 5704 by TMA 113 us; 1085
-// rows (swapped double tiles) 69 -> 41, 70 -> 46, 40 us; 9676 x 194 x 192, one tile a CTA: 22.6 -> 11.9 us, 192 columns 9.0 us.
+// rows (swapped double tiles) 69 -> 41, 70 -> 46, 40 us; 9676 x 194 x 192, one tile a CTA: 22.6 -> 11.9 us, 192 columns 9.0 us; K = 880, 6408 rows:
+// 14082 columns 428 -> 148 us, 14081 441 -> 210 (263 with a choice per row), 14080 131 us.
 CATCOC_DEVICE void flush_staged(uint32_t stg, int lane, uint8_t* base, int64_t pitch,
                                 int rows_valid, int cols_valid, int elt, bool vec_ok,
                                 uint8_t* mc, uint8_t* const* peer_bases, int64_t off, int rank,
