@@ -555,14 +555,14 @@ struct RowsPlan {
 // Rows of a CTA. 64 rows read every page half as often, but the page's slots are its only ones: the loads of the next page wait
 // for the second product, a pass takes 1.3 to 1.5 times as long, and a piece leaves twice the partial sums. In a loop, bf16,
 // chunks of 32 -> of 64 rows, by the passes of 32 rows over a page that an SM makes:
-//   an even number of chunks, four or more: 2 to 5 passes 22.5 -> 24.2 us, 27.7 -> 29.5; 6 passes 26.6 -> 27.9; 7 passes 27.7 -> 27.3, 28.0 -> 27.2; 14
+//   an even number of chunks, four or more: 2 to 5 passes 22.5 -> 24.2 us, 27.7 -> 29.5; 6 passes 26.6 -> 27.9; 7 passes 27.7 -> 27.3, 28.0 -> 27.2; 11 passes 46.6 -> 48.4; 14
 //     passes 44.6 -> 40.9, 43.7 -> 38.4; 55 passes 135 -> 104; 221 passes 507 -> 344
 //   two: 5 passes 31.2 -> 34.0, 14 passes 48.9 -> 50.1, 28 passes 80.2 -> 71.7; 110 passes 335 -> 262
 //   three (a quarter of the rows is padding): 10 passes 34.9 -> 38.6, 21 passes 64.5 -> 68.3, 41 passes 105 -> 101
 int chunk_rows(int rows_per_item, int64_t page_slots, int sms) {
   if (rows_per_item <= 32) return rows_per_item <= 16 ? 16 : 32;
   const int chunks = (rows_per_item + 31) / 32;
-  const int64_t line = chunks >= 4 && chunks % 2 == 0 ? 8 : 24;
+  const int64_t line = chunks >= 4 && chunks % 2 == 0 ? 12 : 24;
   return page_slots * chunks > line * sms ? 64 : 32;
 }
 RowsPlan rows_plan(int rows_per_item, int64_t page_slots) {
