@@ -55,7 +55,8 @@ typedef struct CatcocTiling {
                       32 from 64 to 256; 0 = one accumulator                                         */
   int swap;        /* ... with the output's columns along the tiles' rows: 256 columns x 2 bn rows of the output; 16-bit
                       and int8 operands, no C; over ragged groups the halves are made for each group (bn 256) */
-  int cut_slices;  /* ... and the units of 256 x bn past the last full wave cut along K into this many slices */
+  int cut_slices;  /* ... and the units of 256 x bn past the last full wave cut along K into this many slices;
+                      block-scaled fp8: with bn 192 only                                             */
   int cut_k;       /*     of cut_k elements (catcoc_double_launch); 0 = not cut                       */
 } CatcocTiling;
 

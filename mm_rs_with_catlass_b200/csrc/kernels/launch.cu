@@ -337,6 +337,10 @@ extern "C" int catcoc_sched_get_tile(int M, int N, int bm, int bn, int W, int se
 
 int max_active_pairs(int kind);
 
+// Units that are cut along K are as wide as the caller says, which sizes their planes and steers their fold; block-scaled ones
+// have one width.
+static bool cut_width_fits(const CatcocOpArgs& a, int kind) { return kind != KIND_MX || a.tiling.bn == static_cast<int>(dtile::kMxBN); }
+
 // Fills the parameter block; shared by the normal and the allocation-free entry points.
 int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out, int* grid_out, int* pair_out) {
   if (args == nullptr) { set_error("null args"); return CATCOC_E_BAD_ARG; }
@@ -381,6 +385,10 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
               static_cast<int64_t>(a.tiling.cut_k) * (a.tiling.cut_slices - 1) >= a.K || static_cast<int64_t>(a.tiling.cut_k) * a.tiling.cut_slices < a.K)) {
     set_error("double tiles: %d slices of %d elements do not cut K=%d into whole blocks of a local product", a.tiling.cut_slices, a.tiling.cut_k, a.K);
     return CATCOC_E_BAD_ARG;
+  }
+  if (cut && !cut_width_fits(a, rf.kind)) {
+    set_error("double tiles: the cut units of a block-scaled product are %d columns wide (got bn=%d)", static_cast<int>(dtile::kMxBN), a.tiling.bn);
+    return CATCOC_E_UNSUPPORTED;
   }
   if (swap && (!twice || (rf.kind != KIND_F16 && rf.kind != KIND_I8) || a.c_src != nullptr ||
                (a.num_groups > 0 && (a.tiling.bn != kMaxBN || a.num_groups > kMaxTokenGroups || o.M >= (1 << 24) || o.trans_a || a.g_a_row_back != 0 || a.g_a_k != 0)))) {
@@ -1323,7 +1331,7 @@ int double_workers(const CatcocOpArgs& a, int kind) {
 extern "C" int64_t catcoc_double_workspace_bytes(const CatcocOpArgs* args) {
   Resolved rf;
   if (args == nullptr || args->M <= 0 || args->N <= 0 || args->tiling.cut_slices < 2 || args->tiling.bn < 64 || args->tiling.bn > kMaxBN ||
-      resolve_format(args->in_fmt, &rf) != 0)
+      resolve_format(args->in_fmt, &rf) != 0 || !cut_width_fits(*args, rf.kind))
     return -1;
   const int workers = double_workers(*args, rf.kind);
   if (workers < 1) return -1;
