@@ -4,6 +4,7 @@
 //
 // Reference counterparts: examples/dynamic_tiling/impl/kernel_fp16.cpp:22-86 (layout dispatch +
 // launch) and examples/dynamic_tiling/impl/kernel/matmul_allreduce.h:152-212 (tiling -> params).
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include "catcoc/capi.h"
@@ -336,6 +337,15 @@ extern "C" int catcoc_sched_get_tile(int M, int N, int bm, int bn, int W, int se
 }
 
 int max_active_pairs(int kind);
+
+// Grid of a launch with units cut along K, which are more than its tiles: all the SMs that the caller leaves it, in whole pairs, one
+// at least. The launch, its workspace and its fold all deal out by it.
+static int cut_grid(const CatcocOpArgs& a, int kind) {
+  int device = 0;
+  cudaGetDevice(&device);
+  const int sms = sm_count(device), ctas = a.tiling.num_ctas > 0 ? imin(a.tiling.num_ctas, sms) : sms;
+  return std::max(2, imin(ctas, 2 * max_active_pairs(kind)) & ~1);
+}
 
 // Units that are cut along K are as wide as the caller says, which sizes their planes and steers their fold; block-scaled ones
 // have one width.
@@ -800,7 +810,7 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   }
   if (grid < 1) grid = 1;
   if (twice && !grouped) {
-    if (cut) grid = imin(imin(sms, a.tiling.num_ctas > 0 ? a.tiling.num_ctas : sms), 2 * max_active_pairs(rf.kind)) & ~1;   // more slices than units
+    if (cut) grid = cut_grid(a, rf.kind);
     p->dt.plan = make_double_plan(p->sched, bn, grid / 2, a.tiling.cut_slices, a.tiling.cut_k);
     if (p->dt.plan.doubles == 0) {
       // one block of B per stage: more stages (what single units wait for is the latency of their loads)
@@ -1319,13 +1329,6 @@ __global__ void __launch_bounds__(256, 6) double_fold_kernel(const FoldParams p,
       fold_store<INT>(p, planes + (static_cast<int64_t>(r) * p.pitch + c) * 4, p.plane * 4, p.slices, ti.m0 + r, ti.n0 + c, min(4, ti.cols - c));
   }
 }
-
-int double_workers(const CatcocOpArgs& a, int kind) {
-  int device = 0;
-  cudaGetDevice(&device);
-  const int sms = sm_count(device);
-  return imin(a.tiling.num_ctas > 0 ? imin(a.tiling.num_ctas, sms) : sms, 2 * max_active_pairs(kind)) / 2;
-}
 }  // namespace
 
 extern "C" int64_t catcoc_double_workspace_bytes(const CatcocOpArgs* args) {
@@ -1333,8 +1336,7 @@ extern "C" int64_t catcoc_double_workspace_bytes(const CatcocOpArgs* args) {
   if (args == nullptr || args->M <= 0 || args->N <= 0 || args->tiling.cut_slices < 2 || args->tiling.bn < 64 || args->tiling.bn > kMaxBN ||
       resolve_format(args->in_fmt, &rf) != 0 || !cut_width_fits(*args, rf.kind))
     return -1;
-  const int workers = double_workers(*args, rf.kind);
-  if (workers < 1) return -1;
+  const int workers = cut_grid(*args, rf.kind) / 2;
   const TileSched s = args->tiling.swap ? make_double_sched(args->N, args->M, args->tiling.bn, 1) : make_double_sched(args->M, args->N, args->tiling.bn, 1);
   return static_cast<int64_t>(make_double_plan(s, args->tiling.bn, workers, args->tiling.cut_slices, 1).cut) * args->tiling.cut_slices * 2 * kBM * args->tiling.bn * 4;
 }
@@ -1358,7 +1360,7 @@ extern "C" int catcoc_double_launch(const CatcocOpArgs* args, void* workspace, v
   if (rc != 0) return rc;
   const bool swap = a.tiling.swap != 0;
   const TileSched s = make_double_sched(swap ? a.N : a.M, swap ? a.M : a.N, a.tiling.bn, a.tiling.swizzle > 0 ? a.tiling.swizzle : 8);
-  const DoublePlan plan = make_double_plan(s, a.tiling.bn, double_workers(a, rf.kind), a.tiling.cut_slices, a.tiling.cut_k);
+  const DoublePlan plan = make_double_plan(s, a.tiling.bn, cut_grid(a, rf.kind) / 2, a.tiling.cut_slices, a.tiling.cut_k);
   if (plan.cut == 0) return CATCOC_OK;
   FoldParams f = fold_params(a);
   f.parts = static_cast<const uint8_t*>(workspace);

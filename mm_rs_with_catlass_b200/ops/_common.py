@@ -274,7 +274,10 @@ def launch_double(args: N.OpArgs, device: torch.device) -> None:
     args.timeout_ns = default_timeout_ns()
     args.events, args.events_cap = _event_ring
     lib = N.lib()
-    ws = torch.empty(max(1, int(lib.catcoc_double_workspace_bytes(C.byref(args)))), dtype=torch.uint8, device=device)
+    need = int(lib.catcoc_double_workspace_bytes(C.byref(args)))
+    if need < 0:
+        raise ValueError("double tiles: no workspace for %d x %d in %d slices, bn=%d" % (args.M, args.N, args.tiling.cut_slices, args.tiling.bn))
+    ws = torch.empty(max(1, need), dtype=torch.uint8, device=device)
     N.check(lib.catcoc_double_launch(C.byref(args), ws.data_ptr(), C.c_void_p(stream_of(device))))
     global _launches
     _launches += 1
