@@ -255,12 +255,17 @@ def _split_k(m: int, n: int, k: int, elt: int, direct: TilingConfig):
     return best, whole if best is None else best_time
 
 
-@functools.lru_cache(maxsize=4096)
 def slice_k_groups(groups: int, m: int, n: int, k_total: int, dtype: torch.dtype) -> TilingConfig:
     """Tiling of the products of ``groups`` K ranges, [m, n] each, in one launch (16-bit).
 
     A double tile takes 1.77 times as long as a pair tile: 32 ranges of 440 rows, 2048 x 4096: 294 -> 260 us, 32 of 234, 2048 x
     2048: 111 -> 88 us."""
+    return _slice_k_groups(groups, m, n, k_total, dtype, os.environ.get("CATCOC_CTA_PAIR"))
+
+
+@functools.lru_cache(maxsize=4096)
+def _slice_k_groups(groups: int, m: int, n: int, k_total: int, dtype: torch.dtype, forced: Optional[str]) -> TilingConfig:
+    # (`forced` is read by the heuristic: a choice made under it is not one without it)
     t = heuristic("matmul", groups * m, n, k_total, 1, dtype)
     if t.cta_pair == 2 and math.ceil(m / 256) * 256 > 1.18 * math.ceil(m / 128) * 128:
         t = t.with_(cta_pair=1)

@@ -3,6 +3,7 @@ allows them, narrower tiles where wide ones leave most SMs idle."""
 import pytest
 import torch
 
+from mm_rs_with_catlass_b200.tiling import chooser
 from mm_rs_with_catlass_b200.tiling.chooser import grouped
 
 
@@ -25,3 +26,22 @@ def test_choice_follows_the_waves():
     assert [grouped(8 * 512, r, 8192, torch.bfloat16).cta_pair for r in (512.0, 512, 512.0)] == [
         grouped(8 * 512, float(512), 8192, torch.bfloat16).cta_pair, 2, grouped(8 * 512, 512.0, 8192, torch.bfloat16).cta_pair]
     assert grouped(14080, 440, 4096, torch.bfloat16) is not grouped(14080, 440.0, 4096, torch.bfloat16)
+
+
+@pytest.mark.parametrize("case,order", list(enumerate([("1", None), (None, "1"), ("1", "2"), ("2", "1")])))
+def test_choices_follow_the_forced_cta_count(monkeypatch, case, order):
+    """A choice made with CATCOC_CTA_PAIR set is not kept for calls without it, nor the other way round."""
+    tokens = 14080 + 64 * case             # sizes of its own: what an earlier order left behind serves no later one
+    rules = {"ranges along K": lambda: chooser.slice_k_groups(32, 2048, 4096, tokens, torch.bfloat16),
+             "groups of rows": lambda: chooser.token_groups(tokens, 32, 4096, 2048, torch.bfloat16),
+             "one product": lambda: chooser.choose("matmul", 4096 + tokens, 4096, 4096, 1, torch.bfloat16, tails=True, doubles=True)}
+    for name, rule in rules.items():
+        seen = []
+        for forced in order:
+            if forced is None:
+                monkeypatch.delenv("CATCOC_CTA_PAIR", raising=False)
+            else:
+                monkeypatch.setenv("CATCOC_CTA_PAIR", forced)
+            seen.append(rule())
+        for forced, t in zip(order, seen):
+            assert (t.cta_pair == 1) == (forced == "1"), (name, order, t)
