@@ -359,7 +359,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
   if (warp == kIssuerWarp) ptx::tmem_dealloc(tmem, kTmemCols);
 }
 
-// The slices of a row, a warp each; every row has a slice that it sees something of unless it sees nothing at all
+// The slices of a row, a warp each; every row has a slice that it sees something of unless it sees nothing at all. A slice of which
+// the row sees nothing is left out, not weighed with zero: its piece is zero times values that the row's tile may not see either, where
+// an infinity makes a NaN. (A sum that is not zero, a NaN, is no such slice.)
 template <int D, int FMT>
 __global__ void __launch_bounds__(128) flash_slices_kernel(const float* part_o, const float* part_ml, void* out, int64_t rows, int slices) {
   constexpr int kPer = D / 32;                     // columns per lane
@@ -372,6 +374,7 @@ __global__ void __launch_bounds__(128) flash_slices_kernel(const float* part_o, 
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   const float w = ml.x == -INFINITY ? 0.0f : ptx::ex2_approx(ml.x - mx);
+  const uint32_t seen = __ballot_sync(0xffffffffu, !(ml.x == -INFINITY && ml.y == 0.0f));
   float l = w * ml.y, acc[kPer];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
@@ -381,9 +384,11 @@ __global__ void __launch_bounds__(128) flash_slices_kernel(const float* part_o, 
   for (int c = 0; c < slices; ++c) {
     const float wc = __shfl_sync(0xffffffffu, w, c);
     const float* src = part_o + (c * rows + r) * D + lane * kPer;
-    float o[kPer];
-    if constexpr (kPer == 4) *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(src);
-    else *reinterpret_cast<float2*>(o) = *reinterpret_cast<const float2*>(src);
+    float o[kPer] = {};
+    if ((seen >> c) & 1u) {
+      if constexpr (kPer == 4) *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(src);
+      else *reinterpret_cast<float2*>(o) = *reinterpret_cast<const float2*>(src);
+    }
 #pragma unroll
     for (int e = 0; e < kPer; ++e) acc[e] += wc * o[e];
   }

@@ -38,3 +38,24 @@ def test_against_the_reference(case, d):
 def test_moving_reference_maxima(gain):
     for d in (64, 128):
         _run(1, 8, 2, 160, 3000, d, torch.bfloat16, True, seed=5, key_gain=gain)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("b,h,sq,sk,first", [(1, 1, 2300, 2301, 1280), (1, 2, 1900, 1900, 896), (2, 1, 1500, 4096, 3200)])
+def test_values_behind_a_tile_do_not_reach_its_rows(b, h, sq, sk, first, bad):
+    """Values that are no numbers from key ``first`` on, over several slices: tiles of 128 rows that see none of these keys give the
+    bits that they give without them, as they do where the keys are not cut. A query that is no number still shows."""
+    import mm_rs_with_catlass_b200 as catcoc
+    for d in (64, 128):
+        assert _scratch(b, h, h, sq, sk, d, True) > 0
+        g = torch.Generator(device="cuda").manual_seed(d)
+        q, k, v = (torch.randn(b, h, s, d, device="cuda", generator=g).bfloat16() for s in (sq, sk, sk))
+        want = catcoc.flash_attention(q, k, v, causal=True)
+        v[:, :, first:] = bad
+        got = catcoc.flash_attention(q, k, v, causal=True)
+        clean = sum(1 for t in range(0, sq, 128) if min(sk, t + 128 + sk - sq) <= first) * 128
+        assert 0 < clean < sq and torch.equal(got[:, :, :clean], want[:, :, :clean])
+        assert not got[:, :, -1].isfinite().any()
+        q[:, :, 5] = float("nan")
+        assert catcoc.flash_attention(q, k, v, causal=True)[:, :, 5].isnan().all()
