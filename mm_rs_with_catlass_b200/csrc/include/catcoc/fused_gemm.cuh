@@ -218,7 +218,7 @@ CATCOC_DEVICE float silu_corrected(float x, bool& plain) {
   const float d = 1.0f + __expf(-x), r = ptx::rcp_approx(d);
   const float q = x * r;
   plain = plain || !(d <= 0x1p125f) || !(fabsf(x) <= 0x1p125f);
-  return fmaf(fmaf(-q, d, x), r, q);
+  return copysignf(fmaf(fmaf(-q, d, x), r, q), x);   // (the residual of -0 is +0)
 }
 
 // The same for 32 values. What a tile's first pass costs is the fetch of its instructions: the choice is made once and not per value, and

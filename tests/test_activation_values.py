@@ -42,3 +42,15 @@ def test_values(tiling, act):
     ok = ~bad & v.isfinite() & (want.abs() < 1e37)
     assert bool(((got - want).abs()[ok] <= tol[ok]).all()), ((got - want).abs() - tol)[ok].max()
     assert bool((got[v == math.inf] == math.inf).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tiling", sorted(TILINGS))
+def test_silu_keeps_the_sign_of_zero(tiling):
+    # minus one times an accumulator of zero, and a bias: minus zero where the bias is
+    x = torch.tensor([-0.0, 0.0, -1e-38, 1e-38, -2.0, -0.0, 3.0, -0.0] * 12).cuda()
+    m, n, k = 40, x.numel(), 16
+    a, b = torch.zeros(m, k, device="cuda", dtype=torch.bfloat16), torch.zeros(n, k, device="cuda", dtype=torch.bfloat16)
+    out = catcoc.matmul(a, b, trans_b=True, activation="silu", out_dtype=torch.float32, alpha=-1.0, bias_f32=x,
+                        tiling=TilingConfig(swizzle=2, **TILINGS[tiling]))
+    assert torch.equal(out.signbit(), x.signbit().expand(m, n))
