@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
   struct Item { TileInfo ti; int bn, bn1, parts, half, k_off, k_len, plane; };
   struct TokenWalk { int g, tile_base; };
   using Walk = typename std::conditional<kTok, TokenWalk, GroupWalk>::type;
+  auto event_id = [&](int i) { return static_cast<uint32_t>(worker + i * num_workers); };
   auto walk_begin = [&]() {
     if constexpr (kTok) return TokenWalk{0, 0};
     else return group_walk_begin(p);
@@ -322,6 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
     Walk walk = walk_begin();
     Item it;
     for (int i = 0; ok && get_item(i, walk, it); ++i) {
+      if (is_a && lane == 0) emit_event(p, EV_PRODUCER, EV_BEGIN, event_id(i));
       const TileInfo& ti = it.ti;
       const int parts = is_a ? 1 : it.parts;                        // each half has a block of B of its own
       int k_off = it.k_off;
@@ -508,6 +510,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
         };
         if (it.parts == 1) {
           wait_acc(it.half);
+          if (ok && lane == 0) emit_event(p, EV_MMA, EV_BEGIN, event_id(i));
           for (int kb = 0; ok && kb < tile_kb; ++kb) {
             wait_full(kb);
             if (!ok) break;
@@ -515,6 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
             __syncwarp();
             next0(); next1();
           }
+          if (ok && lane == 0) emit_event(p, EV_MMA, EV_END, event_id(i));
           continue;
         }
         // half 0 leads at both ends of the tile; in between the halves take turns and a stage is free after one block of each
@@ -530,7 +534,10 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
             ++kb;
             continue;
           }
-          if (kb == 0) wait_acc(0);
+          if (kb == 0) {
+            wait_acc(0);
+            if (ok && lane == 0) emit_event(p, EV_MMA, EV_BEGIN, event_id(i));
+          }
           for (int j = 0; ok && j < count; ++j) {
             wait_full(kb + j);
             if (!ok) break;
@@ -546,6 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
           }
           kb += count;
         }
+        if (ok && lane == 0) emit_event(p, EV_MMA, EV_END, event_id(i));
       }
       tick.lap(c_issue);
       if (tr) { atomicAdd(p.trace + 2, c_full); atomicAdd(p.trace + 3, c_acc); atomicAdd(p.trace + 4, c_issue); }
@@ -596,6 +604,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
       }
       acc_phase ^= 1u;
       ptx::tcgen05_fence_after();
+      if (lane == 0 && q == 0) emit_event(p, h == 0 ? EV_EPILOGUE : EV_EPILOGUE_2, EV_BEGIN, event_id(i));
       const int64_t pitch = p.ldc * st_elt;
       if constexpr (SWAP) {
         // The accumulator's lanes are features, its columns tokens. 32-bit values are staged token by token, 32 features of a
@@ -686,6 +695,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&tail->acc_empty[h]), 0u));
         }
+        if (lane == 0 && q == 0) emit_event(p, h == 0 ? EV_EPILOGUE : EV_EPILOGUE_2, EV_END, event_id(i));
         continue;
       }
       uint8_t* base = static_cast<uint8_t*>(p.out) + (static_cast<int64_t>(ti.m0 + row_base) * p.ldc + n0) * st_elt;
@@ -786,6 +796,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&tail->acc_empty[h]), 0u));
       }
+      if (lane == 0 && q == 0) emit_event(p, h == 0 ? EV_EPILOGUE : EV_EPILOGUE_2, EV_END, event_id(i));
     }
     if (lane == 0) ptx::bulk_wait_group_all();   // every TMA store of this warp is performed before the kernel ends
     __syncwarp();

@@ -123,10 +123,12 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
         from ..tiling import chooser
         # [N, K] storage, or a column-major view of [K, N], which as_operand folds into it
         b_k_major = trans_b != (b.stride(-1) != 1 and b.stride(0) == 1 and min(b.shape) > 1)
-        tails = _group is None and trace is None and a.dtype in (torch.float16, torch.bfloat16, torch.int8)
-        tiling = chooser.choose("matmul", m, n, k, 1, a.dtype,
-                                b_k_major=b_k_major and _group is None, tails=tails, doubles=tails,
-                                swap=c is None or beta == 0.0)
+        tails = _group is None and a.dtype in (torch.float16, torch.bfloat16, torch.int8)
+        where = dict(b_k_major=b_k_major and _group is None)
+        tiling = chooser.choose("matmul", m, n, k, 1, a.dtype, tails=tails, doubles=tails, swap=c is None or beta == 0.0, **where)
+        if trace is not None and not tiling.twice:   # (the counters are of one kernel: tiles of one accumulator are then not cut)
+            tails = False
+            tiling = chooser.choose("matmul", m, n, k, 1, a.dtype, **where)
         if _group is None and trace is None and not tiling.twice:
             split = chooser.split_k(m, n, k, a.element_size(), tiling)
             if split is not None:

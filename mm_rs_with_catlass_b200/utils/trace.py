@@ -22,7 +22,7 @@ import torch
 
 from ..ops import _common as cm
 
-ROLES = {0: "tma_producer", 1: "mma", 2: "epilogue", 3: "comm", 4: "reducer"}
+ROLES = {0: "tma_producer", 1: "mma", 2: "epilogue", 3: "comm", 4: "reducer", 5: "epilogue_2"}   # 5: second half of a double tile
 PHASES = {0: "B", 1: "E", 2: "i"}
 
 

@@ -180,3 +180,50 @@ def test_event_ring_gives_a_chrome_trace_with_matched_begin_and_end_records(tmp_
     with open(path) as fh:
         trace = json.load(fh)
     assert len([e for e in trace["traceEvents"] if e.get("ph") in ("B", "E")]) == r["events"]
+
+
+def test_event_ring_of_double_tiles():
+    out = _child("""
+        import json, torch
+        import mm_rs_with_catlass_b200 as catcoc
+        from mm_rs_with_catlass_b200.utils.trace import EventTrace
+        dev = torch.device("cuda:0")
+        a, b = (torch.randn(1000, 512, device=dev).bfloat16() for _ in range(2))
+        for swap in (False, True):
+            for cut in (dict(), dict(cut_slices=2, cut_k=256, num_ctas=14)):
+                with EventTrace(capacity=4096) as tr:
+                    catcoc.matmul(a, b, trans_b=True, tiling=catcoc.TilingConfig(bn=128, cta_pair=2, twice=True, swap=swap, **cut))
+                by = {}
+                for r in tr.records():
+                    by.setdefault((r["cta"], r["role"], r["tile"]), []).append(r["phase"])
+                count = lambda role: len([k for k in by if k[1] == role])
+                print(json.dumps({"cut": bool(cut), "producers": count(0), "mma": count(1), "epilogues": count(2) + count(5), "dropped": tr.dropped,
+                                  "paired": all(sorted(v) == [0, 1] for k, v in by.items() if k[1] != 0)}))
+    """)
+    # 4 x 8 units of 256 x 128: on 74 pairs 32 single units; on 7 pairs 4 of them are cut in two and the others are 14 double
+    # tiles. Producers and epilogues of both CTAs, one issuer a pair.
+    assert len(out) == 4
+    for r in out:
+        items, halves = (14 + 8, 28 + 8) if r["cut"] else (32, 32)
+        assert r["paired"] and r["dropped"] == 0, r
+        assert (r["mma"], r["producers"], r["epilogues"]) == (items, 2 * items, 2 * halves), r
+
+
+def test_trace_counters_are_those_of_the_kernel_that_a_plain_call_runs():
+    out = _child("""
+        import json, torch
+        import mm_rs_with_catlass_b200 as catcoc
+        from mm_rs_with_catlass_b200.ops import gemm
+        dev = torch.device("cuda:0")
+        for m, n, k in ((1024, 5120, 6144), (300, 200, 264)):
+            a, b = torch.randn(m, k, device=dev).bfloat16(), torch.randn(n, k, device=dev).bfloat16()
+            trace, twice = torch.zeros(16, dtype=torch.int64, device=dev), []
+            for t in (None, trace):
+                gemm._plans.clear()
+                catcoc.matmul(a, b, trans_b=True, trace=t)
+                twice.append([p[0].tiling.twice for p in gemm._plans.values()])
+            print(json.dumps({"twice": twice, "trace": trace.tolist()}))
+    """, {"CATCOC_CHECKED": "0"})
+    assert [r["twice"] for r in out] == [[[1], [1]], [[0], [0]]], out
+    # lifetimes of the CTAs, and the double tile's second half
+    assert all(r["trace"][8] > 0 for r in out) and out[0]["trace"][14] > 0 and out[0]["trace"][15] > 0, out
