@@ -787,7 +787,7 @@ __global__ void __launch_bounds__(kThreads, 1) double_tile_kernel(const __grid_c
           prev_tma = true;
         } else {
           __syncwarp();
-          flush_staged(stg, lane, base + static_cast<int64_t>(win) * 128, pitch, rows_valid, min(per_win, cols - c0), st_elt, vec_ok, nullptr, nullptr, 0, 0, 1);
+          flush_staged<false>(stg, lane, base + static_cast<int64_t>(win) * 128, pitch, rows_valid, min(per_win, cols - c0), st_elt, vec_ok, nullptr, nullptr, 0, 0, 1);
         }
         __syncwarp();
       }

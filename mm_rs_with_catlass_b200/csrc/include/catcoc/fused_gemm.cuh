@@ -52,7 +52,7 @@ constexpr int kThreads = 256;          // warps 0-6 are the GEMM roles, warp 7 a
 // it carries two more communication warps: the push of the A shard is latency bound per warp and
 // one warp per SM could not feed the link (measured 173 GB/s per GPU, the GEMM waited on it).
 constexpr int kThreadsPlain = 384;
-CATCOC_HD constexpr int threads_for(int epi) { return (epi == EPI_PLAIN || epi == EPI_PULL) ? kThreadsPlain : kThreads; }
+CATCOC_HD constexpr int threads_for(int epi) { return ((epi & ~EPI_WHOLE_ROWS) == EPI_PLAIN || epi == EPI_PULL) ? kThreadsPlain : kThreads; }
 constexpr int kTmemCols = 512;
 constexpr int kPullStrips = 4;   // pull flavour: a 32-row quarter is reduced in this many strips (one reducer task each)
 constexpr int kMaxStages = 6;
@@ -359,6 +359,12 @@ CATCOC_DEVICE void store_rows_by_word(int lane, int width, uint8_t* dst, int64_t
 // 4096 rows: 5706 columns 174 -> 116 us, 5705 (every other row begins inside a word) 172 -> 120 us, 5704 by TMA 113 us; 1085
 // rows (swapped double tiles) 69 -> 41, 70 -> 46, 40 us; 9676 x 194 x 192, one tile a CTA: 22.6 -> 11.9 us, 192 columns 9.0 us; K = 880, 6408 rows:
 // 14082 columns 428 -> 148 us, 14081 441 -> 210 (263 with a choice per row), 14080 131 us.
+//
+// WHOLE: the caller has no others, and their code is left out, as is the unrolling of the few stores that TMA does not do. Never run, that
+// code still cost 1 to 2 % of a launch bound by its stores (bf16 16000 x 1024 x 192: 20.6 us, 20.2 without) and 5 % with the dequantising
+// epilogue (int8, 16 groups of 2000 rows, 4096 x 1024: 299, 282 without). Out of line, the stores of the others take 15 % longer
+// (bf16 5690 x 3341 x 144: 51 -> 59 us).
+template <bool WHOLE>
 CATCOC_DEVICE void flush_staged(uint32_t stg, int lane, uint8_t* base, int64_t pitch,
                                 int rows_valid, int cols_valid, int elt, bool vec_ok,
                                 uint8_t* mc, uint8_t* const* peer_bases, int64_t off, int rank,
@@ -367,7 +373,7 @@ CATCOC_DEVICE void flush_staged(uint32_t stg, int lane, uint8_t* base, int64_t p
   const int per_unit = 16 / elt;
   const int c0 = unit * per_unit;
   const int ndst = (peer_bases != nullptr) ? W : 1;
-  if (mc == nullptr && (!vec_ok || cols_valid % per_unit != 0)) {
+  if (!WHOLE && mc == nullptr && (!vec_ok || cols_valid % per_unit != 0)) {
     for (int d = 0; d < ndst; ++d) {
       uint8_t* dst = (peer_bases != nullptr) ? peer_bases[peer_for_push_rs(rank, d, W)] + off : base;
       store_rows_by_word(lane, 32, dst, pitch, rows_valid, cols_valid, elt, [&](int row) {
@@ -376,7 +382,7 @@ CATCOC_DEVICE void flush_staged(uint32_t stg, int lane, uint8_t* base, int64_t p
     }
     return;
   }
-#pragma unroll
+#pragma unroll (WHOLE ? 1 : 8)
   for (int it = 0; it < 8; ++it) {
     const int row = it * 4 + (lane >> 3);
     const uint4 v = ptx::ld_shared_v4(stg + row * 128 + ((unit ^ (row & 7)) << 4));
@@ -432,8 +438,8 @@ CATCOC_DEVICE const CUtensorMap* push_map(const FusedParamsTail& p, bool tail, i
 // ---------------------------------------------------------------------------------------
 // The kernel
 // ---------------------------------------------------------------------------------------
-template <int KIND, bool CTA2, int EPI, class Params = FusedParams>
-__global__ void __launch_bounds__(threads_for(EPI), 1)
+template <int KIND, bool CTA2, int EPI_CODE, class Params = FusedParams>
+__global__ void __launch_bounds__(threads_for(EPI_CODE), 1)
 fused_gemm_kernel(const __grid_constant__ Params p) {
   constexpr bool kGk = std::is_same<Params, FusedParamsGk>::value;   // every group has a K range of its own
   constexpr bool kTail = std::is_same<Params, FusedParamsTail>::value;   // the last tiles are cut along K
@@ -452,6 +458,8 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
     }
   };
   // Epilogue variant (see EpiVariant in params.h): stages a launch cannot need are compiled out.
+  constexpr int EPI = EPI_CODE & ~EPI_WHOLE_ROWS;
+  constexpr bool kWholeRows = (EPI_CODE & EPI_WHOLE_ROWS) != 0;
   constexpr bool kReduce = (EPI == EPI_REDUCE || EPI == EPI_FULL);   // push flavour of RS / AR: peers' partials, pushes, stamps
   constexpr bool kScale = (EPI == EPI_FULL);      // int32 bias, dequantisation, alpha / beta / C / fp32 bias
   constexpr bool kPull = (EPI == EPI_PULL);       // pull flavour of RS / AR: local partials, stamps, reducer warps
@@ -1360,7 +1368,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
               }
             }
           } else {
-            flush_staged(stg, lane, base != nullptr ? base + wb : nullptr, pitch, rows_valid,
+            flush_staged<kWholeRows>(stg, lane, base != nullptr ? base + wb : nullptr, pitch, rows_valid,
                          cols_valid, st_elt, vec_ok, mc != nullptr ? mc + wb : nullptr, peer_bases,
                          off + wb, p.rank, p.W);
           }

@@ -5,6 +5,7 @@
 //   EPI_REDUCE  + the owner-side fold of the peers' partial tiles (reduce-scatter, all-reduce)
 //   EPI_FULL    + int32 bias, per-row / per-column scales, alpha / beta / C / fp32 bias
 //   EPI_PULL    16-bit kinds only: partial tiles stay local, reducer warps sum them through the switch
+//   EPI_PLAIN and EPI_FULL also with EPI_WHOLE_ROWS: a local output whose rows are whole 16-byte units (flush_staged)
 // The variants exist because the optional stages, although skipped at run time, slow the plain
 // path down measurably (code size and register pressure in the epilogue warps).
 #pragma once
@@ -123,7 +124,7 @@ cudaError_t launch_double_slice_k(const FusedParamsGk& p, int grid, cudaStream_t
   }                                                                                                   \
   } }
 
-// Four variants: the three above and the pull flavour of reduce-scatter / all-reduce.
+// The three above, the pull flavour of reduce-scatter / all-reduce, and plain and full for whole rows.
 #define CATCOC_DEFINE_UNIT_4(NAME, KIND, CTA2)                                                        \
   namespace catcoc { namespace inst {                                                                 \
   static cudaError_t NAME##_prepare() {                                                               \
@@ -131,12 +132,16 @@ cudaError_t launch_double_slice_k(const FusedParamsGk& p, int grid, cudaStream_t
     if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_REDUCE>();                                \
     if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_FULL>();                                  \
     if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_PULL>();                                  \
+    if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_PLAIN | EPI_WHOLE_ROWS>();                \
+    if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_FULL | EPI_WHOLE_ROWS>();                 \
     return e;                                                                                         \
   }                                                                                                   \
   static cudaError_t NAME##_launch(int epi, const FusedParams& p, int grid, int threads, cudaStream_t s) { \
     if (epi == EPI_PLAIN) return launch_one<KIND, CTA2, EPI_PLAIN>(p, grid, threads, s);              \
     if (epi == EPI_REDUCE) return launch_one<KIND, CTA2, EPI_REDUCE>(p, grid, threads, s);            \
     if (epi == EPI_PULL) return launch_one<KIND, CTA2, EPI_PULL>(p, grid, threads, s);                \
+    if (epi == (EPI_PLAIN | EPI_WHOLE_ROWS)) return launch_one<KIND, CTA2, EPI_PLAIN | EPI_WHOLE_ROWS>(p, grid, threads, s); \
+    if (epi == (EPI_FULL | EPI_WHOLE_ROWS)) return launch_one<KIND, CTA2, EPI_FULL | EPI_WHOLE_ROWS>(p, grid, threads, s);   \
     return launch_one<KIND, CTA2, EPI_FULL>(p, grid, threads, s);                                     \
   }                                                                                                   \
   static int NAME##_clusters() { return CTA2 ? query_clusters<KIND, EPI_FULL>() : 0; }                \
@@ -146,16 +151,20 @@ cudaError_t launch_double_slice_k(const FusedParamsGk& p, int grid, cudaStream_t
   }                                                                                                   \
   } }
 
-// Two variants: plain and full (the full one also serves reduce-only launches).
+// Plain and full (the full one also serves reduce-only launches), each for any rows and for whole ones.
 #define CATCOC_DEFINE_UNIT_2(NAME, KIND, CTA2)                                                        \
   namespace catcoc { namespace inst {                                                                 \
   static cudaError_t NAME##_prepare() {                                                               \
     cudaError_t e = set_smem_attr<KIND, CTA2, EPI_PLAIN>();                                           \
     if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_FULL>();                                  \
+    if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_PLAIN | EPI_WHOLE_ROWS>();                \
+    if (e == cudaSuccess) e = set_smem_attr<KIND, CTA2, EPI_FULL | EPI_WHOLE_ROWS>();                 \
     return e;                                                                                         \
   }                                                                                                   \
   static cudaError_t NAME##_launch(int epi, const FusedParams& p, int grid, int threads, cudaStream_t s) {         \
     if (epi == EPI_PLAIN) return launch_one<KIND, CTA2, EPI_PLAIN>(p, grid, threads, s);                       \
+    if (epi == (EPI_PLAIN | EPI_WHOLE_ROWS)) return launch_one<KIND, CTA2, EPI_PLAIN | EPI_WHOLE_ROWS>(p, grid, threads, s); \
+    if (epi == (EPI_FULL | EPI_WHOLE_ROWS)) return launch_one<KIND, CTA2, EPI_FULL | EPI_WHOLE_ROWS>(p, grid, threads, s);   \
     return launch_one<KIND, CTA2, EPI_FULL>(p, grid, threads, s);                                              \
   }                                                                                                   \
   static int NAME##_clusters() { return CTA2 ? query_clusters<KIND, EPI_FULL>() : 0; }                \

@@ -37,6 +37,7 @@ enum EpiVariant {
   EPI_FULL = 2,     // + int32 bias, per-row / per-column scales, alpha / beta / C / fp32 bias
   EPI_PULL = 3,     // plain stores of partial tiles into the local heap + stamps; extra warps reduce the
                     // owned tiles through the switch (multimem.ld_reduce) and store / broadcast them
+  EPI_WHOLE_ROWS = 4,   // with EPI_PLAIN or EPI_FULL: a local output whose rows are whole 16-byte units, with nothing for others
 };
 
 // Element-wise function on finished (owned) tiles, after scales / affine terms.

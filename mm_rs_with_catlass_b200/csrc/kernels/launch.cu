@@ -876,6 +876,9 @@ int max_active_pairs(int kind) {
   return cached[kind];
 }
 
+// A local output whose rows are whole 16-byte units in memory
+static bool whole_rows(const FusedParams& p) { return p.W <= 1 && p.out_vec_ok != 0 && p.sched.N * fmt_bytes(p.out_fmt) % 16 == 0; }
+
 // The leanest epilogue variant that covers this launch.
 static int pick_epi(const FusedParams& p) {
   if (p.pull) return EPI_PULL;
@@ -898,7 +901,7 @@ int catcoc_launch_params(const FusedParams& p, int kind, int grid, int pair, int
   }
   const inst::Unit* u = unit_for(kind, pair != 0);
   if (u == nullptr) { set_error("no kernel for kind %d with cta_pair=%d", kind, pair ? 2 : 1); return CATCOC_E_UNSUPPORTED; }
-  e = u->launch(pick_epi(p), p, grid, threads, stream);
+  e = u->launch(pick_epi(p) | (whole_rows(p) ? EPI_WHOLE_ROWS : 0), p, grid, threads, stream);
   if (e != cudaSuccess) {
     set_error("kernel launch failed: %s", cudaGetErrorString(e));
     return -1000 - static_cast<int>(e);
