@@ -83,8 +83,9 @@ CATCOC_DEVICE void fail(const AttnParams& p, uint32_t what, uint32_t a, uint32_t
 }
 
 // D: head dimension; FMT: operand and output dtype (compile time: the softmax loop packs 64 pairs per row and block);
-// CUT: a CTA takes the key blocks of slice blockIdx.y only and leaves a piece
-template <int D, int FMT, bool CUT>
+// CUT: a CTA takes the key blocks of slice blockIdx.y only and leaves a piece; LATE: a block's softmax waits for the product with V of
+// the block before where it needs it, to rescale O or to write P, else ahead of its exponentials (D = 64, see attn_plan)
+template <int D, int FMT, bool CUT, bool LATE>
 __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_constant__ AttnParams p) {
   constexpr int kDB = D / 64;                    // 128-byte blocks along the head dimension
   constexpr int kQBytes = kDB * kBlockBytes;     // one Q tile
@@ -305,9 +306,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_attn_kernel(const __grid_co
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->s_free[t]);
       }, [&](bool move, float alpha) {
-        if (!kOneS || move) previous();
+        if (!LATE || move) previous();
         if (move && j > 0) rescale_o<D>(t_o, alpha);
-      }, [&] { if constexpr (kOneS) previous(); }, [&] {
+      }, [&] { if constexpr (LATE) previous(); }, [&] {
         if constexpr (!kOneS) {
           ptx::tcgen05_wait_st();
           ptx::tcgen05_fence_before();
@@ -405,32 +406,42 @@ using namespace catcoc;
 using namespace catcoc::host;
 
 namespace {
+// D = 64: does a softmax wait for the product before late? That is the faster form while the two tiles of a CTA are out of step, from
+// its start on (10 blocks of keys: 2 x 32 / 8 heads x 300 over 1200 keys 22.1 -> 20.1 us) and where the mask gives them different numbers
+// of blocks, at least a third of the keys (load 17, 3 x 600 over 1200: 40.6 -> 39.8; 22, 4 x 32 / 4 x 500 over 1500: 43.7 -> 41.6; 35,
+// 2 x 2048: 65.9 -> 64.8). In step the other one is: load 22, 8 x 300 over 1200 59.2 -> 61.0; 46, 6 x 1000, not causal, 96.5 -> 102.6; 57,
+// 1 x 32 x 4096 105 -> 107; 221, 2 x 4096, not causal, 349 -> 367. `load`: key blocks of the busiest SM.
+bool late_wait(double load, int64_t ctas, int causal, int pos, int Sk) {
+  return load <= (causal && 3ll * pos >= Sk ? 35.0 : ctas <= 148 ? 16.0 : 0.0);
+}
+
 struct AttnPlan {
   int Hq, Sq;          // as the kernel sees them (the query heads of a KV head may be packed)
   int tiles;
   int slices, per;     // keys cut into slices of `per` blocks
+  double load;         // key blocks of the busiest SM
 };
 
 AttnPlan attn_plan(int B, int Hq, int Hk, int Sq, int Sk, int causal, bool cut) {
   const int group = Hq / Hk, rows_cta = attn::kTiles * attn::kBQ, pos = Sq;
   auto blocks = [&](int hi) { return static_cast<double>((causal ? std::min<int64_t>(Sk, static_cast<int64_t>(hi) + Sk - pos) : Sk) + 127) / 128; };
   const double longest = blocks(pos);
-  AttnPlan d{Hq, Sq, (Sq + rows_cta - 1) / rows_cta, 1, 0}, packed = d;
+  AttnPlan d{Hq, Sq, (Sq + rows_cta - 1) / rows_cta, 1, 0, 0.0}, packed = d;
+  double plain = 0.0;
+  for (int i = 0; i < d.tiles; ++i) plain += blocks(std::min((i + 1) * rows_cta, pos));
+  d.load = std::max(longest, static_cast<double>(B) * Hq * plain / 148.0);
   bool pack = false;
   // A call of few query positions: the query heads of a KV head are contiguous rows, so they can fill tiles together. It
   // costs the keys that a head's early tiles would have skipped; in units of (CTA, 128-key block), a launch takes its
   // total over the SMs or its longest CTA. 16 x 32 / 4 heads x 100 positions over 2000 keys: 154 -> 71 us,
   // 16 x 32 / 8 x 64 over 1000 (D = 64): 78 -> 20 us.
   if (group > 1 && static_cast<int64_t>(group) * Sq <= (1 << 24)) {
-    double plain = 0.0;
     packed.Sq = group * Sq;
     packed.Hq = Hk;
     packed.tiles = (packed.Sq + rows_cta - 1) / rows_cta;
     pack = true;
-    for (int i = 0; i < d.tiles; ++i) plain += blocks(std::min((i + 1) * rows_cta, pos));
-    const double heads = static_cast<double>(B) * Hk;
-    const double t_plain = std::max(longest, heads * group * plain / 148.0), t_packed = std::max(longest, heads * packed.tiles * longest / 148.0);
-    if (t_packed < 0.95 * t_plain) d = packed;
+    packed.load = std::max(longest, static_cast<double>(B) * Hk * packed.tiles * longest / 148.0);
+    if (packed.load < 0.95 * d.load) d = packed;
   }
   // Few tiles over many keys leave SMs idle: the keys are then cut into slices, which a second kernel merges. In us, a CTA takes 5
   // and 1.55 a block of keys, the merge 4 and its bytes at 3 TB/s. In a loop, D = 128: 32 heads x 131 positions over 3404 keys 46 ->
@@ -536,14 +547,16 @@ extern "C" int catcoc_flash_attention_cut(const void* q, const void* k, const vo
   const bool bf = fmt == CATCOC_FMT_BF16;
   int lrc;
   if (d.slices > 1) {
-    if (D == 128) lrc = bf ? launch(attn::flash_attn_kernel<128, FMT_BF16, true>) : launch(attn::flash_attn_kernel<128, FMT_F16, true>);
-    else lrc = bf ? launch(attn::flash_attn_kernel<64, FMT_BF16, true>) : launch(attn::flash_attn_kernel<64, FMT_F16, true>);
+    if (D == 128) lrc = bf ? launch(attn::flash_attn_kernel<128, FMT_BF16, true, true>) : launch(attn::flash_attn_kernel<128, FMT_F16, true, true>);
+    else lrc = bf ? launch(attn::flash_attn_kernel<64, FMT_BF16, true, true>) : launch(attn::flash_attn_kernel<64, FMT_F16, true, true>);
     if (lrc == 0 && D == 128) lrc = bf ? merge(attn::flash_slices_kernel<128, FMT_BF16>) : merge(attn::flash_slices_kernel<128, FMT_F16>);
     else if (lrc == 0) lrc = bf ? merge(attn::flash_slices_kernel<64, FMT_BF16>) : merge(attn::flash_slices_kernel<64, FMT_F16>);
   } else if (D == 128) {
-    lrc = bf ? launch(attn::flash_attn_kernel<128, FMT_BF16, false>) : launch(attn::flash_attn_kernel<128, FMT_F16, false>);
+    lrc = bf ? launch(attn::flash_attn_kernel<128, FMT_BF16, false, true>) : launch(attn::flash_attn_kernel<128, FMT_F16, false, true>);
+  } else if (late_wait(d.load, ctas, causal, pos, Sk)) {
+    lrc = bf ? launch(attn::flash_attn_kernel<64, FMT_BF16, false, true>) : launch(attn::flash_attn_kernel<64, FMT_F16, false, true>);
   } else {
-    lrc = bf ? launch(attn::flash_attn_kernel<64, FMT_BF16, false>) : launch(attn::flash_attn_kernel<64, FMT_F16, false>);
+    lrc = bf ? launch(attn::flash_attn_kernel<64, FMT_BF16, false, false>) : launch(attn::flash_attn_kernel<64, FMT_F16, false, false>);
   }
   if (lrc != 0) return lrc;
   e = cudaGetLastError();

@@ -59,3 +59,14 @@ def test_values_behind_a_tile_do_not_reach_its_rows(b, h, sq, sk, first, bad):
         assert not got[:, :, -1].isfinite().any()
         q[:, :, 5] = float("nan")
         assert catcoc.flash_attention(q, k, v, causal=True)[:, :, 5].isnan().all()
+
+
+# D = 64: launches on either side of the line between the two forms of a block's wait: one wave, more, masks over much and over little
+WAITS = [(2, 32, 8, 300, 600, True), (8, 32, 8, 300, 1200, True), (3, 32, 8, 600, 1200, True), (6, 32, 8, 1000, 1000, False), (1, 4, 4, 130, 300, False)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", WAITS)
+def test_both_forms_of_the_wait(case):
+    assert _scratch(*case[:5], 64, case[5]) == 0
+    _run(*case[:5], 64, torch.bfloat16, case[5], seed=case[3])
