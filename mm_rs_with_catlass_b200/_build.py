@@ -42,6 +42,7 @@ SOURCES = [
     "kernels/inst/f8_single.cu",
     "kernels/inst/f8_pair.cu",
     "kernels/inst/mx_single.cu",
+    "kernels/inst/mx_pair.cu",
     "kernels/shmem_prims.cu",
     "kernels/no_alloc.cu",
     "kernels/blas_prims.cu",

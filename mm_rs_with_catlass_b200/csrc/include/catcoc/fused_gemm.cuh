@@ -494,14 +494,13 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
   const int b_cols_cta = CTA2 ? BN / 2 : BN;   // columns of the B tile this CTA loads
   const uint32_t b_stage_bytes = static_cast<uint32_t>(b_cols_cta) * 128u;
   const int qpt = sched.BM / 32;               // 32-row quarters per tile: 4 (single) or 8 (pair)
-  // TMEM columns: two accumulators at 0 and acc_stride. The block-scaled kind runs tiles of 128 columns (on one CTA; pairs:
+  // TMEM columns: two accumulators at 0 and acc_stride. The block-scaled kind runs tiles of 128 columns (pairs of one wave: 192; others:
   // double_tile.cuh) so that the columns behind the accumulators stay free for the scale factors of the K-blocks in flight.
-  static_assert(KIND != KIND_MX || !CTA2, "block-scaled pairs run double tiles");
-  constexpr uint32_t kMxBN = 128;
+  constexpr uint32_t kMxBN = CTA2 ? 192 : 128;
   const uint32_t acc_stride = (KIND == KIND_MX) ? kMxBN : static_cast<uint32_t>(kMaxBN);
   constexpr uint32_t kSfTmemCol = 2 * kMxBN;   // + slot * 16: SFA 4 columns, SFB 4 columns per 128 of N
-  // inside a K-block's part of the stage, after A and B: SFA, then SFB
-  constexpr int kSfSmemOff = kABytes + static_cast<int>(kMxBN) * 128;
+  // inside a K-block's part of the stage, after A and B: SFA, then one (pair: two) blocks of SFB
+  constexpr int kSfSmemOff = kABytes + static_cast<int>(CTA2 ? kMxBN / 2 : kMxBN) * 128;
   const bool grouped = (p.num_groups > 0);
   if (grouped) ptx::grid_dependency_wait();   // the group list may be the predecessor's result
   int total_tiles = grouped ? grouped_total_tiles(p, lane) : sched.total_tiles;
@@ -656,7 +655,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
           // CTAs' copies are credited to the leader's barrier and only the leader arms it, with
           // the bytes of the whole pair. K-blocks past the end of K are not fetched: no MMA reads them.
           const int nsub = min(kps, tile_sub - kb * kps);
-          if (KIND == KIND_MX) {
+          if (KIND == KIND_MX && !CTA2) {
             // A block + the 512-byte scale-factor block of (this 128-row tile, this K-block)
             ptx::mbar_expect_tx(&tail->full[stage], kABytes + 512);
             const int row_tile = a_row / kBM;
@@ -664,13 +663,15 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
                               p.sfa + (static_cast<int64_t>(row_tile) * p.sf_k_blocks + kb) * 512, 512,
                               &tail->full[stage]);
           } else if (!CTA2) ptx::mbar_expect_tx(&tail->full[stage], nsub * kABytes);
-          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * nsub * kABytes);
+          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * nsub * (kABytes + (KIND == KIND_MX ? 512 : 0)));
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             if (j >= nsub) break;
             uint8_t* sa = smem + stage * kStageBytes + j * sub_bytes;
             const int k0 = (kb * kps + j) * p.bk + a_k_off;
             // (a block past the last row or K-block only fills the stage: its MMAs are skipped or its rows not stored)
+            if (KIND == KIND_MX && CTA2)
+              ptx::tma_load_3d_pair(sa + kSfSmemOff, &p.tm_a_gath[0], bar, 0, (kb * kps + j) * 4, a_row / kBM);
             if (!CTA2) {
               if (!p.a_mn_major) {
                 ptx::tma_load_2d(sa, tma, &tail->full[stage], k0, a_row);
@@ -733,6 +734,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
       unsigned long long c_full = 0, c_acc = 0, c_issue = 0;
       Tick tick(tr);
       bool probed = false;
+      uint32_t mx_slot = 0;
       GroupWalk walk = group_walk_begin(p);
       for (int t = worker; ok && t < total_tiles; t += num_workers) {
         int tile_k = K, tile_kb = num_kb;
@@ -748,6 +750,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
             tile_kb = ceil_div(tile_k, p.bk * kps);
           }
         }
+        const int mx_n0 = (KIND == KIND_MX && CTA2) ? walk_tile(p, t, walk).n0 : 0;
         tick.lap(c_issue);
         const bool got_acc = ptx::mbar_wait(&tail->acc_empty[acc], acc_phase ^ 1u, p.timeout_ns, abort_flag);
         tick.lap(c_acc);
@@ -787,7 +790,34 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
             const uint32_t np = (stage + 1 == kStages) ? (phase ^ 1u) : phase;
             probed = ptx::mbar_test_wait(&tail->full[ns], np);
           }
-          if (KIND == KIND_MX) {
+          if (KIND == KIND_MX && CTA2) {
+            if (ptx::elect_one()) {
+              const uint32_t sfb_off = static_cast<uint32_t>((mx_n0 >> 5) & 3);   // an odd tile starts in the middle of a block
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk) {
+                const int j = kk >> 2, k = kk & 3;
+                if (k_first + kk < k_mmas) {
+                  const uint32_t sf_tmem = tmem_base + kSfTmemCol + ((mx_slot + j) & 3u) * 16u;
+                  if (k == 0) {
+                    // scale factors of this K-block: shared -> TMEM in both CTAs. Four slots: a copy never overwrites
+                    // columns that an earlier, still running MMA may read
+                    const uint32_t sf_smem = ptx::smem_u32(smem + stage * kStageBytes + j * kSubBytes + kSfSmemOff);
+#pragma unroll
+                    for (int b = 0; b < 3; ++b)
+                      ptx::tmem_cp_32x128b_warpx4_pair(sf_tmem + 4u * b, ptx::make_smem_desc_noswizzle(sf_smem + 512u * b, 128u, 128u));
+                  }
+                  const uint64_t dak = da + static_cast<uint64_t>(j * (kSubBytes >> 4) + k * a_kinc);
+                  const uint64_t dbk = db + static_cast<uint64_t>(j * (kSubBytes >> 4) + k * b_kinc);
+                  const uint32_t sel = static_cast<uint32_t>(k) << 30;
+                  ptx::umma_mxf8_pair(tmem_d, dak, dbk, ptx::with_sf_ids(idesc, k, k), sf_tmem | sel, (sf_tmem + 4u + sfb_off) | sel,
+                                      (k_first + kk) != 0 ? 1u : 0u);
+                }
+              }
+              ptx::tcgen05_commit_pair(&tail->empty[stage], 3);
+              if (kb == tile_kb - 1) ptx::tcgen05_commit_pair(&tail->acc_full[acc], 3);
+            }
+            mx_slot += 2u;
+          } else if (KIND == KIND_MX) {
             if (ptx::elect_one()) {
               // scale factors of this stage: shared -> TMEM (slot alternates with the stage so a
               // copy never overwrites columns an earlier, still running MMA may read)
@@ -1527,7 +1557,7 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
           const int per_box = 128 / p.elt_bytes_a;
           const int nsub = min(kps, tile_sub - kb * kps);
           const uint32_t bar = CTA2 ? ptx::map_to_cta(ptx::smem_u32(&tail->full[stage]), 0u) : 0u;
-          if (KIND == KIND_MX) {
+          if (KIND == KIND_MX && !CTA2) {
             const int nblk = BN / 128;
             ptx::mbar_expect_tx(&tail->full[stage], b_stage_bytes + nblk * 512);
             for (int j = 0; j < nblk; ++j)
@@ -1535,12 +1565,16 @@ fused_gemm_kernel(const __grid_constant__ Params p) {
                                 p.sfb + (static_cast<int64_t>(b_col / 128 + j) * p.sf_k_blocks + kb) * 512, 512,
                                 &tail->full[stage]);
           } else if (!CTA2) ptx::mbar_expect_tx(&tail->full[stage], nsub * b_stage_bytes);
-          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * nsub * b_stage_bytes);
+          else if (leader) ptx::mbar_expect_tx(&tail->full[stage], 2u * nsub * (b_stage_bytes + (KIND == KIND_MX ? 1024 : 0)));
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             if (j >= nsub) break;
             uint8_t* sb = smem + stage * kStageBytes + j * sub_bytes + kABytes;
             const int k0 = (kb * kps + j) * p.bk + b_k_off;
+            if (KIND == KIND_MX && CTA2) {
+              // both CTAs hold the scales of all 192 columns: two blocks, wherever the tile starts
+              ptx::tma_load_3d_pair(smem + stage * kStageBytes + j * kSubBytes + kSfSmemOff + 512, &p.tm_a_gath[1], bar, 0, (kb * kps + j) * 4, ti.n0 / 128);
+            }
             if (!CTA2) {
               if (!p.b_mn_major) {
                 ptx::tma_load_2d(sb, tmb, &tail->full[stage], k0, b_col);

@@ -83,6 +83,7 @@ const Unit& unit_i8_pair();
 const Unit& unit_f8_single();
 const Unit& unit_f8_pair();
 const Unit& unit_mx_single();
+const Unit& unit_mx_pair();
 
 // 16-bit products over ragged K ranges (kernels/inst/f16_slice_k.cu)
 cudaError_t prepare_slice_k();
@@ -168,6 +169,20 @@ cudaError_t launch_double_slice_k(const FusedParamsGk& p, int grid, cudaStream_t
     return launch_one<KIND, CTA2, EPI_FULL>(p, grid, threads, s);                                              \
   }                                                                                                   \
   static int NAME##_clusters() { return CTA2 ? query_clusters<KIND, EPI_FULL>() : 0; }                \
+  const Unit& unit_##NAME() {                                                                         \
+    static const Unit u = {NAME##_prepare, NAME##_launch, NAME##_clusters};                           \
+    return u;                                                                                         \
+  }                                                                                                   \
+  } }
+
+// The plain variant alone (local launches without epilogue stages).
+#define CATCOC_DEFINE_UNIT_PLAIN(NAME, KIND, CTA2)                                                    \
+  namespace catcoc { namespace inst {                                                                 \
+  static cudaError_t NAME##_prepare() { return set_smem_attr<KIND, CTA2, EPI_PLAIN>(); }              \
+  static cudaError_t NAME##_launch(int epi, const FusedParams& p, int grid, int threads, cudaStream_t s) { \
+    return (epi & ~EPI_WHOLE_ROWS) == EPI_PLAIN ? launch_one<KIND, CTA2, EPI_PLAIN>(p, grid, threads, s) : cudaErrorNotSupported; \
+  }                                                                                                   \
+  static int NAME##_clusters() { return CTA2 ? query_clusters<KIND, EPI_PLAIN>() : 0; }               \
   const Unit& unit_##NAME() {                                                                         \
     static const Unit u = {NAME##_prepare, NAME##_launch, NAME##_clusters};                           \
     return u;                                                                                         \

@@ -384,11 +384,15 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
   // MMAs; 256 x 192 on a pair: 29.5 KiB per 384, the double tile: 42 KiB per 768): 4096 x 8192 x 7168 e4m3 with its quantisation
   // 361, 256 and 222 us. Up to 128 rows: where the caller wants the units cut along K.
   const bool mx_pair = mx && !fused && (a.M > kBM || a.tiling.cut_slices > 0) && a.scale_m == nullptr && a.scale_n == nullptr && !a.affine && a.act == 0;
+  // Where every pair has at most one unit of 256 x 192 to itself and none is cut, no double tile runs, and the one-accumulator kernel
+  // with its stages of two K blocks feeds a unit faster (600 cycles a K block against 640): 256 x 7384 x 14336 47.0 -> 44.1 us, 512 x 4096 x
+  // 14336 47.2 -> 42.2, 2000 x 1408 x 7168 28.3 -> 25.2.
+  const bool mx_one_wave = mx_pair && a.tiling.cut_slices <= 0 && ceil_div(a.M, 2 * kBM) * ceil_div(a.N, static_cast<int>(dtile::kMxBN)) <= cut_grid(a, rf.kind) / 2;
   // 192-column tiles: pairs of local products (no workspace geometry knows them) with a B stored [N, K]; a [K, N] one comes
   // in 128-byte column blocks, of which a CTA's half would hold one and a half
   const bool bn192 = a.tiling.bn == 192 && !fused && a.trans_b && a.tiling.cta_pair == 2;
   // Double tiles (double_tile.cuh): 256 x 2 bn, local products on pairs
-  const bool twice = a.tiling.twice != 0 || mx_pair;
+  const bool twice = mx_pair ? !mx_one_wave : a.tiling.twice != 0;
   const bool cut = a.tiling.cut_slices > 0;
   if (cut && (!twice || a.num_groups > 0 || a.mode != CATCOC_MODE_LOCAL || a.part == nullptr || (reinterpret_cast<uintptr_t>(a.part) & 127) != 0 ||
               a.tiling.cut_slices < 2 || a.tiling.cut_k <= 0 || (a.tiling.cut_k * rf.elt) % 128 != 0 ||
@@ -445,7 +449,7 @@ int catcoc_build_params(const CatcocOpArgs* args, FusedParams* p, int* kind_out,
     // tensor copies can do
     const int rt_a = (a.M + 127) / 128, rt_b = (a.N + 127) / 128;
     rc = encode_scales(&p->tm_a_gath[0], a.sfa, rt_a, a.sf_k_blocks, 1);
-    if (rc == 0) rc = encode_scales(&p->tm_a_gath[1], a.sfb, rt_b, a.sf_k_blocks, 3);
+    if (rc == 0) rc = encode_scales(&p->tm_a_gath[1], a.sfb, rt_b, a.sf_k_blocks, mx_one_wave ? 2 : 3);
     if (rc != 0) return rc;
   }
   p->elt_bytes_a = rf.elt;
@@ -838,7 +842,7 @@ static const inst::Unit* unit_for(int kind, bool pair) {
     case KIND_F16: return pair ? &inst::unit_f16_pair() : &inst::unit_f16_single();
     case KIND_I8: return pair ? &inst::unit_i8_pair() : &inst::unit_i8_single();
     case KIND_F8: return pair ? &inst::unit_f8_pair() : &inst::unit_f8_single();
-    case KIND_MX: return pair ? nullptr : &inst::unit_mx_single();   // (pairs: double tiles)
+    case KIND_MX: return pair ? &inst::unit_mx_pair() : &inst::unit_mx_single();
     default: return nullptr;
   }
 }
@@ -867,7 +871,7 @@ int max_active_pairs(int kind) {
   if (kind < 0 || kind > KIND_MX) return 1;
   if (cached[kind] < 0) {
     if (prepare_kernels() != cudaSuccess) return 1;
-    int n = unit_for(kind == KIND_MX ? KIND_F8 : kind, true)->max_clusters();
+    int n = unit_for(kind, true)->max_clusters();
     int device = 0;
     cudaGetDevice(&device);
     if (n <= 0) n = sm_count(device) / 2;
