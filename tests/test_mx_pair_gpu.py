@@ -28,7 +28,7 @@ def test_pair_tiles(m, n, k, fmt):
     assert ((out.double() - gold).abs() <= 2.0 ** -8 * gold.abs() + k * 2.0 ** -23 * mag).all()
 
 
-@pytest.mark.parametrize("m,n,k", [(256, 192 * 74, 272), (200, 192 * 74 + 8, 272), (300, 192 * 80 - 40, 144), (700, 192 * 50, 400)])
+@pytest.mark.parametrize("m,n,k", [(256, 192 * 74, 288), (200, 192 * 74 + 8, 288), (300, 192 * 80 - 40, 160), (700, 192 * 50, 416)])
 def test_one_wave_of_units_and_more(m, n, k):
     # on 74 pairs: the last launch whose units are one to a pair (one accumulator each), the first with more, and double tiles
     import mm_rs_with_catlass_b200 as catcoc
