@@ -52,6 +52,84 @@ def test_local_kernels_pass_under_the_checked_build():
     assert out and out[-1]["ok"]
 
 
+def test_double_tiles_pass_under_the_checked_build():
+    out = _child("""
+        import json, torch
+        import mm_rs_with_catlass_b200 as catcoc
+        from mm_rs_with_catlass_b200 import _native as N
+        from mm_rs_with_catlass_b200.ops._common import local_status, raise_on_status
+        from mm_rs_with_catlass_b200.utils.verify import assert_close
+        T = catcoc.TilingConfig
+        assert N.lib().catcoc_is_checked_build() == 1
+        dev = torch.device("cuda:0")
+        def r(*s):
+            return torch.randn(*s, device=dev).bfloat16()
+        def i8(*s):
+            return torch.randint(-127, 128, s, device=dev, dtype=torch.int32).to(torch.int8)
+        for swap in (False, True):
+            for (m, n, k, bn, kw) in [(256, 512, 128, 256, {}), (300, 1001, 72, 224, {}), (1, 64, 64, 64, {}), (1024, 2368, 2048, 128, dict(cut_slices=4, cut_k=512)),
+                                      (700, 703, 1024, 96, dict(cut_slices=2, cut_k=512, num_ctas=14))]:
+                a, b = r(m, k), r(n, k) * 0.1
+                t = T(bn=bn, cta_pair=2, twice=True, swap=swap, **kw)
+                for dt in (torch.bfloat16, torch.float32):
+                    assert_close(catcoc.matmul(a, b, trans_b=True, tiling=t, out_dtype=dt), a.float() @ b.float().t(), k=k, dtype=dt, what=str((m, n, k, swap)))
+                x, w = i8(m, -(-k // 16) * 16), i8(n, -(-k // 16) * 16)
+                assert torch.equal(catcoc.matmul(x, w, trans_b=True, tiling=t).cpu().long(), x.cpu().long() @ w.cpu().long().t())
+            sizes = [0, 1, 33, 300, 256, 513]
+            ends = torch.tensor(sizes).cumsum(0).to(torch.int32).to(dev)
+            a, b = r(sum(sizes), 256), r(len(sizes), 256, 336) * 0.1
+            got, at = catcoc.grouped_matmul(a, b, ends, tiling=T(bn=256, cta_pair=2, twice=True, swap=swap)), 0
+            for i, s in enumerate(sizes):
+                if s:
+                    assert_close(got[at:at + s], a[at:at + s].float() @ b[i].float(), k=256, dtype=torch.bfloat16, what="group %d" % i)
+                at += s
+        a, b = r(900, 264), r(900, 520) * 0.1
+        got = catcoc.grouped_matmul_slice_k(a, b, [70, 70, 900], tiling=T(bn=256, cta_pair=2, twice=True))
+        for i, (x, y) in enumerate(((0, 70), (70, 900))):
+            assert_close(got[2 * i], a[x:y].float().t() @ b[x:y].float(), k=900, dtype=torch.bfloat16, what="range %d" % i)
+        assert not got[1].any()
+        for m, n, k in ((300, 584, 1056), (100, 1000, 16384), (300, 15320, 160)):
+            qs = [catcoc.quantize_mxf8(torch.randn(s, k, device=dev)) for s in (m, n)]
+            want = catcoc.ops.mx.dequantize_mxf8(*qs[0]) @ catcoc.ops.mx.dequantize_mxf8(*qs[1]).t()
+            assert_close(catcoc.mxf8_matmul(qs[0][0], catcoc.pack_scales(qs[0][1]), qs[1][0], catcoc.pack_scales(qs[1][1])), want, k=k, dtype=torch.bfloat16, what="mx")
+        torch.cuda.synchronize()
+        raise_on_status(local_status(dev), "checked build")
+        print(json.dumps({"ok": True}))
+    """)
+    assert out and out[-1]["ok"]
+
+
+@pytest.mark.parametrize("swap", [0, 1])
+def test_double_tiles_report_an_understated_output_extent(swap):
+    out = _child("""
+        import json, torch
+        from mm_rs_with_catlass_b200 import _native as N
+        from mm_rs_with_catlass_b200.ops import _common as cm
+        dev = torch.device("cuda:0")
+        m, n, k = 512, 512, 128
+        a, b = (torch.randn(m, k, device=dev).bfloat16() for _ in range(2))
+        out = torch.full((m, n), 7.0, device=dev, dtype=torch.bfloat16)
+        status = torch.zeros(8, dtype=torch.int32, device=dev)
+        args = N.OpArgs()
+        args.mode, args.in_fmt = N.MODE_LOCAL, N.IN_BF16
+        args.M, args.N, args.K = m, n, k
+        args.trans_b = 1
+        args.a, args.lda, args.b, args.ldb = a.data_ptr(), k, b.data_ptr(), k
+        args.out, args.ldc, args.out_fmt, args.partial_fmt = out.data_ptr(), n, N.FMT_BF16, N.FMT_BF16
+        args.tiling.bn, args.tiling.cta_pair, args.tiling.twice, args.tiling.swap = 128, 2, 1, %d
+        args.rank, args.W = 0, 1
+        args.status = status.data_ptr()
+        args.limit[N.LIM_OUT] = 256 * n * 2            # the caller claims half of the rows
+        cm.launch(args, dev)
+        torch.cuda.synchronize()
+        print(json.dumps({"status": status.cpu().tolist(), "tail_untouched": bool((out[256:] == 7.0).all().item()),
+                          "head_written": bool((out[:256] != 7.0).any().item())}))
+    """ % swap, {"CATCOC_OUT_TMA": "0"})
+    r = out[-1]
+    assert r["status"][0] == 7 and r["status"][2] == 13 and r["status"][3] == 256 * 512 * 2, r
+    assert r["tail_untouched"] and r["head_written"], r
+
+
 def test_an_understated_output_extent_is_reported_and_nothing_is_written_past_it():
     out = _child("""
         import ctypes as C, json, torch

@@ -155,10 +155,11 @@ def test_block_scaled_cut_units(monkeypatch, m, n, k):
     import mm_rs_with_catlass_b200 as catcoc
     from mm_rs_with_catlass_b200.ops import mx
     g = torch.Generator(device="cuda").manual_seed(k)
-    ops = []
+    ops, scaled = [], []
     for rows in (m, n):
         q, s = catcoc.quantize_mxf8(torch.randn(rows, k, device="cuda", generator=g), "e4m3")
         ops += [q, catcoc.pack_scales(s)]
+        scaled.append((q, s))
     res = []
     for cut in (None, (2, -(-k // 256) * 128)) if k > 128 else (None,):
         monkeypatch.setattr(mx, "double_plan", lambda *a: (0.0, cut))
@@ -167,6 +168,8 @@ def test_block_scaled_cut_units(monkeypatch, m, n, k):
         _check("block-scaled")
     # fp32 sums in another order, as above; the operands' magnitudes are about one
     assert (res[0] - res[-1]).abs().max().item() < k * 2.0 ** -24 * 4 * k ** 0.5
+    a, b = (catcoc.ops.mx.dequantize_mxf8(*x).double() for x in scaled)
+    assert all((r - a @ b.t()).abs().max().item() < k * 2.0 ** -24 * 4 * k ** 0.5 for r in res)
 
 
 @pytest.mark.gpu
@@ -259,3 +262,87 @@ def test_kept_argument_blocks_serve_other_buffers():
         assert (got.float() - want).abs().max().item() < 2.0 ** -7 * want.abs().max().item()
         _check("kept blocks")
     assert blas._group_blocks and blas._slice_k_blocks and mx._blocks
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", [torch.float8_e4m3fn, torch.float8_e5m2])
+@pytest.mark.parametrize("m,n,k,bn", [(1, 64, 64, 64), (300, 1008, 208, 224), (513, 336, 1296, 160), (256, 512, 256, 256)])
+def test_fp8(fmt, m, n, k, bn):
+    # by an explicit tiling alone: no rule sends fp8 without block scales here
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    s1, s2 = torch.rand(m, device="cuda", generator=g) + 0.5, torch.rand(n, device="cuda", generator=g) + 0.5
+    for tb in (True, False):
+        a, b = _operand(g, fmt, m, k), _operand(g, fmt, *((n, k) if tb else (k, n)))
+        for kw in (dict(out_dtype=torch.float32), dict(scale_m=s1, scale_n=s2)):
+            got, want = (catcoc.matmul(a, b, trans_b=tb, tiling=TilingConfig(bn=x, cta_pair=p, twice=p == 2), **kw) for x, p in ((bn, 2), (256, 1)))
+            _check("fp8")
+            assert torch.equal(got, want), (tb, kw.keys())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.int8])
+@pytest.mark.parametrize("bn", [96, 256])
+def test_groups_of_rows_without_swapped_roles(dtype, bn):
+    # ragged and uniform groups, by an explicit tiling alone; bn 96 leaves half a window behind the last whole one
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(bn)
+    t, ref = TilingConfig(bn=bn, cta_pair=2, twice=True), TilingConfig(bn=256, cta_pair=1)
+    sizes = [0, 1, 31, 300, 256, 0, 513]
+    total, n, k = sum(sizes), 848, 256
+    ends = torch.tensor(sizes).cumsum(0).to(torch.int32).cuda()
+    for tb in (False, True):
+        a, b = _operand(g, dtype, total, k), _operand(g, dtype, *((len(sizes), n, k) if tb else (len(sizes), k, n)))
+        s1, s2 = torch.rand(total, device="cuda", generator=g), torch.rand(len(sizes), n, device="cuda", generator=g)
+        got, want = (catcoc.grouped_quant_matmul(a, b, s1, s2, ends, trans_b=tb, tiling=x) if dtype == torch.int8 else
+                     catcoc.grouped_matmul(a, b, ends, trans_b=tb, tiling=x) for x in (t, ref))
+        _check("groups of rows")
+        assert torch.equal(got, want), tb
+        for ta in (False, True):
+            a = _operand(g, dtype, *((3, k, 304) if ta else (3, 304, k)))
+            got, want = (catcoc.batched_matmul(a, b[:3].contiguous(), trans_a=ta, trans_b=tb, tiling=x) for x in (t, ref))
+            _check("uniform groups")
+            assert torch.equal(got, want), (ta, tb)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("swap", [False, True])
+def test_infinities_beside_a_group_or_behind_k_stay_outside(swap):
+    import mm_rs_with_catlass_b200 as catcoc
+    g = torch.Generator(device="cuda").manual_seed(21)
+    t = TilingConfig(bn=256, cta_pair=2, twice=True, swap=swap)
+    # groups of rows: those of one group
+    sizes, n, k = [70, 200, 33, 300], 336, 200
+    ends, bounds = torch.tensor(sizes).cumsum(0).to(torch.int32).cuda(), [0, 70, 270, 303, 603]
+    a, b = _operand(g, torch.bfloat16, 640, k), _operand(g, torch.bfloat16, len(sizes), n, k)     # (K is no whole number of MMAs)
+    a[603:] = float("inf")                                     # rows of no group
+    want = catcoc.grouped_matmul(a, b, ends, trans_b=True, tiling=t)[:603].clone()
+    assert want.isfinite().all()
+    for i in range(len(sizes)):
+        x = a.clone()
+        x[bounds[i]:bounds[i + 1]] = float("inf")
+        got = catcoc.grouped_matmul(x, b, ends, trans_b=True, tiling=t)
+        for j in range(len(sizes)):
+            if j != i:
+                assert torch.equal(got[bounds[j]:bounds[j + 1]], want[bounds[j]:bounds[j + 1]]), (i, j)
+    # ranges along K: those of one range, which end inside a K block
+    if not swap:
+        a, b = _operand(g, torch.bfloat16, 640, 264), _operand(g, torch.bfloat16, 640, 520)
+        want = catcoc.grouped_matmul_slice_k(a, b, bounds[1:], tiling=t)
+        for i in range(len(sizes)):
+            x, y = a.clone(), b.clone()
+            x[bounds[i]:bounds[i + 1]] = float("inf")
+            y[bounds[i]:bounds[i + 1]] = float("nan")
+            got = catcoc.grouped_matmul_slice_k(x, y, bounds[1:], tiling=t)
+            assert all(torch.equal(got[j], want[j]) for j in range(len(sizes)) if j != i), i
+    # columns behind K of operands inside wider buffers, whole and in slices
+    for k in (72, 1096):
+        wide = [torch.full((r, 1280), float("inf"), device="cuda", dtype=torch.bfloat16) for r in (600, 700)]
+        for w in wide:
+            w[:, :k] = _operand(g, torch.bfloat16, w.shape[0], k)
+        for cut in (dict(), dict(cut_slices=3, cut_k=384)) if k > 72 else (dict(),):
+            tc = TilingConfig(bn=96, cta_pair=2, twice=True, swap=swap, **cut)
+            got, want = (catcoc.matmul(x, y, trans_b=True, out_dtype=torch.float32, tiling=tc)
+                         for x, y in ([w[:, :k] for w in wide], [w[:, :k].contiguous() for w in wide]))
+            assert want.isfinite().all() and torch.equal(got, want), (k, cut)
+    _check("infinities")

@@ -9,7 +9,7 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mm_rs_with_catlass_b200", "csrc")
 # files whose kernels (and device functions) all belong to overlapped launches
 WHOLE = ["kernels/flash_attn.cu", "kernels/flash_decode.cu", "kernels/mla_rows.cu", "kernels/mx_quant.cu", "kernels/launch.cu",
-         "include/catcoc/fused_gemm.cuh", "include/catcoc/softmax_row.cuh"]
+         "include/catcoc/fused_gemm.cuh", "include/catcoc/double_tile.cuh", "include/catcoc/softmax_row.cuh"]
 FILES = WHOLE + ["kernels/blas_prims.cu"]
 
 

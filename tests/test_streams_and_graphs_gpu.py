@@ -3,6 +3,8 @@ captured call replays on new contents of its inputs."""
 import pytest
 import torch
 
+from mm_rs_with_catlass_b200.tiling.config import TilingConfig
+
 pytestmark = pytest.mark.gpu
 
 
@@ -26,6 +28,31 @@ def _call(name, seed):
     if name == "slice_k":
         a, b = _randn(g, 700, 512), _randn(g, 700, 256)
         return [a, b], lambda: catcoc.grouped_matmul_slice_k(a, b, [100, 100, 431, 700])
+    if name == "attention_cut":                      # few tiles of queries over many keys
+        from mm_rs_with_catlass_b200 import _native as N
+        assert N.lib().catcoc_flash_attention_workspace_bytes(1, 8, 2, 160, 3000, 128, 1) > 0
+        q, k, v = _randn(g, 1, 8, 160, 128), _randn(g, 1, 2, 3000, 128), _randn(g, 1, 2, 3000, 128)
+        return [q, k], lambda: catcoc.flash_attention(q, k, v, causal=True)
+    if name == "token_groups":
+        a, b = _randn(g, 2000, 512), _randn(g, 8, 512, 1024)
+        ends = torch.tensor([10, 300, 300, 800, 1001, 1500, 1600, 2000], device="cuda", dtype=torch.int32)
+        t = TilingConfig(bn=256, cta_pair=2, twice=True, swap=True)
+        return [a, b], lambda: catcoc.grouped_matmul(a, b, ends, tiling=t)
+    if name == "mx_cut":
+        from mm_rs_with_catlass_b200.ops import mx
+        assert mx._cut(100, 1000, 16384) is not None
+        x, w = _randn(g, 100, 16384), _randn(g, 1000, 16384)
+        wq, ws = catcoc.quantize_mxf8(w)
+        ws = catcoc.pack_scales(ws)
+
+        def quantised():
+            q, s = catcoc.quantize_mxf8(x)
+            return catcoc.mxf8_matmul(q, catcoc.pack_scales(s), wq, ws)
+        return [x], quantised
+    if name.startswith("double_cut"):
+        a, b = _randn(g, 1024, 2048), _randn(g, 2368, 2048)
+        t = TilingConfig(bn=128, cta_pair=2, twice=True, swap=name.endswith("swapped"), cut_slices=4, cut_k=512)
+        return [a, b], lambda: catcoc.matmul(a, b, trans_b=True, tiling=t)
     m, n, k = {"split_k": (64, 1024, 8192), "tail_cut": (1024, 5120, 6144), "padded_a": (200, 1000, 601),
                "padded_both": (200, 999, 601)}[name]
     a, b = _randn(g, m, k), _randn(g, k, n)
@@ -37,7 +64,8 @@ def _call(name, seed):
     return [a, b], lambda: catcoc.matmul(a, b)
 
 
-ROUTES = ["split_k", "tail_cut", "padded_a", "padded_both", "flash_decode", "mla_rows", "slice_k"]
+ROUTES = ["split_k", "tail_cut", "padded_a", "padded_both", "flash_decode", "mla_rows", "slice_k", "double_cut", "double_cut_swapped",
+          "attention_cut", "token_groups", "mx_cut"]
 
 
 def _status():
