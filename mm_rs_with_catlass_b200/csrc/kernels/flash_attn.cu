@@ -1,7 +1,7 @@
 // Flash attention forward on tcgen05: one CTA per 256 query rows (two tiles of 128) of one (batch, head).
 //
 //   warps 0..3  softmax of tile 0 : one query row per thread: tcgen05.ld the scores, row maximum, exp2, row sum,
-//   warps 4..7  softmax of tile 1   P (operand dtype) written back over the scores with tcgen05.st, O rescaled in
+//   warps 4..7  softmax of tile 1   P (operand dtype) written to columns of its own with tcgen05.st, O rescaled in
 //                                   TMEM when the running maximum moved by more than 2^8, final O / l and the store
 //   warp 8      TMA producer      : both Q tiles once, then K and V blocks of 128 keys through one ring of slots
 //   warp 9      MMA issuer        : S_t = Q_t K^T into TMEM, O_t += P_t V with P read from TMEM (the A operand of
@@ -14,7 +14,7 @@
 //
 // Bound by the steps of one row: of 2930 cycles a block (D = 128, per tile, cycle counters) 260 go to reading the scores, 300 to
 // the maximum, 1840 to the exponentials beside the other tile's (the special-function unit alone: 1024), 400 to waiting for
-// the next scores; tensor cores and special-function unit are 70 % busy. With P on top of S_t and one issuer for both tiles, whose
+// the next scores; tensor cores and special-function unit are 65 % busy (1 x 32 x 4096, not causal). With P on top of S_t and one issuer for both tiles, whose
 // products waited behind the other tile's softmax, a block took 3490. Causal, 2 x 32 / 8 heads x 8192, D = 128: 855 -> 770 us
 // at full clock (operands of zeros), 1040 -> 980 us in a loop, which the power limit holds.
 //
@@ -44,7 +44,7 @@ namespace attn {
 constexpr int kBQ = 128;          // query rows per tile == TMEM lanes
 constexpr int kTiles = 2;         // query tiles per CTA
 constexpr int kBKV = 128;         // keys per block
-constexpr int kThreads = 384;     // 2 x 4 softmax warps, producer, issuer, two warps that only complete the warpgroup
+constexpr int kThreads = 384;     // 2 x 4 softmax warps, producer, one or (D = 128) two issuers; the others only complete the warpgroup
 // Registers: a softmax thread keeps 128 scores and their probabilities. The block is launched with 168 a thread; the
 // third warpgroup gives up what the first two take: 2 x 216 + 72 = 3 x 168.
 constexpr int kSoftmaxRegs = 216, kOtherRegs = 72;
